@@ -36,9 +36,11 @@ UNITS = {
     "f16_gemm_sm100.cu": [],
     "ops_rows.cu": [],
     "linear_rows.cu": [],
+    "linear_f32.cu": [],
     "latent_attn.cu": [],
     "latent_prefill.cu": [],
     "window_attn.cu": [],
+    "window_f32.cu": [],
     "window_prefill.cu": [],
     "window_attn_sm100.cu": [],
     "channel_delta.cu": [],

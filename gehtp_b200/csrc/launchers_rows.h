@@ -43,6 +43,8 @@ struct LinearArgs {
 void k_linear(cudaStream_t st, const LinearArgs& a, uint32_t M, bool exact, unsigned int* status);
 // tcgen05 form (bf16 x): false = shape or alignment not taken, nothing launched
 bool k_linear_sm100(cudaStream_t st, const LinearArgs& a, uint32_t M, unsigned int* status);
+// fp32 x (linear_f32.cu): false = alignment not taken, nothing launched
+bool k_linear_f32(cudaStream_t st, const LinearArgs& a, uint32_t M);
 
 // ---- latent attention (latent_attn.cu, latent_prefill.cu)
 struct LatentArgs {

@@ -6,6 +6,7 @@
 // Columns at or past N are left out.
 #pragma once
 #include <type_traits>
+#include "launchers_rows.h"
 #include "rows_common.cuh"
 
 namespace gehtp {
@@ -193,6 +194,15 @@ inline EpiTanh<A> make_epi_tanh(const float* p, const float* x, const float* nex
     const uintptr_t al = (uintptr_t)p | (uintptr_t)x | (uintptr_t)next | (uintptr_t)x_out;
     e.vec = width % 4 == 0 && act_ld % 4 == 0 && (al & 15u) == 0 && ((uintptr_t)act & (sizeof(typename A::T) == 2 ? 7u : 15u)) == 0;
     return e;
+}
+
+// the epilogue of `a`, outputs in the activation type of YB
+template <bool YB, class F>
+inline void with_epilogue(const LinearArgs& a, F&& f) {
+    if (a.tanh) f(make_epi_tanh<typename std::conditional<YB, ActBf16, ActF32>::type>(a.p, a.res, a.next, a.x_out, a.act, a.N, a.act_ld));
+    else if (a.gelu_gate) f(EpiGelu<YB>{a.y, a.ys});
+    else if (YB && a.y_bf16) { if (a.relu2) f(EpiPlain<YB, true>{a.y, a.ys, a.bias}); else f(EpiPlain<YB, false>{a.y, a.ys, a.bias}); }
+    else { if (a.relu2) f(EpiPlain<false, true>{a.y, a.ys, a.bias}); else f(EpiPlain<false, false>{a.y, a.ys, a.bias}); }
 }
 
 }  // namespace gehtp

@@ -3,8 +3,8 @@
 //   bf16 x, few rows    streaming product on mma.sync m16n8k16 (lin_stream_kernel): a warp owns 8 output columns and a
 //                       share of K, the shares of a column group meet in shared memory
 //   bf16 x, more rows   the TMA-fed tcgen05 GEMM (f16_gemm_sm100.cu)
-//   fp32 x, shapes whose rows are no multiple of 16 bytes, and the one-kernel-per-op plan: fp32 FMA tiles
-#include <type_traits>
+//   fp32 x              linear_f32.cu
+//   shapes whose rows are no multiple of 16 bytes, and the one-kernel-per-op plan: fp32 FMA tiles
 #include "launchers_rows.h"
 #include "linear_epi.cuh"
 #include "mma_bf16.cuh"
@@ -174,20 +174,15 @@ void launch_fma(cudaStream_t st, const LinearArgs& a, const E& epi, uint32_t M) 
     g_launches++;
 }
 
-// the epilogue of `a`, outputs in the activation type of YB
-template <bool YB, class F>
-void with_epilogue(const LinearArgs& a, F&& f) {
-    if (a.tanh) f(make_epi_tanh<typename std::conditional<YB, ActBf16, ActF32>::type>(a.p, a.res, a.next, a.x_out, a.act, a.N, a.act_ld));
-    else if (a.gelu_gate) f(EpiGelu<YB>{a.y, a.ys});
-    else if (YB && a.y_bf16) { if (a.relu2) f(EpiPlain<YB, true>{a.y, a.ys, a.bias}); else f(EpiPlain<YB, false>{a.y, a.ys, a.bias}); }
-    else { if (a.relu2) f(EpiPlain<false, true>{a.y, a.ys, a.bias}); else f(EpiPlain<false, false>{a.y, a.ys, a.bias}); }
-}
-
 }  // namespace
 
 void k_linear(cudaStream_t st, const LinearArgs& a, uint32_t M, bool exact, unsigned int* status) {
     if (!M) return;
-    if (!a.x_bf16) { with_epilogue<false>(a, [&](const auto& epi) { launch_fma<ActF32>(st, a, epi, M); }); return; }
+    if (!a.x_bf16) {
+        if (!exact && k_linear_f32(st, a, M)) return;
+        with_epilogue<false>(a, [&](const auto& epi) { launch_fma<ActF32>(st, a, epi, M); });
+        return;
+    }
     const bool vec = a.K % 8 == 0 && a.xs % 8 == 0 && (((uintptr_t)a.x | (uintptr_t)a.w) & 15u) == 0;
     with_epilogue<true>(a, [&](const auto& epi) {
         if (!exact && vec) {

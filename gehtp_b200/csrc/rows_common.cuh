@@ -41,6 +41,25 @@ __device__ __forceinline__ float block_sum(float v, float* part) {
     return s;
 }
 
+// Sums NV values (a power of two up to 32) over the warp; lane l is left with the sum of value l / (32 / NV).
+template <int NV>
+__device__ __forceinline__ float fold_sum(float (&v)[NV]) {
+    const uint32_t lane = threadIdx.x & 31;
+    int off = 16;
+#pragma unroll
+    for (int n = NV; n > 1; n /= 2, off /= 2) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < n / 2; i++) {
+            const float keep = up ? v[i + n / 2] : v[i], send = up ? v[i] : v[i + n / 2];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+    float s = v[0];
+    for (; off > 0; off /= 2) s += __shfl_xor_sync(0xffffffffu, s, off);
+    return s;
+}
+
 // Cluster barrier in two halves: all threads of the cluster's CTAs arrive, then wait.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }

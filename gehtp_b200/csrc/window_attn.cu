@@ -6,6 +6,7 @@
 //   window_step_kernel    few bf16 rows: a cluster of CTAs per (key head, row) shares the window out, the partial results
 //                         meet through distributed shared memory; for one row the append is part of it
 //   more bf16 rows        window_attn_sm100.cu, window_prefill.cu
+//   fp32 rows             window_f32.cu
 #include <cooperative_groups.h>
 #include "launchers_rows.h"
 #include "mma_bf16.cuh"
@@ -537,6 +538,7 @@ bool step(cudaStream_t st, const WindowArgs& a, uint32_t rows) {
 
 bool k_window_sm100(cudaStream_t st, const WindowArgs& a, uint32_t rows);
 bool k_window_flash(cudaStream_t st, const WindowArgs& a, uint32_t rows);
+bool k_window_f32(cudaStream_t st, const WindowArgs& a, uint32_t rows);
 
 void k_heads_append(cudaStream_t st, const WindowArgs& a, uint32_t rows) {
     if (!rows) return;
@@ -568,6 +570,7 @@ void k_window_attend(cudaStream_t st, const WindowArgs& a, uint32_t rows, bool e
         if (rows <= kStepRows && step<false>(st, a, rows)) return;
         if (k_window_sm100(st, a, rows) || k_window_flash(st, a, rows)) return;
     }
+    if (!a.bf16 && !exact && k_window_f32(st, a, rows)) return;
     const size_t smem = (size_t)(a.dim + a.vdim) * 4;
     static int have_b[64] = {}, have_f[64] = {};
     if (a.bf16) {
