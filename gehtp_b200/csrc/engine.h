@@ -50,6 +50,7 @@ struct PlanOp {
     uint32_t span = 0;
     uint32_t stat = 0;          // index into the stats struct, 0 = none
     bool uses_internal = false; // touches a temp that has no memory in a fused plan
+    bool wanted_now = false;        // scratch of want_temp
     bool dead_when_fused = false;   // its result is read only by ops that fused chains replace: skipped in whole fused runs
     // a data-movement op whose inputs are weight slots (or results of such ops) and whose output nobody else writes:
     // its result is a constant of the blob, made by the first run that reaches it and kept

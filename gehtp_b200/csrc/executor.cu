@@ -209,6 +209,29 @@ void drop_graphs() {
     g.graphs.clear();
 }
 
+// A caller asks for a temp that whole fused runs leave out (dead_when_fused): its op and the left-out ops in front of it
+// are launched from now on. now: launch them here too, behind a run that left them out.
+static void want_temp(uint32_t id, bool now) {
+    if (!g.planned || id >= kMaxTemps) return;
+    std::vector<uint8_t> want(kMaxTemps, 0);
+    want[id] = 1;
+    bool any = false;
+    for (uint32_t i = (uint32_t)g.plan.size(); i-- > 0;) {
+        PlanOp& p = g.plan[i];
+        if (!p.dead_when_fused || p.out_id[0] == kNoOff || !want[p.out_id[0]]) continue;
+        const uint32_t src = g.blob->ops[i].args[0];
+        if (!(src & 0xC000u) && src < kMaxTemps) want[src] = 1;
+        p.dead_when_fused = false;
+        p.wanted_now = any = true;
+    }
+    if (!any) return;
+    drop_graphs();
+    for (PlanOp& p : g.plan) {
+        if (p.wanted_now && now && p.launch) p.launch(g.stream);
+        p.wanted_now = false;
+    }
+}
+
 static void note_outputs(const PlanOp& p) {
     for (int k = 0; k < 2; k++) {
         uint32_t id = p.out_id[k];
@@ -376,6 +399,7 @@ static int run_impl(const wt_blob* b, uint32_t first, uint32_t count, const void
     if ((uint64_t)first + count > b->n_ops) { set_err(err, errn, "range oob"); return -1; }
     if (ensure_plan(b, err, errn) != 0) return -1;
 
+    if (out_host || out_dev) want_temp(out_temp, false);
     const bool timing = op_us || g.ts_buf;
     const bool whole = first == 0 && count == b->n_ops;
     const bool has_in = in_host || in_dev;
@@ -554,6 +578,7 @@ int gehtp_cuda_run_dev(const struct wt_blob* b, const void* in_dev, void* out_de
 
 uint8_t* wt_exec_temp(uint32_t id) {
     if (!g.dev_ok || id >= kMaxTemps || !g.temp_cap[id] || !g.temp_dev[id]) return nullptr;
+    want_temp(id, true);
     auto& m = g.mirrors[id];
     size_t need = g.temp_cap[id];
     if (m.second < need) {
@@ -672,7 +697,12 @@ uint32_t gehtp_cuda_fused_ops(void) { return g.fused_ops; }
 uint32_t gehtp_cuda_const_ops(void) { return g.const_ops; }
 uint32_t gehtp_cuda_demoted_temps(void) { return g.demoted_temps; }
 void* gehtp_cuda_stream(void) { return ensure_device(nullptr, 0) ? (void*)g.stream : nullptr; }
-void* gehtp_cuda_temp_dev(uint32_t id) { return (id < kMaxTemps && g.temp_cap[id]) ? g.temp_dev[id] : nullptr; }
+void* gehtp_cuda_temp_dev(uint32_t id) {
+    if (id >= kMaxTemps || !g.temp_cap[id]) return nullptr;
+    cudaSetDevice(g.device);
+    want_temp(id, true);
+    return g.temp_dev[id];
+}
 int gehtp_cuda_sync(void) {
     if (!g.dev_ok) return -1;
     cudaSetDevice(g.device);

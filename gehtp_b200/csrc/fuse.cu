@@ -166,6 +166,10 @@ struct Span {
     // decode attention: index of the W4A16 q|k|v projection when it sits right before the chain and
     // nothing but the chain reads its output (its epilogue can then do the rotary + append), else -1
     int qkv_lin = -1;
+    // decode attention: the operand is one row of a slot that a BROADCAST repeats for every head; the chain reads that
+    // row where it lies (tables: all four of them) and the broadcast is not launched
+    bool mask_row = false, table_row = false;
+    uint32_t mask_off = 0, tab_off[4] = {};       // first element in the slot
     // kind 5, split + rotary of a prefill block: qkv in, q_out / k_out / v_out, B = tokens
     // kind 6, SwiGLU around two GEMMs: ops gate_op and up_op keep their launches, a_ref/y as kind 1, n values
     uint32_t k_out, v_out, gate_op, up_op, gate_t, up_t;
@@ -206,6 +210,36 @@ bool const_scalar(const Graph& G, int bc_op, float& v) {
     } else if (e == 31u) bits = sign | 0x7f800000u | (m << 13);
     else bits = sign | ((e + 112u) << 23) | (m << 13);
     std::memcpy(&v, &bits, 4);
+    return true;
+}
+
+// The slot row behind operand temp of op `user` (argument `arg`): BROADCAST (1, 1, 1, n) -> (1, 1, R, n) of a slot or of a
+// contiguous rank-1 SLICE of one (the faces of the merged input). Slots keep their bytes for a whole run unless a
+// memory-planner op writes them.
+bool slot_row(const Graph& G, int bc, uint32_t n, uint32_t rows, uint32_t& slot_ref, uint32_t& first) {
+    const wt_blob* b = G.b;
+    if (bc < 0 || b->ops[bc].opcode != OP_BROADCAST_F16) return false;
+    const wt_op& o = b->ops[bc];
+    const uint32_t in[4] = {1, 1, 1, n}, out[4] = {1, 1, rows, n};
+    if (o.args[3] != n) return false;
+    for (int k = 0; k < 4; k++) if (o.args[4 + k] != in[k] || o.args[8 + k] != out[k]) return false;
+    uint32_t src = o.args[0];
+    first = 0;
+    const int sl = (src & 0x8000u) ? -1 : G.producer_of_arg[0][bc];
+    if (sl >= 0) {
+        const wt_op& q = b->ops[sl];
+        if (q.opcode != OP_STRIDED_SLICE_F16 || q.args[3] != 1 || q.args[2] != n || q.args[10] > 1 || q.args[7] != q.args[4] + n || q.args[7] > q.args[13]) return false;
+        src = q.args[0];
+        first = q.args[4];
+    }
+    if (!(src & 0x8000u) || (src & 0x4000u)) return false;
+    const uint32_t s = src & 0x7FFFu;
+    if (s >= b->n_slots || (b->slots[s].addr != 0 && b->slots[s].addr != WT_SLOT_EXT_IN) || ((uint64_t)first + n) * 2 > b->slots[s].len) return false;
+    for (uint32_t i = 0; i < b->n_ops; i++) {
+        const uint32_t oc = b->ops[i].opcode;
+        if (oc == OP_SPILL || oc == OP_FILL || oc == OP_DMA) return false;
+    }
+    slot_ref = src;
     return true;
 }
 
@@ -282,6 +316,15 @@ bool match_attention(const Graph& G, uint32_t ia, Span& sp) {
     sp.q_out = b->ops[rq.out_op].args[2]; sp.mask = ad.args[1]; sp.ctx = pv.args[2]; sp.state = si;
     sp.B = B; sp.nh = nh; sp.kvh = kvh; sp.hd = hd; sp.nslots = nslots; sp.pos = ap.args[3];
     sp.scale = scale; sp.scale_div = bi.args[4] == 3;
+    uint32_t ref = 0;
+    if (slot_row(G, G.producer_of_arg[1][j + 2], nslots, H, ref, sp.mask_off)) { sp.mask_row = true; sp.mask = ref; }
+    // cosine and sine operands: argument 1 of the two products of a rotary chain (its first and last but one op)
+    uint32_t refs[4];
+    const int tab_ops[4] = {(int)rq.ops[0], (int)rq.ops[5], (int)rk.ops[0], (int)rk.ops[5]};
+    const uint32_t tab_rows[4] = {H, H, B * kvh, B * kvh};
+    sp.table_row = true;
+    for (int k = 0; k < 4; k++) sp.table_row = sp.table_row && slot_row(G, G.producer_of_arg[1][tab_ops[k]], hd, tab_rows[k], refs[k], sp.tab_off[k]);
+    if (sp.table_row) { sp.cos_q = refs[0]; sp.sin_q = refs[1]; sp.cos_k = refs[2]; sp.sin_k = refs[3]; }
     return true;
 }
 
@@ -725,15 +768,15 @@ void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector
         }
         return true;
     };
-    for (uint32_t i = 0; i < b->n_ops; i++) {
+    for (uint32_t i = b->n_ops; i-- > 0;) {             // from the back: a slice goes with the broadcasts that read it
         if (span_of[i] >= 0 || G.users[i].empty() || meas[i].rc) continue;
         const uint32_t opc = b->ops[i].opcode;
-        if (opc != OP_BROADCAST_F16) continue;          // pure functions of their inputs only
+        if (opc != OP_BROADCAST_F16 && opc != OP_STRIDED_SLICE_F16) continue;     // pure functions of their inputs only
         const uint32_t t = meas[i].out_id[0];
         if (t == kNoOff || meas[i].out_id[1] != kNoOff) continue;
         bool all_dead = true;
         for (uint32_t u : G.users[i])
-            if (span_of[u] < 0 || span_reads(g_spans[span_of[u]], t)) { all_dead = false; break; }
+            if (span_of[u] < 0 ? !dead[u] : span_reads(g_spans[span_of[u]], t)) { all_dead = false; break; }
         if (all_dead) dead[i] = 1;
     }
 }
@@ -815,6 +858,9 @@ void fuse_materialize(const wt_blob* b) {
             const uint16_t* mask = (const uint16_t*)resolve(b, sp.mask);
             uint16_t* ctx = (uint16_t*)resolve(b, sp.ctx);
             if (!qkv || !cq || !sq || !ck || !sk || !q_out || !mask || !ctx) continue;
+            if (sp.table_row) { cq += sp.tab_off[0]; sq += sp.tab_off[1]; ck += sp.tab_off[2]; sk += sp.tab_off[3]; }
+            if (sp.mask_row) mask += sp.mask_off;
+            const bool tab_row = sp.table_row;
             uint32_t si = sp.state;
             uint16_t* ring = (uint16_t*)g.st_buf[si];
             uint32_t* posmap = g.kv[si].posmap;
@@ -823,13 +869,13 @@ void fuse_materialize(const wt_blob* b) {
             AttnDecodeArgs a{};
             a.status = g.d_status;
             a.q = q_out; a.ring = ring; a.counter = ctr; a.n_kv = 0; a.n_kv_add = 1; a.bump_counter = ctr;
-            a.mask = mask; a.mask_seq_stride = nh * nslots; a.kvh_per_seq = kvh;
+            a.mask = mask; a.mask_seq_stride = sp.mask_row ? 0 : nh * nslots; a.kvh_per_seq = kvh;
             a.scale = sp.scale; a.scale_div = sp.scale_div; a.rep = nh / kvh; a.kv_heads = B * kvh; a.nslots = nslots;
             a.nsplit = attn_decode_nsplit(B * kvh, nslots, nh / kvh, hd, 0);
             a.part_o = g_attn_scratch;
             a.part_ml = g_attn_scratch + (size_t)B * kvh * a.nsplit * a.rep * hd;
             head.fused = [=](cudaStream_t st) {
-                k_rope_kv_append(st, qkv, cq, sq, ck, sk, q_out, ring, posmap, ctr, B, nh, kvh, hd, nslots, pos);
+                k_rope_kv_append(st, qkv, cq, sq, ck, sk, q_out, ring, posmap, ctr, B, nh, kvh, hd, nslots, pos, tab_row);
                 k_attn_decode(st, a, hd, ctx, B * kvh);
             };
             // The q|k|v projection right before the chain takes the rotary embedding and the append into
@@ -848,7 +894,7 @@ void fuse_materialize(const wt_blob* b) {
                     W4Epilogue ep;
                     ep.mode = 2;
                     ep.cos_q = cq; ep.sin_q = sq; ep.cos_k = ck; ep.sin_k = sk; ep.q_out = q_out; ep.ring = ring;
-                    ep.posmap = posmap; ep.counter = ctr; ep.nh = nh; ep.kvh = kvh; ep.nslots = nslots; ep.pos_const = pos;
+                    ep.posmap = posmap; ep.counter = ctr; ep.tab_row = tab_row; ep.nh = nh; ep.kvh = kvh; ep.nslots = nslots; ep.pos_const = pos;
                     const uint32_t* pk = it->second.packed;
                     const uint16_t* sc = it->second.scales;
                     lin.fused = [=](cudaStream_t st) {

@@ -38,11 +38,11 @@ size_t attn_decode_scratch_floats(uint32_t kv_heads_total, uint32_t rep, uint32_
 bool k_attn_decode(cudaStream_t st, const AttnDecodeArgs& a, uint32_t hd, uint16_t* out,
                    uint32_t kv_heads_total);
 
-// split + rotary + KV append in one launch (ops_fused.cu)
+// split + rotary + KV append in one launch (ops_fused.cu); tab_row: the tables are one row of hd for every head
 void k_rope_kv_append(cudaStream_t st, const uint16_t* qkv, const uint16_t* cos_q, const uint16_t* sin_q,
                       const uint16_t* cos_k, const uint16_t* sin_k, uint16_t* q_out, uint16_t* ring,
                       uint32_t* posmap, const uint32_t* counter, uint32_t B, uint32_t nh, uint32_t kvh,
-                      uint32_t hd, uint32_t nslots, uint32_t pos_const);
+                      uint32_t hd, uint32_t nslots, uint32_t pos_const, bool tab_row);
 
 // Prefill attention over token-major q [seq_q][nh][hd], k / v [seq_k][kvh][hd] -> out [seq_q][nh*hd]
 // (ops_attn_prefill.cu). `skip` marks (64-row query tile, 64-position key tile) pairs whose mask is -inf

@@ -26,7 +26,8 @@ struct W4Epilogue {
     uint16_t *sum_out = nullptr, *norm_out = nullptr;
     unsigned int* status = nullptr;   // engine status word: the tcgen05 GEMM reports a barrier wait that ran out here
     // mode 2
-    const uint16_t *cos_q = nullptr, *sin_q = nullptr, *cos_k = nullptr, *sin_k = nullptr;   // [M*heads][hd]
+    const uint16_t *cos_q = nullptr, *sin_q = nullptr, *cos_k = nullptr, *sin_k = nullptr;   // [M*heads][hd], or one row
+    bool tab_row = false;             // the tables are one row of hd for every head
     uint16_t *q_out = nullptr, *ring = nullptr;
     uint32_t* posmap = nullptr;
     const uint32_t* counter = nullptr;

@@ -17,7 +17,7 @@ __global__ void rope_kv_append_kernel(const uint16_t* __restrict__ qkv, const ui
                                       const uint16_t* __restrict__ sin_k, uint16_t* __restrict__ q_out,
                                       uint16_t* __restrict__ ring, uint32_t* __restrict__ posmap,
                                       const uint32_t* __restrict__ counter, uint32_t B, uint32_t nh,
-                                      uint32_t kvh, uint32_t hd, uint32_t nslots, uint32_t pos_const) {
+                                      uint32_t kvh, uint32_t hd, uint32_t nslots, uint32_t pos_const, bool tab_row) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t pos = (pos_const == 0xFFFFFFFAu) ? *counter : pos_const;
@@ -34,8 +34,8 @@ __global__ void rope_kv_append_kernel(const uint16_t* __restrict__ qkv, const ui
             const uint16_t* src = qkv + (size_t)b * row_w + (r - d);
             float x = h2f(src[d]);
             float rot = d < h ? -h2f(src[d + h]) : h2f(src[d - h]);
-            float xc = h2f(f2h(__fmul_rn(x, h2f(cos_q[e]))));
-            float xs = h2f(f2h(__fmul_rn(rot, h2f(sin_q[e]))));
+            float xc = h2f(f2h(__fmul_rn(x, h2f(cos_q[tab_row ? d : e]))));
+            float xs = h2f(f2h(__fmul_rn(rot, h2f(sin_q[tab_row ? d : e]))));
             q_out[e] = f2h(__fadd_rn(xc, xs));
         } else if (e < nq + nk) {
             uint32_t i = e - nq;
@@ -43,8 +43,8 @@ __global__ void rope_kv_append_kernel(const uint16_t* __restrict__ qkv, const ui
             const uint16_t* src = qkv + (size_t)b * row_w + nh * hd + (r - d);
             float x = h2f(src[d]);
             float rot = d < h ? -h2f(src[d + h]) : h2f(src[d - h]);
-            float xc = h2f(f2h(__fmul_rn(x, h2f(cos_k[i]))));
-            float xs = h2f(f2h(__fmul_rn(rot, h2f(sin_k[i]))));
+            float xc = h2f(f2h(__fmul_rn(x, h2f(cos_k[tab_row ? d : i]))));
+            float xs = h2f(f2h(__fmul_rn(rot, h2f(sin_k[tab_row ? d : i]))));
             kf[i] = f2h(__fadd_rn(xc, xs));
         } else {
             uint32_t i = e - nq - nk;
@@ -58,12 +58,12 @@ __global__ void rope_kv_append_kernel(const uint16_t* __restrict__ qkv, const ui
 void k_rope_kv_append(cudaStream_t st, const uint16_t* qkv, const uint16_t* cos_q, const uint16_t* sin_q,
                       const uint16_t* cos_k, const uint16_t* sin_k, uint16_t* q_out, uint16_t* ring,
                       uint32_t* posmap, const uint32_t* counter, uint32_t B, uint32_t nh, uint32_t kvh,
-                      uint32_t hd, uint32_t nslots, uint32_t pos_const) {
+                      uint32_t hd, uint32_t nslots, uint32_t pos_const, bool tab_row) {
     uint32_t total = B * (nh + 2 * kvh) * hd;
     uint32_t grid = (total + 255) / 256;
     if (grid > 148 * 8) grid = 148 * 8;
     launch_pdl(rope_kv_append_kernel, dim3(grid), dim3(256), 0, st, qkv, cos_q, sin_q, cos_k, sin_k, q_out, ring, posmap, counter,
-               B, nh, kvh, hd, nslots, pos_const);
+               B, nh, kvh, hd, nslots, pos_const, tab_row);
     g_launches++;
 }
 

@@ -312,9 +312,10 @@ w4a16_skinny_kernel(const uint16_t* __restrict__ a, const uint4* __restrict__ wp
             const uint16_t* st = is_q ? ep.sin_q : ep.sin_k;
             uint16_t* dst = is_q ? ep.q_out : kf;
             const float fa = h2f(xa), fb = h2f(xb);
+            const size_t to = ep.tab_row ? d : o;
             // out[d] = x[d] cos - x[d+64] sin ; out[d+64] = x[d+64] cos + x[d] sin, each product rounded to fp16
-            const float lo = __fadd_rn(h2f(f2h(__fmul_rn(fa, h2f(ct[o])))), h2f(f2h(__fmul_rn(-fb, h2f(st[o])))));
-            const float hi = __fadd_rn(h2f(f2h(__fmul_rn(fb, h2f(ct[o + 64])))), h2f(f2h(__fmul_rn(fa, h2f(st[o + 64])))));
+            const float lo = __fadd_rn(h2f(f2h(__fmul_rn(fa, h2f(ct[to])))), h2f(f2h(__fmul_rn(-fb, h2f(st[to])))));
+            const float hi = __fadd_rn(h2f(f2h(__fmul_rn(fb, h2f(ct[to + 64])))), h2f(f2h(__fmul_rn(fa, h2f(st[to + 64])))));
             dst[o] = f2h(lo);
             dst[o + 64] = f2h(hi);
         }
