@@ -17,7 +17,7 @@
 //   warp 0 : one lane issues the TMA loads of both operand tiles into a STAGES-deep ring
 //   warp 1 : one lane issues tcgen05.mma (4 x k16 per stage and row half) and tcgen05.commit
 //   warp 3 : owns the TMEM allocation
-//   warps 4-7 : epilogue (tcgen05.ld -> fp16 -> 64-byte row segments)
+//   warps 4-11: epilogue (tcgen05.ld -> fp16 -> 64-byte row segments), two warps per 32 rows, every second column chunk
 // All mbarrier waits are bounded; on a timeout the CTA raises the engine's status word, every role
 // stops, in-flight copies are waited for (bounded) and the TMEM is freed.
 #include <cstdlib>
@@ -36,14 +36,17 @@ using namespace sm100;
 
 namespace {
 
-constexpr int BK = 64, HALF_A_BYTES = 128 * BK * 2, NTHREADS = 256, EPI_WARPS = 4, MAX_STAGES = 6;
+constexpr int BK = 64, HALF_A_BYTES = 128 * BK * 2, NTHREADS = 384, EPI_WARPS = 8, MAX_STAGES = 6;
 
 template <int MH, int BN>
 struct FCfg {
     static constexpr int A_BYTES = MH * HALF_A_BYTES, B_BYTES = BN * BK * 2;
-    static constexpr int STAGES = (A_BYTES + B_BYTES) <= 32768 ? 6 : ((A_BYTES + B_BYTES) <= 49152 ? 4 : 3);
-    static constexpr int NBUF = (MH * BN == 512) ? 1 : 2;
-    static constexpr uint32_t ACC_COLS = MH * BN, TMEM_COLS = NBUF * ACC_COLS;
+    static constexpr int STAGES = (A_BYTES + B_BYTES) <= 32768 ? 6 : ((A_BYTES + B_BYTES) <= 57344 ? 4 : 3);
+    // Two accumulator buffers where 512 TMEM columns hold them. Else one, released by row halves: the next tile's products
+    // for the first 128 rows run while the epilogue drains the second.
+    static constexpr int NBUF = MH * BN > 256 ? 1 : 2;
+    static constexpr bool HALVES = NBUF == 1 && MH == 2;
+    static constexpr uint32_t ACC_COLS = MH * BN, TMEM_COLS = NBUF * ACC_COLS > 256 ? 512 : 256;   // a power of two
 };
 
 struct __align__(8) FBarriers {
@@ -70,15 +73,12 @@ struct EpiF16 {
         }
     }
 };
-// Operand type by epilogue. EDGE: N need not be a multiple of the tile width nor K of 64 (the tensor maps zero-fill what
-// lies outside), the epilogue checks its columns.
+// Operand type by epilogue
 template <class E> struct InOf {
-    static constexpr bool EDGE = true;
     static constexpr CUtensorMapDataType MAP = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     static constexpr uint32_t IDESC = (1u << 7) | (1u << 10);      // A and B are bf16
 };
 template <> struct InOf<EpiF16> {
-    static constexpr bool EDGE = false;
     static constexpr CUtensorMapDataType MAP = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     static constexpr uint32_t IDESC = 0;
 };
@@ -86,6 +86,8 @@ template <> struct InOf<EpiF16> {
 template <class E> struct Heavy { static constexpr bool value = false; };
 template <class A> struct Heavy<EpiTanh<A>> { static constexpr bool value = true; };
 
+// N need not be a multiple of the tile width nor K of 64: the tensor maps zero-fill what lies outside, chunks of 32 columns
+// past N are left out and the epilogue checks the columns of the last one (EpiF16: N is a multiple of 128).
 // fp16 outputs: rows ldy elements apart (the SPLIT form writes N columns of a row of N_full).
 template <int MH, int BN, class E>
 __global__ void __launch_bounds__(NTHREADS, 1)
@@ -103,15 +105,15 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     volatile uint32_t* abort_flag = &bars->abort_flag;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t KG = IO::EDGE ? (K + BK - 1) / BK : K / BK;
-    const uint32_t m_tiles = (M + 128 * MH - 1) / (128 * MH), tiles = m_tiles * (IO::EDGE ? (N + BN - 1) / BN : N / BN);
+    const uint32_t KG = (K + BK - 1) / BK;
+    const uint32_t m_tiles = (M + 128 * MH - 1) / (128 * MH), tiles = m_tiles * ((N + BN - 1) / BN);
     // Split K (S > 1): a work item is (tile, run of K/64/S k blocks), item = run * tiles + tile. With `part` a run leaves its
     // fp32 sums in part[run][row][N]; f16_splitk_reduce_kernel adds the runs in order and applies the epilogue.
     const uint32_t items = tiles * S, KGS = KG / S;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
-        for (int s = 0; s < NBUF; s++) { mbar_init(&bars->tmem_full[s], 1); mbar_init(&bars->tmem_empty[s], EPI_WARPS); }
+        for (int s = 0; s < 2; s++) { mbar_init(&bars->tmem_full[s], 1); mbar_init(&bars->tmem_empty[s], EPI_WARPS); }
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -152,6 +154,7 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         bool live = true;
         for (uint32_t item = blockIdx.x; item < items && live; item += gridDim.x, t++) {
             const uint32_t buf = t % NBUF;
+            // tmem_empty: one barrier per buffer, or (HALVES) per row half
             if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&bars->tmem_empty[buf], ((t / NBUF) & 1) ^ 1, abort_flag))) { *abort_flag = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + buf * ACC_COLS;
@@ -160,7 +163,22 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&bars->full[s], ph, abort_flag))) { *abort_flag = 1; live = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da0 = umma_desc(a_base + s * A_BYTES), db0 = umma_desc(b_base + s * B_BYTES);
-                if (lane == 0) {
+                if (C::HALVES && kb == 0) {
+                    // first k block of a tile: the second half's accumulator may still be on its way out
+#pragma unroll
+                    for (int h = 0; h < MH; h++) {
+                        if (h) {
+                            if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&bars->tmem_empty[1], (t & 1) ^ 1, abort_flag))) { *abort_flag = 1; live = false; break; }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        if (lane == 0) {
+#pragma unroll
+                            for (uint32_t k4 = 0; k4 < BK / 16; k4++)
+                                umma_f16(acc + h * BN, da0 + (uint64_t)(h * (HALF_A_BYTES >> 4) + k4 * 2), db0 + (uint64_t)(k4 * 2), idesc_f16(BN) | IO::IDESC, k4);
+                        }
+                    }
+                    if (lane == 0 && live) umma_commit(&bars->empty[s]);
+                } else if (lane == 0) {
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < BK / 16; k4++) {
 #pragma unroll
@@ -171,6 +189,7 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     umma_commit(&bars->empty[s]);
                 }
                 __syncwarp();
+                if (!live) break;
             }
             if (!live) break;
             if (lane == 0) umma_commit(&bars->tmem_full[buf]);
@@ -178,7 +197,7 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
     } else if (warp >= 4) {
         // epilogue: TMEM lane = output row; a warp may touch lanes (warp % 4) * 32 .. +31
-        const uint32_t lane_base = (warp & 3) * 32;
+        const uint32_t lane_base = (warp & 3) * 32, chunk0 = (warp - 4) >> 2;
         uint32_t t = 0;
         asm volatile("griddepcontrol.wait;" ::: "memory");   // y may be memory the predecessor still reads
         for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, t++) {
@@ -193,7 +212,7 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             for (int h = 0; h < MH; h++) {
                 const uint32_t m = m0 + h * 128 + lane_base + lane;
 #pragma unroll 1
-                for (uint32_t c = 0; c < BN / 32; c++) {
+                for (uint32_t c = chunk0; c < BN / 32; c += EPI_WARPS / 4) {
                     uint32_t v[32];
                     const uint32_t taddr = tmem + (lane_base << 16) + buf * ACC_COLS + h * BN + c * 32;
                     asm volatile(
@@ -208,22 +227,24 @@ f16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     const uint32_t n = n0 + c * 32;
                     if (m < M && part) {
                         // rows of the partial sums are N rounded up to 4 floats apart
-                        const uint32_t np = IO::EDGE ? (N + 3) & ~3u : N;
+                        const uint32_t np = (N + 3) & ~3u;
                         uint4* dst = (uint4*)(part + ((size_t)run * M + m) * np + n);
 #pragma unroll
                         for (int q = 0; q < 8; q++)
-                            if (!IO::EDGE || n + 4 * q < np) dst[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                            if (n + 4 * q < np) dst[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     } else if (m < M) {
                         float f[32];
 #pragma unroll
                         for (int q = 0; q < 32; q++) f[q] = __uint_as_float(v[q]);
-                        if (!IO::EDGE || n < N) epi.chunk(m, n, f, N);
+                        if (n < N) epi.chunk(m, n, f, N);
                     }
                 }
+                if (C::HALVES || h == MH - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->tmem_empty[C::HALVES ? h : buf]);
+                }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->tmem_empty[buf]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -287,40 +308,17 @@ SplitScratch* split_scratch(cudaStream_t st, size_t need) {
 
 template <int MH, int BN, class E>
 bool launch(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16_t* w, const E& epi, uint32_t M, uint32_t K, uint32_t N,
-            unsigned int* status, int sms) {
+            unsigned int* status, uint32_t sms, uint32_t S) {
     using C = FCfg<MH, BN>;
     using IO = InOf<E>;
-    // an epilogue that is too much for four warps goes to the reduction kernel even of a single run
+    // an epilogue that reads and writes rows of its own goes to the reduction kernel even of a single run
     using G = typename std::conditional<Heavy<E>::value, EpiPlain<false, false>, E>::type;
     CUtensorMap ta, tw;
     if (!make_map(&ta, IO::MAP, a, M, K, lda, 128) || !make_map(&tw, IO::MAP, w, N, K, K, BN)) return false;
     const size_t smem = 1024 + (size_t)C::STAGES * (C::A_BYTES + C::B_BYTES) + sizeof(FBarriers) + 16;
     static int have[64] = {};
     if (!ensure_dyn_smem(f16_gemm_sm100_kernel<MH, BN, G>, smem, have)) return false;
-    const uint32_t tiles = ((M + 128 * MH - 1) / (128 * MH)) * ((N + BN - 1) / BN), KG = (K + BK - 1) / BK;
-    const uint32_t np = (N + 3) & ~3u;
-    // Split K while the tiles alone leave SMs idle (same rule as the W4A16 GEMM): the divisor of K/64 that makes
-    // (items per CTA) x (k blocks per item + set-up) smallest, a run at least one trip round the ring, partial sums <= 64 MB.
-    uint32_t S = 1;
-    if (tiles < (uint32_t)sms) {
-        float best = (float)(KG + 4);
-        for (uint32_t c = 2; c <= 32 && c <= KG; c++) {
-            if (KG % c || KG / c < (uint32_t)C::STAGES || (size_t)c * M * np * sizeof(float) > ((size_t)64 << 20)) continue;
-            const uint32_t rounds = (tiles * c + sms - 1) / sms;
-            const float cost = (float)rounds * (float)(KG / c + 4) + 0.75f * (float)c + 6.0f;
-            if (cost < best) { best = cost; S = c; }
-        }
-    }
-    // sums that go through memory anyway: also where the tiles fill the SMs but their last round would not
-    if (Heavy<E>::value && tiles >= (uint32_t)sms) {
-        const float run_cost = (float)((double)M * np * sizeof(float) / 2e6);      // one more run to write and read, in k blocks
-        float best = (float)((tiles + sms - 1) / sms) * (float)(KG + 4);
-        for (uint32_t c = 2; c <= 4; c++) {
-            if (KG % c || KG / c < (uint32_t)C::STAGES || (size_t)c * M * np * sizeof(float) > ((size_t)64 << 20)) continue;
-            const float cost = (float)((tiles * c + sms - 1) / sms) * (float)(KG / c + 4) + (float)(c - 1) * run_cost;
-            if (cost < best) { best = cost; S = c; }
-        }
-    }
+    const uint32_t tiles = ((M + 128 * MH - 1) / (128 * MH)) * ((N + BN - 1) / BN), np = (N + 3) & ~3u;
     float* part = nullptr;
     if (S > 1 || Heavy<E>::value) {
         SplitScratch* ss = split_scratch(st, (size_t)S * M * np * sizeof(float));
@@ -330,7 +328,7 @@ bool launch(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16_t* w,
     if constexpr (!Heavy<E>::value) direct = epi;
     else if (!part) return false;
     const uint32_t items = tiles * S;
-    const uint32_t grid = items < (uint32_t)sms ? items : (uint32_t)sms;
+    const uint32_t grid = items < sms ? items : sms;
     if (launch_pdl(f16_gemm_sm100_kernel<MH, BN, G>, dim3(grid), dim3(NTHREADS), smem, st, ta, tw, direct, M, K, N, status, S, part) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -339,7 +337,7 @@ bool launch(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16_t* w,
     if (part) {
         const size_t quads = (size_t)M * np / 4;
         uint32_t rg = (uint32_t)((quads + 255) / 256);
-        if (rg > (uint32_t)sms * 8) rg = (uint32_t)sms * 8;
+        if (rg > sms * 8) rg = sms * 8;
         if (launch_pdl(f16_splitk_reduce_kernel<E>, dim3(rg), dim3(256), 0, st, (const float*)part, epi, M, N, S) != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -478,7 +476,18 @@ bool launch_gemv(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t
     return true;
 }
 
-// tile shape by the number of tiles it gives
+// Tile and split of K. A CTA takes in operand tiles at 110 to 125 GB/s whatever the shape (64 bytes a cycle and SM), so a k
+// block lasts as long as its bytes, a round over the SMs as its k blocks and the part of the epilogue that nothing hides
+// (single accumulator buffer: half of it). Measured on one B200, us per k block and per epilogue:
+//     128 x 128  0.296  0.8      128 x 192  0.316  1.2      128 x 256  0.334  2.5      256 x 160  0.465  5      256 x 192  0.484  6
+// A wide tile brings more products per byte, a narrow one wastes less of the last round; runs of K fill the SMs where tiles
+// alone do not and cost a second launch that reads their fp32 sums. The smallest sum of these is taken; it lies within 10 %
+// of the measured best of 40 combinations at M 77 .. 2048, K 1024 .. 9728, N 1024 .. 19456. 2048 rows, before -> now:
+// 2560 x 10240 105 -> 87 us, gelu 2560 x 19456 178 -> 151, into the residual 4096 x 2560 87 -> 63, 9728 x 2560 146 -> 103.
+// (256 x 128, 256 x 224 and 256 x 256, 0.42, 0.625 and 0.625 us a k block, were never more than 1 % ahead.)
+struct TileCost { uint32_t mh, bn; float kb, epi; };
+constexpr TileCost kTiles[] = {{1, 128, 0.296f, 0.8f}, {1, 192, 0.316f, 1.2f}, {1, 256, 0.334f, 2.5f}, {2, 160, 0.465f, 5.0f}, {2, 192, 0.484f, 6.0f}};
+
 template <class E>
 bool launch_tiles(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16_t* w, const E& epi, uint32_t M, uint32_t K, uint32_t N,
                   unsigned int* status) {
@@ -490,14 +499,29 @@ bool launch_tiles(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 148;
     }
-    const uint32_t t256 = ((M + 255) / 256) * ((N + 255) / 256), t128 = ((M + 255) / 256) * ((N + 127) / 128);
-    // row-count projections: the wider tile where its rounds over the SMs are not worth more than those of the narrow one
-    // (0.55 of its time, and an epilogue that overlaps the next tile's products)
-    const uint32_t r256 = (t256 + sms - 1) / sms, r128 = (t128 + sms - 1) / sms;
-    if (InOf<E>::EDGE && M > 128 && t128 >= (uint32_t)sms && 11 * r128 < 20 * r256) return launch<2, 128, E>(st, a, lda, w, epi, M, K, N, status, sms);
-    if ((InOf<E>::EDGE || N % 256 == 0) && M > 128 && t256 >= (uint32_t)sms) return launch<2, 256, E>(st, a, lda, w, epi, M, K, N, status, sms);
-    if (M > 128 && t128 >= (uint32_t)sms) return launch<2, 128, E>(st, a, lda, w, epi, M, K, N, status, sms);
-    return launch<1, 128, E>(st, a, lda, w, epi, M, K, N, status, sms);
+    const uint32_t KG = (K + BK - 1) / BK, np = (N + 3) & ~3u;
+    const double run_bytes = (double)M * np * sizeof(float);
+    int best = 0;
+    uint32_t S = 1;
+    float best_us = 0.0f;
+    for (int i = 0; i < (int)(sizeof(kTiles) / sizeof(kTiles[0])); i++) {
+        const TileCost& t = kTiles[i];
+        const uint32_t tiles = ((M + 128 * t.mh - 1) / (128 * t.mh)) * ((N + t.bn - 1) / t.bn);
+        for (uint32_t c = 1; c <= 32 && c <= KG; c++) {
+            // a run at least 6 k blocks (one trip round the longest ring), partial sums <= 64 MB
+            if (c > 1 && (KG % c || KG / c < (uint32_t)MAX_STAGES || c * run_bytes > (double)(64u << 20))) continue;
+            float us = (float)((tiles * c + sms - 1) / sms) * ((float)(KG / c) * t.kb + t.epi);
+            if (c > 1 || Heavy<E>::value) us += 2.0f + (float)(c * run_bytes * 2.0 / 5e6);
+            if (best_us == 0.0f || us < best_us) { best_us = us; best = i; S = c; }
+        }
+    }
+    switch (best) {
+        case 0: return launch<1, 128, E>(st, a, lda, w, epi, M, K, N, status, sms, S);
+        case 1: return launch<1, 192, E>(st, a, lda, w, epi, M, K, N, status, sms, S);
+        case 2: return launch<1, 256, E>(st, a, lda, w, epi, M, K, N, status, sms, S);
+        case 3: return launch<2, 160, E>(st, a, lda, w, epi, M, K, N, status, sms, S);
+        default: return launch<2, 192, E>(st, a, lda, w, epi, M, K, N, status, sms, S);
+    }
 }
 
 }  // namespace
