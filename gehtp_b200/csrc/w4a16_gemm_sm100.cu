@@ -2,15 +2,16 @@
 // Y[M,N] = A[M,K] . W, W = fp16((q-8)*scale), fp32 accumulation in TMEM.
 //
 // Persistent kernel, one CTA per SM. A CTA walks output tiles of (128*MH) x BN (MH = 1 or 2 row halves sharing
-// one dequantised B tile, BN = 128 or 256 columns); K is walked in steps of 64 (one scale group, one 128-byte
+// one dequantised B tile, BN = 128 to 256 columns); K is walked in steps of 64 (one scale group, one 128-byte
 // swizzled row per operand row).
 //   warp 0     : one lane issues the TMA loads of the A tile (MH boxes of 128 rows x 64 k, SWIZZLE_128B) into a
 //                STAGES-deep ring. A is [M][K], or [K / d][M][d] read through a three-dimensional map (the
 //                output of a per-head kernel, without a transposed copy).
 //   warp 1     : walks the k loop as a whole warp (uniform counters and descriptors); one lane issues
 //                tcgen05.mma (4 x k16 x MH per stage, M128 x BN) and tcgen05.commit, which frees the stage
-//                when the MMAs have read it. The accumulators are double-buffered in TMEM (except 256 x 256)
-//                so that the epilogue of a tile overlaps the main loop of the next one.
+//                when the MMAs have read it. The accumulators are double-buffered in TMEM (256 rows x 160 and
+//                more columns: single, released by row halves) so that the epilogue of a tile overlaps the main
+//                loop of the next one.
 //   warp 2     : one lane streams the int4 tile of each k block (BN / 16 strip units, contiguous in the
 //                strip-major layout) and its BN group scales with bulk copies into an RSTAGES-deep ring.
 //   warp 3     : owns the TMEM allocation.
@@ -50,30 +51,29 @@ constexpr int HALF_A_BYTES = 128 * BK * 2;
 constexpr int NTHREADS = 768;
 constexpr int DQ_PER_STAGE = 4, EPI_WARPS = 4;   // 16 dequant warps, 4 of them per k block
 
-// Tile configuration: MH row halves of 128 x BN columns per tile.
-//   <1,128>: 128x128, 4 stages, two accumulator buffers   (small M, or N not a multiple of 256)
-//   <2,128>: 256x128, 4 stages, two accumulator buffers
-//   <2,256>: 256x256, 3 stages, one accumulator buffer (all 512 TMEM columns): per FLOP it reads
-//            45 % fewer operand bytes from L2 and a third fewer from shared memory than 256x128;
-//            the epilogue is not overlapped (a few % of a K >= 2048 main loop).
-//   <1,256>: 128x256, 3 stages, two accumulator buffers: the gate | up form (DUAL) at few rows.
+// Tile configurations <MH, BN>: <1,128>, <1,192>, <1,256>, <2,128>, <2,160>, <2,192>, <2,256>; which one: kTiles below.
 // DUAL (BN = 256 only): the B tile of a k block holds 128 columns of a first weight matrix (gate) and the same 128
 // columns of a second one (up); one N = 256 instruction feeds both accumulators and the epilogue writes
 // fp16(fp16(gate * fp16(sigmoid(gate))) * up), 128 output columns per tile: the two projections of a gated FFN and
 // the three elementwise ops behind them in one launch, neither projection's output going through memory.
 template <int MH, int BN>
 struct Cfg {
-    static constexpr int STAGES = BN == 256 ? 3 : 4;
-    static constexpr int NBUF = (MH * BN == 512) ? 1 : 2;
+    static constexpr int A_BYTES = MH * HALF_A_BYTES, B_BYTES = BN * BK * 2;
+    static constexpr int RAW_BYTES = BN * BK / 2, RAW_SLOT = RAW_BYTES + BN * 2;   // nibbles + BN fp16 scales
+    static constexpr int STAGES = 4 * (A_BYTES + B_BYTES + RAW_SLOT) + 2048 <= 227 * 1024 ? 4 : 3;
+    // Two accumulator buffers where 512 TMEM columns hold them. Else one, released by row halves: the next tile's products
+    // for the first 128 rows run while the epilogue drains the second.
+    static constexpr int NBUF = MH * BN > 256 ? 1 : 2;
+    static constexpr bool HALVES = NBUF == 1;
     // One dequant group (4 warps) per operand stage, and one int4/scale slot per group: group q only
     // ever waits on stage q and slot q, so it sees every phase of those barriers in turn. (A parity
     // wait is only sound when the waiter has seen the phase before the one it waits for.)
     static constexpr int GROUPS = STAGES;
     static constexpr int RSTAGES = STAGES;
-    static constexpr int A_BYTES = MH * HALF_A_BYTES, B_BYTES = BN * BK * 2;
-    static constexpr int RAW_BYTES = BN * BK / 2, RAW_SLOT = RAW_BYTES + BN * 2;   // nibbles + BN fp16 scales
+    // three stages leave warps 20-23 without one: they take every second column chunk of the epilogue
+    static constexpr bool EPI2 = GROUPS == 3;
     static constexpr uint32_t ACC_COLS = MH * BN;             // TMEM columns of one accumulator buffer
-    static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS;    // 256 or 512: a power of two
+    static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS > 256 ? 512 : 256;      // a power of two
     // instruction descriptor, kind::f16: A,B fp16 K-major, D fp32, M128 x N = BN
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 };
@@ -128,7 +128,6 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                         uint32_t N, W4Epilogue ep, uint32_t S, float* __restrict__ part, uint32_t a_d) {
     using C = Cfg<MH, BN>;
     static_assert(!DUAL || BN == 256, "the gate | up form pairs two 128-column halves");
-    static_assert(!DUAL || C::GROUPS == 3, "warps 20-23 help the epilogue of the gate | up form: they must own no operand stage");
     constexpr uint32_t BN_OUT = DUAL ? BN / 2 : BN;      // output (and weight) columns of one tile
     constexpr int STAGES = C::STAGES, RSTAGES = C::RSTAGES, NBUF = C::NBUF;
     constexpr int A_BYTES = C::A_BYTES, B_BYTES = C::B_BYTES, RAW_BYTES = C::RAW_BYTES, RAW_SLOT = C::RAW_SLOT;
@@ -147,7 +146,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
     // drains; only the A loads and the epilogue's global accesses order themselves after it.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t m_tiles = (M + 128 * MH - 1) / (128 * MH), n_tiles = N / BN_OUT;
+    const uint32_t m_tiles = (M + 128 * MH - 1) / (128 * MH), n_tiles = (N + BN_OUT - 1) / BN_OUT;
     const uint32_t tiles = m_tiles * n_tiles;
     // Split K: S > 1 cuts the k blocks of every tile into S runs, one work item each (item = run * tiles + tile);
     // a run leaves its fp32 partial sums in `part` ([run][row][N]) and a small kernel behind this one adds the
@@ -160,7 +159,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
             mbar_init(&bars->empty[s], 1);
         }
         for (int s = 0; s < RSTAGES; s++) { mbar_init(&bars->raw_full[s], 1); mbar_init(&bars->raw_empty[s], DQ_PER_STAGE); }
-        for (int s = 0; s < NBUF; s++) { mbar_init(&bars->tmem_full[s], 1); mbar_init(&bars->tmem_empty[s], DUAL ? 2 * EPI_WARPS : EPI_WARPS); }
+        for (int s = 0; s < 2; s++) { mbar_init(&bars->tmem_full[s], 1); mbar_init(&bars->tmem_empty[s], C::EPI2 ? 2 * EPI_WARPS : EPI_WARPS); }
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -207,6 +206,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
         bool live = true;
         for (uint32_t item = blockIdx.x; item < items && live; item += gridDim.x, t++) {
             const uint32_t buf = t % NBUF;
+            // tmem_empty: one barrier per buffer, or (HALVES) per row half
             if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&bars->tmem_empty[buf], ((t / NBUF) & 1) ^ 1, abort_flag))) { *abort_flag = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + buf * ACC_COLS;
@@ -214,7 +214,22 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                 if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&bars->full[s], ph, abort_flag))) { *abort_flag = 1; live = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da0 = da_base + (uint64_t)(s * (A_BYTES >> 4)), db0 = db_base + (uint64_t)(s * (B_BYTES >> 4));
-                if (lane == 0) {
+                if (C::HALVES && kb == 0) {
+                    // first k block of a tile: the second half's accumulator may still be on its way out
+#pragma unroll
+                    for (int h = 0; h < MH; h++) {
+                        if (h) {
+                            if (!__all_sync(0xffffffffu, mbar_wait_or_abort(&bars->tmem_empty[1], (t & 1) ^ 1, abort_flag))) { *abort_flag = 1; live = false; break; }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        if (lane == 0) {
+#pragma unroll
+                            for (uint32_t k4 = 0; k4 < BK / 16; k4++)
+                                umma_f16(acc + h * BN, da0 + (uint64_t)(h * (HALF_A_BYTES >> 4) + k4 * 2), db0 + (uint64_t)(k4 * 2), C::IDESC, k4);
+                        }
+                    }
+                    if (lane == 0 && live) umma_commit(&bars->empty[s]);
+                } else if (lane == 0) {
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < BK / 16; k4++) {
 #pragma unroll
@@ -225,6 +240,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                     umma_commit(&bars->empty[s]);
                 }
                 __syncwarp();
+                if (!live) break;
                 if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
             }
             if (!live) break;
@@ -238,6 +254,9 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
             for (uint32_t item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
                 const uint32_t tile = item % tiles, kb0 = (item / tiles) * KGS;
                 const uint32_t n0 = (tile / m_tiles) * BN_OUT;
+                // the last tile of a row may reach past N: its copies end there, what the slot holds beyond only reaches
+                // accumulator columns that are not stored
+                const uint32_t cols = DUAL ? BN_OUT : min((uint32_t)BN, N - n0);
                 const uint4* wsrc = wp + (size_t)(n0 / 16) * 32;
                 const uint16_t* ssrc = sc + n0;
                 const uint4* wsrc2 = DUAL ? wp2 + (size_t)(n0 / 16) * 32 : nullptr;
@@ -246,26 +265,26 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                     const uint32_t r = it % RSTAGES, ph = (it / RSTAGES) & 1;
                     if (*abort_flag || !mbar_wait(&bars->raw_empty[r], ph ^ 1)) { *abort_flag = 1; break; }
                     unsigned char* dst = sRaw + r * RAW_SLOT;
-                    mbar_expect_tx(&bars->raw_full[r], RAW_SLOT);
+                    mbar_expect_tx(&bars->raw_full[r], DUAL ? RAW_SLOT : cols * (BK / 2 + 2));
                     if (DUAL) {      // strip units 0-7 and scales 0-127 from the first matrix, the rest from the second
                         bulk_load(dst, wsrc + (size_t)kb * NB * 32, RAW_BYTES / 2, &bars->raw_full[r]);
                         bulk_load(dst + RAW_BYTES / 2, wsrc2 + (size_t)kb * NB * 32, RAW_BYTES / 2, &bars->raw_full[r]);
                         bulk_load(dst + RAW_BYTES, ssrc + (size_t)kb * N, BN_OUT * 2, &bars->raw_full[r]);
                         bulk_load(dst + RAW_BYTES + BN_OUT * 2, ssrc2 + (size_t)kb * N, BN_OUT * 2, &bars->raw_full[r]);
                     } else {
-                        bulk_load(dst, wsrc + (size_t)kb * NB * 32, RAW_BYTES, &bars->raw_full[r]);
-                        bulk_load(dst + RAW_BYTES, ssrc + (size_t)kb * N, BN * 2, &bars->raw_full[r]);
+                        bulk_load(dst, wsrc + (size_t)kb * NB * 32, cols * (BK / 2), &bars->raw_full[r]);
+                        bulk_load(dst + RAW_BYTES, ssrc + (size_t)kb * N, cols * 2, &bars->raw_full[r]);
                     }
                 }
             }
             if (*abort_flag)
                 for (uint32_t j = it > (uint32_t)RSTAGES ? it - RSTAGES : 0; j < it; j++) mbar_wait(&bars->raw_full[j % RSTAGES], (j / RSTAGES) & 1);
         }
-    } else if ((warp >= 4 && warp < 8) || (DUAL && warp >= 20)) {
-        // ---- epilogue: TMEM lane = output row; a warp may touch lanes (warp % 4) * 32 .. +31. The gate | up form
-        // (three operand stages: dequant warps 20-23 have no stage) gives those four warps every second column chunk.
+    } else if ((warp >= 4 && warp < 8) || (C::EPI2 && warp >= 20)) {
+        // ---- epilogue: TMEM lane = output row; a warp may touch lanes (warp % 4) * 32 .. +31
         const uint32_t lane_base = (warp & 3) * 32;
-        const uint32_t chunk0 = (DUAL && warp >= 20) ? 1 : 0;
+        const uint32_t chunk0 = warp >= 20 ? 1 : 0;
+        constexpr uint32_t CSTEP = C::EPI2 ? 2 : 1;
         uint32_t t = 0;
         // y (and the residual) may be memory the predecessor still reads or writes
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -306,7 +325,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                 if (DUAL) {
                     // gate in accumulator columns 0-127, up in 128-255: 16 columns of each at a time
 #pragma unroll 1
-                    for (uint32_t c = chunk0; c < BN_OUT / 16; c += 2) {
+                    for (uint32_t c = chunk0; c < BN_OUT / 16; c += CSTEP) {
                         uint32_t vg[16], vu[16];
                         const uint32_t taddr = tmem + (lane_base << 16) + buf * ACC_COLS + h * BN + c * 16;
                         tmem_ld16(taddr, vg);
@@ -332,10 +351,9 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                             dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
                         }
                     }
-                    continue;
                 }
 #pragma unroll 1
-                for (uint32_t c = 0; c < BN / 32; c++) {
+                for (uint32_t c = chunk0; !DUAL && c < BN / 32 && n0 + c * 32 < N; c += CSTEP) {
                     uint32_t v[32];
                     const uint32_t taddr = tmem + (lane_base << 16) + buf * ACC_COLS + h * BN + c * 32;
                     asm volatile(
@@ -356,17 +374,19 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                         for (int q = 0; q < 8; q++) dst[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     }
                 }
+                if (C::HALVES || h == MH - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->tmem_empty[C::HALVES ? h : buf]);
+                }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->tmem_empty[buf]);
         }
     } else if (warp >= 8) {
         // ---- dequant: one group of 4 warps per operand stage; group q takes the k blocks with
-        // it % STAGES == q, and warp j of a group turns strip units UPW*j .. UPW*j+UPW-1 (BN/4
-        // columns) of that block into fp16, two units at a time. A warp so has STAGES k-block
-        // periods for its share, and pays one proxy fence for all of it.
-        constexpr int UPW = BN / 64;       // strip units per warp and k block: 2 or 4
+        // it % STAGES == q, and warp j of a group turns strip units j, j + 4, ... of that block
+        // into fp16, two units at a time. A warp so has STAGES k-block periods for its share, and
+        // pays one proxy fence for all of it.
+        constexpr int UNITS = BN / 16, UPW = (UNITS + 3) / 4;       // strip units per k block and (at most) per warp
         constexpr int GROUPS = C::GROUPS;
         const uint32_t dw = warp - 8, q = dw >> 2, j = dw & 3, g = lane >> 2, t = lane & 3;
         const uint32_t my_items = blockIdx.x < items ? (items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -392,7 +412,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
             uint16_t sl[UPW], sh[UPW];
 #pragma unroll
             for (int u = 0; u < UPW; u++) {
-                const uint32_t unit = UPW * j + u;
+                const uint32_t unit = min(j + 4 * u, (uint32_t)UNITS - 1);      // a warp with one unit less reads the last again
                 asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                              : "=r"(w[u].x), "=r"(w[u].y), "=r"(w[u].z), "=r"(w[u].w) : "r"(raw + (unit * 32 + lane) * 16));
                 asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sl[u]) : "r"(raw + RAW_BYTES + (unit * 16 + g) * 2));
@@ -406,7 +426,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
             for (int up = 0; up < UPW; up += 2) {
                 uint32_t o[2][4][4];
 #pragma unroll
-                for (int u = 0; u < 2; u++) {
+                for (int u = 0; u < 2 && up + u < UPW; u++) {
                     const __half2 slo = __half2half2(__ushort_as_half(sl[up + u])), shi = __half2half2(__ushort_as_half(sh[up + u]));
                     dequant_word(w[up + u].x, slo, shi, o[u][0]);
                     dequant_word(w[up + u].y, slo, shi, o[u][1]);
@@ -418,8 +438,9 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                     stage_free = true;
                 }
 #pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const uint32_t ub = bt + (UPW * j + up + u) * 2048;
+                for (int u = 0; u < 2 && up + u < UPW; u++) {
+                    if (UNITS % 4 && j + 4 * (up + u) >= (uint32_t)UNITS) break;
+                    const uint32_t ub = bt + (j + 4 * (up + u)) * 2048;
                     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(ub + off[0]), "r"(o[u][0][0]), "r"(o[u][0][2]), "r"(o[u][1][0]), "r"(o[u][1][2]) : "memory");
                     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(ub + off[1]), "r"(o[u][2][0]), "r"(o[u][2][2]), "r"(o[u][3][0]), "r"(o[u][3][2]) : "memory");
                     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(ub + off[2]), "r"(o[u][0][1]), "r"(o[u][0][3]), "r"(o[u][1][1]), "r"(o[u][1][3]) : "memory");
@@ -518,34 +539,21 @@ SplitScratch* split_scratch(cudaStream_t st, size_t need) {
 
 template <int MH, int BN, bool DUAL = false>
 bool launch(cudaStream_t st, const CUtensorMap& tmap, const uint32_t* packed, const uint16_t* sc, uint16_t* y,
-            uint32_t M, uint32_t K, uint32_t N, const W4Epilogue& ep, int sms, const uint32_t* packed2 = nullptr,
-            const uint16_t* sc2 = nullptr, uint32_t a_d = 0) {
+            uint32_t M, uint32_t K, uint32_t N, const W4Epilogue& ep, uint32_t sms, uint32_t S, uint32_t a_d,
+            const uint32_t* packed2 = nullptr, const uint16_t* sc2 = nullptr) {
     using C = Cfg<MH, BN>;
     const size_t smem = 1024 + (size_t)C::STAGES * (C::A_BYTES + C::B_BYTES) + (size_t)C::RSTAGES * C::RAW_SLOT + sizeof(Barriers) + 16;
     static int have[64] = {};
     if (!ensure_dyn_smem(w4a16_gemm_sm100_kernel<MH, BN, DUAL>, smem, have)) return false;
-    const uint32_t tiles = ((M + 128 * MH - 1) / (128 * MH)) * (N / (DUAL ? BN / 2 : BN)), KG = K / BK;
-    // Split K when the tiles alone leave SMs idle. A CTA walks a k block in about 0.42 us whatever the shape, so
-    // the launch lasts (items per CTA) x (k blocks per item + set-up); S is the divisor of K/64 that makes that
-    // smallest, a run keeping at least one trip round the operand ring, the partial sums at most 64 MB.
-    static const int split_on = [] { const char* e = std::getenv("GEHTP_CUDA_SPLITK"); return e ? std::atoi(e) : 1; }();
-    uint32_t S = 1;
-    if (split_on && !DUAL && tiles < (uint32_t)sms) {      // the gate | up form keeps its product in the epilogue: no runs
-        float best = (float)(KG + 4);
-        for (uint32_t c = 2; c <= 32 && c <= KG; c++) {
-            if (KG % c || KG / c < (uint32_t)C::STAGES || (size_t)c * M * N * sizeof(float) > ((size_t)64 << 20)) continue;
-            const uint32_t rounds = (tiles * c + sms - 1) / sms;
-            const float cost = (float)rounds * (float)(KG / c + 4) + 0.75f * (float)c + 6.0f;   // + the reduction: one launch, c reads
-            if (cost < best) { best = cost; S = c; }
-        }
-    }
+    constexpr uint32_t BN_OUT = DUAL ? BN / 2 : BN;
+    const uint32_t tiles = ((M + 128 * MH - 1) / (128 * MH)) * ((N + BN_OUT - 1) / BN_OUT);
     float* part = nullptr;
     if (S > 1) {
         SplitScratch* ss = split_scratch(st, (size_t)S * M * N * sizeof(float));
         if (ss) part = ss->part; else S = 1;
     }
     const uint32_t items = tiles * S;
-    const uint32_t grid = items < (uint32_t)sms ? items : (uint32_t)sms;
+    const uint32_t grid = items < sms ? items : sms;
     if (launch_pdl(w4a16_gemm_sm100_kernel<MH, BN, DUAL>, dim3(grid), dim3(NTHREADS), smem, st, tmap, (const uint4*)packed, sc,
                    (const uint4*)packed2, sc2, y, M, K, N, ep, S, part, a_d) != cudaSuccess) {
         cudaGetLastError();
@@ -561,7 +569,7 @@ bool launch(cudaStream_t st, const CUtensorMap& tmap, const uint32_t* packed, co
     } else if (S > 1) {
         const size_t quads = (size_t)M * N / 4;
         uint32_t rg = (uint32_t)((quads + 255) / 256);
-        if (rg > (uint32_t)sms * 8) rg = (uint32_t)sms * 8;
+        if (rg > sms * 8) rg = sms * 8;
         if (launch_pdl(w4a16_splitk_reduce_kernel, dim3(rg), dim3(256), 0, st, (const float*)part, y, M, N, S, ep) != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -593,7 +601,41 @@ bool make_a_map(CUtensorMap* tmap, const uint16_t* a, uint32_t M, uint32_t K, ui
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int sm_count() {
+// Tile and split of K: the configuration with the smallest rounds over the SMs x (k blocks of an item x kb + epi), plus, where
+// K is cut into runs, the launch that adds them (2 us and their fp32 sums written and read at 5 TB/s). kb and epi in us,
+// measured on one B200 at K 1024 .. 9728: a k block is bound by the operand bytes an SM takes in and the dequantisation, so
+// wide tiles bring more products per microsecond, and narrow ones (or 160 and 192 columns) waste less of the last round;
+// epi is what a tile costs beside its k blocks. The choice lies within 10 % of the best of 50 combinations at M 64 .. 2048.
+// Before (the largest tile that gave every SM one) -> now, 2048 rows: 4096 x 2560 78 -> 49 us, 9728 x 2560 168 -> 100,
+// 2560 x 6144 71 -> 63, 2560 x 151936 1451 -> 1267 (N is no multiple of 256); 64 rows: 2560 x 151936 137 -> 97.
+struct TileCost { uint32_t mh, bn; float kb, epi; };
+constexpr TileCost kTiles[] = {{1, 128, 0.347f, 1.0f}, {1, 192, 0.394f, 2.0f}, {1, 256, 0.434f, 3.5f}, {2, 128, 0.511f, 2.2f},
+                               {2, 160, 0.574f, 4.5f}, {2, 192, 0.606f, 6.0f}, {2, 256, 0.677f, 9.0f}};
+constexpr int kTileCount = sizeof(kTiles) / sizeof(kTiles[0]);
+
+// index into kTiles and the number of runs of K; only >= 0: that tile
+int pick_tile(uint32_t M, uint32_t K, uint32_t N, uint32_t sms, int only, uint32_t& S) {
+    static const int split_on = [] { const char* e = std::getenv("GEHTP_CUDA_SPLITK"); return e ? std::atoi(e) : 1; }();
+    const uint32_t KG = K / BK;
+    const double run_bytes = (double)M * N * sizeof(float);
+    int best = 0;
+    float best_us = 0.0f;
+    for (int i = 0; i < kTileCount; i++) {
+        const TileCost& t = kTiles[i];
+        if (only >= 0 && i != only) continue;
+        const uint32_t tiles = ((M + 128 * t.mh - 1) / (128 * t.mh)) * ((N + t.bn - 1) / t.bn);
+        for (uint32_t c = 1; c <= (split_on ? 32u : 1u) && c <= KG; c++) {
+            // a run at least one trip round the longest operand ring, partial sums <= 64 MB
+            if (c > 1 && (KG % c || KG / c < (uint32_t)MAX_STAGES || c * run_bytes > (double)(64u << 20))) continue;
+            float us = (float)((tiles * c + sms - 1) / sms) * ((float)(KG / c) * t.kb + t.epi);
+            if (c > 1) us += 2.0f + (float)(c * run_bytes * 2.0 / 5e6);
+            if (best_us == 0.0f || us < best_us) { best_us = us; best = i; S = c; }
+        }
+    }
+    return best;
+}
+
+uint32_t sm_count() {
     static int sms_of[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -602,7 +644,7 @@ int sm_count() {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 148;
     }
-    return sms;
+    return (uint32_t)sms;
 }
 
 }  // namespace
@@ -616,17 +658,20 @@ bool k_w4a16_gemm_sm100(cudaStream_t st, const uint16_t* a, const uint32_t* pack
     if (ep.mode == 3 && (!ep.res || !ep.gamma || !ep.sum_out || !ep.norm_out || N * sizeof(float) > 48u * 1024u ||
                          (((uintptr_t)ep.res | (uintptr_t)ep.gamma | (uintptr_t)ep.beta | (uintptr_t)ep.sum_out | (uintptr_t)ep.norm_out) & 15)))
         return false;
-    const int sms = sm_count();
+    if (tile == 3 && N % 256) tile = 0;
+    const uint32_t sms = sm_count();
     CUtensorMap tmap;
     if (!make_a_map(&tmap, a, M, K, a_d)) return false;
-    // Largest tile that still gives every SM a tile.
-    const uint32_t t256 = ((M + 255) / 256) * (N / 256);
-    const uint32_t t128 = ((M + 255) / 256) * (N / 128);
-    const int force = tile;   // 0: by shape, 1: 128x128, 2: 256x128, 3: 256x256
-    if (force == 3 ? N % 256 == 0 : (force == 0 && N % 256 == 0 && M > 128 && t256 >= (uint32_t)sms))
-        return launch<2, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, nullptr, nullptr, a_d);
-    if (force == 2 || (force == 0 && M > 128 && t128 >= (uint32_t)sms)) return launch<2, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, nullptr, nullptr, a_d);
-    return launch<1, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, nullptr, nullptr, a_d);
+    uint32_t S = 1;
+    switch (pick_tile(M, K, N, sms, tile == 1 ? 0 : tile == 2 ? 3 : tile == 3 ? 6 : -1, S)) {
+        case 0: return launch<1, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 1: return launch<1, 192>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 2: return launch<1, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 3: return launch<2, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 4: return launch<2, 160>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 5: return launch<2, 192>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        default: return launch<2, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+    }
 }
 
 bool w4a16_gemm_sm100_swiglu_takes(uint32_t M, uint32_t K, uint32_t N) {
@@ -638,14 +683,14 @@ bool k_w4a16_gemm_sm100_swiglu(cudaStream_t st, const uint16_t* a, const uint32_
                                const uint16_t* su, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, unsigned int* status) {
     if (!w4a16_gemm_sm100_swiglu_takes(M, K, N)) return false;
     if (((uintptr_t)a | (uintptr_t)pg | (uintptr_t)sg | (uintptr_t)pu | (uintptr_t)su | (uintptr_t)y) & 15) return false;
-    const int sms = sm_count();
+    const uint32_t sms = sm_count();
     CUtensorMap tmap;
     if (!make_a_map(&tmap, a, M, K)) return false;
     W4Epilogue ep;
     ep.status = status;
     // 256 rows per tile once that still gives every SM a tile
-    if (M > 128 && ((M + 255) / 256) * (N / 128) >= (uint32_t)sms) return launch<2, 256, true>(st, tmap, pg, sg, y, M, K, N, ep, sms, pu, su);
-    return launch<1, 256, true>(st, tmap, pg, sg, y, M, K, N, ep, sms, pu, su);
+    if (M > 128 && ((M + 255) / 256) * (N / 128) >= sms) return launch<2, 256, true>(st, tmap, pg, sg, y, M, K, N, ep, sms, 1, 0, pu, su);
+    return launch<1, 256, true>(st, tmap, pg, sg, y, M, K, N, ep, sms, 1, 0, pu, su);
 }
 
 }  // namespace gehtp
