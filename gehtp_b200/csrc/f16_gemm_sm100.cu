@@ -399,48 +399,59 @@ f16_gemv_nk_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* 
     }
 }
 
-// ---- the same on the tensor cores (mma.sync m16n8k16) for up to 8 rows per CTA row tile: a warp owns 8 output
-// columns and walks K in chunks of 32. Lane (g, t) loads 16 bytes of weight row n0 + g (8 consecutive k values)
+// ---- the same on the tensor cores (mma.sync m16n8k16) for up to 8 rows per CTA row tile. A CTA of 8 warps owns
+// 8 * (8 / KS) output columns: KS warps share a group of 8 columns and walk every KS-th chunk of 32 along K, their sums
+// meet in shared memory in warp order. Lane (g, t) loads 16 bytes of weight row n0 + g (8 consecutive k values)
 // and the 16 bytes at the same k of activation row g from shared memory; the first and the second half of those
 // 8 values feed two MMAs. Which of the 16 k slots of an MMA a value takes does not matter as long as A and B
 // agree, so no shuffling into the fragment order is needed: one 16-byte load per operand and chunk, 2 MMAs,
 // where the scalar form above spends some 140 instructions on the same 8 weights at 8 rows.
 // The first batch of weights (constants) is requested before the dependency wait.
-template <int UNR>
+// Bound by DRAM where the matrix is large (vocabulary) and by the latency of one warp's share of K where it is small:
+// one warp per 8 columns left a projection to 1024 columns on 16 SMs.
+template <int KS, int UNR>
 __global__ void __launch_bounds__(256)
 f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy) {
-    extern __shared__ __align__(16) unsigned char smem_a[];      // [8][K * 2 + 64] bytes: rows 64 bytes apart in the banks
+    extern __shared__ __align__(16) unsigned char smem_a[];      // [rows][K * 2 + 64] bytes: rows 64 bytes apart in the banks
+    __shared__ float part[KS > 1 ? 8 : 1][64];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const uint32_t m0 = blockIdx.y * 8, n0 = (blockIdx.x * 8 + warp) * 8, KC = K / 32, RS = K * 2 + 64;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, ks = warp % KS;
+    const uint32_t m0 = blockIdx.y * 8, rows = min(8u, M - m0), n0 = (blockIdx.x * (8 / KS) + warp / KS) * 8, KC = K / 32, RS = K * 2 + 64;
     const bool active = n0 < N;
     const uint4* wr = (const uint4*)(w + (size_t)min(n0 + g, N - 1) * K) + t;      // chunk kc lies 4 * kc further
     uint4 wq[UNR];
 #pragma unroll
-    for (int u = 0; u < UNR; u++) wq[u] = (active && (uint32_t)u < KC) ? __ldcs(wr + 4 * u) : make_uint4(0, 0, 0, 0);
+    for (int u = 0; u < UNR; u++) wq[u] = (active && ks + u * KS < KC) ? __ldcs(wr + 4 * (ks + u * KS)) : make_uint4(0, 0, 0, 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (uint32_t i = threadIdx.x; i < 8 * (K / 8); i += blockDim.x) {
-        const uint32_t r = i / (K / 8), c = i % (K / 8), m = min(m0 + r, M - 1);       // rows past M repeat row M-1; never stored
-        *(uint4*)(smem_a + r * RS + c * 16) = __ldcg((const uint4*)(a + (size_t)m * K) + c);
+    for (uint32_t i = threadIdx.x; i < rows * (K / 8); i += blockDim.x) {
+        const uint32_t r = i / (K / 8), c = i % (K / 8);
+        *(uint4*)(smem_a + r * RS + c * 16) = __ldcg((const uint4*)(a + (size_t)(m0 + r) * K) + c);
     }
     __syncthreads();
-    if (!active) return;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const unsigned char* arow = smem_a + g * RS + t * 16;
-    for (uint32_t kc0 = 0; kc0 < KC; kc0 += UNR) {
+    const unsigned char* arow = smem_a + min(g, rows - 1) * RS + t * 16;           // rows past M repeat the last; never stored
+    for (uint32_t kc0 = ks; active && kc0 < KC; kc0 += UNR * KS) {
         uint4 nx[UNR];
 #pragma unroll
-        for (int u = 0; u < UNR; u++) nx[u] = kc0 + UNR + u < KC ? __ldcs(wr + 4 * (kc0 + UNR + u)) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < UNR; u++) nx[u] = kc0 + (UNR + u) * KS < KC ? __ldcs(wr + 4 * (kc0 + (UNR + u) * KS)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int u = 0; u < UNR; u++) {
-            if (kc0 + u >= KC) break;
-            const uint4 av = *(const uint4*)(arow + (kc0 + u) * 64);
+            if (kc0 + u * KS >= KC) break;
+            const uint4 av = *(const uint4*)(arow + (kc0 + u * KS) * 64);
             const uint32_t a1[4] = {av.x, 0u, av.y, 0u}, a2[4] = {av.z, 0u, av.w, 0u};    // rows g + 8 of the tile: none
             mma16816(acc, a1, wq[u].x, wq[u].y);
             mma16816(acc, a2, wq[u].z, wq[u].w);
         }
 #pragma unroll
         for (int u = 0; u < UNR; u++) wq[u] = nx[u];
+    }
+    if (KS > 1) {
+        part[warp][g * 8 + 2 * t] = acc[0];
+        part[warp][g * 8 + 2 * t + 1] = acc[1];
+        __syncthreads();
+        if (ks != 0) return;
+#pragma unroll
+        for (int s = 1; s < KS; s++) { acc[0] += part[warp + s][g * 8 + 2 * t]; acc[1] += part[warp + s][g * 8 + 2 * t + 1]; }
     }
     const uint32_t m = m0 + g, n = n0 + 2 * t;
     if (m < M) {
@@ -449,16 +460,27 @@ f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t*
     }
 }
 
+template <int KS>
 bool launch_gemv_mma(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy) {
-    const size_t smem = (size_t)8 * (K * 2 + 64);
+    const size_t smem = (size_t)(M < 8 ? M : 8) * (K * 2 + 64);
     static int have[64] = {};
-    if (K % 32 || smem > 200 * 1024 || (smem > 48 * 1024 && !ensure_dyn_smem(f16_gemv_mma_kernel<8>, smem, have))) return false;
-    if (launch_pdl(f16_gemv_mma_kernel<8>, dim3((N + 63) / 64, (M + 7) / 8), dim3(256), smem, st, a, w, y, M, K, N, ldy) != cudaSuccess) {
+    if (K % 32 || smem > 200 * 1024 || (smem > 40 * 1024 && !ensure_dyn_smem(f16_gemv_mma_kernel<KS, 8>, smem, have))) return false;
+    const uint32_t cols = 8 * (8 / KS);
+    if (launch_pdl(f16_gemv_mma_kernel<KS, 8>, dim3((N + cols - 1) / cols, (M + 7) / 8), dim3(256), smem, st, a, w, y, M, K, N, ldy) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     g_launches++;
     return true;
+}
+
+// K shares per column group: enough CTAs for two per SM, a share of at least one batch of chunks
+bool launch_gemv_mma_any(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy) {
+    const uint32_t KC = K / 32, groups = (N + 7) / 8;
+    if (groups >= 8 * 296 || KC < 16) return launch_gemv_mma<1>(st, a, w, y, M, K, N, ldy);
+    if (groups >= 4 * 296 || KC < 32) return launch_gemv_mma<2>(st, a, w, y, M, K, N, ldy);
+    if (groups >= 2 * 296 || KC < 64) return launch_gemv_mma<4>(st, a, w, y, M, K, N, ldy);
+    return launch_gemv_mma<8>(st, a, w, y, M, K, N, ldy);
 }
 
 template <int MR>
@@ -533,7 +555,7 @@ bool k_matmul_f16_nk(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint
     if (!M || !K || !N || (K & 7u) || ((((uintptr_t)a) | ((uintptr_t)w)) & 15u)) return false;
     if (M < 32) {
         static const int mma_on = [] { const char* e = std::getenv("GEHTP_CUDA_F16_GEMV_MMA"); return e ? std::atoi(e) : 1; }();
-        if (mma_on && launch_gemv_mma(st, a, w, y, M, K, N, ldy)) return true;
+        if (mma_on && launch_gemv_mma_any(st, a, w, y, M, K, N, ldy)) return true;
         return M <= 4 ? launch_gemv<4>(st, a, w, y, M, K, N, ldy) : launch_gemv<8>(st, a, w, y, M, K, N, ldy);
     }
     if (M < 128 || K % BK || N % 128 || (ldy & 7u) || ((uintptr_t)y & 15u)) return false;
