@@ -25,22 +25,28 @@ struct NormLoadGlobal {
     __device__ __forceinline__ uint4 operator()(uint32_t i) const { return __ldcg((const uint4*)(a + i)); }
 };
 
-template <int BLOCK, class Sync, class LoadA>
+// REGS_ONLY: the caller has seen to it that the row fits the register form (norm_in_registers below); the kernel then
+// holds no more than the U * 8 values per thread that its rows need. With room for 32 of them a thread took 122 registers
+// and two CTAs filled an SM: 512 rows of 1024 were two rounds.
+template <int BLOCK, int U>
+inline bool norm_in_registers(uint32_t width, uintptr_t pointers) { return (width & 7u) == 0 && width <= U * BLOCK * 8u && (pointers & 15u) == 0; }
+
+template <int BLOCK, int U = 4, bool REGS_ONLY = false, class Sync, class LoadA>
 __device__ __forceinline__ void rmsnorm_row_t(const uint32_t tid, Sync sync, LoadA load_a, const uint16_t* a, const uint16_t* r,
                                               const uint16_t* __restrict__ g, const uint16_t* __restrict__ b,
                                               uint16_t* sum_out, uint16_t* y, uint32_t width, float* row, double* part,
                                               float* s_rms) {
-    // Rows of up to 4 * BLOCK * 8 values with 16-byte aligned operands: every thread keeps its (up to 32)
+    // Rows of up to U * BLOCK * 8 values with 16-byte aligned operands: every thread keeps its (up to U * 8)
     // values in registers between the two passes. Same loads, sums and roundings as the general path
     // below, without the round trip through the shared row buffer.
-    if ((width & 7u) == 0 && width <= 4u * BLOCK * 8u &&
-        ((((uintptr_t)a) | ((uintptr_t)r) | ((uintptr_t)sum_out) | ((uintptr_t)g) | ((uintptr_t)b) | ((uintptr_t)y)) & 15u) == 0) {
-        float v[4][8];
+    if (REGS_ONLY || ((width & 7u) == 0 && width <= U * BLOCK * 8u &&
+        ((((uintptr_t)a) | ((uintptr_t)r) | ((uintptr_t)sum_out) | ((uintptr_t)g) | ((uintptr_t)b) | ((uintptr_t)y)) & 15u) == 0)) {
+        float v[U][8];
         double acc = 0.0;
         {
-            uint4 qa4[4], qr4[4];
+            uint4 qa4[U], qr4[U];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < U; u++) {
                 const uint32_t i = tid * 8 + u * BLOCK * 8;
                 qa4[u] = make_uint4(0, 0, 0, 0); qr4[u] = make_uint4(0, 0, 0, 0);
                 if (i < width) {
@@ -49,7 +55,7 @@ __device__ __forceinline__ void rmsnorm_row_t(const uint32_t tid, Sync sync, Loa
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < U; u++) {
                 const uint32_t i = tid * 8 + u * BLOCK * 8;
                 if (i >= width) break;
                 const uint32_t wa[4] = {qa4[u].x, qa4[u].y, qa4[u].z, qa4[u].w}, wr[4] = {qr4[u].x, qr4[u].y, qr4[u].z, qr4[u].w};
@@ -72,9 +78,9 @@ __device__ __forceinline__ void rmsnorm_row_t(const uint32_t tid, Sync sync, Loa
             }
         }
         // gamma and beta are requested before the threads meet: their latency hides behind the reduction
-        uint4 qg4[4], qb4[4];
+        uint4 qg4[U], qb4[U];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < U; u++) {
             const uint32_t i = tid * 8 + u * BLOCK * 8;
             qg4[u] = make_uint4(0, 0, 0, 0); qb4[u] = make_uint4(0, 0, 0, 0);
             if (i < width) {
@@ -93,7 +99,7 @@ __device__ __forceinline__ void rmsnorm_row_t(const uint32_t tid, Sync sync, Loa
         sync();
         const float rms = *s_rms;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < U; u++) {
             const uint32_t i = tid * 8 + u * BLOCK * 8;
             if (i >= width) break;
             const uint32_t wg[4] = {qg4[u].x, qg4[u].y, qg4[u].z, qg4[u].w}, wb[4] = {qb4[u].x, qb4[u].y, qb4[u].z, qb4[u].w};
@@ -109,6 +115,7 @@ __device__ __forceinline__ void rmsnorm_row_t(const uint32_t tid, Sync sync, Loa
         }
         return;
     }
+    if constexpr (REGS_ONLY) return;
     double acc = 0.0;
     if ((width & 7u) == 0 && ((((uintptr_t)a) | ((uintptr_t)r) | ((uintptr_t)sum_out)) & 15u) == 0) {
         // 8 values per 16-byte load; the loads of four steps are issued together (one round trip to L2,
@@ -197,11 +204,11 @@ __device__ __forceinline__ void rmsnorm_row_t(const uint32_t tid, Sync sync, Loa
     }
 }
 
-template <int BLOCK>
+template <int BLOCK, int U = 4, bool REGS_ONLY = false>
 __device__ __forceinline__ void rmsnorm_row(const uint16_t* a, const uint16_t* r, const uint16_t* __restrict__ g,
                                             const uint16_t* __restrict__ b, uint16_t* sum_out, uint16_t* y,
                                             uint32_t width, float* row, double* part, float* s_rms) {
-    rmsnorm_row_t<BLOCK>(threadIdx.x, [] { __syncthreads(); }, NormLoadGlobal{a}, a, r, g, b, sum_out, y, width, row, part, s_rms);
+    rmsnorm_row_t<BLOCK, U, REGS_ONLY>(threadIdx.x, [] { __syncthreads(); }, NormLoadGlobal{a}, a, r, g, b, sum_out, y, width, row, part, s_rms);
 }
 
 }  // namespace gehtp

@@ -10,7 +10,7 @@ namespace gehtp {
 
 // ------------------------------------------------------------- RMSNorm
 // One CTA per row (norm_row.cuh).
-template <int BLOCK>
+template <int BLOCK, int U = 4, bool REGS_ONLY = false>
 __global__ void rmsnorm_kernel(const uint16_t* __restrict__ a, const uint16_t* __restrict__ r,
                                const uint16_t* __restrict__ g, const uint16_t* __restrict__ b,
                                uint16_t* __restrict__ sum_out, uint16_t* __restrict__ y,
@@ -21,13 +21,18 @@ __global__ void rmsnorm_kernel(const uint16_t* __restrict__ a, const uint16_t* _
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const size_t base = (size_t)blockIdx.x * width;
-    rmsnorm_row<BLOCK>(a + base, r ? r + base : nullptr, g, b, sum_out ? sum_out + base : nullptr, y + base, width, row, part, &s_rms);
+    rmsnorm_row<BLOCK, U, REGS_ONLY>(a + base, r ? r + base : nullptr, g, b, sum_out ? sum_out + base : nullptr, y + base, width, row, part, &s_rms);
 }
 
 void k_add_rmsnorm(cudaStream_t st, const uint16_t* a, const uint16_t* r, const uint16_t* g,
                    const uint16_t* b, uint16_t* sum_out, uint16_t* y, uint32_t rows, uint32_t width) {
     if (!rows || !width) return;
-    if (width <= 512)
+    const uintptr_t ptrs = (uintptr_t)a | (uintptr_t)r | (uintptr_t)g | (uintptr_t)b | (uintptr_t)sum_out | (uintptr_t)y;
+    if (width > 512 && norm_in_registers<256, 1>(width, ptrs))
+        launch_pdl(rmsnorm_kernel<256, 1, true>, dim3(rows), dim3(256), 0, st, a, r, g, b, sum_out, y, width);
+    else if (width > 512 && norm_in_registers<256, 2>(width, ptrs))
+        launch_pdl(rmsnorm_kernel<256, 2, true>, dim3(rows), dim3(256), 0, st, a, r, g, b, sum_out, y, width);
+    else if (width <= 512)
         launch_pdl(rmsnorm_kernel<64>, dim3(rows), dim3(64), width * sizeof(float), st, a, r, g, b, sum_out, y, width);
     else
         launch_pdl(rmsnorm_kernel<256>, dim3(rows), dim3(256), width * sizeof(float), st, a, r, g, b, sum_out, y, width);

@@ -240,7 +240,7 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                     umma_commit(&bars->empty[s]);
                 }
                 __syncwarp();
-                if (!live) break;
+                if (C::HALVES && !live) break;
                 if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
             }
             if (!live) break;
@@ -494,6 +494,7 @@ struct NormLoadRuns {
     uint16_t* y;            // this row of the GEMM's own output
     __device__ __forceinline__ uint4 operator()(uint32_t i) const {
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
         for (uint32_t r = 0; r < S; r++) {
             const float4 p = __ldcg((const float4*)(part + r * plane + i)), q = __ldcg((const float4*)(part + r * plane + i + 4));
             lo.x += p.x; lo.y += p.y; lo.z += p.z; lo.w += p.w;
@@ -505,6 +506,7 @@ struct NormLoadRuns {
     }
 };
 
+template <int U, bool REGS_ONLY>
 __global__ void __launch_bounds__(256)
 w4a16_splitk_add_rmsnorm_kernel(const float* __restrict__ part, uint16_t* __restrict__ y, uint32_t M, uint32_t N, uint32_t S, W4Epilogue ep) {
     extern __shared__ float row[];      // N floats (rows wider than the register form takes)
@@ -514,7 +516,7 @@ w4a16_splitk_add_rmsnorm_kernel(const float* __restrict__ part, uint16_t* __rest
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const size_t base = (size_t)blockIdx.x * N;
     const NormLoadRuns load{part + base, (size_t)M * N, S, y + base};
-    rmsnorm_row_t<256>(threadIdx.x, [] { __syncthreads(); }, load, (const uint16_t*)nullptr, ep.res + base, ep.gamma, ep.beta, ep.sum_out + base,
+    rmsnorm_row_t<256, U, REGS_ONLY>(threadIdx.x, [] { __syncthreads(); }, load, (const uint16_t*)nullptr, ep.res + base, ep.gamma, ep.beta, ep.sum_out + base,
                        ep.norm_out + base, N, row, red, &s_rms);
 }
 
@@ -561,7 +563,10 @@ bool launch(cudaStream_t st, const CUtensorMap& tmap, const uint32_t* packed, co
     }
     g_launches++;
     if (S > 1 && ep.mode == 3) {
-        if (launch_pdl(w4a16_splitk_add_rmsnorm_kernel, dim3(M), dim3(256), (size_t)N * sizeof(float), st, (const float*)part, y, M, N, S, ep) != cudaSuccess) {
+        auto add = [&](auto kernel, size_t row_bytes) { return launch_pdl(kernel, dim3(M), dim3(256), row_bytes, st, (const float*)part, y, M, N, S, ep); };
+        // every operand is 16-byte aligned here (checked at the entry); rows beyond 4096 go through shared memory
+        if ((N <= 2048 ? add(w4a16_splitk_add_rmsnorm_kernel<1, true>, 0) : N <= 4096 ? add(w4a16_splitk_add_rmsnorm_kernel<2, true>, 0)
+                       : add(w4a16_splitk_add_rmsnorm_kernel<4, false>, (size_t)N * sizeof(float))) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
