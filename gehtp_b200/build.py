@@ -25,6 +25,7 @@ UNITS = {
     "ops_elem.cu": ["--fmad=false"],
     "ops_gdn.cu": ["--fmad=false"],
     "gdn_delta_mma.cu": [],
+    "gdn_scan.cu": [],
     "ops_attn.cu": [],
     "ops_attn_decode.cu": [],
     "ops_attn_prefill.cu": [],

@@ -194,6 +194,8 @@ void fuse_materialize(const wt_blob* b);
 // Marks the ops whose result is a constant of the blob (PlanOp::const_fold). addr / maxb: device address and capacity
 // of every temp id of the plan.
 void fold_constants(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb);
+// Chunks of the delta rule that carry one state: their launches gathered at the first of them (behind fold_constants).
+void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb);
 bool fuse_all_materialized();
 void fuse_release();
 

@@ -23,7 +23,8 @@
 //   tanh residual       LINEAR + TANH_RESID of a row-count runlist -> the projection's epilogue
 //   picked norm         PICK_ROWS + TANH_RESID of a row-count runlist -> one kernel
 //   delta rule          LINEAR x2 (low-rank decay, gate), SHORT_CONV, CHANNEL_DELTA, GATED_NORM -> for few rows: one kernel
-// and marks the data-movement ops whose result is a constant of the blob (fold_constants).
+// marks the data-movement ops whose result is a constant of the blob (fold_constants), and gathers the delta-rule chunks
+// of a sequence (fuse_delta_runs).
 //
 // A chain is fused only when every intermediate temp is consumed inside the
 // chain and the chain's ops are contiguous in the list. Temps that exist only
@@ -35,6 +36,7 @@
 #include <map>
 #include <utility>
 #include "engine.h"
+#include "launchers.h"
 #include "launchers_attn.h"
 #include "launchers_rows.h"
 #include "launchers_w4.h"
@@ -650,6 +652,7 @@ bool match_picked_norm(const Graph& G, uint32_t i, Span& sp) {
 
 std::vector<Span> g_spans;
 float* g_attn_scratch = nullptr;
+std::vector<void*> g_delta_bufs;                                 // chunk tables and scratch of fuse_delta_runs
 std::map<std::pair<uint32_t, uint64_t>, uint8_t*> g_skip_maps;   // (mask slot, S<<32|Sk) -> device tile-skip bitmap
 
 const uint8_t* resolve(const wt_blob* b, uint32_t arg) {
@@ -1167,6 +1170,125 @@ void fold_constants(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb
     }
 }
 
+// Runs of DELTA_CHUNK ops that carry one state over chunks of 64 tokens. Between two of them the emitter leaves the windows
+// of their operands (constants of the blob, see above) and what is done with a chunk's result (transposition, projection).
+// The chunks' rule then goes in two launches for all of them (gdn_scan.cu), the ops in between follow in list order.
+// Taken when no op of the run but the chunks touches a state, when every chunk reads slots, constants or temps made before
+// the run, and when the memory an op of the run writes is no chunk's operand and not another chunk's result.
+void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb) {
+    if (g.exact_ops) return;
+    auto mem = [&](uint32_t t, const uint8_t*& lo, const uint8_t*& hi) { lo = t < kMaxTemps ? addr[t] : nullptr; hi = lo ? lo + maxb[t] : nullptr; return lo && maxb[t]; };
+    auto overlap = [&](uint32_t s, uint32_t t) {
+        const uint8_t *a0, *a1, *b0, *b1;
+        return mem(s, a0, a1) && mem(t, b0, b1) && a0 < b1 && b0 < a1;
+    };
+    for (uint32_t first = 0; first < b->n_ops; first++) {
+        const wt_op& d0 = b->ops[first];
+        if (d0.opcode != OP_DELTA_CHUNK_F16 || d0.args[7] != 64 || (d0.args[10] != 64 && d0.args[10] != 128) || g.plan[first].rc || g.plan[first].fused) continue;
+        std::vector<uint32_t> deltas, others, consts;      // ops of the run; `deltas` end it
+        std::vector<uint32_t> open_o, open_c;              // behind the last chunk so far
+        auto operands_ok = [&](uint32_t i) {               // slots, or temps no op of the run but constants writes
+            for (int k = 0; k < 5; k++) {
+                const uint32_t a = b->ops[i].args[k];
+                if (!is_temp_ref(a)) { if ((a & 0xC000u) != 0x8000u) return false; continue; }
+                for (const auto* v : {&deltas, &others, &open_o})
+                    for (uint32_t o : *v)
+                        for (int w = 0; w < 2; w++)
+                            if (g.plan[o].out_id[w] != kNoOff && overlap(g.plan[o].out_id[w], a)) return false;
+            }
+            // and its result is nobody else's memory in the run
+            for (const auto* v : {&deltas, &others, &open_o, &consts, &open_c})
+                for (uint32_t o : *v)
+                    for (int w = 0; w < 2; w++)
+                        if (g.plan[o].out_id[w] != kNoOff && overlap(g.plan[o].out_id[w], b->ops[i].args[5])) return false;
+            for (const auto* v : {&deltas, &others, &open_o})
+                for (uint32_t o : *v) {
+                    int ia[8];
+                    const int n = input_args(b->ops[o], ia);
+                    for (int k = 0; k < n; k++)
+                        if (is_temp_ref(b->ops[o].args[ia[k]]) && overlap(b->ops[o].args[ia[k]], b->ops[i].args[5])) return false;
+                }
+            return true;
+        };
+        for (uint32_t i = first; i < b->n_ops; i++) {
+            const PlanOp& p = g.plan[i];
+            const wt_op& op = b->ops[i];
+            if (p.rc || !p.launch || p.dead_when_fused) break;
+            if (op.opcode == OP_DELTA_CHUNK_F16) {
+                bool same = op.args[6] == d0.args[6];
+                for (int k = 7; k < 12; k++) same = same && op.args[k] == d0.args[k];
+                if (!same || p.uses_internal || !operands_ok(i)) break;
+                deltas.push_back(i);
+                others.insert(others.end(), open_o.begin(), open_o.end());
+                consts.insert(consts.end(), open_c.begin(), open_c.end());
+                open_o.clear(); open_c.clear();
+            } else if (p.const_fold) {
+                open_c.push_back(i);
+            } else if (op.opcode == OP_TRANSPOSE_GEN_F16 || op.opcode == OP_MATMUL_W4A16 || op.opcode == OP_MATMUL_F16) {
+                // its output must leave the operands of the chunks in front of it alone: they are read before it either way
+                open_o.push_back(i);
+            } else {
+                break;
+            }
+        }
+        if (deltas.size() < 2) continue;
+        const uint32_t last = deltas.back(), n = (uint32_t)deltas.size(), ntok = d0.args[8], H = d0.args[9], D = d0.args[10], q_raw = d0.args[11];
+        std::vector<DeltaChunk> table;
+        uintptr_t bits = 0;
+        bool ok = (d0.args[6] & 0xE000u) == WT_REF_STATE_FLAG;
+        for (uint32_t i : deltas) {
+            const wt_op& op = b->ops[i];
+            const uint16_t* r[6];
+            for (int k = 0; k < 6; k++) { r[k] = (const uint16_t*)resolve(b, op.args[k]); ok = ok && r[k]; }
+            table.push_back({r[0], r[1], r[2], r[3], r[4], (uint16_t*)r[5]});
+            bits |= (uintptr_t)r[0] | (uintptr_t)r[1] | (uintptr_t)r[2] | (uintptr_t)r[5];
+        }
+        // an op whose temp has no memory is only launched as part of its own chain, whose head and end lie in the run
+        std::vector<uint32_t> heads;
+        for (size_t k = 0; k < others.size() && ok;) {
+            const uint32_t i = others[k];
+            const PlanOp& p = g.plan[i];
+            const uint32_t span = p.fused && p.span ? p.span : 1;
+            if (span == 1 && !p.fused && p.uses_internal) ok = false;
+            for (uint32_t j = 0; j < span && ok; j++) ok = k + j < others.size() && others[k + j] == i + j;
+            heads.push_back(i);
+            k += span;
+        }
+        float* S = (float*)g.st_buf[d0.args[6] & 0x1FFFu];
+        if (!ok || !S || ((bits | (uintptr_t)S) & 15u)) continue;
+        DeltaChunk* d_table = nullptr;
+        void* scratch = nullptr;
+        if (cudaMalloc(&d_table, n * sizeof(DeltaChunk)) != cudaSuccess || cudaMalloc(&scratch, delta_scan_scratch_bytes(n, H)) != cudaSuccess) {
+            cudaGetLastError();
+            if (d_table) cudaFree(d_table);
+            continue;
+        }
+        g_delta_bufs.push_back(d_table);
+        g_delta_bufs.push_back(scratch);
+        cudaMemcpyAsync(d_table, table.data(), n * sizeof(DeltaChunk), cudaMemcpyHostToDevice, g.stream);
+        cudaStreamSynchronize(g.stream);
+        // what follows the last chunk keeps its own place in the list
+        g.plan[first].fused = [=](cudaStream_t st) {
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            const bool capturing = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+            for (uint32_t i : consts) {
+                PlanOp& p = g.plan[i];
+                if (p.const_done) continue;
+                p.launch(st);
+                if (!capturing) p.const_done = true;
+            }
+            if (!k_delta_scan(st, d_table, scratch, S, n, ntok, H, D, q_raw))
+                for (uint32_t i : deltas) g.plan[i].launch(st);
+            for (uint32_t i : heads) {
+                PlanOp& p = g.plan[i];
+                if (p.fused) p.fused(st); else p.launch(st);
+            }
+        };
+        g.plan[first].span = last - first + 1;
+        first = last;
+    }
+}
+
 bool fuse_all_materialized() {
     for (const Span& sp : g_spans)
         if (!g.plan[sp.first].fused || g.plan[sp.first].span != sp.count) return false;
@@ -1175,6 +1297,8 @@ bool fuse_all_materialized() {
 
 void fuse_release() {
     if (g_attn_scratch) { cudaFree(g_attn_scratch); g_attn_scratch = nullptr; }
+    for (void* p : g_delta_bufs) cudaFree(p);
+    g_delta_bufs.clear();
     for (auto& kv : g_skip_maps) cudaFree(kv.second);
     g_skip_maps.clear();
     g_spans.clear();

@@ -82,6 +82,12 @@ void k_conv1d_step(cudaStream_t st, const uint16_t* x, const uint16_t* w, uint16
 // Tensor-core form of the chunked delta rule (gdn_delta_mma.cu): head dim 64 or 128. false: shape not taken.
 bool k_delta_chunk_mma(cudaStream_t st, const uint16_t* k, const uint16_t* v, const uint16_t* q, const uint16_t* beta,
                        const uint16_t* g, uint16_t* y, float* S, uint32_t c, uint32_t ntok, uint32_t H, uint32_t D, uint32_t q_raw);
+// The same over n chunks of 64 tokens that carry one state (gdn_scan.cu); `chunks` lies on the device, operands 16-byte
+// aligned. false: head dim other than 64 or 128, or the launch was refused before anything ran.
+struct DeltaChunk { const uint16_t *k, *v, *q, *beta, *g; uint16_t* y; };
+size_t delta_scan_scratch_bytes(uint32_t n, uint32_t H);
+bool k_delta_scan(cudaStream_t st, const DeltaChunk* chunks, void* scratch, float* S, uint32_t n, uint32_t ntok, uint32_t H,
+                  uint32_t D, uint32_t q_raw);
 void k_delta_chunk(cudaStream_t st, const uint16_t* k, const uint16_t* v, const uint16_t* q,
                    const uint16_t* beta, const uint16_t* g, uint16_t* y, float* S, uint32_t c,
                    uint32_t ntok, uint32_t H, uint32_t D, uint32_t q_raw);

@@ -824,6 +824,7 @@ int build_plan(const wt_blob* b, char* err, size_t errn) {
         if (fuse_all_materialized())
             for (uint32_t i = 0; i < b->n_ops && i < dead_ops.size(); i++) g.plan[i].dead_when_fused = dead_ops[i] != 0;
         fold_constants(b, P.addr, P.maxb);
+        fuse_delta_runs(b, P.addr, P.maxb);
     }
     cudaError_t ce = cudaStreamSynchronize(g.stream);
     if (ce != cudaSuccess) { std::snprintf(err, errn, "plan upload: %s", cudaGetErrorString(ce)); return -1; }
