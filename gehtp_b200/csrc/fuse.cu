@@ -1267,7 +1267,50 @@ void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* max
         g_delta_bufs.push_back(scratch);
         cudaMemcpyAsync(d_table, table.data(), n * sizeof(DeltaChunk), cudaMemcpyHostToDevice, g.stream);
         cudaStreamSynchronize(g.stream);
-        // what follows the last chunk keeps its own place in the list
+        // Every chunk's result goes [head][row][d] -> [row][head * d] -> one W4A16 matrix: with results and outputs each the
+        // same distance apart, one GEMM over all chunks behind the walk (a chunk's 64 rows alone fill half of a tile).
+        uint32_t span = last - first + 1;
+        std::function<bool(cudaStream_t)> project;
+        {
+            bool one = ntok == 64 && g.tp_world <= 1 && others.size() == 2 * (size_t)(n - 1) && last + 2 < b->n_ops;
+            std::vector<uint32_t> pair(others);
+            pair.push_back(last + 1);
+            pair.push_back(last + 2);
+            const wt_op* mm0 = one ? &b->ops[pair[1]] : nullptr;
+            std::vector<uint32_t> outs;
+            for (uint32_t c = 0; c < n && one; c++) {
+                const uint32_t it = pair[2 * c], im = pair[2 * c + 1];
+                const wt_op &tr = b->ops[it], &mm = b->ops[im];
+                const PlanOp& p = g.plan[it];
+                one = tr.opcode == OP_TRANSPOSE_GEN_F16 && mm.opcode == OP_MATMUL_W4A16 && im == it + 1 && p.fused && p.span == 2 && !p.rc && !g.plan[im].rc &&
+                      tr.args[0] == b->ops[deltas[c]].args[5] && tr.args[2] == 3 && tr.args[3] == H && tr.args[4] == 64 && tr.args[5] == D &&
+                      mm.args[0] == tr.args[1] && mm.args[1] == mm0->args[1] && mm.args[3] == 64 && mm.args[4] == H * D && mm.args[5] == mm0->args[5];
+                outs.push_back(mm.args[2]);
+            }
+            for (uint32_t c = 0; c < n && one; c++)
+                for (uint32_t e = 0; e < n && one; e++)
+                    one = !overlap(outs[c], b->ops[deltas[e]].args[5]) && (c == e || !overlap(outs[c], outs[e]));
+            if (one) {
+                const uint32_t K = H * D, N = mm0->args[5];
+                auto it = g.w4.find((uint64_t)(mm0->args[1] & 0x7FFFu) | ((uint64_t)K << 16) | ((uint64_t)N << 40));
+                uint16_t* y0 = (uint16_t*)resolve(b, outs[0]);
+                const ptrdiff_t a_block = table[1].y - table[0].y, y_block = (const uint16_t*)resolve(b, outs[1]) - y0;
+                one = it != g.w4.end() && y0 && a_block > 0 && y_block > 0;
+                for (uint32_t c = 0; c < n && one; c++)
+                    one = table[c].y == table[0].y + (ptrdiff_t)c * a_block && (const uint16_t*)resolve(b, outs[c]) == y0 + (ptrdiff_t)c * y_block;
+                if (one) {
+                    const uint16_t *a = table[0].y, *sc = it->second.scales;
+                    const uint32_t* pk = it->second.packed;
+                    W4Epilogue ep;
+                    ep.status = g.d_status;
+                    ep.y_block = (size_t)y_block;
+                    project = [=](cudaStream_t st) { return k_w4a16_gemm_sm100_blocks(st, a, (size_t)a_block, D, pk, sc, y0, n, K, N, ep); };
+                    heads.push_back(last + 1);
+                    span += 2;
+                }
+            }
+        }
+        // (without that GEMM, what follows the last chunk keeps its own place in the list)
         g.plan[first].fused = [=](cudaStream_t st) {
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
             const bool capturing = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
@@ -1279,13 +1322,14 @@ void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* max
             }
             if (!k_delta_scan(st, d_table, scratch, S, n, ntok, H, D, q_raw))
                 for (uint32_t i : deltas) g.plan[i].launch(st);
+            if (project && project(st)) return;
             for (uint32_t i : heads) {
                 PlanOp& p = g.plan[i];
                 if (p.fused) p.fused(st); else p.launch(st);
             }
         };
-        g.plan[first].span = last - first + 1;
-        first = last;
+        g.plan[first].span = span;
+        first += span - 1;
     }
 }
 

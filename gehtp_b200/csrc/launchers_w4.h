@@ -24,6 +24,8 @@ struct W4Epilogue {
     // mode 3
     const uint16_t *gamma = nullptr, *beta = nullptr;
     uint16_t *sum_out = nullptr, *norm_out = nullptr;
+    // tcgen05 GEMM over blocks of 64 rows (mode 0): rows 64 c .. 64 c + 63 of the output lie at y + c * y_block
+    size_t y_block = 0;
     unsigned int* status = nullptr;   // engine status word: the tcgen05 GEMM reports a barrier wait that ran out here
     // mode 2
     const uint16_t *cos_q = nullptr, *sin_q = nullptr, *cos_k = nullptr, *sin_k = nullptr;   // [M*heads][hd], or one row
@@ -73,6 +75,10 @@ void k_w4a16_skinny_swiglu(cudaStream_t st, const uint16_t* a, const uint32_t* p
 bool k_w4a16_gemm_sm100(cudaStream_t st, const uint16_t* a, const uint32_t* packed,
                         const uint16_t* sc, uint16_t* y, uint32_t M, uint32_t K, uint32_t N,
                         const W4Epilogue& ep, int tile = 0, uint32_t a_d = 0);
+// One matrix for `blocks` blocks of 64 rows that lie apart: block c of the activations at a + c * a_block, stored
+// [K / a_d][64][a_d], its output [64][N] at y + c * ep.y_block (elements; both multiples of 8). false: nothing launched.
+bool k_w4a16_gemm_sm100_blocks(cudaStream_t st, const uint16_t* a, size_t a_block, uint32_t a_d, const uint32_t* packed, const uint16_t* sc,
+                               uint16_t* y, uint32_t blocks, uint32_t K, uint32_t N, const W4Epilogue& ep);
 // Gate and up projections of a gated FFN plus its three elementwise ops on the same kernel: y[M, N] =
 // fp16(fp16(g * fp16(sigmoid(g))) * u), g = a . Wg, u = a . Wu (both [K, N]), neither g nor u written to memory.
 // `takes`: the shape test alone (N a multiple of 128, K of 64); the launcher also wants

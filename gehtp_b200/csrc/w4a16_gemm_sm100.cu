@@ -186,7 +186,12 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
                     mbar_expect_tx(&bars->full[s], A_BYTES);
 #pragma unroll
                     for (int h = 0; h < MH; h++)
-                        if (a_d)     // A stored [head][row][a_d]: column kb * 64 of A is column (kb * 64) % a_d of head (kb * 64) / a_d
+                        if (ep.y_block) {     // A in blocks of 64 rows, each stored [K / a_d][64][a_d]: two blocks per 128 rows
+#pragma unroll
+                            for (int j = 0; j < 2; j++)
+                                tma_load_4d(sA + s * A_BYTES + h * HALF_A_BYTES + j * (HALF_A_BYTES / 2), &tmap_a, (int)((kb * BK) % a_d), 0,
+                                            (int)((kb * BK) / a_d), (int)((m0 + h * 128) / 64 + j), &bars->full[s]);
+                        } else if (a_d)     // A stored [head][row][a_d]: column kb * 64 of A is column (kb * 64) % a_d of head (kb * 64) / a_d
                             tma_load_3d(sA + s * A_BYTES + h * HALF_A_BYTES, &tmap_a, (int)((kb * BK) % a_d), (int)(m0 + h * 128), (int)((kb * BK) / a_d),
                                         &bars->full[s]);
                         else
@@ -290,7 +295,8 @@ w4a16_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint4*
         asm volatile("griddepcontrol.wait;" ::: "memory");
         // 32 accumulator values of row m from column n on their way to y
         auto emit = [&](uint32_t m, uint32_t n, const uint32_t (&v)[32]) {
-            const size_t o = (size_t)m * N + n;       // 64-byte aligned: N and n are multiples of 32
+            // 64-byte aligned (16 with y_block): N and n are multiples of 32
+            const size_t o = ep.y_block ? (size_t)(m / 64) * ep.y_block + (size_t)(m % 64) * N + n : (size_t)m * N + n;
             uint4* dst = (uint4*)(y + o);
             if (ep.mode == 1) {
                 const uint4* res = (const uint4*)(ep.res + o);
@@ -480,6 +486,11 @@ w4a16_splitk_reduce_kernel(const float* __restrict__ part, uint16_t* __restrict_
         } else {
             o = make_uint2(pack_out(acc.x, acc.y), pack_out(acc.z, acc.w));
         }
+        if (ep.y_block) {
+            const size_t m = i * 4 / N, n = i * 4 % N;
+            *(uint2*)(y + (m / 64) * ep.y_block + (m % 64) * N + n) = o;
+            continue;
+        }
         *((uint2*)y + i) = o;
     }
 }
@@ -652,6 +663,20 @@ uint32_t sm_count() {
     return (uint32_t)sms;
 }
 
+bool pick_and_launch(cudaStream_t st, const CUtensorMap& tmap, const uint32_t* packed, const uint16_t* sc, uint16_t* y, uint32_t M, uint32_t K,
+                     uint32_t N, const W4Epilogue& ep, uint32_t sms, int only, uint32_t a_d) {
+    uint32_t S = 1;
+    switch (pick_tile(M, K, N, sms, only, S)) {
+        case 0: return launch<1, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 1: return launch<1, 192>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 2: return launch<1, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 3: return launch<2, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 4: return launch<2, 160>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        case 5: return launch<2, 192>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+        default: return launch<2, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
+    }
+}
+
 }  // namespace
 
 bool k_w4a16_gemm_sm100(cudaStream_t st, const uint16_t* a, const uint32_t* packed, const uint16_t* sc,
@@ -667,16 +692,23 @@ bool k_w4a16_gemm_sm100(cudaStream_t st, const uint16_t* a, const uint32_t* pack
     const uint32_t sms = sm_count();
     CUtensorMap tmap;
     if (!make_a_map(&tmap, a, M, K, a_d)) return false;
-    uint32_t S = 1;
-    switch (pick_tile(M, K, N, sms, tile == 1 ? 0 : tile == 2 ? 3 : tile == 3 ? 6 : -1, S)) {
-        case 0: return launch<1, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-        case 1: return launch<1, 192>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-        case 2: return launch<1, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-        case 3: return launch<2, 128>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-        case 4: return launch<2, 160>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-        case 5: return launch<2, 192>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-        default: return launch<2, 256>(st, tmap, packed, sc, y, M, K, N, ep, sms, S, a_d);
-    }
+    return pick_and_launch(st, tmap, packed, sc, y, M, K, N, ep, sms, tile == 1 ? 0 : tile == 2 ? 3 : tile == 3 ? 6 : -1, a_d);
+}
+
+bool k_w4a16_gemm_sm100_blocks(cudaStream_t st, const uint16_t* a, size_t a_block, uint32_t a_d, const uint32_t* packed, const uint16_t* sc,
+                               uint16_t* y, uint32_t blocks, uint32_t K, uint32_t N, const W4Epilogue& ep) {
+    if (!blocks || !K || K % BK || N % 128 || !a_d || a_d % BK || K % a_d || ep.mode != 0 || !ep.y_block || ((a_block | ep.y_block) & 7u)) return false;
+    if (((uintptr_t)a | (uintptr_t)packed | (uintptr_t)sc | (uintptr_t)y) & 15) return false;
+    EncodeTiledFn enc = encode_fn();
+    CUtensorMap tmap;
+    cuuint64_t dims[4] = {a_d, 64, K / a_d, blocks};
+    cuuint64_t strides[3] = {(cuuint64_t)a_d * 2, (cuuint64_t)64 * a_d * 2, (cuuint64_t)a_block * 2};
+    cuuint32_t box[4] = {BK, 64, 1, 1}, estr[4] = {1, 1, 1, 1};
+    if (!enc || enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void*)a, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    const uint32_t sms = sm_count(), M = blocks * 64;
+    return pick_and_launch(st, tmap, packed, sc, y, M, K, N, ep, sms, -1, a_d);
 }
 
 bool w4a16_gemm_sm100_swiglu_takes(uint32_t M, uint32_t K, uint32_t N) {

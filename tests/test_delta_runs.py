@@ -64,3 +64,20 @@ def test_delta_run_against_op_by_op(cuda, H, D, n, ntok, q_raw, shared):
         for c in range(n):
             sel = (slice(None),) if shared == "operand" and ntok == 64 else rows
             assert_fp16_close(got[r][c].view(np.float16).reshape(ntok, H, D)[sel], want[r][c].view(np.float16).reshape(ntok, H, D)[sel], "run %d chunk %d" % (r, c))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,D,chunks,hidden", [(2, 128, 2, 128), (4, 64, 5, 384), (16, 128, 9, 1024)])
+def test_projection_of_all_chunks(cuda, H, D, chunks, hidden):
+    """The layer's out-projections run as one GEMM over blocks of 64 rows that lie apart in memory: every chunk's output
+    against the one-kernel-per-op plan, an odd number of blocks among them (half of the last tile is missing)."""
+    from gehtp_b200.runlists import build_gdn_runlist
+    blob, man = build_gdn_runlist(64 * chunks, hidden, 256, 4, H, D, 64)
+    x = np.random.default_rng(4).standard_normal((64 * chunks, hidden)).astype(np.float16)
+    temps = [man["conv_temp"]] + man["chunk_out"]
+    got, launches = _run(cuda, blob, temps, 1, 3, x)
+    want, _ = _run(cuda, blob, temps, 0, 3, x)
+    assert launches <= 7                                         # two projections (each with a reduction), convolution, the two of the rule
+    for r in range(3):
+        for c, t in enumerate(temps):
+            assert_fp16_close(got[r][c].view(np.float16), want[r][c].view(np.float16), "run %d temp %d" % (r, t))
