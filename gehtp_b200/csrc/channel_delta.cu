@@ -3,8 +3,8 @@
 //   short_conv_kernel    causal depthwise convolution + silu; the last taps - 1 inputs are kept in the state, two banks:
 //                        a run reads the bank of its parity and writes the other, so that no CTA overwrites what
 //                        another still reads
-//   delta_prep_kernel    unit vectors, decays, step sizes and the products of neighbouring tokens' vectors, fp32
-//   delta_scan_kernel    the recurrence, two tokens at a time: S lives in registers, all reductions of both tokens run side
+//   delta_prep_kernel    unit vectors, decays, step sizes and the products of the vectors of four tokens, fp32
+//   delta_scan_kernel    the recurrence, four tokens at a time: S lives in registers, all reductions of the four run side
 //                        by side
 //   gated_norm_kernel    RMS norm of a head's read-out, weight, sigmoid gate
 //   delta_step_kernel    all of it for up to 4 rows, with the second halves of the low-rank decay and gate projections
@@ -64,8 +64,10 @@ short_conv_kernel(const typename A::T* y, const float* __restrict__ w, float* st
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
-// work: k [rows][KH][D], q [rows][KH][D], decay [rows][H][D], {step, k . q, (g k') . k, (g k') . q} [rows][H][4] with k' the
-// key of the row before (odd rows only)
+// work: k [rows][KH][D], q [rows][KH][D], decay [rows][H][D], {step, m0, m1, m2, k . q, n0, n1, n2} [rows][H][8]. Rows are
+// taken in blocks of BT; m_i and n_i are the products of k and q with the key of row i of the block, decayed up to this row
+// (0 from this row on).
+constexpr uint32_t BT = 4, BK = 8;
 struct DeltaWork { float *k, *q, *g, *bk; };
 __host__ __device__ inline size_t up4(size_t n) { return (n + 3) & ~(size_t)3; }
 inline DeltaWork work_of(const DeltaArgs& a, uint32_t rows) {
@@ -77,7 +79,7 @@ inline DeltaWork work_of(const DeltaArgs& a, uint32_t rows) {
     return w;
 }
 
-// A warp per head and pair of rows (2 p, 2 p + 1), the head's vectors in registers (DR values per lane).
+// A warp per head and block of BT rows, the head's vectors in registers (DR values per lane).
 template <class A, int DR>
 __global__ void __launch_bounds__(256)
 delta_prep_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
@@ -85,13 +87,11 @@ delta_prep_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
     pdl_wait();
     const uint32_t h = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, D = a.dim, KH = a.kv_heads, H = a.heads;
     if (h >= H) return;
-    const uint32_t rep = H / KH, kh = h / rep, r0 = blockIdx.y * 2;
+    const uint32_t rep = H / KH, kh = h / rep, r0 = blockIdx.y * BT;
     const float qs = 1.0f / sqrtf((float)D), ea = expf(__ldg(a.a_log + h));
-    float kp[DR], k[DR], q[DR], g[DR];
+    float kd[BT][DR], q[DR], g[DR];                 // kd: keys of the block's rows, decayed up to the row in hand
 #pragma unroll
-    for (int j = 0; j < DR; j++) kp[j] = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
+    for (int e = 0; e < (int)BT; e++) {
         const uint32_t r = r0 + e;
         if (r >= rows) break;
         const float *qx = a.qkv + (size_t)r * a.channels() + kh * D, *kx = qx + KH * D, *ax = a.a + ((size_t)r * H + h) * D;
@@ -101,33 +101,39 @@ delta_prep_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
             const uint32_t i = lane + 32 * j;
             const bool in = i < D;
             q[j] = in ? __ldcg(qx + i) : 0.0f;
-            k[j] = in ? __ldcg(kx + i) : 0.0f;
+            kd[e][j] = in ? __ldcg(kx + i) : 0.0f;
             g[j] = in ? __ldcg(ax + i) + __ldg(a.dt_bias + h * D + i) : 0.0f;
-            qq = fmaf(q[j], q[j], qq); kk = fmaf(k[j], k[j], kk); qk = fmaf(q[j], k[j], qk);
+            qq = fmaf(q[j], q[j], qq); kk = fmaf(kd[e][j], kd[e][j], kk); qk = fmaf(q[j], kd[e][j], qk);
         }
         qq = warp_sum(qq); kk = warp_sum(kk); qk = warp_sum(qk);
         const float iq = qs / sqrtf(qq + 1e-6f), ik = 1.0f / sqrtf(kk + 1e-6f);
-        float m = 0.0f, n = 0.0f;
+        float m[BT] = {}, n[BT] = {};
 #pragma unroll
         for (int j = 0; j < DR; j++) {
             const uint32_t i = lane + 32 * j;
             g[j] = expf(-ea * softplus_f(g[j]));
-            q[j] *= iq; k[j] *= ik;
-            m = fmaf(g[j] * kp[j], k[j], m);
-            n = fmaf(g[j] * kp[j], q[j], n);
+            q[j] *= iq; kd[e][j] *= ik;
+#pragma unroll
+            for (int b = 0; b < e; b++) {
+                kd[b][j] *= g[j];
+                m[b] = fmaf(kd[b][j], kd[e][j], m[b]);
+                n[b] = fmaf(kd[b][j], q[j], n[b]);
+            }
             if (i < D) {
                 wk.g[((size_t)r * H + h) * D + i] = g[j];
                 if (h % rep == 0) {
                     wk.q[((size_t)r * KH + kh) * D + i] = q[j];
-                    wk.k[((size_t)r * KH + kh) * D + i] = k[j];
+                    wk.k[((size_t)r * KH + kh) * D + i] = kd[e][j];
                 }
             }
-            kp[j] = k[j];
         }
-        if (e) { m = warp_sum(m); n = warp_sum(n); }
+#pragma unroll
+        for (int b = 0; b < e; b++) { m[b] = warp_sum(m[b]); n[b] = warp_sum(n[b]); }
         if (lane == 0) {
             const float b = A::ld((const typename A::T*)a.y + (size_t)r * a.ys + a.b_col + h);
-            *(float4*)(wk.bk + ((size_t)r * H + h) * 4) = make_float4(sigmoid_f(b), qk * iq * ik, m, n);
+            float4* d = (float4*)(wk.bk + ((size_t)r * H + h) * BK);
+            d[0] = make_float4(sigmoid_f(b), m[0], m[1], m[2]);
+            d[1] = make_float4(qk * iq * ik, n[0], n[1], n[2]);
         }
     }
 }
@@ -138,34 +144,38 @@ __device__ __forceinline__ float sum2(uint64_t v) { float a, b; asm("mov.b64 {%0
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
-// 16 lanes hold 2 neighbouring columns of S, RPL rows each (as RPL / 2 pairs of values); a warp holds 4 columns, a CTA NW
-// warps of one head. Tokens are taken two at a time: with P = g1 S, R = g2 P,
-//   u1 = b1 (v1 - P^T k1)                 o1 = P^T q1 + u1 (k1 . q1)
-//   u2 = b2 (v2 - R^T k2 - u1 m)          o2 = R^T q2 + u1 n + u2 (k2 . q2)       m = (g2 k1) . k2, n = (g2 k1) . q2
-//   S  = R + (g2 k1) u1^T + k2 u2^T
-// so that the four sums of both tokens are reduced together. The eight sums of a lane (4 per column) are reduced over its
-// 16 lanes by halving - an exchange leaves a lane with half of the sums it had - until lane (token, k or q, column, -)
-// holds one. Tokens come in chunks of TC through shared memory (cp.async, two stages; VEC = 16-byte copies); a last odd
-// token is paired with one that changes nothing (decay 1, key, query and step 0).
+// L lanes (16 or 32) hold 2 neighbouring columns of S, RPL rows each (as RPL / 2 pairs of values); a CTA is NW warps of one
+// head. Tokens are taken four at a time: with R_j = g_j R_(j-1), R_0 = S, and K_ij the key of token i decayed up to j,
+//   u_j = b_j (v_j - R_j^T k_j - sum_(i<j) u_i m_ij)     o_j = R_j^T q_j + sum_(i<j) u_i n_ij + u_j (k_j . q_j)
+//   S' = R_4 + sum_i K_i4 u_i^T                          m_ij = K_ij . k_j, n_ij = K_ij . q_j
+// so that the eight sums of the four tokens are reduced together. The sixteen sums of a lane (8 per column) are reduced over
+// its L lanes by halving - an exchange leaves a lane with half of the sums it had - until lane (token, k or q, column) holds
+// one. Tokens come in chunks of TC through shared memory (cp.async, two stages; VEC = 16-byte copies); a last block is filled
+// up with tokens that change nothing (decay 1, key, query and step 0).
+// Bound by the chain of a block - products, five exchanges, the four u, the update - of which little overlaps. With 32 lanes
+// of 4 rows (128 channels) two warps share a scheduler and a lane's part is half of what it is with 16 of 8.
+// 2048 tokens, 16 heads of 128 x 128: two tokens at a time, 16 lanes 493 us; 32 lanes 427; four at a time 372 (16 lanes 446, the next block's
+// operands held in registers ahead 441): shared-memory reads and exchanges of eight warps, then the chain they cannot hide.
 constexpr uint32_t TC = 16;
-template <int RPL, int NW, bool VEC>
+template <int L, int RPL, int NW, bool VEC>
 __global__ void __launch_bounds__(NW * 32)
 delta_scan_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
-    constexpr uint32_t DP = 16 * RPL, NC = NW * 4, NT = NW * 32;
+    constexpr uint32_t DP = L * RPL, NC = NW * (32 / L) * 2, NT = NW * 32;
+    static_assert(NC <= 32, "one warp copies a token's values");
     extern __shared__ __align__(16) float sm[];
     float* s_kqg = sm;                                // [2][TC][3][DP]
     float* s_v = s_kqg + 2 * TC * 3 * DP;             // [2][TC][NC]
-    float* s_bk = s_v + 2 * TC * NC;                  // [2][TC][4]
+    float* s_bk = s_v + 2 * TC * NC;                  // [2][TC][BK]
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, H = a.heads, D = a.dim, V = a.vdim;
     const uint32_t h = blockIdx.y, kh = h / (H / a.kv_heads), c0 = blockIdx.x * NC;
-    const uint32_t l = lane & 15, base = lane & 16, cl = warp * 4 + (lane >> 4) * 2;      // first of this lane's columns, within the CTA
+    const uint32_t l = lane & (L - 1), base = lane & (32 - L), cl = (warp * (32 / L) + lane / L) * 2;      // first of this lane's columns, within the CTA
     const uint32_t C = a.channels(), voff = 2 * a.kv_heads * D + h * V;
     for (uint32_t i = tid; i < 2 * TC * 3 * DP; i += NT)
         if (i % DP >= D) s_kqg[i] = 0.0f;             // rows past D: S stays zero there
     for (uint32_t i = tid; i < 2 * TC * NC; i += NT)
         if (c0 + i % NC >= V) s_v[i] = 0.0f;          // columns past V, which no copy writes
     float* Sg = a.S + (size_t)h * D * V;
-    auto row_of = [&](int i) -> uint32_t { return (i / 4) * 64 + l * 4 + (i & 3); };
+    auto row_of = [&](int i) -> uint32_t { return (i / 4) * (4 * L) + l * 4 + (i & 3); };
     uint64_t S[RPL / 2][2];
 #pragma unroll
     for (int i = 0; i < RPL; i += 2) {
@@ -197,76 +207,93 @@ delta_scan_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
             if (lane < NC && c0 + lane < V)
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(s_v + (stg * TC + t) * NC + lane)),
                              "l"(a.qkv + (size_t)(t0 + t) * C + voff + c0 + lane) : "memory");
-            if (lane == 0) cp16(smem_addr(s_bk + (stg * TC + t) * 4), wk.bk + ((size_t)(t0 + t) * H + h) * 4, 16);
+            if (lane < 2) cp16(smem_addr(s_bk + (stg * TC + t) * BK + lane * 4), wk.bk + ((size_t)(t0 + t) * H + h) * BK + lane * 4, 16);
         }
-        if ((nt & 1u) && warp == (nt % NW)) {         // the idle partner of a last odd token
-            for (uint32_t c = lane; c < D; c += 32) { float* dt = d + nt * 3 * DP; dt[c] = 0.0f; dt[DP + c] = 0.0f; dt[2 * DP + c] = 1.0f; }
-            if (lane < NC) s_v[(stg * TC + nt) * NC + lane] = 0.0f;
-            if (lane < 4) s_bk[(stg * TC + nt) * 4 + lane] = 0.0f;
+        for (uint32_t t = nt + (warp + NW - nt % NW) % NW; t < ((nt + BT - 1) & ~(BT - 1)); t += NW) {       // idle tokens of a last block
+            for (uint32_t c = lane; c < D; c += 32) { float* dt = d + t * 3 * DP; dt[c] = 0.0f; dt[DP + c] = 0.0f; dt[2 * DP + c] = 1.0f; }
+            if (lane < NC) s_v[(stg * TC + t) * NC + lane] = 0.0f;
+            if (lane < BK) s_bk[(stg * TC + t) * BK + lane] = 0.0f;
         }
         cp_commit();
     };
     fetch(0, 0);
-    const bool second = l & 8, isq = l & 4, odd = l & 2;      // the sum this lane ends up with: token, S^T q or S^T k, column
+    // the sum this lane ends up with: token, S^T q or S^T k, column
+    const bool hi = l & (L / 2), lo = l & (L / 4), isq = l & (L / 8), odd = l & (L / 16);
+    const uint32_t mine = (hi ? 2 : 0) + (lo ? 1 : 0);
     for (uint32_t t0 = 0, stg = 0; t0 < rows; t0 += TC, stg ^= 1) {
         fetch(t0 + TC, stg ^ 1);
         cp_wait<1>();
         __syncthreads();
         const uint32_t nt = min(TC, rows - t0);
         const float* kqg = s_kqg + stg * TC * 3 * DP + l * 4;
-        for (uint32_t t = 0; t < nt; t += 2) {
-            const float *p1 = kqg + t * 3 * DP, *p2 = p1 + 3 * DP;
-            const float4 bk1 = *(const float4*)(s_bk + (stg * TC + t) * 4), bk2 = *(const float4*)(s_bk + (stg * TC + t + 1) * 4);
-            const float2 v1 = *(const float2*)(s_v + (stg * TC + t) * NC + cl), v2 = *(const float2*)(s_v + (stg * TC + t + 1) * NC + cl);
-            uint64_t ka[RPL / 2], kb[RPL / 2], a1[2], b1[2], a2[2], b2[2];
+        for (uint32_t t = 0; t < nt; t += BT) {
+            const float *p = kqg + t * 3 * DP, *bk = s_bk + (stg * TC + t) * BK, *vs = s_v + (stg * TC + t) * NC + cl;
+            uint64_t kd[BT][RPL / 2], sk[BT][2], sq[BT][2];
 #pragma unroll
             for (int i = 0; i < RPL; i += 4) {
-                const ulonglong2 k1 = *(const ulonglong2*)(p1 + i * 16), q1 = *(const ulonglong2*)(p1 + DP + i * 16), g1 = *(const ulonglong2*)(p1 + 2 * DP + i * 16);
-                const ulonglong2 k2 = *(const ulonglong2*)(p2 + i * 16), q2 = *(const ulonglong2*)(p2 + DP + i * 16), g2 = *(const ulonglong2*)(p2 + 2 * DP + i * 16);
-                ka[i / 2] = mul2(g2.x, k1.x); ka[i / 2 + 1] = mul2(g2.y, k1.y);
-                kb[i / 2] = k2.x; kb[i / 2 + 1] = k2.y;
 #pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    uint64_t x = mul2(S[i / 2][c], g1.x), y = mul2(S[i / 2 + 1][c], g1.y);
-                    a1[c] = i == 0 ? mul2(x, k1.x) : fma2(x, k1.x, a1[c]);
-                    b1[c] = i == 0 ? mul2(x, q1.x) : fma2(x, q1.x, b1[c]);
-                    a1[c] = fma2(y, k1.y, a1[c]);
-                    b1[c] = fma2(y, q1.y, b1[c]);
-                    x = mul2(x, g2.x); y = mul2(y, g2.y);
-                    a2[c] = i == 0 ? mul2(x, k2.x) : fma2(x, k2.x, a2[c]);
-                    b2[c] = i == 0 ? mul2(x, q2.x) : fma2(x, q2.x, b2[c]);
-                    a2[c] = fma2(y, k2.y, a2[c]);
-                    b2[c] = fma2(y, q2.y, b2[c]);
-                    S[i / 2][c] = x; S[i / 2 + 1][c] = y;
+                for (int j = 0; j < (int)BT; j++) {
+                    const float* pj = p + j * 3 * DP + i * L;
+                    const ulonglong2 k = *(const ulonglong2*)pj, q = *(const ulonglong2*)(pj + DP), g = *(const ulonglong2*)(pj + 2 * DP);
+#pragma unroll
+                    for (int b = 0; b < j; b++) { kd[b][i / 2] = mul2(kd[b][i / 2], g.x); kd[b][i / 2 + 1] = mul2(kd[b][i / 2 + 1], g.y); }
+                    kd[j][i / 2] = k.x; kd[j][i / 2 + 1] = k.y;
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        const uint64_t x = mul2(S[i / 2][c], g.x), y = mul2(S[i / 2 + 1][c], g.y);
+                        sk[j][c] = i == 0 ? mul2(x, k.x) : fma2(x, k.x, sk[j][c]);
+                        sq[j][c] = i == 0 ? mul2(x, q.x) : fma2(x, q.x, sq[j][c]);
+                        sk[j][c] = fma2(y, k.y, sk[j][c]);
+                        sq[j][c] = fma2(y, q.y, sq[j][c]);
+                        S[i / 2][c] = x; S[i / 2 + 1][c] = y;
+                    }
                 }
             }
-            float e4[4], e2[2], e;
-            {
-                const float x0 = sum2(a1[0]), x1 = sum2(a1[1]), x2 = sum2(b1[0]), x3 = sum2(b1[1]);
-                const float y0 = sum2(a2[0]), y1 = sum2(a2[1]), y2 = sum2(b2[0]), y3 = sum2(b2[1]);
-                e4[0] = (second ? y0 : x0) + __shfl_xor_sync(0xffffffffu, second ? x0 : y0, 8);
-                e4[1] = (second ? y1 : x1) + __shfl_xor_sync(0xffffffffu, second ? x1 : y1, 8);
-                e4[2] = (second ? y2 : x2) + __shfl_xor_sync(0xffffffffu, second ? x2 : y2, 8);
-                e4[3] = (second ? y3 : x3) + __shfl_xor_sync(0xffffffffu, second ? x3 : y3, 8);
-            }
-            e2[0] = (isq ? e4[2] : e4[0]) + __shfl_xor_sync(0xffffffffu, isq ? e4[0] : e4[2], 4);
-            e2[1] = (isq ? e4[3] : e4[1]) + __shfl_xor_sync(0xffffffffu, isq ? e4[1] : e4[3], 4);
-            e = (odd ? e2[1] : e2[0]) + __shfl_xor_sync(0xffffffffu, odd ? e2[0] : e2[1], 2);
-            e += __shfl_xor_sync(0xffffffffu, e, 1);
-            // S^T k of both tokens and columns to every lane
-            const float s10 = __shfl_sync(0xffffffffu, e, base), s11 = __shfl_sync(0xffffffffu, e, base | 2);
-            const float s20 = __shfl_sync(0xffffffffu, e, base | 8), s21 = __shfl_sync(0xffffffffu, e, base | 10);
-            const float u10 = bk1.x * (v1.x - s10), u11 = bk1.x * (v1.y - s11);
-            const float u20 = bk2.x * (v2.x - fmaf(u10, bk2.z, s20)), u21 = bk2.x * (v2.y - fmaf(u11, bk2.z, s21));
-            const uint64_t w10 = pk2(u10, u10), w11 = pk2(u11, u11), w20 = pk2(u20, u20), w21 = pk2(u21, u21);
+            float e8[2][2][2], e4[2][2], e2[2], e;
 #pragma unroll
-            for (int i = 0; i < RPL / 2; i++) {
-                S[i][0] = fma2(kb[i], w20, fma2(ka[i], w10, S[i][0]));
-                S[i][1] = fma2(kb[i], w21, fma2(ka[i], w11, S[i][1]));
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const float k0 = sum2(sk[j][c]), k1 = sum2(sk[j + 2][c]), q0 = sum2(sq[j][c]), q1 = sum2(sq[j + 2][c]);
+                    e8[j][0][c] = (hi ? k1 : k0) + __shfl_xor_sync(0xffffffffu, hi ? k0 : k1, L / 2);
+                    e8[j][1][c] = (hi ? q1 : q0) + __shfl_xor_sync(0xffffffffu, hi ? q0 : q1, L / 2);
+                }
+#pragma unroll
+            for (int w = 0; w < 2; w++)
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+                    e4[w][c] = (lo ? e8[1][w][c] : e8[0][w][c]) + __shfl_xor_sync(0xffffffffu, lo ? e8[0][w][c] : e8[1][w][c], L / 4);
+#pragma unroll
+            for (int c = 0; c < 2; c++) e2[c] = (isq ? e4[1][c] : e4[0][c]) + __shfl_xor_sync(0xffffffffu, isq ? e4[0][c] : e4[1][c], L / 8);
+            e = (odd ? e2[1] : e2[0]) + __shfl_xor_sync(0xffffffffu, odd ? e2[0] : e2[1], L / 16);
+            if (L == 32) e += __shfl_xor_sync(0xffffffffu, e, 1);
+            float u[BT][2];
+#pragma unroll
+            for (int j = 0; j < (int)BT; j++) {
+                const float4 b = *(const float4*)(bk + j * BK);          // step, m0, m1, m2
+                const float2 v = *(const float2*)(vs + j * NC);
+                const uint32_t from = base | (j & 2 ? L / 2 : 0) | (j & 1 ? L / 4 : 0);
+                float s0 = __shfl_sync(0xffffffffu, e, from), s1 = __shfl_sync(0xffffffffu, e, from | (L / 16));
+                if (j > 0) { s0 = fmaf(u[0][0], b.y, s0); s1 = fmaf(u[0][1], b.y, s1); }
+                if (j > 1) { s0 = fmaf(u[1][0], b.z, s0); s1 = fmaf(u[1][1], b.z, s1); }
+                if (j > 2) { s0 = fmaf(u[2][0], b.w, s0); s1 = fmaf(u[2][1], b.w, s1); }
+                u[j][0] = b.x * (v.x - s0);
+                u[j][1] = b.x * (v.y - s1);
             }
-            if (isq && !(l & 1) && c0 + cl + odd < V && t + second < nt) {
-                const float u1 = odd ? u11 : u10, u2 = odd ? u21 : u20;
-                a.o[((size_t)(t0 + t + second) * H + h) * V + c0 + cl + odd] = second ? fmaf(u2, bk2.y, fmaf(u1, bk2.w, e)) : fmaf(u1, bk1.y, e);
+#pragma unroll
+            for (int j = 0; j < (int)BT; j++) {
+                const uint64_t w0 = pk2(u[j][0], u[j][0]), w1 = pk2(u[j][1], u[j][1]);
+#pragma unroll
+                for (int i = 0; i < RPL / 2; i++) {
+                    S[i][0] = fma2(kd[j][i], w0, S[i][0]);
+                    S[i][1] = fma2(kd[j][i], w1, S[i][1]);
+                }
+            }
+            if (isq && (L == 16 || !(l & 1)) && c0 + cl + odd < V && t + mine < nt) {
+                const float4 n = *(const float4*)(bk + mine * BK + 4);   // k . q, n0, n1, n2
+                const float x0 = odd ? u[0][1] : u[0][0], x1 = odd ? u[1][1] : u[1][0], x2 = odd ? u[2][1] : u[2][0], x3 = odd ? u[3][1] : u[3][0];
+                const float own = hi ? (lo ? x3 : x2) : (lo ? x1 : x0);
+                a.o[((size_t)(t0 + t + mine) * H + h) * V + c0 + cl + odd] = fmaf(own, n.x, fmaf(x2, n.w, fmaf(x1, n.z, fmaf(x0, n.y, e))));
             }
         }
         __syncthreads();
@@ -536,7 +563,7 @@ bool launch_step(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
 
 template <class A>
 void launch_prep(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32_t rows) {
-    const dim3 grid((a.heads + 7) / 8, (rows + 1) / 2);
+    const dim3 grid((a.heads + 7) / 8, (rows + BT - 1) / BT);
     if (a.dim <= 64) launch_pdl(delta_prep_kernel<A, 2>, grid, dim3(256), 0, st, a, w, rows);
     else if (a.dim <= 128) launch_pdl(delta_prep_kernel<A, 4>, grid, dim3(256), 0, st, a, w, rows);
     else launch_pdl(delta_prep_kernel<A, 16>, grid, dim3(256), 0, st, a, w, rows);
@@ -545,20 +572,23 @@ void launch_prep(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32
 
 // Ordinary launch: CTAs that come up while the kernel before still holds SMs pile up on the ones it has left, and the
 // recurrence then runs at the pace of the fullest SM.
-template <int RPL, int NW, bool VEC>
+template <int L, int RPL, int NW, bool VEC>
 void launch_scan_t(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32_t rows) {
-    const size_t smem = (size_t)2 * TC * (3 * 16 * RPL + NW * 4 + 4) * 4;
+    constexpr uint32_t NC = NW * (32 / L) * 2;
+    const size_t smem = (size_t)2 * TC * (3 * L * RPL + NC + BK) * 4;
     static int have[64] = {};
-    ensure_dyn_smem(delta_scan_kernel<RPL, NW, VEC>, smem, have);
-    delta_scan_kernel<RPL, NW, VEC><<<dim3((a.vdim + NW * 4 - 1) / (NW * 4), a.heads), NW * 32, smem, st>>>(a, w, rows);
+    ensure_dyn_smem(delta_scan_kernel<L, RPL, NW, VEC>, smem, have);
+    delta_scan_kernel<L, RPL, NW, VEC><<<dim3((a.vdim + NC - 1) / NC, a.heads), NW * 32, smem, st>>>(a, w, rows);
     g_launches++;
 }
-template <int RPL>
+// 32 columns per CTA, or 16 while CTAs of 32 would leave half of the SMs without one, and where 16 warps of 32 columns have no
+// registers for 8 rows a lane and more
+template <int L, int RPL>
 void launch_scan(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32_t rows) {
-    if (a.dim % 4) { launch_scan_t<RPL, 8, false>(st, a, w, rows); return; }
-    // narrower CTAs while those of 8 warps would leave half of the SMs without one
-    if ((a.vdim + 31) / 32 * a.heads <= 74) launch_scan_t<RPL, 4, true>(st, a, w, rows);
-    else launch_scan_t<RPL, 8, true>(st, a, w, rows);
+    constexpr int NARROW = L / 4, WIDE = RPL > 4 ? L / 4 : L / 2;
+    if (a.dim % 4) { launch_scan_t<L, RPL, NARROW, false>(st, a, w, rows); return; }
+    if ((a.vdim + 31) / 32 * a.heads <= 74) launch_scan_t<L, RPL, NARROW, true>(st, a, w, rows);
+    else launch_scan_t<L, RPL, WIDE, true>(st, a, w, rows);
 }
 
 }  // namespace
@@ -573,7 +603,7 @@ void k_short_conv(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
 }
 
 size_t delta_work_floats(const DeltaArgs& a, uint32_t rows) {
-    return 2 * up4((size_t)rows * a.kv_heads * a.dim) + up4((size_t)rows * a.heads * a.dim) + (size_t)rows * a.heads * 4;
+    return 2 * up4((size_t)rows * a.kv_heads * a.dim) + up4((size_t)rows * a.heads * a.dim) + (size_t)rows * a.heads * BK;
 }
 
 void k_channel_delta(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
@@ -581,10 +611,10 @@ void k_channel_delta(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
     const DeltaWork w = work_of(a, rows);
     if (a.bf16) launch_prep<ActBf16>(st, a, w, rows);
     else launch_prep<ActF32>(st, a, w, rows);
-    if (a.dim <= 64) launch_scan<4>(st, a, w, rows);
-    else if (a.dim <= 128) launch_scan<8>(st, a, w, rows);
-    else if (a.dim <= 256) launch_scan<16>(st, a, w, rows);
-    else launch_scan<32>(st, a, w, rows);
+    if (a.dim <= 64) launch_scan<16, 4>(st, a, w, rows);
+    else if (a.dim <= 128) launch_scan<32, 4>(st, a, w, rows);
+    else if (a.dim <= 256) launch_scan<32, 8>(st, a, w, rows);
+    else launch_scan<32, 16>(st, a, w, rows);
 }
 
 bool k_delta_step(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
