@@ -793,8 +793,8 @@ int gehtp_cuda_state_load(const struct wt_blob* b, uint32_t idx, const void* src
 int gehtp_cuda_state_set_count(uint32_t idx, uint32_t n_positions) {
     if (!g.dev_ok || idx >= g.n_states || !g.kv[idx].ready || n_positions > g.kv[idx].nslots) return -1;
     cudaSetDevice(g.device);
-    cudaMemcpyAsync(g.d_st_count + idx, &n_positions, 4, cudaMemcpyHostToDevice, g.stream);
-    cudaStreamSynchronize(g.stream);
+    // in stream order behind the runs queued so far; a copy and a wait per state took 8 us (228 us for 28 layers)
+    if (!k_set_count(g.stream, g.d_st_count + idx, n_positions)) return -1;
     g.st_count[idx] = n_positions;
     return 0;
 }

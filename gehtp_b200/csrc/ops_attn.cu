@@ -129,6 +129,14 @@ __global__ void kv_append_kernel(const uint16_t* __restrict__ k, const uint16_t*
     }
 }
 
+__global__ void set_count_kernel(uint32_t* counter, uint32_t n) { *counter = n; }
+
+bool k_set_count(cudaStream_t st, uint32_t* counter, uint32_t n) {
+    set_count_kernel<<<1, 1, 0, st>>>(counter, n);
+    g_launches++;
+    return cudaGetLastError() == cudaSuccess;
+}
+
 void k_kv_append(cudaStream_t st, const uint16_t* k, const uint16_t* v, uint16_t* ring,
                  uint32_t* posmap, uint32_t* counter, uint32_t kv_elems, uint32_t nslots,
                  uint32_t pos_const) {
