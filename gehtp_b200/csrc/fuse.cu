@@ -893,7 +893,7 @@ void fuse_materialize(const wt_blob* b) {
                 const uint16_t* act = (const uint16_t*)resolve(b, lo.args[0]);
                 if (it != g.w4.end() && act && !lin.fused && !lin.rc && lin.launch && !lin.uses_internal && !reduced &&
                     lo.args[3] == B && N == (nh + 2 * kvh) * hd && K % 512 == 0 && K / 512 <= 10 &&
-                    N / 32 >= 148) {     // one CTA per pair of strips: worth it only while every SM still gets one
+                    N / 32 >= 120) {     // one CTA per pair of strips: worth it while nearly every SM still gets one (128 pairs: 780 -> 755 us a step of 28 layers)
                     W4Epilogue ep;
                     ep.mode = 2;
                     ep.cos_q = cq; ep.sin_q = sq; ep.cos_k = ck; ep.sin_k = sk; ep.q_out = q_out; ep.ring = ring;
