@@ -68,7 +68,7 @@ latent_append_kernel(const LatentArgs a) {
     }
 }
 
-// Plain attention of one (row, head): the query through the key up-projection, scores against the cached rows, running
+// Plain attention of one (row, head), for the one-kernel-per-op plan and sizes the others do not take: the query through the key up-projection, scores against the cached rows, running
 // softmax over blocks of 128 keys, the weighted latent through the value up-projection. Dynamic shared memory:
 // [rank + rot] query, [rank] latent, fp32.
 template <class A>
@@ -130,6 +130,148 @@ latent_exact_kernel(const LatentArgs a) {
         s = warp_sum(s);
         if (lane == 0) A::st(out + v, s * g);
     }
+}
+
+// fp32 rows: a CTA of 8 warps takes one head and 8 rows, so that the up-projections and every cached row are read once for the
+// eight. Queries into latent space (a thread per column); per block of 64 keys the scores (a warp per 4 keys, lanes along the
+// latent, 32 sums folded over the lanes), the running softmax (a warp per row) and the weighted latent (a thread per column,
+// NC of them in registers); the value up-projection with lanes along the latent. Sums are fp32 FMAs, in shorter chains than
+// one after the other. Bound by shared-memory reads and FMAs; a CTA per (row, head) read 256 KB of weights each and cached rows
+// with a stride. 16 heads, rank 512, 77 rows: 500 -> 78 us; two such layers, 300 + 3 tokens, of a model: 9.6 -> 2.8 ms.
+constexpr uint32_t FR = 8, FK = 64;
+template <int NC>
+__global__ void __launch_bounds__(256)
+latent_f32_kernel(const LatentArgs a, uint32_t rows) {
+    extern __shared__ float sm[];
+    __shared__ __align__(16) float sp[FK * FR];          // scores, then weights: [key][row]
+    __shared__ float s_corr[FR], s_l[FR];
+    pdl_release();
+    pdl_wait();
+    const uint32_t h = blockIdx.x, r0 = blockIdx.y * FR, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t nr = min(FR, rows - r0), past = *a.counter, n = past + r0 + nr, hd = a.dim + a.rot, ls = a.ls(), qw = a.rank + a.rot;
+    float *qa = sm, *q = qa + FR * qw;                   // [FR][qw] (later the latent), [FR][dim]
+    for (uint32_t i = tid; i < FR * hd; i += 256) {
+        const uint32_t r = i / hd, c = i % hd;
+        const float v = r < nr ? __ldcg((const float*)a.q + ((size_t)(r0 + r) * a.heads + h) * hd + c) : 0.0f;
+        if (c < a.dim) q[r * a.dim + c] = v; else qa[r * qw + a.rank + c - a.dim] = v;
+    }
+    __syncthreads();
+    for (uint32_t c = tid; c < a.rank; c += 256) {
+        float s[FR] = {};
+        const uint16_t* w = a.w_kv + (size_t)h * a.dim * a.rank + c;
+#pragma unroll 4
+        for (uint32_t d = 0; d < a.dim; d++) {
+            const float wv = bf2f(__ldg(w + (size_t)d * a.rank));
+#pragma unroll
+            for (int r = 0; r < (int)FR; r++) s[r] = fmaf(q[r * a.dim + d], wv, s[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < (int)FR; r++) qa[r * qw + c] = s[r];
+    }
+    __syncthreads();
+    const float* state = (const float*)a.state;
+    const uint32_t mine = past + r0 + min(warp, nr - 1) + 1;       // keys that row `warp` sees (rows past the last repeat it)
+    float ctx[NC][FR], m = -INFINITY, l = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NC; i++)
+#pragma unroll
+        for (int r = 0; r < (int)FR; r++) ctx[i][r] = 0.0f;
+    for (uint32_t j0 = 0; j0 < n; j0 += FK) {
+        const uint32_t cnt = min(FK, n - j0);
+        for (uint32_t k0 = warp * 4; k0 < cnt; k0 += 32) {
+            float acc[4 * FR] = {};
+            const float* row[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) row[k] = state + (size_t)min(j0 + k0 + k, n - 1) * ls;
+            for (uint32_t c = lane; c < qw; c += 32) {
+                float x[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) x[k] = __ldcg(row[k] + c);
+#pragma unroll
+                for (int r = 0; r < (int)FR; r++) {
+                    const float v = qa[r * qw + c];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) acc[k * FR + r] = fmaf(v, x[k], acc[k * FR + r]);
+                }
+            }
+            sp[k0 * FR + lane] = fold_sum<4 * FR>(acc) * a.scale;  // lane = (key, row)
+        }
+        __syncthreads();
+        {
+            float s[2], bm = m;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const uint32_t k = lane + 32 * i;
+                s[i] = k < cnt && j0 + k < mine ? sp[k * FR + warp] : -INFINITY;
+                bm = fmaxf(bm, s[i]);
+            }
+            bm = warp_max(bm);                                       // key 0 is visible to every row: finite
+            const float corr = expf(m - bm), e0 = expf(s[0] - bm), e1 = expf(s[1] - bm);
+            m = bm;
+            l = l * corr + warp_sum(e0 + e1);
+            sp[lane * FR + warp] = e0;
+            sp[(lane + 32) * FR + warp] = e1;
+            if (lane == 0) s_corr[warp] = corr;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NC; i++)
+#pragma unroll
+            for (int r = 0; r < (int)FR; r++) ctx[i][r] *= s_corr[r];
+#pragma unroll 4
+        for (uint32_t k = 0; k < cnt; k++) {
+            const float4 p0 = *(const float4*)(sp + k * FR), p1 = *(const float4*)(sp + k * FR + 4);
+            const float p[FR] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const uint32_t c = tid + 256 * i;
+                const float x = c < a.rank ? __ldcg(state + (size_t)(j0 + k) * ls + c) : 0.0f;
+#pragma unroll
+                for (int r = 0; r < (int)FR; r++) ctx[i][r] = fmaf(p[r], x, ctx[i][r]);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        const uint32_t c = tid + 256 * i;
+        if (c >= a.rank) break;
+#pragma unroll
+        for (int r = 0; r < (int)FR; r++) qa[r * qw + c] = ctx[i][r];  // the queries have been used
+    }
+    if (lane == 0) s_l[warp] = l;
+    __syncthreads();
+    for (uint32_t v0 = warp * 4; v0 < a.vdim; v0 += 32) {
+        float acc[4 * FR] = {};
+        const uint16_t* w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = a.w_kv + ((size_t)a.heads * a.dim + (size_t)h * a.vdim + min(v0 + k, a.vdim - 1)) * a.rank;
+        for (uint32_t c = lane; c < a.rank; c += 32) {
+            float x[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) x[k] = bf2f(__ldg(w[k] + c));
+#pragma unroll
+            for (int r = 0; r < (int)FR; r++) {
+                const float v = qa[r * qw + c];
+#pragma unroll
+                for (int k = 0; k < 4; k++) acc[k * FR + r] = fmaf(v, x[k], acc[k * FR + r]);
+            }
+        }
+        const float s = fold_sum<4 * FR>(acc);
+        const uint32_t v = v0 + lane / FR, r = lane % FR;
+        if (v < a.vdim && r < nr)
+            ((float*)a.out)[((size_t)(r0 + r) * a.heads + h) * a.vdim + v] = s * (a.gate[(size_t)(r0 + r) * a.heads + h] / s_l[r]);
+    }
+}
+
+template <int NC>
+bool launch_f32(cudaStream_t st, const LatentArgs& a, uint32_t rows) {
+    static int have[64] = {};
+    const size_t smem = (size_t)FR * (a.rank + a.rot + a.dim) * 4;
+    if (smem > 200 * 1024 || !ensure_dyn_smem(latent_f32_kernel<NC>, smem, have)) return false;
+    if (launch_pdl(latent_f32_kernel<NC>, dim3(a.heads, (rows + FR - 1) / FR), dim3(256), smem, st, a, rows) != cudaSuccess) { cudaGetLastError(); return false; }
+    g_launches++;
+    return true;
 }
 
 // Few rows: q of every head into latent space, times the score scale, stored as hi + lo bf16 rows like the cached ones.
@@ -548,6 +690,7 @@ void k_latent_append(cudaStream_t st, const LatentArgs& a, uint32_t rows) {
 void k_latent_attend(cudaStream_t st, const LatentArgs& a, uint32_t rows, uint32_t n_past, bool exact) {
     if (!rows) return;
     if (a.bf16 && !exact && k_latent_prefill(st, a, rows, n_past)) return;
+    if (!a.bf16 && !exact && a.rank <= 1024 && (a.rank <= 512 ? launch_f32<2>(st, a, rows) : launch_f32<4>(st, a, rows))) return;
     const size_t smem = (size_t)(2 * a.rank + a.rot) * 4;
     static int have_b[64] = {}, have_f[64] = {};
     if (a.bf16) {

@@ -190,7 +190,7 @@ void plan_rows_op(Planner& P, const wt_op& op, PlanOp& p) {
             // runs that may be captured take the kernel that reads the position count on the device
             if (P.build) p.launch = [=](cudaStream_t st) {
                 const uint32_t n = rows_of(rows);
-                k_latent_attend(st, l, n, g.st_count[l.state_idx], !g.opt_fuse || g.exact_ops || n <= kGraphRows);
+                k_latent_attend(st, l, n, g.st_count[l.state_idx], !g.opt_fuse || g.exact_ops || (l.bf16 && n <= kGraphRows));
             };
         }
         p.rows_args->lat = l;
