@@ -50,8 +50,10 @@ struct PlanOp {
     uint32_t span = 0;
     uint32_t stat = 0;          // index into the stats struct, 0 = none
     bool uses_internal = false; // touches a temp that has no memory in a fused plan
-    bool wanted_now = false;        // scratch of want_temp
-    bool dead_when_fused = false;   // its result is read only by ops that fused chains replace: skipped in whole fused runs
+    // its result is read only by ops that fused chains replace: skipped in whole fused runs. again: launched behind such a
+    // run it leaves what it would have left inside (fuse_left_out); left_out: the last run skipped it; left_src: temp it reads
+    bool dead_when_fused = false, again = false, left_out = false;
+    uint32_t left_src = kNoOff;
     // a data-movement op whose inputs are weight slots (or results of such ops) and whose output nobody else writes:
     // its result is a constant of the blob, made by the first run that reaches it and kept
     bool const_fold = false, const_done = false;
@@ -194,6 +196,8 @@ void fuse_materialize(const wt_blob* b);
 // Marks the ops whose result is a constant of the blob (PlanOp::const_fold). addr / maxb: device address and capacity
 // of every temp id of the plan.
 void fold_constants(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb);
+// Marks the ops that whole fused runs leave out (PlanOp::dead_when_fused), of those that fuse_analyze found dead.
+void fuse_left_out(const wt_blob* b, const std::vector<uint8_t>& dead, uint8_t* const* addr, const uint64_t* maxb);
 // Chunks of the delta rule that carry one state: their launches gathered at the first of them (behind fold_constants).
 void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb);
 bool fuse_all_materialized();

@@ -209,27 +209,37 @@ void drop_graphs() {
     g.graphs.clear();
 }
 
+// Launches what the last run left out, all of it or (ids) the writers of those temps, and waits: whoever reads the bytes
+// may do so from any stream. The caller's current device stays as it is.
+static void make_up(const std::vector<uint8_t>* ids) {
+    int device = -1;
+    for (PlanOp& p : g.plan) {
+        if (!p.left_out || !p.again || !p.launch || (ids && !(*ids)[p.out_id[0]])) continue;
+        if (device < 0) { cudaGetDevice(&device); cudaSetDevice(g.device); }
+        p.launch(g.stream);
+        p.left_out = false;
+    }
+    if (device < 0) return;
+    cudaStreamSynchronize(g.stream);
+    cudaSetDevice(device);
+}
+
 // A caller asks for a temp that whole fused runs leave out (dead_when_fused): its op and the left-out ops in front of it
 // are launched from now on. now: launch them here too, behind a run that left them out.
 static void want_temp(uint32_t id, bool now) {
     if (!g.planned || id >= kMaxTemps) return;
-    std::vector<uint8_t> want(kMaxTemps, 0);
-    want[id] = 1;
-    bool any = false;
+    std::vector<uint8_t> want;
     for (uint32_t i = (uint32_t)g.plan.size(); i-- > 0;) {
         PlanOp& p = g.plan[i];
-        if (!p.dead_when_fused || p.out_id[0] == kNoOff || !want[p.out_id[0]]) continue;
-        const uint32_t src = g.blob->ops[i].args[0];
-        if (!(src & 0xC000u) && src < kMaxTemps) want[src] = 1;
+        if (!p.dead_when_fused || !p.again || (want.empty() ? p.out_id[0] != id : !want[p.out_id[0]])) continue;
+        want.resize(kMaxTemps, 0);
+        want[id] = 1;
+        if (p.left_src != kNoOff) want[p.left_src] = 1;
         p.dead_when_fused = false;
-        p.wanted_now = any = true;
     }
-    if (!any) return;
+    if (want.empty()) return;
     drop_graphs();
-    for (PlanOp& p : g.plan) {
-        if (p.wanted_now && now && p.launch) p.launch(g.stream);
-        p.wanted_now = false;
-    }
+    if (now) make_up(&want);
 }
 
 static void note_outputs(const PlanOp& p) {
@@ -285,7 +295,8 @@ static int queue_range(uint32_t first, uint32_t count, bool fuse, bool per_op_sy
             if (!rc) {
                 if (use_fused) p.fused(g.stream);
                 else for (PlanOp* q : pending) {
-                    if (!q->launch || (g.skip_dead && q->dead_when_fused)) continue;
+                    if (!q->launch) continue;
+                    if ((q->left_out = g.skip_dead && q->dead_when_fused)) continue;
                     if (q->const_fold && q->const_done) continue;        // a constant of the blob, made by an earlier run
                     q->launch(g.stream);
                     if (q->const_fold && !capturing) q->const_done = true;   // inside a capture the launch has not run yet
@@ -427,6 +438,7 @@ static int run_impl(const wt_blob* b, uint32_t first, uint32_t count, const void
             g.st.ops++;
             note_outputs(q);
             host_advance(q, 1);
+            q.left_out = q.dead_when_fused;
         }
         if (in_host) {
             for (auto& kv : g.d_ext)
@@ -442,6 +454,8 @@ static int run_impl(const wt_blob* b, uint32_t first, uint32_t count, const void
         if (rc == 0 && out_host && out_temp < kMaxTemps) std::memcpy(out_host, g.h_out, g.temp_last[out_temp]);
         return rc;
     }
+
+    if (!whole) make_up(nullptr);       // a range may read any temp, with the bytes the last run gave it
 
     // a run that could be graphed later is captured on its second eager pass
     const uint64_t warm_key = (uint64_t)rows << 32 | sel;
@@ -578,6 +592,7 @@ int gehtp_cuda_run_dev(const struct wt_blob* b, const void* in_dev, void* out_de
 
 uint8_t* wt_exec_temp(uint32_t id) {
     if (!g.dev_ok || id >= kMaxTemps || !g.temp_cap[id] || !g.temp_dev[id]) return nullptr;
+    cudaSetDevice(g.device);
     want_temp(id, true);
     auto& m = g.mirrors[id];
     size_t need = g.temp_cap[id];
@@ -587,7 +602,6 @@ uint8_t* wt_exec_temp(uint32_t id) {
         if (cudaMallocHost(&m.first, need) != cudaSuccess) { m.second = 0; return nullptr; }
         m.second = need;
     }
-    cudaSetDevice(g.device);
     cudaStreamSynchronize(g.stream);
     if (cudaMemcpy(m.first, g.temp_dev[id], need, cudaMemcpyDeviceToHost) != cudaSuccess) return nullptr;
     return m.first;
@@ -699,7 +713,6 @@ uint32_t gehtp_cuda_demoted_temps(void) { return g.demoted_temps; }
 void* gehtp_cuda_stream(void) { return ensure_device(nullptr, 0) ? (void*)g.stream : nullptr; }
 void* gehtp_cuda_temp_dev(uint32_t id) {
     if (id >= kMaxTemps || !g.temp_cap[id]) return nullptr;
-    cudaSetDevice(g.device);
     want_temp(id, true);
     return g.temp_dev[id];
 }

@@ -1103,6 +1103,73 @@ void fuse_materialize(const wt_blob* b) {
     }
 }
 
+namespace {
+
+// Who writes the temps of a planned list, and which of them share memory
+struct TempMemory {
+    uint8_t* const* addr;
+    const uint64_t* maxb;
+    std::vector<int> writers;
+    bool planner_ops = false;       // SPILL, FILL, DMA: they write slots and parts of temps
+    TempMemory(const wt_blob* b, uint8_t* const* a, const uint64_t* m) : addr(a), maxb(m), writers(kMaxTemps, 0) {
+        for (uint32_t i = 0; i < b->n_ops; i++) {
+            const uint32_t oc = b->ops[i].opcode;
+            if (oc == OP_SPILL || oc == OP_FILL || oc == OP_DMA) planner_ops = true;
+            for (uint32_t id : g.plan[i].out_id)
+                if (id != kNoOff && id < kMaxTemps) writers[id]++;
+        }
+    }
+    // one op writes it, and its memory overlaps no other temp's
+    bool own(uint32_t id) const {
+        if (id >= kMaxTemps || writers[id] != 1 || !addr[id] || !maxb[id]) return false;
+        const uint8_t *lo = addr[id], *hi = lo + maxb[id];
+        for (uint32_t t = 0; t < kMaxTemps; t++)
+            if (t != id && addr[t] && maxb[t] && addr[t] < hi && lo < addr[t] + maxb[t]) return false;
+        return true;
+    }
+};
+
+}  // namespace
+
+// A dead op may be left out of a run only if nobody can tell afterwards. Either it can be launched again behind the run
+// and leaves what it would have left inside: nothing but it writes its result's memory, and what it reads is a slot, or a
+// temp that keeps its value as well. Or its result is gone at the end of a run anyway: a later op writes over all of it (an
+// id used again, a static table that lays temps on one another). Any other stays in the run, and so does what it reads.
+void fuse_left_out(const wt_blob* b, const std::vector<uint8_t>& dead, uint8_t* const* addr, const uint64_t* maxb) {
+    const TempMemory mem(b, addr, maxb);
+    std::vector<int> made_by(kMaxTemps, -1), source(b->n_ops, -1);
+    for (uint32_t i = 0; i < b->n_ops; i++) {
+        PlanOp& p = g.plan[i];
+        if (dead[i]) {
+            const uint32_t src = b->ops[i].args[0];
+            if (is_temp_ref(src)) { p.left_src = src; source[i] = made_by[src]; }
+            const bool stays = is_temp_ref(src) ? source[i] >= 0 && mem.own(src) && (!dead[source[i]] || g.plan[source[i]].again) : (src & 0xC000u) == 0x8000u;
+            p.again = stays && !mem.planner_ops && mem.own(p.out_id[0]);
+        }
+        for (uint32_t id : p.out_id)
+            if (id != kNoOff && id < kMaxTemps) made_by[id] = (int)i;
+    }
+    auto written_over = [&](uint32_t i) {
+        const uint8_t* lo = addr[g.plan[i].out_id[0]];
+        const size_t n = g.plan[i].out_bytes[0];
+        for (uint32_t j = i + 1; lo && j < b->n_ops; j++) {
+            const PlanOp& q = g.plan[j];
+            for (int k = 0; k < 2; k++) {
+                const uint32_t id = q.out_id[k];
+                if (id != kNoOff && !q.rc && !q.out_row_bytes[k] && addr[id] && addr[id] <= lo && lo + n <= addr[id] + q.out_bytes[k]) return true;
+            }
+        }
+        return false;
+    };
+    std::vector<uint8_t> read(b->n_ops, 0);             // by an op that stays
+    for (uint32_t i = b->n_ops; i-- > 0;) {
+        if (!dead[i]) continue;
+        PlanOp& p = g.plan[i];
+        p.dead_when_fused = !read[i] && (p.again || written_over(i));
+        if (!p.dead_when_fused && source[i] >= 0) read[source[i]] = 1;
+    }
+}
+
 // Constant results. Compiled runlists slice, transpose and broadcast tables that live in weight slots (rotary tables,
 // masks, per-chunk windows of a constant tensor) with one op per ONNX node; such an op gives the same bytes on every
 // run. It is marked when: it only moves data; every tensor it reads is a weight slot with data in the blob or the
@@ -1112,18 +1179,13 @@ void fuse_materialize(const wt_blob* b) {
 // captured graph - skip it.
 void fold_constants(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb) {
     g.const_ops = 0;
-    for (uint32_t i = 0; i < b->n_ops; i++) {
-        const uint32_t oc = b->ops[i].opcode;
-        if (oc == OP_SPILL || oc == OP_FILL || oc == OP_DMA) return;
-    }
+    const TempMemory mem(b, addr, maxb);
+    if (mem.planner_ops) return;
     for (uint32_t s = 0; s < b->n_slots; s++)
         if (b->slots[s].addr == WT_SLOT_TEMPOFF) return;
-    std::vector<int> writers(kMaxTemps, 0);
     std::vector<uint8_t> in_span(b->n_ops, 0), const_temp(kMaxTemps, 0);
     for (uint32_t i = 0; i < b->n_ops; i++) {
         const PlanOp& p = g.plan[i];
-        for (int k = 0; k < 2; k++)
-            if (p.out_id[k] != kNoOff && p.out_id[k] < kMaxTemps) writers[p.out_id[k]]++;
         if (p.fused && p.span)
             for (uint32_t k = 0; k < p.span && i + k < b->n_ops; k++) in_span[i + k] = 1;
     }
@@ -1156,10 +1218,7 @@ void fold_constants(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb
             const uint32_t id = p.out_id[k];
             if (id == kNoOff) continue;
             outs++;
-            if (id >= kMaxTemps || writers[id] != 1 || !addr[id] || !maxb[id]) { ok = false; break; }
-            const uint8_t *lo = addr[id], *hi = lo + maxb[id];
-            for (uint32_t t = 0; t < kMaxTemps && ok; t++)
-                if (t != id && addr[t] && maxb[t] && addr[t] < hi && lo < addr[t] + maxb[t]) ok = false;
+            ok = mem.own(id);
         }
         if (!ok || !outs) continue;
         p.const_fold = true;

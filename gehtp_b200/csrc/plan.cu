@@ -821,8 +821,7 @@ int build_plan(const wt_blob* b, char* err, size_t errn) {
     if (fusing) {
         fuse_materialize(b);
         // only when every chain really got its kernel: a chain left op-by-op still reads those results
-        if (fuse_all_materialized())
-            for (uint32_t i = 0; i < b->n_ops && i < dead_ops.size(); i++) g.plan[i].dead_when_fused = dead_ops[i] != 0;
+        if (fuse_all_materialized()) fuse_left_out(b, dead_ops, P.addr, P.maxb);
         fold_constants(b, P.addr, P.maxb);
         fuse_delta_runs(b, P.addr, P.maxb);
     }
