@@ -205,8 +205,9 @@ latent_f32_kernel(const LatentArgs a, uint32_t rows) {
                 s[i] = k < cnt && j0 + k < mine ? sp[k * FR + warp] : -INFINITY;
                 bm = fmaxf(bm, s[i]);
             }
-            bm = warp_max(bm);                                       // key 0 is visible to every row: finite
-            const float corr = expf(m - bm), e0 = expf(s[0] - bm), e1 = expf(s[1] - bm);
+            bm = warp_max(bm);
+            const float base = bm == -INFINITY ? 0.0f : bm;          // scores of -inf alone so far: weights of zero
+            const float corr = expf(m - base), e0 = expf(s[0] - base), e1 = expf(s[1] - base);
             m = bm;
             l = l * corr + warp_sum(e0 + e1);
             sp[lane * FR + warp] = e0;
@@ -218,8 +219,7 @@ latent_f32_kernel(const LatentArgs a, uint32_t rows) {
         for (int i = 0; i < NC; i++)
 #pragma unroll
             for (int r = 0; r < (int)FR; r++) ctx[i][r] *= s_corr[r];
-#pragma unroll 4
-        for (uint32_t k = 0; k < cnt; k++) {
+        auto add = [&](uint32_t k, uint32_t from) {                  // key j0 + k to the rows from `from` on
             const float4 p0 = *(const float4*)(sp + k * FR), p1 = *(const float4*)(sp + k * FR + 4);
             const float p[FR] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
@@ -227,9 +227,13 @@ latent_f32_kernel(const LatentArgs a, uint32_t rows) {
                 const uint32_t c = tid + 256 * i;
                 const float x = c < a.rank ? __ldcg(state + (size_t)(j0 + k) * ls + c) : 0.0f;
 #pragma unroll
-                for (int r = 0; r < (int)FR; r++) ctx[i][r] = fmaf(p[r], x, ctx[i][r]);
+                for (int r = 0; r < (int)FR; r++) ctx[i][r] = fmaf(p[r], (uint32_t)r < from ? 0.0f : x, ctx[i][r]);
             }
-        }
+        };
+        const uint32_t all = min(cnt, past + r0 + 1 > j0 ? past + r0 + 1 - j0 : 0);      // keys that every row sees
+#pragma unroll 4
+        for (uint32_t k = 0; k < all; k++) add(k, 0);
+        for (uint32_t k = all; k < cnt; k++) add(k, j0 + k - past - r0);                  // a row's result holds nothing of keys behind it, whatever they are
         __syncthreads();
     }
 #pragma unroll
