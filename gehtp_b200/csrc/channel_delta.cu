@@ -277,8 +277,9 @@ delta_scan_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
                 if (j > 0) { s0 = fmaf(u[0][0], b.y, s0); s1 = fmaf(u[0][1], b.y, s1); }
                 if (j > 1) { s0 = fmaf(u[1][0], b.z, s0); s1 = fmaf(u[1][1], b.z, s1); }
                 if (j > 2) { s0 = fmaf(u[2][0], b.w, s0); s1 = fmaf(u[2][1], b.w, s1); }
-                u[j][0] = b.x * (v.x - s0);
-                u[j][1] = b.x * (v.y - s1);
+                const bool token = t + j < nt;                           // an idle one adds nothing, whatever S holds
+                u[j][0] = token ? b.x * (v.x - s0) : 0.0f;
+                u[j][1] = token ? b.x * (v.y - s1) : 0.0f;
             }
 #pragma unroll
             for (int j = 0; j < (int)BT; j++) {
@@ -293,7 +294,11 @@ delta_scan_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
                 const float4 n = *(const float4*)(bk + mine * BK + 4);   // k . q, n0, n1, n2
                 const float x0 = odd ? u[0][1] : u[0][0], x1 = odd ? u[1][1] : u[1][0], x2 = odd ? u[2][1] : u[2][0], x3 = odd ? u[3][1] : u[3][0];
                 const float own = hi ? (lo ? x3 : x2) : (lo ? x1 : x0);
-                a.o[((size_t)(t0 + t + mine) * H + h) * V + c0 + cl + odd] = fmaf(own, n.x, fmaf(x2, n.w, fmaf(x1, n.z, fmaf(x0, n.y, e))));
+                float o = e;                                             // tokens behind this one are left out, not weighted with their zeros
+                if (mine > 0) o = fmaf(x0, n.y, o);
+                if (mine > 1) o = fmaf(x1, n.z, o);
+                if (mine > 2) o = fmaf(x2, n.w, o);
+                a.o[((size_t)(t0 + t + mine) * H + h) * V + c0 + cl + odd] = fmaf(own, n.x, o);
             }
         }
         __syncthreads();

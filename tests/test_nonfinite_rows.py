@@ -28,3 +28,18 @@ def test_latent_rows_before_a_bad_token(cuda, value, past, rows, bad):
     got = s.feed(tok[past:] + [mt[0]["vocab"] - 1] * (rows - bad), range(bad))
     s.close()
     assert rip.close(got[:, :-1], want, "float32")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("bad", [1, 6, 7, 17])
+def test_delta_rows_before_a_bad_token(cuda, value, bad):
+    """Channel-decay recurrence: tokens of a block of four in front of one that is no number."""
+    mt = _with_bad_token(rip.make([rip.delta(heads=2, kv_heads=2, dim=128, vdim=40, ff=None)], seed=bad, slow=2.0), value)
+    tok = rip.ids(bad, seed=bad)
+    want = ripidra_oracle.run(*mt, tok)[0][:, :-1]
+    for dtype in rip.DTYPES:
+        s = rip.session(cuda, mt, dtype, max_tokens=64)
+        got = s.feed(tok + [mt[0]["vocab"] - 1] * 5, range(bad))
+        s.close()
+        assert rip.close(got[:, :-1], want, dtype), dtype
