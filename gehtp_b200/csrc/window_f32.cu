@@ -79,7 +79,8 @@ window_f32_kernel(const WindowArgs a, uint32_t rows, uint32_t hg) {
         float mn = fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, LPV));
         mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2 * LPV));
         mn = fmaxf(m, mn);
-        const float corr = m == -INFINITY ? 0.0f : expf(m - mn), e = seen ? expf(sc - mn) : 0.0f;
+        const float base = mn == -INFINITY ? 0.0f : mn;            // scores of -inf alone so far: weights of zero
+        const float corr = expf(m - base), e = expf(sc - base);
         l = l * corr + e;
         m = mn;
         const uint32_t see = __ballot_sync(0xffffffffu, seen);

@@ -4,7 +4,9 @@ import numpy as np
 import pytest
 
 import ripidra_oracle
+import supevik_oracle
 import test_ripidra as rip
+import test_supevik as sup
 
 
 def _with_bad_token(mt, value):
@@ -43,3 +45,27 @@ def test_delta_rows_before_a_bad_token(cuda, value, bad):
         got = s.feed(tok + [mt[0]["vocab"] - 1] * 5, range(bad))
         s.close()
         assert rip.close(got[:, :-1], want, dtype), dtype
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv_heads", [(6, 2), (2, 2), (8, 1)])
+def test_window_keys_with_scores_of_minus_infinity(cuda, heads, kv_heads):
+    """fp32 window attention: keys whose scores are -inf fill a warp's positions, or are the last a row sees."""
+    cfg, t = sup.make([sup.layer(heads=heads, kv_heads=kv_heads, ff=None)], seed=heads)
+    at, w, H, G = 20, 5, heads, kv_heads                          # a component the rotation leaves alone; a component of the input
+    marked = cfg["vocab"] - 1
+    t["embed"][:, w] = 0.0
+    t["embed"][marked, w] = 4.0
+    t["l0.norm1.b"][w], t["l0.norm1"][w] = 0.0, 1.0
+    q, k = (t["l0.mix." + n].reshape(r, 24, -1) for n, r in (("q", H), ("k", G)))
+    q[:, at], k[:, at], k[:, at, w] = 0.0, 0.0, -100.0            # 0 for every token but the marked one
+    t["l0.mix.q.b"].reshape(H, 24)[:, at], t["l0.mix.k.b"].reshape(G, 24)[:, at] = 1.0, 0.0
+    t["l0.mix.q.norm"][at], t["l0.mix.k.norm"][at] = 1.0, 3e38    # its key: -sqrt(24) 3e38
+    tok = [i % (marked - 1) for i in sup.ids(44, seed=2)]
+    for p in (8, 9, 10, 11, 21, 32, 33, 34, 35, 36, 37, 43):
+        tok[p] = marked
+    want = supevik_oracle.run(cfg, t, tok)[0]
+    s = sup.session(cuda, (cfg, t), "float32", max_tokens=64)
+    for cut in ([44], [9, 1, 1, 10, 23], [12, 20, 1, 1, 1, 9]):
+        assert sup.close(sup.run_cut(s, tok, cut), want, "float32"), cut
+    s.close()
