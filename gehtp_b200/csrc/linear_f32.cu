@@ -2,7 +2,9 @@
 //
 //   up to 16 rows   lin_f32_rows_kernel: weights streamed 16 bytes a lane, fp32 FMA
 //   more rows       lin_f32_mma_kernel: an fp32 value is the exact sum of three bf16 values (8 + 8 + 8 bits of its 24), so three
-//                   bf16 MMAs make the exact products of the fp32 ones; only the order of the sums differs from FMA tiles
+//                   bf16 MMAs make the exact products of the fp32 ones; only the order of the sums differs from FMA tiles.
+//                   An infinite weight has no such products (infinity times a middle part of 0): sums that come out as no
+//                   number are made again in fp32 FMA
 #include <cooperative_groups.h>
 #include "linear_epi.cuh"
 #include "mma_bf16.cuh"
@@ -122,6 +124,12 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
     lo = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
 }
 
+__device__ __noinline__ float dot_f32(const float* x, const uint16_t* w, uint32_t K) {
+    float s = 0.0f;
+    for (uint32_t k = 0; k < K; k++) s = fmaf(__ldcg(x + k), bf2f(__ldg(w + k)), s);
+    return s;
+}
+
 // A CTA of 8 warps owns a 64 x 64 tile: 2 x 2 warp tiles of 32 x 32, and the two halves of every 32-deep k step. Lane (g, t)
 // holds k = 4t .. 4t + 3 of a 16-deep step in the MMA's k slots 2t, 2t + 1, 2t + 8, 2t + 9 of both operands. The tensor core
 // adds without rounding to nearest, so its sums run over 64 k of a warp at most and are added to fp32 registers. gridDim.z CTAs
@@ -220,6 +228,9 @@ lin_f32_mma_kernel(const float* x, const uint16_t* __restrict__ w, const E epi, 
                 v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
             }
         }
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++)
+            if (isnan(v[i]) && n0 + c + i < N) v[i] = dot_f32(x + (size_t)(m0 + r) * xs, w + (size_t)(n0 + c + i) * K, K);
         epi.quad(m0 + r, n0 + c, v, N);
     }
     if (KZ > 1) cluster.sync();                                 // nobody leaves while its sums are being read

@@ -7,6 +7,10 @@ import ripidra_oracle
 import supevik_oracle
 import test_ripidra as rip
 import test_supevik as sup
+from gehtp_b200.checkpoint import bf16_to_f32, f32_to_bf16
+from gehtp_b200.rowlists import RowsEmitter
+from gehtp_b200.wtop import OP, ROWS_AUTO, Engine
+from test_f32_rows import f32_bits
 
 
 def _with_bad_token(mt, value):
@@ -69,3 +73,36 @@ def test_window_keys_with_scores_of_minus_infinity(cuda, heads, kv_heads):
     for cut in ([44], [9, 1, 1, 10, 23], [12, 20, 1, 1, 1, 9]):
         assert sup.close(sup.run_cut(s, tok, cut), want, "float32"), cut
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K,N", [(264, 66), (3072, 130)])
+def test_infinite_weights(cuda, K, N):
+    """fp32 projection: weights of +-inf against x of few and of many bits, of either sign, and zero (no number then). Bound of
+    the finite sums: every one of the K products and sums rounds by at most 2^-24 of what has been added up (2^-23 where
+    the tensor core truncates)."""
+    rng = np.random.default_rng(K)
+    scale = np.float32(1 / 3)
+    tab = bf16_to_f32(f32_to_bf16(rng.standard_normal((150, K)).astype(np.float32)))
+    tab[:, 9] = np.resize(np.float32([1.0, -2.0, 0.5, 0.0, -1.0, 2.0, -0.5, 0.0]), 150)
+    tab[::2, 9] *= 3.0                                            # times scale: one bit in every other row, all 24 in the rest
+    w = bf16_to_f32(f32_to_bf16(rng.standard_normal((N, K)).astype(np.float32)))
+    w[3, 9], w[64, 9], w[N - 1, 9], w[5, 9], w[5, K - 1] = np.inf, -np.inf, np.inf, np.inf, -np.inf
+    e = RowsEmitter("float32", 256, 150, 1)
+    t, ws = e.slot("t", lambda: f32_bits(tab)), e.slot("w", lambda: f32_bits(w))
+    e.embed(t, 150, K, scale=scale)
+    e.op(OP.LINEAR, [e.temp("x"), ws, e.temp("y"), ROWS_AUTO, K, N, 0, 0, 0, 0])
+    eng = Engine(cuda, e.finish())
+    face = np.zeros(151, np.int32)
+    face[:150] = np.arange(150)
+    x = (tab * scale).astype(np.float32).astype(np.float64)
+    with np.errstate(invalid="ignore"):
+        want, size = np.stack([(x * w[n].astype(np.float64)).sum(1) for n in range(N)], 1), np.abs(x) @ np.abs(np.where(np.isinf(w), 0, w)).T.astype(np.float64)
+    for rows in (2, 16, 17, 64, 150):
+        eng.set_rows(rows, 1)
+        eng.run_io(face, e.temp("y"), None)
+        got = eng.temp(e.temp("y"), np.float32).reshape(rows, N).astype(np.float64)
+        fine = np.isfinite(want[:rows])
+        assert np.array_equal(got[~fine], want[:rows][~fine], equal_nan=True), rows
+        assert (np.abs(got[fine] - want[:rows][fine]) <= (K + 2) * 2.0 ** -23 * size[:rows][fine]).all(), rows
+    eng.shutdown()
