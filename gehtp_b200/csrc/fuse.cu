@@ -1233,7 +1233,8 @@ void fold_constants(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb
 // of their operands (constants of the blob, see above) and what is done with a chunk's result (transposition, projection).
 // The chunks' rule then goes in two launches for all of them (gdn_scan.cu), the ops in between follow in list order.
 // Taken when no op of the run but the chunks touches a state, when every chunk reads slots, constants or temps made before
-// the run, and when the memory an op of the run writes is no chunk's operand and not another chunk's result.
+// the run, when the memory an op of the run writes is no later chunk's operand and not another chunk's result, and when no
+// chunk's result lies on what an op of the run reads.
 void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* maxb) {
     if (g.exact_ops) return;
     auto mem = [&](uint32_t t, const uint8_t*& lo, const uint8_t*& hi) { lo = t < kMaxTemps ? addr[t] : nullptr; hi = lo ? lo + maxb[t] : nullptr; return lo && maxb[t]; };
@@ -1260,14 +1261,19 @@ void fuse_delta_runs(const wt_blob* b, uint8_t* const* addr, const uint64_t* max
                 for (uint32_t o : *v)
                     for (int w = 0; w < 2; w++)
                         if (g.plan[o].out_id[w] != kNoOff && overlap(g.plan[o].out_id[w], b->ops[i].args[5])) return false;
+            // nor what an op of the run reads: a head's CTAs walk the chunks at their own pace, and one may still read an
+            // earlier chunk when another writes this result
+            auto reads = [&](uint32_t o) {
+                int ia[8];
+                const int n = input_args(b->ops[o], ia);
+                for (int k = 0; k < n; k++)
+                    if (is_temp_ref(b->ops[o].args[ia[k]]) && overlap(b->ops[o].args[ia[k]], b->ops[i].args[5])) return true;
+                return false;
+            };
             for (const auto* v : {&deltas, &others, &open_o})
-                for (uint32_t o : *v) {
-                    int ia[8];
-                    const int n = input_args(b->ops[o], ia);
-                    for (int k = 0; k < n; k++)
-                        if (is_temp_ref(b->ops[o].args[ia[k]]) && overlap(b->ops[o].args[ia[k]], b->ops[i].args[5])) return false;
-                }
-            return true;
+                for (uint32_t o : *v)
+                    if (reads(o)) return false;
+            return !reads(i);
         };
         for (uint32_t i = first; i < b->n_ops; i++) {
             const PlanOp& p = g.plan[i];

@@ -55,9 +55,9 @@ void k_rmsnorm(cudaStream_t st, const uint16_t* x, const uint16_t* g, const uint
 void k_add_rmsnorm(cudaStream_t st, const uint16_t* a, const uint16_t* r, const uint16_t* g,
                    const uint16_t* b, uint16_t* sum_out, uint16_t* y, uint32_t rows, uint32_t width);
 void k_softmax(cudaStream_t st, const uint16_t* x, uint16_t* y, uint32_t rows, uint32_t n);
-// pos_const == 0xFFFFFFFA: position = *counter, and the counter is advanced.
 // *counter = n, in stream order
 bool k_set_count(cudaStream_t st, uint32_t* counter, uint32_t n);
+// pos_const == 0xFFFFFFFA: position = *counter, and the counter is advanced.
 void k_kv_append(cudaStream_t st, const uint16_t* k, const uint16_t* v, uint16_t* ring,
                  uint32_t* posmap, uint32_t* counter, uint32_t kv_elems, uint32_t nslots,
                  uint32_t pos_const);
