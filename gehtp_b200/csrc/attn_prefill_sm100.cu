@@ -313,7 +313,6 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         const uint32_t qrow = q0 + row;
         const uint32_t lane_addr = (quarter * 32) << 16;
         const uint16_t* mrow = A.mask ? A.mask + (size_t)head * A.mask_head_stride + (size_t)min(qrow, A.seq_q - 1) * A.seq_k : nullptr;
-        const uintptr_t mask_end = (uintptr_t)(A.mask + (A.mask_head_stride ? (size_t)(A.nh - 1) * A.mask_head_stride : 0) + (size_t)A.seq_q * A.seq_k);
         const bool mvec = ((A.seq_k & 7u) == 0) && (((uintptr_t)A.mask & 15u) == 0);
         const float rscale = A.scale_div ? 1.0f / A.scale : A.scale;   // s * (1 / scale): within an fp32 step of s / scale before the fp16 rounding
         float m_run = -INFINITY, l_run = 0.0f;
@@ -336,30 +335,40 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
                 for (int q4 = 0; q4 < 8; q4++) mk[q4] = __ldg((const uint4*)(mrow + key0) + q4);
                 return;
             }
-            // Rows that start on no 16-byte boundary, or end inside the tile: nine aligned 16-byte pieces, moved into place by
+            if (mrow && mvec) {                                 // a piece lies inside the row or past its end
+#pragma unroll
+                for (uint32_t q4 = 0; q4 < 8; q4++)
+                    mk[q4] = key0 + q4 * 8 < A.seq_k ? __ldg((const uint4*)(mrow + key0) + q4) : make_uint4(0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u);
+                return;
+            }
+            // Rows that start on no 16-byte boundary: nine aligned 16-byte pieces, moved into place by
             // 8, 4 and 2 bytes. (One 2-byte load per position took 64 requests of 32 rows each, twice per tile: 16 heads x 333
             // positions 35 us a layer; now 17.) Pieces outside the mask tensor are never read.
             const uint32_t past = A.seq_k > key0 ? A.seq_k - key0 : 0;                  // positions of the tile before the end
             const uintptr_t at = (uintptr_t)(mrow + key0), lo = at & ~(uintptr_t)15;
+            const uintptr_t mask_end = (uintptr_t)(A.mask + (A.mask_head_stride ? (size_t)(A.nh - 1) * A.mask_head_stride : 0) + (size_t)A.seq_q * A.seq_k);
             if (mrow && past && lo >= (uintptr_t)A.mask && lo + 144 <= mask_end) {
-                uint32_t w[36];
-#pragma unroll
-                for (int q4 = 0; q4 < 9; q4++) {
-                    const uint4 p = __ldg((const uint4*)lo + q4);
-                    w[4 * q4] = p.x; w[4 * q4 + 1] = p.y; w[4 * q4 + 2] = p.z; w[4 * q4 + 3] = p.w;
-                }
                 const uint32_t by = (uint32_t)(at & 15);
-#pragma unroll
-                for (int i = 0; i < 34; i++) w[i] = by & 8u ? w[i + 2] : w[i];
-#pragma unroll
-                for (int i = 0; i < 33; i++) w[i] = by & 4u ? w[i + 1] : w[i];
                 uint32_t* m32 = (uint32_t*)mk;
 #pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    uint32_t x = by & 2u ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
-                    if (2u * i >= past) x = 0xFC00FC00u;                                // positions past the sequence count as masked out
-                    else if (2u * i + 1 >= past) x = (x & 0xFFFFu) | 0xFC000000u;
-                    m32[i] = x;
+                for (int h = 0; h < 2; h++) {                                           // 32 positions at a time: the registers allow no more
+                    uint32_t w[20];
+#pragma unroll
+                    for (int q4 = 0; q4 < 5; q4++) {
+                        const uint4 p = __ldg((const uint4*)lo + 4 * h + q4);
+                        w[4 * q4] = p.x; w[4 * q4 + 1] = p.y; w[4 * q4 + 2] = p.z; w[4 * q4 + 3] = p.w;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 18; i++) w[i] = by & 8u ? w[i + 2] : w[i];
+#pragma unroll
+                    for (int i = 0; i < 17; i++) w[i] = by & 4u ? w[i + 1] : w[i];
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        uint32_t x = by & 2u ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
+                        if (32u * h + 2u * i >= past) x = 0xFC00FC00u;                  // positions past the sequence count as masked out
+                        else if (32u * h + 2u * i + 1 >= past) x = (x & 0xFFFFu) | 0xFC000000u;
+                        m32[16 * h + i] = x;
+                    }
                 }
             } else {
                 uint16_t* m16 = (uint16_t*)mk;
