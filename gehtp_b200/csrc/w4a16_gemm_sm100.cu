@@ -575,9 +575,11 @@ bool launch(cudaStream_t st, const CUtensorMap& tmap, const uint32_t* packed, co
     g_launches++;
     if (S > 1 && ep.mode == 3) {
         auto add = [&](auto kernel, size_t row_bytes) { return launch_pdl(kernel, dim3(M), dim3(256), row_bytes, st, (const float*)part, y, M, N, S, ep); };
-        // every operand is 16-byte aligned here (checked at the entry); rows beyond 4096 go through shared memory
-        if ((N <= 2048 ? add(w4a16_splitk_add_rmsnorm_kernel<1, true>, 0) : N <= 4096 ? add(w4a16_splitk_add_rmsnorm_kernel<2, true>, 0)
-                       : add(w4a16_splitk_add_rmsnorm_kernel<4, false>, (size_t)N * sizeof(float))) != cudaSuccess) {
+        // Every operand is 16-byte aligned here (checked at the entry). The forms of few registers for more rows than two per SM:
+        // their CTAs come up beside the GEMM's, and fewer of them pile up on the SMs it has left. Prompt of 160 tokens (28-layer
+        // shape, 8 layers) 618 -> 599 us, of 64 511 -> 504 with the wide form; 512 rows would take two rounds in it.
+        if ((M <= 2 * sms || N > 4096 ? add(w4a16_splitk_add_rmsnorm_kernel<4, false>, (size_t)N * sizeof(float))
+                                      : N <= 2048 ? add(w4a16_splitk_add_rmsnorm_kernel<1, true>, 0) : add(w4a16_splitk_add_rmsnorm_kernel<2, true>, 0)) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
