@@ -575,9 +575,9 @@ bool launch(cudaStream_t st, const CUtensorMap& tmap, const uint32_t* packed, co
     g_launches++;
     if (S > 1 && ep.mode == 3) {
         auto add = [&](auto kernel, size_t row_bytes) { return launch_pdl(kernel, dim3(M), dim3(256), row_bytes, st, (const float*)part, y, M, N, S, ep); };
-        // Every operand is 16-byte aligned here (checked at the entry). The forms of few registers for more rows than two per SM:
-        // their CTAs come up beside the GEMM's, and fewer of them pile up on the SMs it has left. Prompt of 160 tokens (28-layer
-        // shape, 8 layers) 618 -> 599 us, of 64 511 -> 504 with the wide form; 512 rows would take two rounds in it.
+        // Every operand is 16-byte aligned here (checked at the entry). Up to two rows an SM take the form with room for 32 values a
+        // thread: CTAs of the others fit beside the GEMM's and pile up on the SMs it has left. Prompt of 160 tokens (28-layer
+        // shape, 8 layers) 618 -> 599 us, of 64 511 -> 504. More rows would take two rounds of it.
         if ((M <= 2 * sms || N > 4096 ? add(w4a16_splitk_add_rmsnorm_kernel<4, false>, (size_t)N * sizeof(float))
                                       : N <= 2048 ? add(w4a16_splitk_add_rmsnorm_kernel<1, true>, 0) : add(w4a16_splitk_add_rmsnorm_kernel<2, true>, 0)) != cudaSuccess) {
             cudaGetLastError();
@@ -620,15 +620,19 @@ bool make_a_map(CUtensorMap* tmap, const uint16_t* a, uint32_t M, uint32_t K, ui
 }
 
 // Tile and split of K: the configuration with the smallest rounds over the SMs x (k blocks of an item x kb + epi), plus, where
-// K is cut into runs, the launch that adds them (2 us and their fp32 sums written and read at 5 TB/s). kb and epi in us,
-// measured on one B200 at K 1024 .. 9728: a k block is bound by the operand bytes an SM takes in and the dequantisation, so
-// wide tiles bring more products per microsecond, and narrow ones (or 160 and 192 columns) waste less of the last round;
-// epi is what a tile costs beside its k blocks. The choice lies within 10 % of the best of 50 combinations at M 64 .. 2048.
+// K is cut into runs, the launch that adds them (1.6 us and their fp32 sums written and read at 7 TB/s). A last round that is
+// not full counts for 0.89 and its share, since fewer CTAs bring their operands in faster. More runs or a wider tile have to
+// be 3 % ahead. kb and epi in us are fitted to
+// whole prompts of 64 to 512 tokens, captured, with one projection's tile and runs changed at a time (983 of them, K 1024 ..
+// 9728, N 1024 .. 151936): alone and back to back, small launches cost other times than between the ones they depend on. A k
+// block is bound by the operand bytes an SM takes in and the dequantisation, so wide tiles bring more products per
+// microsecond, and narrow ones (or 160 and 192 columns) waste less of the last round; epi is what a tile costs beside its k
+// blocks. With 700 to 2048 rows among them the choice lies within 1.6 us a launch of the best measured in 66 of 67 cases.
 // Before (the largest tile that gave every SM one) -> now, 2048 rows: 4096 x 2560 78 -> 49 us, 9728 x 2560 168 -> 100,
 // 2560 x 6144 71 -> 63, 2560 x 151936 1451 -> 1267 (N is no multiple of 256); 64 rows: 2560 x 151936 137 -> 97.
 struct TileCost { uint32_t mh, bn; float kb, epi; };
-constexpr TileCost kTiles[] = {{1, 128, 0.347f, 1.0f}, {1, 192, 0.394f, 2.0f}, {1, 256, 0.434f, 3.5f}, {2, 128, 0.511f, 2.2f},
-                               {2, 160, 0.574f, 4.5f}, {2, 192, 0.606f, 6.0f}, {2, 256, 0.677f, 9.0f}};
+constexpr TileCost kTiles[] = {{1, 128, 0.368f, 0.7f}, {1, 192, 0.378f, 2.5f}, {1, 256, 0.410f, 3.9f}, {2, 128, 0.487f, 2.4f},
+                               {2, 160, 0.562f, 5.0f}, {2, 192, 0.582f, 6.2f}, {2, 256, 0.613f, 8.7f}};
 constexpr int kTileCount = sizeof(kTiles) / sizeof(kTiles[0]);
 
 // index into kTiles and the number of runs of K; only >= 0: that tile
@@ -645,9 +649,11 @@ int pick_tile(uint32_t M, uint32_t K, uint32_t N, uint32_t sms, int only, uint32
         for (uint32_t c = 1; c <= (split_on ? 32u : 1u) && c <= KG; c++) {
             // a run at least one trip round the longest operand ring, partial sums <= 64 MB
             if (c > 1 && (KG % c || KG / c < (uint32_t)MAX_STAGES || c * run_bytes > (double)(64u << 20))) continue;
-            float us = (float)((tiles * c + sms - 1) / sms) * ((float)(KG / c) * t.kb + t.epi);
-            if (c > 1) us += 2.0f + (float)(c * run_bytes * 2.0 / 5e6);
-            if (best_us == 0.0f || us < best_us) { best_us = us; best = i; S = c; }
+            const uint32_t items = tiles * c;
+            const float rounds = 0.89f * (float)((items + sms - 1) / sms) + 0.11f * (items > sms ? (float)items / (float)sms : 1.0f);
+            float us = rounds * ((float)(KG / c) * t.kb + t.epi);
+            if (c > 1) us += 1.6f + (float)(c * run_bytes * 2.0 / 7e6);
+            if (best_us == 0.0f || us < best_us * 0.97f) { best_us = us; best = i; S = c; }
         }
     }
     return best;
