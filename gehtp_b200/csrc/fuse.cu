@@ -893,7 +893,10 @@ void fuse_materialize(const wt_blob* b) {
                 const uint16_t* act = (const uint16_t*)resolve(b, lo.args[0]);
                 if (it != g.w4.end() && act && !lin.fused && !lin.rc && lin.launch && !lin.uses_internal && !reduced &&
                     lo.args[3] == B && N == (nh + 2 * kvh) * hd && K % 512 == 0 && K / 512 <= 10 &&
-                    N / 32 >= 120) {     // one CTA per pair of strips: worth it while nearly every SM still gets one (128 pairs: 780 -> 755 us a step of 28 layers)
+                    N / 32 >= 120) {
+                    // One CTA per pair of strips: worth it while nearly every SM still gets one. Against a launch of its own, a layer
+                    // (hidden 1024, 2560): 120 pairs 0.81, 0.66 us less at batch 1 and the same at batch 8; 128 pairs 0.85, 0.07 and
+                    // 0.43, 0.12 less; 144 pairs 0.83, 0.66 and the same; 96 pairs 0.95, 0.79 less at batch 1, 0.66, 0.31 more at 8.
                     W4Epilogue ep;
                     ep.mode = 2;
                     ep.cos_q = cq; ep.sin_q = sq; ep.cos_k = ck; ep.sin_k = sk; ep.q_out = q_out; ep.ring = ring;
