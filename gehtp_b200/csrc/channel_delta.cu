@@ -294,8 +294,8 @@ delta_scan_kernel(const DeltaArgs a, const DeltaWork wk, uint32_t rows) {
                 const float x0 = odd ? u[0][1] : u[0][0], x1 = odd ? u[1][1] : u[1][0], x2 = odd ? u[2][1] : u[2][0], x3 = odd ? u[3][1] : u[3][0];
                 const float own = hi ? (lo ? x3 : x2) : (lo ? x1 : x0);
                 // Tokens behind this one are left out, whatever their u are. Their factors n are zero: a sum that came out as no
-                // number is made again without them, or (16 lanes of 8 rows, where it costs nothing) they are not in it. With
-                // 32 lanes of 4 rows 2048 tokens of 16 heads took 447 us instead of 370 that way.
+                // number is made again without them, or (16 lanes of 8 rows, where it costs nothing) they are not in it. 2048
+                // tokens of 16 heads, 32 lanes of 4 rows: 434 us with the check, 447 with selects, 370 without either.
                 float o;
                 if (L == 16 && RPL == 8) {
                     o = fmaf(own, n.x, fmaf(mine > 2 ? x2 : 0.0f, n.w, fmaf(mine > 1 ? x1 : 0.0f, n.z, fmaf(mine > 0 ? x0 : 0.0f, n.y, e))));
@@ -608,8 +608,8 @@ void launch_scan(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32
 
 // Up to 128 channels: 32 lanes of 4 rows while CTAs of 16 columns fit one to an SM. Beyond that the SM's issue slots count, and
 // 16 lanes of 8 rows spend fewer exchanges on a token; of their two widths the one with less of a last round. 1024 tokens,
-// heads of 128 x 128, us: 16 heads 185 (16 lanes, 32 columns: 259; 16 lanes, 16 columns: 221), 32 heads 278 (259; 278),
-// 48 heads 445 (413; 355), 64 heads 549 (413; 445).
+// heads of 128 x 128, us: 16 heads 217 (16 lanes, 32 columns: 252; 16 lanes, 16 columns: 218), 32 heads 296 (253; 272),
+// 64 heads 591 (403; 441); two tokens at a time, before: 249, 263, 410.
 void launch_scan_128(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32_t rows) {
     const uint32_t n16 = (a.vdim + 15) / 16 * a.heads, n32 = (a.vdim + 31) / 32 * a.heads;
     if (a.dim % 4) launch_scan_t<32, 4, 8, false>(st, a, w, rows);
