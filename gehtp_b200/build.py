@@ -45,6 +45,7 @@ UNITS = {
     "window_prefill.cu": [],
     "window_attn_sm100.cu": [],
     "channel_delta.cu": [],
+    "channel_chunks.cu": [],
     "tp.cu": [],
     "tp_p2p.cu": [],
 }

@@ -10,6 +10,7 @@
 //   delta_step_kernel    all of it for up to 4 rows, with the second halves of the low-rank decay and gate projections
 //
 // All of it is fp32, token after token: a cut of the prompt changes nothing but roundings.
+#include <algorithm>
 #include <cooperative_groups.h>
 #include "launchers_rows.h"
 #include "mma_bf16.cuh"
@@ -630,11 +631,13 @@ void k_short_conv(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
 }
 
 size_t delta_work_floats(const DeltaArgs& a, uint32_t rows) {
-    return 2 * up4((size_t)rows * a.kv_heads * a.dim) + up4((size_t)rows * a.heads * a.dim) + (size_t)rows * a.heads * BK;
+    const size_t tokens = 2 * up4((size_t)rows * a.kv_heads * a.dim) + up4((size_t)rows * a.heads * a.dim) + (size_t)rows * a.heads * BK;
+    return std::max(tokens, delta_chunks_floats(a, rows));
 }
 
 void k_channel_delta(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
     if (!rows) return;
+    if (delta_chunks_take(a, rows)) { k_delta_chunks(st, a, rows); return; }
     const DeltaWork w = work_of(a, rows);
     if (a.bf16) launch_prep<ActBf16>(st, a, w, rows);
     else launch_prep<ActF32>(st, a, w, rows);

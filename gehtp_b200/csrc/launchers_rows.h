@@ -99,11 +99,16 @@ struct DeltaArgs {
     const float* norm_w; const float* gate; void* out; float eps; bool bf16;
     // one-kernel step: second halves of the low-rank decay and gate projections, columns of their first halves in y
     const uint16_t *a2, *g2; uint32_t rank_a, rank_g, a_col, g_col;
+    unsigned int* status;
     __host__ __device__ uint32_t channels() const { return 2 * kv_heads * dim + heads * vdim; }
 };
 void k_short_conv(cudaStream_t st, const DeltaArgs& a, uint32_t rows);
 size_t delta_work_floats(const DeltaArgs& a, uint32_t max_rows);
 void k_channel_delta(cudaStream_t st, const DeltaArgs& a, uint32_t rows);
+// the same in chunks of tokens (channel_chunks.cu), for the sizes it takes; floats of work it needs
+bool delta_chunks_take(const DeltaArgs& a, uint32_t rows);
+size_t delta_chunks_floats(const DeltaArgs& a, uint32_t max_rows);
+void k_delta_chunks(cudaStream_t st, const DeltaArgs& a, uint32_t rows);
 // all of the above for up to 4 rows in one launch, the low-rank projections included; false: sizes not taken
 bool k_delta_step(cudaStream_t st, const DeltaArgs& a, uint32_t rows);
 void k_gated_norm(cudaStream_t st, const DeltaArgs& a, uint32_t rows);

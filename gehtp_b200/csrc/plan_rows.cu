@@ -282,6 +282,7 @@ void plan_rows_op(Planner& P, const wt_op& op, PlanOp& p) {
             !temp_holds(P, a[2], mr * d.ys * (d.bf16 ? 2u : 4u))) FAIL("channel delta input too small");
         d.a_log = (const float*)P.ref(a[3]); d.dt_bias = (const float*)P.ref(a[4]);
         d.S = (float*)g.st_buf[si];
+        d.status = g.d_status;
         d.o = (float*)temp_rows(P, a[6], rows, (uint64_t)d.heads * d.vdim * 4u, p);
         d.work = (float*)P.temp_get(a[7], delta_work_floats(d, (uint32_t)mr) * 4u, p);
         if (!d.qkv || !d.a || !d.y || !d.a_log || !d.dt_bias || !d.o || !d.work) FAIL("channel delta ref fail");
