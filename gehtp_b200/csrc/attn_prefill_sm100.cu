@@ -5,26 +5,28 @@
 // fp16 before they meet V; the division by the row sum is applied to the fp32 output accumulator (the reference's
 // SOFTMAX op, oplist_exec.c:1163-1194, divides first and rounds then: a difference of rounding only).
 //
-// One CTA = one query head x 128 query rows. Key/value tiles of 128 positions; tiles whose mask is -inf
-// everywhere (upper triangle of a causal mask) are skipped. Two passes over the live tiles:
-//   pass 1  S = Q K^T per tile -> row maximum (on tiles whose mask is +0 everywhere: the maximum of the raw dot
-//           products, pushed through the roundings once per row; nothing is kept of S);
-//   pass 2  S again -> P = f16(exp(s - max)), row sum -> O += P V; O / sum at the end.
-// Recomputing S costs tensor time, which is plentiful here; it removes the rescaling of the output
-// accumulator that an online softmax needs (O stays in TMEM untouched until the end).
+// One CTA = one query head x 128 query rows. Key/value tiles of 128 positions; tiles whose mask is -inf everywhere (upper
+// triangle of a causal mask) are skipped, the others are dealt out in turn to two groups of four softmax warps, each with its
+// own S, O, row maximum and row sum. While one group works on its scores the tensor core runs the products of the other; the
+// two halves of the result are added at the end. Halving the chain of a row tile this way is what a prompt of a few hundred
+// tokens needs (64 CTAs of up to four tiles at 512 tokens and 16 heads: no CTA has a second one beside it on its SM).
 //
-// Operands: Q, K token-major (head_dim contiguous) are K-major for S = Q K^T; for O = P V the
-// contraction runs over key positions: V is read as it lies in memory ([position][head_dim]) and declared
-// an MN-major B operand (instruction descriptor bit 16; boxes of 64 positions x 64 head_dim values, see
-// umma_desc_v), and P is written by the softmax warps into shared memory in the 128-byte-swizzled K-major
-// form tcgen05.mma reads.
+//   S = Q K^T   tcgen05.mma into TMEM
+//   P           one thread per row: score roundings on half2 pairs (a scale that fp16 holds multiplies them as half2: the
+//               product of two fp16 values, rounded once, is what the fp32 product rounds to), maximum, 2^(s - m) rounded to
+//               fp16 and written over S
+//   O += P V    tcgen05.mma with P as the A operand from TMEM
+// The maximum a row is referred to is raised - and its O rescaled - only when a tile exceeds it by more than 2^8.
+// Bound by the exponentials (16 a cycle and SM) and the ALU work beside them.
 //
-//   warp 0     TMA producer: Q once, then K tiles (both passes) and V tiles (pass 2), 2-stage rings
+// Operands: Q, K token-major (head_dim contiguous) are K-major for S = Q K^T; for O = P V the contraction runs over key
+// positions: V is read as it lies in memory ([position][head_dim]) and declared an MN-major B operand (instruction
+// descriptor bit 16; boxes of 64 positions x 64 head_dim values, see umma_desc_v).
+//
+//   warp 0     TMA producer: Q once, then the K and V tiles, one buffer of each per group
 //   warp 1     one lane issues tcgen05.mma / tcgen05.commit
-//   warp 2     owns the TMEM allocation (512 columns: two S buffers, O)
-//   warps 4-11 softmax: warp w works on TMEM lanes 32 (w % 4) .. +31 (one query row per thread) and on
-//              the key columns 64 ((w - 4) / 4) .. +63 of a tile; the two warps of a row exchange their
-//              tile maxima through shared memory.
+//   warp 2     owns the TMEM allocation (512 columns: S / P and O of both groups)
+//   warps 4-11 softmax: warp w works on TMEM lanes 32 (w % 4) .. +31, one query row per thread, group (w - 4) / 4
 // Every mbarrier wait is bounded; on a timeout the CTA raises the engine's status word and winds down.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -42,13 +44,12 @@ namespace {
 constexpr int BQ = 128, BKV = 128, HD = 128, TILE_BYTES = 128 * 64 * 2;   // one 128 x 64 fp16 box
 constexpr int NTHREADS = 384;
 
+constexpr float RAISE = 8.0f;
+
 struct __align__(8) ABars {
-    uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full, p_empty, o_full;
-    uint64_t pair[4];         // the two softmax warps of a row quarter meet here (bounded, unlike bar.sync)
+    uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full, merge;
     uint32_t tmem_base, abort_flag;
     unsigned long long live, zero;   // bit kt: tile (qt, kt) has a live entry / a mask of +0 everywhere (n_kt <= 64)
-    float xmax[2][128];       // tile maxima of the two column halves of a row
-    float xsum[2][128];
 };
 
 struct SmArgs {
@@ -63,32 +64,15 @@ struct SmArgs {
     unsigned int* status;
 };
 
-__device__ __forceinline__ float round_h(float x) { return __half2float(__float2half_rn(x)); }
-__device__ __forceinline__ float score_of(float dot, float rscale, float maskv) {
-    float s = round_h(dot);
-    s = round_h(__fmul_rn(s, rscale));
-    return round_h(__fadd_rn(s, maskv));
-}
-
-// Two fp32 values -> one half2 word (low half = a) in one instruction, and back. The softmax warps are bound by
-// the ALU pipe: the score roundings run on pairs.
+// Two fp32 values -> one half2 word (low half = a) in one instruction, and back.
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     uint32_t r;
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
     return r;
 }
-__device__ __forceinline__ float2 unpack_h2(uint32_t h) { return __half22float2(*(const __half2*)&h); }
-// the scores of two neighbouring positions with the roundings of the op chain; mk = their two mask values (half2 word)
-template <bool MASKED>
-__device__ __forceinline__ float2 score2(float d0, float d1, float rscale, uint32_t mk) {
-    float2 f = unpack_h2(pack_h2(d0, d1));
-    f = unpack_h2(pack_h2(__fmul_rn(f.x, rscale), __fmul_rn(f.y, rscale)));
-    if (MASKED) {
-        const float2 m = unpack_h2(mk);
-        f = unpack_h2(pack_h2(__fadd_rn(f.x, m.x), __fadd_rn(f.y, m.y)));
-    }
-    return f;
-}
+__device__ __forceinline__ __half2 as_h2(uint32_t w) { return *(const __half2*)&w; }
+__device__ __forceinline__ uint32_t as_u32(__half2 h) { return *(const uint32_t*)&h; }
+__device__ __forceinline__ float2 unpack_h2(uint32_t h) { return __half22float2(as_h2(h)); }
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -104,32 +88,91 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+          "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+        :: "memory");
+}
+// waits for the loads in flight; the registers of the last one pass through, so that nothing reads them ahead of it
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+          "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+          "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+          "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+        :: "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};"
+        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+        " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
 }
 
-// P of one row for 64 positions: 2^(s log2e + m_off) rounded to fp16, eight 16-byte chunks; adds the unrounded values to l
-template <bool MASKED>
-__device__ __forceinline__ void probs64(uint32_t taddr, const uint4 (&mk)[8], float rscale, float m_off, float& l, uint4 (&pk)[8]) {
-    const float LOG2E = 1.4426950408889634f;
+// piece `p` of row `row` (16 bytes) in a tile of 32 rows of 16 pieces: rows of a piece and pieces of a row lie on different banks
+__device__ __forceinline__ uint32_t mask_at(uint32_t row, uint32_t p) { return row * 16 + (p ^ (row & 15)); }
+
+// the scores of 32 positions of a row from its 32 dot products, as 16 half2 words
+template <bool HALF_SCALE>
+__device__ __forceinline__ void scores32(const uint32_t (&v)[32], uint32_t* h, bool masked, const uint4* mask, uint32_t row, uint32_t piece, float rscale, uint32_t rscale2) {
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-        uint32_t v[32];
-        tmem_ld32(taddr + c * 32, v);
-        const uint32_t* m32 = (const uint32_t*)mk + c * 16;
+    for (int i = 0; i < 16; i++) {
+        uint32_t w = pack_h2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+        if (HALF_SCALE) {
+            w = as_u32(__hmul2_rn(as_h2(w), as_h2(rscale2)));
+        } else {
+            const float2 f = unpack_h2(w);
+            w = pack_h2(__fmul_rn(f.x, rscale), __fmul_rn(f.y, rscale));
+        }
+        h[i] = w;
+    }
+    if (masked) {
 #pragma unroll
-        for (int ch = 0; ch < 4; ch++) {
-            uint32_t w[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int e0 = ch * 8 + 2 * i;
-                const float2 sc = score2<MASKED>(__uint_as_float(v[e0]), __uint_as_float(v[e0 + 1]), rscale, MASKED ? m32[e0 >> 1] : 0u);
-                const float p0 = ex2(fmaf(sc.x, LOG2E, m_off)), p1 = ex2(fmaf(sc.y, LOG2E, m_off));
-                l += p0 + p1;
-                w[i] = pack_h2(p0, p1);
-            }
-            pk[c * 4 + ch] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int q = 0; q < 4; q++) {
+            const uint4 p = mask[mask_at(row, piece + q)];
+            h[4 * q] = as_u32(__hadd2_rn(as_h2(h[4 * q]), as_h2(p.x)));
+            h[4 * q + 1] = as_u32(__hadd2_rn(as_h2(h[4 * q + 1]), as_h2(p.y)));
+            h[4 * q + 2] = as_u32(__hadd2_rn(as_h2(h[4 * q + 2]), as_h2(p.z)));
+            h[4 * q + 3] = as_u32(__hadd2_rn(as_h2(h[4 * q + 3]), as_h2(p.w)));
         }
     }
+}
+
+// D[tmem] (+)= A[tmem] B[smem]
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // true: the 128 x 128 tile (qt, kt) has no live entry
@@ -167,34 +210,95 @@ __device__ __forceinline__ uint64_t umma_desc_v(uint32_t saddr) {
     return d;
 }
 
+// Mask values of 32 rows (row0 on; past the last: of the last) for the 128 positions from key0 on into shared memory, by one
+// warp. Positions past the sequence count as masked out; bytes outside the mask tensor are never read. Code that runs once
+// in a CTA costs its fetch (about 3 ns an instruction): loops stay rolled, and the function is no part of the score loop.
+__device__ __noinline__ void mask_tile(const uint16_t* mask, const uint16_t* end, uint32_t row0, uint32_t rows, uint32_t key0, uint32_t seq_k, uint4* out) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint4 none = make_uint4(0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u);
+    if (mask && (seq_k & 7u) == 0 && ((uintptr_t)mask & 15u) == 0) {
+        // pieces of 16 bytes lie inside a row or past its end; 16 lanes to a row, all requests in flight
+        const uint32_t p = lane & 15, k = key0 + 8 * p;
+#pragma unroll 1
+        for (uint32_t r = lane >> 4; r < 32; r += 2) {
+            if (k < seq_k)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(out + mask_at(r, p))), "l"(mask + (size_t)min(row0 + r, rows - 1) * seq_k + k) : "memory");
+            else
+                out[mask_at(r, p)] = none;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        return;
+    }
+    // Rows that start on no 16-byte boundary, one to a lane: five aligned pieces for 32 positions, moved into place by 8, 4 and 2
+    // bytes. (One 2-byte load per position: 16 heads x 333 positions twice the time of the layer.)
+    const uint16_t* mrow = mask ? mask + (size_t)min(row0 + lane, rows - 1) * seq_k : nullptr;
+#pragma unroll 1
+    for (uint32_t c = 0; c < 4; c++, key0 += 32) {
+        uint32_t mk[16];
+        const uint32_t past = seq_k > key0 ? seq_k - key0 : 0;                          // positions of the piece before the end
+        const uintptr_t at = (uintptr_t)(mrow + key0), lo = at & ~(uintptr_t)15;
+        if (mrow && past && lo >= (uintptr_t)mask && lo + 80 <= (uintptr_t)end) {
+            const uint32_t by = (uint32_t)(at & 15);
+            uint32_t w[20];
+#pragma unroll
+            for (int q4 = 0; q4 < 5; q4++) {
+                const uint4 p = __ldg((const uint4*)lo + q4);
+                w[4 * q4] = p.x; w[4 * q4 + 1] = p.y; w[4 * q4 + 2] = p.z; w[4 * q4 + 3] = p.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 18; i++) w[i] = by & 8u ? w[i + 2] : w[i];
+#pragma unroll
+            for (int i = 0; i < 17; i++) w[i] = by & 4u ? w[i + 1] : w[i];
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                uint32_t x = by & 2u ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
+                if (2u * i >= past) x = 0xFC00FC00u;
+                else if (2u * i + 1 >= past) x = (x & 0xFFFFu) | 0xFC000000u;
+                mk[i] = x;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const uint32_t k = key0 + 2 * i;
+                const uint32_t lo16 = k < seq_k ? (mrow ? mrow[k] : 0u) : 0xFC00u, hi16 = k + 1 < seq_k ? (mrow ? mrow[k + 1] : 0u) : 0xFC00u;
+                mk[i] = lo16 | (hi16 << 16);
+            }
+        }
+#pragma unroll
+        for (uint32_t q4 = 0; q4 < 4; q4++) out[mask_at(lane, c * 4 + q4)] = make_uint4(mk[4 * q4], mk[4 * q4 + 1], mk[4 * q4 + 2], mk[4 * q4 + 3]);
+    }
+    __syncwarp();
+}
+
+// HALF_SCALE: the scale is an fp16 value
+template <bool HALF_SCALE>
 __global__ void __launch_bounds__(NTHREADS, 1)
 attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                           const __grid_constant__ CUtensorMap tmap_v, const SmArgs A) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sQ = smem;                          // 2 boxes (head_dim halves)
-    unsigned char* sK = sQ + 2 * TILE_BYTES;           // 2 stages x 2 boxes
-    unsigned char* sV = sK + 4 * TILE_BYTES;           // 2 stages x 2 boxes (position halves)
-    unsigned char* sP = sV + 4 * TILE_BYTES;           // 2 boxes (position halves)
-    ABars* bars = (ABars*)(sP + 2 * TILE_BYTES);
+    unsigned char* sK = sQ + 2 * TILE_BYTES;           // 2 groups x 2 boxes
+    unsigned char* sV = sK + 4 * TILE_BYTES;           // 2 groups x 2 boxes (position halves)
+    unsigned char* sM = sV + 4 * TILE_BYTES;           // 2 groups x 4 warps x 32 rows x 128 mask values
+    ABars* bars = (ABars*)(sM + 4 * TILE_BYTES);
     volatile uint32_t* abort_flag = &bars->abort_flag;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t qt = gridDim.x - 1 - blockIdx.x;     // the longest rows first
-    const uint32_t head = blockIdx.y, kvhd = head / (A.nh / A.kvh);
+    const uint32_t qt = gridDim.y - 1 - blockIdx.y;     // the longest rows of all heads first
+    const uint32_t head = blockIdx.x, kvhd = head / (A.nh / A.kvh);
     const uint32_t q0 = qt * BQ;
     const uint32_t n_kt = (A.seq_k + BKV - 1) / BKV;
     const uint32_t nq64 = (A.seq_q + 63) / 64, nk64 = (A.seq_k + 63) / 64;
 
     if (threadIdx.x == 0) {
-        mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->q_full, 1); mbar_init(&bars->o_full, 1); mbar_init(&bars->merge, 8);
         for (int s = 0; s < 2; s++) {
             mbar_init(&bars->k_full[s], 1); mbar_init(&bars->k_empty[s], 1);
             mbar_init(&bars->v_full[s], 1); mbar_init(&bars->v_empty[s], 1);
-            mbar_init(&bars->s_full[s], 1); mbar_init(&bars->s_empty[s], 8);
+            mbar_init(&bars->s_full[s], 1); mbar_init(&bars->p_full[s], 4);
         }
-        mbar_init(&bars->p_full, 8); mbar_init(&bars->p_empty, 1); mbar_init(&bars->o_full, 1);
-        for (int s = 0; s < 4; s++) mbar_init(&bars->pair[s], 2);
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -202,6 +306,8 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (threadIdx.x == 32)
+        for (const CUtensorMap* map : {&tmap_q, &tmap_k, &tmap_v}) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
     if (warp == 3) {
         // which key tiles this CTA works on, read once (the tables are constants: no need to wait for the predecessor)
         unsigned long long lv = 0, zr = 0;
@@ -216,264 +322,225 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = bars->tmem_base;
-    const uint32_t tm_o = tmem + 256;
     const unsigned long long live = bars->live, zero_tiles = bars->zero;
+    const uint32_t n_live = (uint32_t)__popcll(live);   // tile number i (in order) belongs to group i % 2, as its i / 2 th
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (lane == 0 && n_live) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
             mbar_expect_tx(&bars->q_full, 2 * TILE_BYTES);
             tma_load_2d(sQ, &tmap_q, (int)(head * HD), (int)q0, &bars->q_full);
             tma_load_2d(sQ + TILE_BYTES, &tmap_q, (int)(head * HD + 64), (int)q0, &bars->q_full);
-            uint32_t ik = 0, iv = 0;
-            for (int pass = 0; pass < 2 && !*abort_flag; pass++)
-                for (uint32_t kt = 0; kt < n_kt && !*abort_flag; kt++) {
-                    if (!((live >> kt) & 1ull)) continue;
-                    {
-                        const uint32_t s = ik & 1, ph = (ik >> 1) & 1;
-                        if (!mbar_wait(&bars->k_empty[s], ph ^ 1)) { *abort_flag = 1; break; }
-                        mbar_expect_tx(&bars->k_full[s], 2 * TILE_BYTES);
-                        tma_load_2d(sK + s * 2 * TILE_BYTES, &tmap_k, (int)(kvhd * HD), (int)(kt * BKV), &bars->k_full[s]);
-                        tma_load_2d(sK + s * 2 * TILE_BYTES + TILE_BYTES, &tmap_k, (int)(kvhd * HD + 64), (int)(kt * BKV), &bars->k_full[s]);
-                        ik++;
-                    }
-                    if (pass == 1) {
-                        const uint32_t s = iv & 1, ph = (iv >> 1) & 1;
-                        if (!mbar_wait(&bars->v_empty[s], ph ^ 1)) { *abort_flag = 1; break; }
-                        mbar_expect_tx(&bars->v_full[s], 2 * TILE_BYTES);
-                        // [position half][head_dim half][64 positions x 128 bytes]
-#pragma unroll
-                        for (uint32_t b4 = 0; b4 < 4; b4++)
-                            tma_load_2d(sV + s * 2 * TILE_BYTES + b4 * (TILE_BYTES / 2), &tmap_v, (int)(kvhd * HD + (b4 & 1) * 64),
-                                        (int)(kt * BKV + (b4 >> 1) * 64), &bars->v_full[s]);
-                        iv++;
-                    }
+            unsigned long long rest = live;
+            uint32_t kn = 0, vn = 0;                    // tiles requested
+            while (vn < n_live && !*abort_flag) {
+                uint32_t kt[2];
+                const uint32_t n = min(2u, n_live - vn);
+                for (uint32_t t = 0; t < n; t++) { kt[t] = (uint32_t)__ffsll((long long)rest) - 1; rest &= rest - 1; }
+                for (uint32_t t = 0; t < n; t++) {
+                    if (!mbar_wait_or_abort(&bars->k_empty[t], ((kn >> 1) & 1) ^ 1, abort_flag)) { *abort_flag = 1; break; }
+                    mbar_expect_tx(&bars->k_full[t], 2 * TILE_BYTES);
+                    tma_load_2d(sK + t * 2 * TILE_BYTES, &tmap_k, (int)(kvhd * HD), (int)(kt[t] * BKV), &bars->k_full[t]);
+                    tma_load_2d(sK + t * 2 * TILE_BYTES + TILE_BYTES, &tmap_k, (int)(kvhd * HD + 64), (int)(kt[t] * BKV), &bars->k_full[t]);
+                    kn++;
                 }
+                for (uint32_t t = 0; t < n && !*abort_flag; t++) {
+                    if (!mbar_wait_or_abort(&bars->v_empty[t], ((vn >> 1) & 1) ^ 1, abort_flag)) { *abort_flag = 1; break; }
+                    mbar_expect_tx(&bars->v_full[t], 2 * TILE_BYTES);
+                    // [position half][head_dim half][64 positions x 128 bytes]
+#pragma unroll
+                    for (uint32_t b4 = 0; b4 < 4; b4++)
+                        tma_load_2d(sV + t * 2 * TILE_BYTES + b4 * (TILE_BYTES / 2), &tmap_v, (int)(kvhd * HD + (b4 & 1) * 64),
+                                    (int)(kt[t] * BKV + (b4 >> 1) * 64), &bars->v_full[t]);
+                    vn++;
+                }
+            }
             if (*abort_flag) {   // copies already requested must land before the CTA may go away
-                for (uint32_t j = ik > 2 ? ik - 2 : 0; j < ik; j++) mbar_wait(&bars->k_full[j & 1], (j >> 1) & 1);
-                for (uint32_t j = iv > 2 ? iv - 2 : 0; j < iv; j++) mbar_wait(&bars->v_full[j & 1], (j >> 1) & 1);
+                mbar_wait(&bars->q_full, 0);
+                for (uint32_t j = kn > 2 ? kn - 2 : 0; j < kn; j++) mbar_wait(&bars->k_full[j & 1], (j >> 1) & 1);
+                for (uint32_t j = vn > 2 ? vn - 2 : 0; j < vn; j++) mbar_wait(&bars->v_full[j & 1], (j >> 1) & 1);
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t q_base = smem_u32(sQ), k_base = smem_u32(sK), v_base = smem_u32(sV), p_base = smem_u32(sP);
-            bool ok = mbar_wait(&bars->q_full, 0);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t ik = 0, is = 0;
-            // S[buf] = Q K_tile^T : 2 head_dim halves x 4 steps of k16
-            auto issue_s = [&]() -> bool {
-                const uint32_t s = ik & 1, buf = is & 1;
-                if (!mbar_wait(&bars->k_full[s], (ik >> 1) & 1)) return false;
-                if (!mbar_wait(&bars->s_empty[buf], ((is >> 1) & 1) ^ 1)) return false;
+        if (lane == 0 && n_live) {
+            const uint32_t q_base = smem_u32(sQ), k_base = smem_u32(sK), v_base = smem_u32(sV);
+            bool ok = true;
+            auto wait = [&](uint64_t* bar, uint32_t parity) {
+                if (ok) ok = mbar_wait_or_abort(bar, parity, abort_flag);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                for (uint32_t kb = 0; kb < 2; kb++)
-#pragma unroll
-                    for (uint32_t k4 = 0; k4 < 4; k4++)
-                        umma_f16(tmem + buf * 128, umma_desc(q_base + kb * TILE_BYTES) + (uint64_t)(k4 * 2),
-                                 umma_desc(k_base + s * 2 * TILE_BYTES + kb * TILE_BYTES) + (uint64_t)(k4 * 2), idesc_f16(128), (kb | k4) ? 1u : 0u);
-                umma_commit(&bars->k_empty[s]);
-                umma_commit(&bars->s_full[buf]);
-                ik++; is++;
-                return true;
+                return ok;
             };
-            // pass 1
-            for (uint32_t kt = 0; ok && kt < n_kt && !*abort_flag; kt++) {
-                if (!((live >> kt) & 1ull)) continue;
-                ok = issue_s();
-            }
-            // pass 2: S of the next live tile is issued before P V of the current one
-            const uint32_t n_live = (uint32_t)__popcll(live);
-            if (ok && n_live && !*abort_flag) ok = issue_s();
-            for (uint32_t j = 0; ok && j < n_live && !*abort_flag; j++) {
-                if (j + 1 < n_live) ok = issue_s();
-                if (!ok) break;
-                const uint32_t s = j & 1;
-                if (!mbar_wait(&bars->v_full[s], (j >> 1) & 1) || !mbar_wait(&bars->p_full, j & 1)) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // S of tile i: 2 head_dim halves x 4 steps of k16
+            auto issue_s = [&](uint32_t i) {
+                const uint32_t t = i & 1;
+                if (!wait(&bars->k_full[t], (i >> 1) & 1)) return;
 #pragma unroll
                 for (uint32_t kb = 0; kb < 2; kb++)
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < 4; k4++)
-                        // 16 positions = two 8-position groups = 2048 bytes per step; bit 16: B is MN-major
-                        umma_f16(tm_o, umma_desc(p_base + kb * TILE_BYTES) + (uint64_t)(k4 * 2),
-                                 umma_desc_v(v_base + s * 2 * TILE_BYTES + kb * TILE_BYTES + k4 * 2048), idesc_f16(128) | (1u << 16), (j | kb | k4) ? 1u : 0u);
-                umma_commit(&bars->v_empty[s]);
-                umma_commit(&bars->p_empty);
+                        umma_f16(tmem + t * 128, umma_desc(q_base + kb * TILE_BYTES) + (uint64_t)(k4 * 2),
+                                 umma_desc(k_base + t * 2 * TILE_BYTES + kb * TILE_BYTES) + (uint64_t)(k4 * 2), idesc_f16(128), (kb | k4) ? 1u : 0u);
+                umma_commit(&bars->k_empty[t]);
+                umma_commit(&bars->s_full[t]);
+            };
+            if (wait(&bars->q_full, 0)) {
+                issue_s(0);
+                if (n_live > 1) issue_s(1);
             }
-            if (ok && !*abort_flag) umma_commit(&bars->o_full);
-            if (!ok) *abort_flag = 1;
+            for (uint32_t i = 0; ok && i < n_live; i++) {
+                const uint32_t t = i & 1, ph = (i >> 1) & 1;
+                if (!wait(&bars->v_full[t], ph) || !wait(&bars->p_full[t], ph)) break;
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++)                // 16 positions = two 8-position groups = 2048 bytes; bit 16: B is MN-major
+                    umma_f16_ta(tmem + 256 + t * 128, tmem + t * 128 + k * 8, umma_desc_v(v_base + t * 2 * TILE_BYTES + (k >> 2) * TILE_BYTES + (k & 3) * 2048),
+                                idesc_f16(128) | (1u << 16), (i > 1 || k) ? 1u : 0u);
+                umma_commit(&bars->v_empty[t]);
+                if (i + 2 < n_live) issue_s(i + 2);             // over the P just read: products run in the order they are issued
+            }
+            if (ok) umma_commit(&bars->o_full);
+            else *abort_flag = 1;
         }
     } else if (warp >= 4) {
-        // ------------------------------------------------------------ softmax and epilogue
-        const uint32_t quarter = warp & 3, half = (warp - 4) >> 2;
-        const uint32_t row = quarter * 32 + lane;              // query row of the tile = TMEM lane
-        const uint32_t qrow = q0 + row;
-        const uint32_t lane_addr = (quarter * 32) << 16;
-        const uint16_t* mrow = A.mask ? A.mask + (size_t)head * A.mask_head_stride + (size_t)min(qrow, A.seq_q - 1) * A.seq_k : nullptr;
-        const bool mvec = ((A.seq_k & 7u) == 0) && (((uintptr_t)A.mask & 15u) == 0);
+        // ------------------------------------------------------------ softmax and output: one thread per query row and group
+        const uint32_t quarter = warp & 3, t = (warp - 4) >> 2;
+        // query row of the tile = TMEM lane = quarter * 32 + lane
+        const uint32_t ts = tmem + ((quarter * 32) << 16) + t * 128, to = ts + 256;
+        const uint16_t* mask = A.mask ? A.mask + (size_t)head * A.mask_head_stride : nullptr;
+        const uint16_t* mask_end = mask + (size_t)A.seq_q * A.seq_k;
+        uint4* mbuf = (uint4*)sM + (t * 4 + quarter) * 512;    // this warp's rows of a mask tile
         const float rscale = A.scale_div ? 1.0f / A.scale : A.scale;   // s * (1 / scale): within an fp32 step of s / scale before the fp16 rounding
-        float m_run = -INFINITY, l_run = 0.0f;
-        uint32_t is = 0, pair_phase = 0;
+        const uint32_t rscale2 = pack_h2(rscale, rscale);
+        const float LOG2E = 1.4426950408889634f;
+        float m = -INFINITY;                                   // in powers of two
+        float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         bool ok = true;
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        // the two warps of a row quarter wait for each other; shared-memory writes before it are visible after it
-        auto pair_sync = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->pair[quarter]);
-            const bool done = __all_sync(0xffffffffu, mbar_wait(&bars->pair[quarter], pair_phase));
-            pair_phase ^= 1;
-            return done;
-        };
-        // mask values of this row for 64 positions from tile column c0 (requested before the scores are waited for)
-        auto mask64 = [&](uint32_t kt, uint32_t c0, uint4 (&mk)[8]) {
-            const uint32_t key0 = kt * BKV + c0;
-            if (mrow && mvec && key0 + 64 <= A.seq_k) {
+        unsigned long long rest = live;
+        for (uint32_t i = 0; i < n_live; i++) {
+            const uint32_t kt = (uint32_t)__ffsll((long long)rest) - 1;
+            rest &= rest - 1;
+            if ((i & 1) != t) continue;
+            // a tile whose mask is +0 everywhere and that lies inside the sequence needs no mask values
+            const bool masked = !((!mask || ((zero_tiles >> kt) & 1ull)) && (kt + 1) * BKV <= A.seq_k);
+            if (masked) mask_tile(mask, mask_end, q0 + quarter * 32, A.seq_q, kt * BKV, A.seq_k, mbuf);
+            ok = !__any_sync(0xffffffffu, *abort_flag != 0) && __all_sync(0xffffffffu, mbar_wait_or_abort(&bars->s_full[t], (i >> 1) & 1, abort_flag));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // scores, two to a word, over the columns already read (64 words: where P goes), and their maximum
+            __half2 mx[4] = {as_h2(0xFC00FC00u), as_h2(0xFC00FC00u), as_h2(0xFC00FC00u), as_h2(0xFC00FC00u)};
+#pragma unroll 1
+            for (uint32_t c = 0; c < 2; c++) {
+                uint32_t va[32], vb[32], h[32];
+                tmem_ld32(ts + c * 64, va);
+                tmem_ld_wait(va);
+                tmem_ld32(ts + c * 64 + 32, vb);
+                scores32<HALF_SCALE>(va, h, masked, mbuf, lane, c * 8, rscale, rscale2);
+                tmem_ld_wait(vb);
+                scores32<HALF_SCALE>(vb, h + 16, masked, mbuf, lane, c * 8 + 4, rscale, rscale2);
+                tmem_st32(ts + c * 32, h);
 #pragma unroll
-                for (int q4 = 0; q4 < 8; q4++) mk[q4] = __ldg((const uint4*)(mrow + key0) + q4);
-                return;
+                for (int e = 0; e < 32; e++) mx[e & 3] = __hmax2(mx[e & 3], as_h2(h[e]));
             }
-            if (mrow && mvec) {                                 // a piece lies inside the row or past its end
+            mx[0] = __hmax2(__hmax2(mx[0], mx[1]), __hmax2(mx[2], mx[3]));
+            const float mt = fmaxf(__low2float(mx[0]), __high2float(mx[0])) * LOG2E;
+            tmem_st_wait();
+            // s_full of this tile came after this group's products of the tile before: its O is at rest
+            const bool raise = mt > m + RAISE;
+            if (__any_sync(0xffffffffu, raise)) {
+                const float f = raise ? (m == -INFINITY ? 0.0f : ex2(m - mt)) : 1.0f;
+                if (raise) m = mt;
 #pragma unroll
-                for (uint32_t q4 = 0; q4 < 8; q4++)
-                    mk[q4] = key0 + q4 * 8 < A.seq_k ? __ldg((const uint4*)(mrow + key0) + q4) : make_uint4(0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u, 0xFC00FC00u);
-                return;
-            }
-            // Rows that start on no 16-byte boundary: nine aligned 16-byte pieces, moved into place by
-            // 8, 4 and 2 bytes. (One 2-byte load per position took 64 requests of 32 rows each, twice per tile: 16 heads x 333
-            // positions 35 us a layer; now 17.) Pieces outside the mask tensor are never read.
-            const uint32_t past = A.seq_k > key0 ? A.seq_k - key0 : 0;                  // positions of the tile before the end
-            const uintptr_t at = (uintptr_t)(mrow + key0), lo = at & ~(uintptr_t)15;
-            const uintptr_t mask_end = (uintptr_t)(A.mask + (A.mask_head_stride ? (size_t)(A.nh - 1) * A.mask_head_stride : 0) + (size_t)A.seq_q * A.seq_k);
-            if (mrow && past && lo >= (uintptr_t)A.mask && lo + 144 <= mask_end) {
-                const uint32_t by = (uint32_t)(at & 15);
-                uint32_t* m32 = (uint32_t*)mk;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {                                           // 32 positions at a time: the registers allow no more
-                    uint32_t w[20];
-#pragma unroll
-                    for (int q4 = 0; q4 < 5; q4++) {
-                        const uint4 p = __ldg((const uint4*)lo + 4 * h + q4);
-                        w[4 * q4] = p.x; w[4 * q4 + 1] = p.y; w[4 * q4 + 2] = p.z; w[4 * q4 + 3] = p.w;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 18; i++) w[i] = by & 8u ? w[i + 2] : w[i];
-#pragma unroll
-                    for (int i = 0; i < 17; i++) w[i] = by & 4u ? w[i + 1] : w[i];
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        uint32_t x = by & 2u ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
-                        if (32u * h + 2u * i >= past) x = 0xFC00FC00u;                  // positions past the sequence count as masked out
-                        else if (32u * h + 2u * i + 1 >= past) x = (x & 0xFFFFu) | 0xFC000000u;
-                        m32[16 * h + i] = x;
-                    }
-                }
-            } else {
-                uint16_t* m16 = (uint16_t*)mk;
-#pragma unroll
-                for (int i = 0; i < 64; i++) m16[i] = key0 + i < A.seq_k ? (mrow ? mrow[key0 + i] : (uint16_t)0) : (uint16_t)0xFC00u;
-            }
-        };
-        for (int pass = 0; pass < 2 && ok; pass++) {
-            uint32_t jp = 0;
-            for (uint32_t kt = 0; kt < n_kt && ok; kt++) {
-                if (!((live >> kt) & 1ull)) continue;
-                // a tile whose mask is +0 everywhere and that lies inside the sequence needs no mask values
-                const bool plain = (!mrow || ((zero_tiles >> kt) & 1ull)) && (kt + 1) * BKV <= A.seq_k;
-                uint4 mk[8];
-                if (!plain) mask64(kt, half * 64, mk);
-                const uint32_t buf = is & 1;
-                ok = !__any_sync(0xffffffffu, *abort_flag != 0);
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[buf], (is >> 1) & 1));
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (pass == 0) {
-                    // row maximum of the tile. Rounding to fp16 and a positive scale keep the order, so without a mask
-                    // the maximum of the scores is the score of the largest dot product.
-                    float mt = -INFINITY;
-#pragma unroll
-                    for (int c = 0; c < 2; c++) {
+                for (int c = 0; c < 2; c++) { l2[c].x *= f; l2[c].y *= f; }
+                if (i > 1) {
+#pragma unroll 1
+                    for (int c = 0; c < 4; c++) {
                         uint32_t v[32];
-                        tmem_ld32(tmem + lane_addr + buf * 128 + half * 64 + c * 32, v);
-                        if (plain) {
+                        tmem_ld32(to + c * 32, v);
+                        tmem_ld_wait(v);
 #pragma unroll
-                            for (int i = 0; i < 32; i++) mt = fmaxf(mt, __uint_as_float(v[i]));
-                        } else {
-                            const uint32_t* m32 = (const uint32_t*)mk + c * 16;
-#pragma unroll
-                            for (int i = 0; i < 16; i++) {
-                                const float2 sc = score2<true>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]), rscale, m32[i]);
-                                mt = fmaxf(mt, fmaxf(sc.x, sc.y));
-                            }
-                        }
+                        for (int e = 0; e < 32; e++) v[e] = __float_as_uint(__uint_as_float(v[e]) * f);
+                        tmem_st32(to + c * 32, v);
                     }
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->s_empty[buf]);
-                    if (plain) mt = score_of(mt, rscale, 0.0f);
-                    m_run = fmaxf(m_run, mt);
-                } else {
-                    if (jp == 0) {
-                        // the two column halves of a row agree on the row maximum once, before the second pass
-                        bars->xmax[half][row] = m_run;
-                        if (!pair_sync()) { ok = false; break; }
-                        m_run = fmaxf(bars->xmax[0][row], bars->xmax[1][row]);
-                    }
-                    // P of this warp's 64 columns: 8 chunks of 8 positions, 16 bytes each, swizzled by row. The values are
-                    // formed first; the buffer (still read by P V of the tile before) is waited for only then.
-                    uint4 pk[8];
-                    // exp(s - m) as 2^(s log2e - m log2e); a row with no live position (m = -inf) gives zeros through m_off = 0
-                    const float m_off = m_run == -INFINITY ? 0.0f : -m_run * 1.4426950408889634f;
-                    if (plain) probs64<false>(tmem + lane_addr + buf * 128 + half * 64, mk, rscale, m_off, l_run, pk);
-                    else probs64<true>(tmem + lane_addr + buf * 128 + half * 64, mk, rscale, m_off, l_run, pk);
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->s_empty[buf]);
-                    if (!__all_sync(0xffffffffu, mbar_wait(&bars->p_empty, (jp & 1) ^ 1))) { ok = false; break; }
-                    unsigned char* prow = sP + half * TILE_BYTES + row * 128;
-#pragma unroll
-                    for (uint32_t chunk = 0; chunk < 8; chunk++) *(uint4*)(prow + ((chunk ^ (row & 7u)) << 4)) = pk[chunk];
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->p_full);
-                    jp++;
+                    tmem_st_wait();
                 }
-                is++;
             }
+            const float off = m == -INFINITY ? 0.0f : -m;        // a row that has seen no live position yet: zeros
+#pragma unroll 1
+            for (uint32_t c = 0; c < 2; c++) {
+                uint32_t h[32];
+                tmem_ld32(ts + c * 32, h);
+                tmem_ld_wait(h);
+#pragma unroll
+                for (int e = 0; e < 32; e++) {
+                    const float2 x = fma2(unpack_h2(h[e]), make_float2(LOG2E, LOG2E), make_float2(off, off));
+                    const float2 p = make_float2(ex2(x.x), ex2(x.y));
+                    l2[e & 1] = add2(l2[e & 1], p);
+                    h[e] = pack_h2(p.x, p.y);
+                }
+                tmem_st32(ts + c * 32, h);
+            }
+            tmem_st_wait();
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->p_full[t]);
         }
-        // ---- O / row sum -> fp16 -> out; this warp stores head_dim columns 64 half .. +63 of its rows
-        float inv_l = 0.0f;
+        // ---- the two groups' halves together: every thread takes head_dim columns 64 t .. +63 of its row out of both
         if (ok) {
-            bars->xsum[half][row] = l_run;
-            ok = pair_sync();
-            const float l = bars->xsum[0][row] + bars->xsum[1][row];
-            inv_l = l > 0.0f ? 1.0f / l : 0.0f;
+            __syncwarp();                                       // the warp's mask values have been read
+            ((float2*)mbuf)[lane] = make_float2(m, (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y));      // row maximum and sum, for the other group
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->merge);
+            ok = __all_sync(0xffffffffu, mbar_wait_or_abort(&bars->merge, 0, abort_flag));
         }
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_full, 0));
+        if (ok && n_live) ok = __all_sync(0xffffffffu, mbar_wait_or_abort(&bars->o_full, 0, abort_flag));
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float2 ml0 = ((const float2*)((const uint4*)sM + quarter * 512))[lane], ml1 = ((const float2*)((const uint4*)sM + (4 + quarter) * 512))[lane];
+            const float M = fmaxf(ml0.x, ml1.x);
+            float f0 = ml0.x == -INFINITY ? 0.0f : ex2(ml0.x - M), f1 = ml1.x == -INFINITY ? 0.0f : ex2(ml1.x - M);
+            const float l = ml0.y * f0 + ml1.y * f1;
+            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+            f0 *= inv; f1 *= inv;
+            const uint32_t ta = tmem + ((quarter * 32) << 16) + 256 + t * 64;
+            // the warp's 32 rows of 128 bytes by way of shared memory: 8 lanes to a row, a request touches four (a row to a lane touched
+            // 32, 1.2 us). Q has been read by all products.
+            uint4* stage = (uint4*)sQ + (t * 4 + quarter) * 256;
 #pragma unroll 1
-            for (int c = 0; c < 2; c++) {
-                uint32_t v[32];
-                tmem_ld32(tm_o + lane_addr + half * 64 + c * 32, v);
-                if (qrow < A.seq_q) {
-                    uint4* dst = (uint4*)(A.out + ((size_t)qrow * A.nh + head) * HD + half * 64 + c * 32);
+            for (int c = 0; c < 4; c++) {
+                uint32_t v[16], u[16];
+                tmem_ld16(ta + c * 16, v);
+                tmem_ld16(ta + 128 + c * 16, u);
+                tmem_ld_wait(v);
+                tmem_ld_wait(u);
+                const bool two = n_live > 1;                     // a group without a tile has nothing in its O
+                float o[16], sum = 0.0f;
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; q4++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++)      // a row without a live position never reached the accumulator: zeros
-                            w[i] = inv_l == 0.0f ? 0u : (uint32_t)f2h(__uint_as_float(v[8 * q4 + 2 * i]) * inv_l) |
-                                                        ((uint32_t)f2h(__uint_as_float(v[8 * q4 + 2 * i + 1]) * inv_l) << 16);
-                        dst[q4] = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
+                for (int e = 0; e < 16; e++) {
+                    o[e] = __uint_as_float(v[e]) * f0;
+                    if (two) o[e] = fmaf(__uint_as_float(u[e]), f1, o[e]);
+                    if (inv == 0.0f) o[e] = 0.0f;                // a row without a live position, whatever values it would have weighed
+                    sum += o[e];
                 }
+                uint32_t w[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) w[e] = pack_h2(o[2 * e], o[2 * e + 1]);
+                if (isnan(sum)) {                                // the reference's conversion of NaN, which the instruction does not know
+#pragma unroll
+                    for (int e = 0; e < 8; e++) w[e] = (uint32_t)f2h(o[2 * e]) | ((uint32_t)f2h(o[2 * e + 1]) << 16);
+                }
+#pragma unroll
+                for (int q = 0; q < 2; q++) stage[lane * 8 + ((c * 2 + q) ^ (lane & 7))] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
             }
-        } else {
-            *abort_flag = 1;
+            __syncwarp();
+            const uint32_t p = lane & 7;
+#pragma unroll 2
+            for (uint32_t r = lane >> 3; r < 32; r += 4)
+                if (q0 + quarter * 32 + r < A.seq_q)
+                    ((uint4*)(A.out + ((size_t)(q0 + quarter * 32 + r) * A.nh + head) * HD + t * 64))[p] = stage[r * 8 + (p ^ (r & 7))];
         }
+        if (!ok) *abort_flag = 1;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -508,11 +575,14 @@ bool k_attn_prefill_sm100(cudaStream_t st, const uint16_t* q, const uint16_t* k,
     if (!make_map(&tq, q, (uint64_t)nh * hd, seq_q, (uint64_t)nh * hd) || !make_map(&tk, k, (uint64_t)kvh * hd, seq_k, (uint64_t)kvh * hd) ||
         !make_map(&tv, v, (uint64_t)kvh * hd, seq_k, (uint64_t)kvh * hd, 64))
         return false;
-    const size_t smem = 1024 + 12 * (size_t)TILE_BYTES + sizeof(ABars) + 16;
-    static int have[64] = {};
-    if (!ensure_dyn_smem(attn_prefill_sm100_kernel, smem, have)) return false;
+    const size_t smem = 1024 + 14 * (size_t)TILE_BYTES + sizeof(ABars) + 16;
+    const float rscale = scale_div ? 1.0f / scale : scale;
+    const bool half_scale = __half2float(__float2half_rn(rscale)) == rscale;
+    static int have[2][64] = {};
+    auto kernel = half_scale ? attn_prefill_sm100_kernel<true> : attn_prefill_sm100_kernel<false>;
+    if (!ensure_dyn_smem(kernel, smem, have[half_scale])) return false;
     SmArgs a{mask, mask_head_stride, skip, zero, out, seq_q, seq_k, nh, kvh, scale, scale_div, status};
-    if (launch_pdl(attn_prefill_sm100_kernel, dim3((seq_q + BQ - 1) / BQ, nh), dim3(NTHREADS), smem, st, tq, tk, tv, a) != cudaSuccess) {
+    if (launch_pdl(kernel, dim3(nh, (seq_q + BQ - 1) / BQ), dim3(NTHREADS), smem, st, tq, tk, tv, a) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
