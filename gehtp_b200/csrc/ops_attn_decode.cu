@@ -695,22 +695,19 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap, AttnDecodeArgs 
 }
 
 // out[h][d] = sum_s O_s[d] e^{m_s - m} / sum_s l_s e^{m_s - m}.
-// One CTA of 16 warps per query head. Warp w folds the slices w, w+16, ... (eight at a time, all their loads in
-// flight together) into a running (max, sum, vector) of its own; the 16 warp results are then combined in warp
-// order. Every slice of the scratch buffers is written by the split-KV kernel (an empty one as max = -inf,
-// sum = 0), so nothing here depends on the position counter and the first loads leave right after the wait.
-// MERGE_WARPS warps share the slices of one query head (8 slices in flight per warp and pass); their partial
-// results meet in shared memory. Few slices want few warps: the closing combination walks all of them.
+// One CTA per query head, or one warp (MERGE_WARPS = 1, eight to a CTA) while there are no more than eight slices. A warp takes eight neighbouring slices at a time, their vectors requested before anything else;
+// beside them every warp reads the maxima and sums of all slices, lanes along the slices, and has the common maximum and the
+// denominator to itself: warps meet once, to add their vectors. Every slice of the scratch buffers is written by the split-KV
+// kernel (an empty one as max = -inf, sum = 0), so nothing here depends on the position counter.
+// Bound by two trips to L2, the launch and the fetch of its code.
 template <int MERGE_WARPS>
-__global__ void __launch_bounds__(MERGE_WARPS * 32)
-attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* out, uint32_t rep, uint32_t hd,
+__global__ void __launch_bounds__(MERGE_WARPS == 1 ? 256 : MERGE_WARPS * 32)
+attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* out, uint32_t heads, uint32_t rep, uint32_t hd,
                          uint32_t nsplit, uint32_t* bump_counter) {
-    __shared__ float s_acc[MERGE_WARPS][128];
-    __shared__ float s_l[MERGE_WARPS];
-    __shared__ float s_m[MERGE_WARPS];
-    const uint32_t h = blockIdx.x;           // query head, = kvh * rep + r
+    __shared__ __align__(16) float s_acc[MERGE_WARPS][128];
+    const uint32_t warp = MERGE_WARPS == 1 ? 0 : threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t h = MERGE_WARPS == 1 ? min(blockIdx.x * 8 + threadIdx.x / 32, heads - 1) : blockIdx.x;      // query head, = kvh * rep + r
     const uint32_t kvh = h / rep, r = h % rep;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // The kernels behind this one start their weight loads as soon as they are allowed on an SM. They are
     // released only once the split-KV kernel has finished. Released at entry (measured on B200, batch 8,
     // context 8192), they came up beside that kernel's last CTAs, and with their loads in flight the P.V
@@ -720,60 +717,65 @@ attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* ou
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const size_t row0 = ((size_t)kvh * nsplit) * rep + r;     // slice s is at row0 + s*rep
-    const uint32_t per_lane = hd / 32;       // 4 for head_dim 128, 2 for 64
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float m_run = -INFINITY, l_run = 0.0f;
-    for (uint32_t s0 = warp; s0 < nsplit; s0 += MERGE_WARPS * 8) {
-        float ms[8], ls[8], ov[8][4];
+    const uint32_t at = lane * (hd / 32);                     // 4 values a lane for head_dim 128, 2 for 64
+    const float2* ml = (const float2*)part_ml + row0;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f}, m = -INFINITY, den = 0.0f;
+#pragma unroll 1
+    for (uint32_t s0 = warp * 8; s0 < nsplit || s0 == warp * 8; s0 += MERGE_WARPS * 8) {
+        float4 ov[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const uint32_t s = s0 + MERGE_WARPS * u;
-            const bool ok = s < nsplit;
-            const size_t base = row0 + (size_t)(ok ? s : s0) * rep;
-            ms[u] = ok ? __ldcg(part_ml + base * 2) : -INFINITY;
-            ls[u] = ok ? __ldcg(part_ml + base * 2 + 1) : 0.0f;
-            const float* po = part_o + base * hd + lane * per_lane;
-            if (per_lane == 4) {
-                float4 v = __ldcg((const float4*)po);
-                ov[u][0] = v.x; ov[u][1] = v.y; ov[u][2] = v.z; ov[u][3] = v.w;
-            } else {
-                float2 v = __ldcg((const float2*)po);
-                ov[u][0] = v.x; ov[u][1] = v.y; ov[u][2] = 0.0f; ov[u][3] = 0.0f;
+        for (uint32_t u = 0; u < 8; u++) {
+            const float* po = part_o + (row0 + (size_t)(s0 + u) * rep) * hd + at;
+            ov[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (s0 + u >= nsplit) continue;
+            if (hd == 128) ov[u] = __ldcg((const float4*)po);
+            else { const float2 v = __ldcg((const float2*)po); ov[u].x = v.x; ov[u].y = v.y; }
+        }
+        float own = -INFINITY;                                // maximum of slice s0 + lane (lanes 0 - 7)
+        if (lane < 8 && s0 + lane < nsplit) own = __ldcg(ml + (size_t)(s0 + lane) * rep).x;
+        if (s0 == warp * 8) {
+#pragma unroll 1
+            for (uint32_t b = 0; b < nsplit; b += 128) {
+                float2 v[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) {
+                    const uint32_t s = b + u * 32 + lane;
+                    v[u] = s < nsplit ? __ldcg(ml + (size_t)s * rep) : make_float2(-INFINITY, 0.0f);
+                }
+                const float m_new = fmaxf(m, warp_max(fmaxf(fmaxf(v[0].x, v[1].x), fmaxf(v[2].x, v[3].x))));
+                den *= m == -INFINITY ? 0.0f : __expf(m - m_new);
+                m = m_new;
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) den += v[u].x == -INFINITY ? 0.0f : v[u].y * __expf(v[u].x - m);
             }
+            den = warp_sum(den);
         }
-        float m_new = m_run;
+        const float w = own == -INFINITY ? 0.0f : __expf(own - m);
 #pragma unroll
-        for (int u = 0; u < 8; u++) m_new = fmaxf(m_new, ms[u]);
-        if (m_new == -INFINITY) continue;                      // nothing but empty slices so far
-        const float keep = (m_run == -INFINITY) ? 0.0f : __expf(m_run - m_new);
-        l_run *= keep;
-#pragma unroll
-        for (int k = 0; k < 4; k++) acc[k] *= keep;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (ms[u] == -INFINITY) continue;                   // empty slice: its vector may be stale memory
-            const float w = __expf(ms[u] - m_new);
-            l_run += ls[u] * w;
-#pragma unroll
-            for (int k = 0; k < 4; k++) acc[k] += ov[u][k] * w;
+        for (uint32_t u = 0; u < 8; u++) {
+            const float wu = __shfl_sync(0xffffffffu, w, u);
+            if (__shfl_sync(0xffffffffu, own, u) == -INFINITY) continue;      // empty slice: its vector may be stale memory
+            acc[0] = fmaf(ov[u].x, wu, acc[0]); acc[1] = fmaf(ov[u].y, wu, acc[1]);
+            acc[2] = fmaf(ov[u].z, wu, acc[2]); acc[3] = fmaf(ov[u].w, wu, acc[3]);
         }
-        m_run = m_new;
     }
-    for (uint32_t k = 0; k < per_lane; k++) s_acc[warp][lane * per_lane + k] = acc[k];
-    if (lane == 0) { s_l[warp] = l_run; s_m[warp] = m_run; }
-    __syncthreads();
-    if (threadIdx.x < hd) {
+    if (MERGE_WARPS == 1) {                                   // heads past the last: the last one again, the same values
+        uint16_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) o[e] = f2h(den > 0.0f ? acc[e] / den : 0.0f);
+        uint32_t* dst = (uint32_t*)(out + (size_t)h * hd + at);
+        dst[0] = o[0] | ((uint32_t)o[1] << 16);
+        if (hd == 128) dst[1] = o[2] | ((uint32_t)o[3] << 16);
+    } else {
+        if (hd == 128) *(float4*)&s_acc[warp][at] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        else *(float2*)&s_acc[warp][at] = make_float2(acc[0], acc[1]);
+        __syncthreads();
+    }
+    if (MERGE_WARPS > 1 && threadIdx.x < hd) {
         const uint32_t d = threadIdx.x;
-        float mt = -INFINITY;
+        float num = 0.0f;
 #pragma unroll
-        for (int w = 0; w < MERGE_WARPS; w++) mt = fmaxf(mt, s_m[w]);
-        float num = 0.0f, den = 0.0f;
-#pragma unroll
-        for (int w = 0; w < MERGE_WARPS; w++) {
-            const float f = (s_m[w] == -INFINITY) ? 0.0f : __expf(s_m[w] - mt);
-            num += s_acc[w][d] * f;
-            den += s_l[w] * f;
-        }
+        for (int w = 0; w < MERGE_WARPS; w++) num += s_acc[w][d];
         out[(size_t)h * hd + d] = f2h(den > 0.0f ? num / den : 0.0f);
     }
     // all readers of the counter in this launch must be done before it moves: the
@@ -914,13 +916,15 @@ bool k_attn_decode(cudaStream_t st, const AttnDecodeArgs& a, uint32_t hd, uint16
     if (!ok) { cudaGetLastError(); return false; }
     {
         static const int forced = [] { const char* e = std::getenv("GEHTP_CUDA_MERGE_WARPS"); return e ? std::atoi(e) : 0; }();
-        const int mw = forced ? forced : (a.nsplit <= 32 ? 4 : a.nsplit <= 64 ? 8 : 16);
-        const dim3 grid(kv_heads_total * a.rep);
+        // a warp a head up to eight slices, then as many warps as leave each eight
+        const int mw = forced ? forced : (a.nsplit <= 8 ? 1 : a.nsplit <= 32 ? 4 : a.nsplit <= 64 ? 8 : 16);
+        const uint32_t heads = kv_heads_total * a.rep;
         const float *po = (const float*)a.part_o, *pml = (const float*)a.part_ml;
         cudaError_t ce;
-        if (mw <= 4) ce = launch_pdl(attn_decode_merge_kernel<4>, grid, dim3(128), 0, st, po, pml, out, a.rep, hd, a.nsplit, a.bump_counter);
-        else if (mw <= 8) ce = launch_pdl(attn_decode_merge_kernel<8>, grid, dim3(256), 0, st, po, pml, out, a.rep, hd, a.nsplit, a.bump_counter);
-        else ce = launch_pdl(attn_decode_merge_kernel<16>, grid, dim3(512), 0, st, po, pml, out, a.rep, hd, a.nsplit, a.bump_counter);
+        if (mw <= 1 && ((uintptr_t)out & 3u) == 0) ce = launch_pdl(attn_decode_merge_kernel<1>, dim3((heads + 7) / 8), dim3(256), 0, st, po, pml, out, heads, a.rep, hd, a.nsplit, a.bump_counter);
+        else if (mw <= 4) ce = launch_pdl(attn_decode_merge_kernel<4>, dim3(heads), dim3(128), 0, st, po, pml, out, heads, a.rep, hd, a.nsplit, a.bump_counter);
+        else if (mw <= 8) ce = launch_pdl(attn_decode_merge_kernel<8>, dim3(heads), dim3(256), 0, st, po, pml, out, heads, a.rep, hd, a.nsplit, a.bump_counter);
+        else ce = launch_pdl(attn_decode_merge_kernel<16>, dim3(heads), dim3(512), 0, st, po, pml, out, heads, a.rep, hd, a.nsplit, a.bump_counter);
         ok = ce == cudaSuccess;
     }
     if (!ok) { cudaGetLastError(); return false; }
