@@ -2,11 +2,11 @@
 // (flags bit 1, the layout the reference's emitter gives every FullyConnected weight,
 // compiler/tools/wtop_ops/op_matmul.cpp:50):
 //
-//   M >= 128 : TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
+//   M >= 32  : TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
 //              tile of W (BN rows x 64 k) land in shared memory by cp.async.bulk.tensor with the 128-byte
 //              swizzle that tcgen05.mma reads; accumulators live in TMEM, double-buffered so that the
 //              epilogue of a tile overlaps the main loop of the next. The reference takes its matrix
-//              unit for the same shapes (exec_matmul_f16_hmx, kernels/src/runtime/oplist_exec.c:1600-1706).
+//              unit from 128 rows on (exec_matmul_f16_hmx, kernels/src/runtime/oplist_exec.c:1600-1706).
 //   M <  32  : streaming GEMV, one warp per output column, 16-byte loads along K, fp32 accumulation,
 //              shuffle reduction (exec_matmul_f16_gemv, :1483-1590).
 //
@@ -36,6 +36,7 @@ using namespace sm100;
 
 namespace {
 
+constexpr uint32_t kF16GemmRows = 32;
 constexpr int BK = 64, HALF_A_BYTES = 128 * BK * 2, NTHREADS = 384, EPI_WARPS = 8, MAX_STAGES = 6;
 
 template <int MH, int BN>
@@ -409,16 +410,21 @@ f16_gemv_nk_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* 
 // The first batch of weights (constants) is requested before the dependency wait.
 // Bound by DRAM where the matrix is large (vocabulary) and by the latency of one warp's share of K where it is small:
 // one warp per 8 columns left a projection to 1024 columns on 16 SMs.
-template <int KS, int UNR>
+// DUAL: the gate and the up matrix of a gated feed-forward in one launch, as many warps again behind each group for the
+// second matrix; y = f16(f16(g f16(sigmoid(g))) u) with g and u rounded to fp16 (and stored) as the two products round them.
+struct GemvDual { const uint16_t* w; uint16_t *gate, *up; };
+template <int KS, int UNR, bool DUAL>
 __global__ void __launch_bounds__(256)
-f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy) {
+f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, const GemvDual du) {
     extern __shared__ __align__(16) unsigned char smem_a[];      // [rows][K * 2 + 64] bytes: rows 64 bytes apart in the banks
-    __shared__ float part[KS > 1 ? 8 : 1][64];
+    __shared__ float part[KS > 1 || DUAL ? 8 : 1][64];
+    constexpr int WG = DUAL ? 2 * KS : KS;                       // warps of a group of 8 columns
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, ks = warp % KS;
-    const uint32_t m0 = blockIdx.y * 8, rows = min(8u, M - m0), n0 = (blockIdx.x * (8 / KS) + warp / KS) * 8, KC = K / 32, RS = K * 2 + 64;
+    const uint32_t m0 = blockIdx.y * 8, rows = min(8u, M - m0), n0 = (blockIdx.x * (8 / WG) + warp / WG) * 8, KC = K / 32, RS = K * 2 + 64;
     const bool active = n0 < N;
-    const uint4* wr = (const uint4*)(w + (size_t)min(n0 + g, N - 1) * K) + t;      // chunk kc lies 4 * kc further
+    const uint16_t* wm = DUAL && warp % WG >= KS ? du.w : w;
+    const uint4* wr = (const uint4*)(wm + (size_t)min(n0 + g, N - 1) * K) + t;     // chunk kc lies 4 * kc further
     uint4 wq[UNR];
 #pragma unroll
     for (int u = 0; u < UNR; u++) wq[u] = (active && ks + u * KS < KC) ? __ldcs(wr + 4 * (ks + u * KS)) : make_uint4(0, 0, 0, 0);
@@ -445,28 +451,45 @@ f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t*
 #pragma unroll
         for (int u = 0; u < UNR; u++) wq[u] = nx[u];
     }
-    if (KS > 1) {
+    const uint32_t m = m0 + g, n = n0 + 2 * t;
+    if (KS > 1 || DUAL) {
         part[warp][g * 8 + 2 * t] = acc[0];
         part[warp][g * 8 + 2 * t + 1] = acc[1];
         __syncthreads();
-        if (ks != 0) return;
+        if (warp % WG) return;
 #pragma unroll
         for (int s = 1; s < KS; s++) { acc[0] += part[warp + s][g * 8 + 2 * t]; acc[1] += part[warp + s][g * 8 + 2 * t + 1]; }
     }
-    const uint32_t m = m0 + g, n = n0 + 2 * t;
+    if (DUAL) {
+        if (m >= M) return;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            if (n + e >= N) break;
+            float u = part[warp + KS][g * 8 + 2 * t + e];
+#pragma unroll
+            for (int s = 1; s < KS; s++) u += part[warp + KS + s][g * 8 + 2 * t + e];
+            const size_t i = (size_t)m * ldy + n + e;
+            const uint16_t gh = f2h(acc[e]), uh = f2h(u);
+            const float gt = h2f(gh), sg = h2f(f2h(1.0f / (1.0f + expf(-gt))));
+            du.gate[i] = gh;
+            du.up[i] = uh;
+            y[i] = f2h(__fmul_rn(h2f(f2h(__fmul_rn(gt, sg))), h2f(uh)));
+        }
+        return;
+    }
     if (m < M) {
         if (n < N) y[(size_t)m * ldy + n] = f2h(acc[0]);
         if (n + 1 < N) y[(size_t)m * ldy + n + 1] = f2h(acc[1]);
     }
 }
 
-template <int KS>
-bool launch_gemv_mma(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy) {
+template <int KS, bool DUAL = false>
+bool launch_gemv_mma(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, const GemvDual& du = {}) {
     const size_t smem = (size_t)(M < 8 ? M : 8) * (K * 2 + 64);
     static int have[64] = {};
-    if (K % 32 || smem > 200 * 1024 || (smem > 40 * 1024 && !ensure_dyn_smem(f16_gemv_mma_kernel<KS, 8>, smem, have))) return false;
-    const uint32_t cols = 8 * (8 / KS);
-    if (launch_pdl(f16_gemv_mma_kernel<KS, 8>, dim3((N + cols - 1) / cols, (M + 7) / 8), dim3(256), smem, st, a, w, y, M, K, N, ldy) != cudaSuccess) {
+    if (K % 32 || smem > 200 * 1024 || (smem > 40 * 1024 && !ensure_dyn_smem(f16_gemv_mma_kernel<KS, 8, DUAL>, smem, have))) return false;
+    const uint32_t cols = 8 * (8 / KS) / (DUAL ? 2 : 1);
+    if (launch_pdl(f16_gemv_mma_kernel<KS, 8, DUAL>, dim3((N + cols - 1) / cols, (M + 7) / 8), dim3(256), smem, st, a, w, y, M, K, N, ldy, du) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -548,17 +571,29 @@ bool launch_tiles(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16
 
 }  // namespace
 
+// y = gated feed-forward of two matrices of one shape, M < 32; gate and up get the two products. false: not taken
+bool k_matmul_f16_swiglu(cudaStream_t st, const uint16_t* a, const uint16_t* wg, const uint16_t* wu, uint16_t* gate, uint16_t* up, uint16_t* y,
+                         uint32_t M, uint32_t K, uint32_t N) {
+    if (!M || M >= kF16GemmRows || !K || !N || (K & 31u) || ((((uintptr_t)a) | ((uintptr_t)wg) | ((uintptr_t)wu)) & 15u)) return false;
+    const GemvDual du{wu, gate, up};
+    // the shares of launch_gemv_mma_any, up to what a CTA of 8 warps has for two matrices: the same sums
+    const uint32_t KC = K / 32, groups = (N + 7) / 8;
+    if (groups >= 8 * 296 || KC < 16) return launch_gemv_mma<1, true>(st, a, wg, y, M, K, N, N, du);
+    if (groups >= 4 * 296 || KC < 32) return launch_gemv_mma<2, true>(st, a, wg, y, M, K, N, N, du);
+    return launch_gemv_mma<4, true>(st, a, wg, y, M, K, N, N, du);
+}
+
 // Y[M, N] (rows ldy apart) = A[M, K] . W^T, W stored [N, K]. false: shape or alignment outside what the
 // tensor-core forms take (the caller then runs the exact kernel); nothing launched.
 bool k_matmul_f16_nk(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N,
                      uint32_t ldy, unsigned int* status) {
     if (!M || !K || !N || (K & 7u) || ((((uintptr_t)a) | ((uintptr_t)w)) & 15u)) return false;
-    if (M < 32) {
+    if (M < kF16GemmRows) {
         static const int mma_on = [] { const char* e = std::getenv("GEHTP_CUDA_F16_GEMV_MMA"); return e ? std::atoi(e) : 1; }();
         if (mma_on && launch_gemv_mma_any(st, a, w, y, M, K, N, ldy)) return true;
         return M <= 4 ? launch_gemv<4>(st, a, w, y, M, K, N, ldy) : launch_gemv<8>(st, a, w, y, M, K, N, ldy);
     }
-    if (M < 128 || K % BK || N % 128 || (ldy & 7u) || ((uintptr_t)y & 15u)) return false;
+    if (K % BK || N % 128 || (ldy & 7u) || ((uintptr_t)y & 15u)) return false;
     return launch_tiles(st, a, K, w, EpiF16{y, ldy}, M, K, N, status);
 }
 

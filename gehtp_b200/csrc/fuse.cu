@@ -175,6 +175,7 @@ struct Span {
     // kind 5, split + rotary of a prefill block: qkv in, q_out / k_out / v_out, B = tokens
     // kind 6, SwiGLU around two GEMMs: ops gate_op and up_op keep their launches, a_ref/y as kind 1, n values
     uint32_t k_out, v_out, gate_op, up_op, gate_t, up_t;
+    bool f16;                     // kind 6: fp16 weights stored [N, K]
     std::vector<uint32_t> keep;   // ops inside the span whose outputs stay materialised (besides the last)
 };
 
@@ -456,22 +457,26 @@ bool match_qkv_split_rope(const Graph& G, const std::vector<PlanOp>& meas, uint3
     return true;
 }
 
-// The SwiGLU chain of match_swiglu with more rows than the fused GEMV form takes: the two
+// The SwiGLU chain of match_swiglu with more rows than the fused GEMV form takes, or with fp16 weights: the two
 // projections keep their own launches (GEMMs) and the three elementwise ops become one kernel.
 bool match_swiglu_tail(const Graph& G, uint32_t ip, Span& sp) {
     const wt_blob* b = G.b;
     const wt_op& pr = b->ops[ip];
     if (pr.opcode != OP_BINARY_F16 || pr.args[4] != 2) return false;
     int act = G.producer_of_arg[0][ip], up = G.producer_of_arg[1][ip];
-    if (act < 0 || up < 0 || b->ops[act].opcode != OP_BINARY_F16 || b->ops[act].args[4] != 2 || b->ops[up].opcode != OP_MATMUL_W4A16) return false;
+    if (act < 0 || up < 0 || b->ops[act].opcode != OP_BINARY_F16 || b->ops[act].args[4] != 2) return false;
+    const uint16_t proj = b->ops[up].opcode;
+    if (proj != OP_MATMUL_W4A16 && proj != OP_MATMUL_F16) return false;
     int gate = G.producer_of_arg[0][act], sig = G.producer_of_arg[1][act];
-    if (gate < 0 || sig < 0 || b->ops[gate].opcode != OP_MATMUL_W4A16 || b->ops[sig].opcode != OP_UNARY_F16 || b->ops[sig].args[3] != 8) return false;
+    if (gate < 0 || sig < 0 || b->ops[gate].opcode != proj || b->ops[sig].opcode != OP_UNARY_F16 || b->ops[sig].args[3] != 8) return false;
     if (G.producer_of_arg[0][sig] != gate) return false;
     const wt_op &gt = b->ops[gate], &u = b->ops[up];
     if (gt.args[3] != u.args[3] || gt.args[5] != u.args[5]) return false;
+    // fp16 weights: one matrix each, stored [N, K]
+    if (proj == OP_MATMUL_F16 && (gt.args[6] != 2u || u.args[6] != 2u)) return false;
     const uint64_t n64 = (uint64_t)gt.args[3] * gt.args[5];
     const uint32_t n = (uint32_t)n64;
-    if (n64 > 0xFFFFFFFFull || (gt.args[3] <= 64 && gt.args[3] < w4_gemm_min_rows()) || pr.args[3] != n || b->ops[act].args[3] != n || b->ops[sig].args[2] != n) return false;
+    if (n64 > 0xFFFFFFFFull || (proj == OP_MATMUL_W4A16 && gt.args[3] <= 64 && gt.args[3] < w4_gemm_min_rows()) || pr.args[3] != n || b->ops[act].args[3] != n || b->ops[sig].args[2] != n) return false;
     if (!is_temp_ref(gt.args[2]) || !is_temp_ref(u.args[2]) || !is_temp_ref(pr.args[2])) return false;
     std::vector<uint32_t> ops = {(uint32_t)gate, (uint32_t)sig, (uint32_t)act, (uint32_t)up, ip};
     uint32_t first;
@@ -481,7 +486,7 @@ bool match_swiglu_tail(const Graph& G, uint32_t ip, Span& sp) {
     sp.a_ref = gt.args[0]; sp.y = pr.args[2]; sp.n = n;
     // one input and one K: the pair can also run as the gate | up GEMM
     sp.M = gt.args[3]; sp.N = gt.args[5]; sp.K = (gt.args[0] == u.args[0] && gt.args[4] == u.args[4]) ? gt.args[4] : 0;
-    sp.wg = gt.args[1]; sp.wu = u.args[1];
+    sp.wg = gt.args[1]; sp.wu = u.args[1]; sp.f16 = proj == OP_MATMUL_F16;
     return true;
 }
 
@@ -666,6 +671,9 @@ const uint8_t* resolve(const wt_blob* b, uint32_t arg) {
     if (!is_temp_ref(arg)) return nullptr;
     return g.temp_dev[arg];
 }
+
+// some of the n and m elements share memory
+bool touch(const uint16_t* a, size_t n, const uint16_t* b, size_t m) { return a < b + m && b < a + n; }
 
 }  // namespace
 
@@ -920,7 +928,7 @@ void fuse_materialize(const wt_blob* b) {
                 return it == g.w4.end() ? nullptr : &it->second;
             };
             const W4Packed *wg = find(sp.wg), *wu = find(sp.wu);
-            if (!act || !y || !wg || !wu) continue;
+            if (!act || !y || !wg || !wu || touch(y, (size_t)sp.M * sp.N, act, (size_t)sp.M * sp.K)) continue;
             const uint32_t *pg = wg->packed, *pu = wu->packed;
             const uint16_t *sg = wg->scales, *su = wu->scales;
             uint32_t M = sp.M, K = sp.K, N = sp.N;
@@ -981,15 +989,28 @@ void fuse_materialize(const wt_blob* b) {
             if ((((uintptr_t)gt) | ((uintptr_t)up) | ((uintptr_t)y)) & 15u) continue;
             auto lg = pg.launch, lu = pu.launch;
             size_t n = sp.n;
-            // both projections and the elementwise tail on one tcgen05 kernel when they share input and shape
+            // the result may lie where the gate lay, whole; where it covers the gate in part, the ops stay apart
+            if (y != gt && touch(y, n, gt, n)) continue;
+            // both projections and the elementwise tail in one launch when they share input and shape, and the result does not lie
+            // on the input, which other CTAs still read
             const uint16_t* act = sp.K ? (const uint16_t*)resolve(b, sp.a_ref) : nullptr;
+            if (act && touch(y, n, act, (size_t)sp.M * sp.K)) act = nullptr;
             auto find = [&](uint32_t wref) -> const W4Packed* {
                 uint64_t key = (uint64_t)(wref & 0x7FFFu) | ((uint64_t)sp.K << 16) | ((uint64_t)sp.N << 40);
                 auto it = g.w4.find(key);
                 return it == g.w4.end() ? nullptr : &it->second;
             };
-            const W4Packed *wg = act ? find(sp.wg) : nullptr, *wu = act ? find(sp.wu) : nullptr;
-            if (wg && wu && !g.exact_ops && w4a16_gemm_sm100_swiglu_takes(sp.M, sp.K, sp.N) && !(((uintptr_t)act) & 15u)) {
+            if (sp.f16) {
+                const uint16_t *wg = act ? (const uint16_t*)resolve(b, sp.wg) : nullptr, *wu = act ? (const uint16_t*)resolve(b, sp.wu) : nullptr;
+                uint16_t *gw = (uint16_t*)gt, *uw = (uint16_t*)up;
+                const uint32_t M = sp.M, K = sp.K, N = sp.N;
+                head.fused = [=](cudaStream_t st) {
+                    if (wg && wu && !g.exact_ops && k_matmul_f16_swiglu(st, act, wg, wu, gw, uw, y, M, K, N)) return;
+                    lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n);
+                };
+            }
+            const W4Packed *wg = act && !sp.f16 ? find(sp.wg) : nullptr, *wu = act && !sp.f16 ? find(sp.wu) : nullptr;
+            if (!sp.f16 && wg && wu && !g.exact_ops && w4a16_gemm_sm100_swiglu_takes(sp.M, sp.K, sp.N) && !(((uintptr_t)act) & 15u)) {
                 const uint32_t *qg = wg->packed, *qu = wu->packed;
                 const uint16_t *sg = wg->scales, *su = wu->scales;
                 const uint32_t M = sp.M, K = sp.K, N = sp.N;
@@ -998,7 +1019,7 @@ void fuse_materialize(const wt_blob* b) {
                     if (k_w4a16_gemm_sm100_swiglu(st, act, qg, sg, qu, su, y, M, K, N, status)) return;
                     lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n);
                 };
-            } else {
+            } else if (!sp.f16) {
                 head.fused = [=](cudaStream_t st) { lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n); };
             }
         } else if (sp.kind == 4) {
