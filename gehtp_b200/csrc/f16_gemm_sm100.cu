@@ -2,12 +2,12 @@
 // (flags bit 1, the layout the reference's emitter gives every FullyConnected weight,
 // compiler/tools/wtop_ops/op_matmul.cpp:50):
 //
-//   M >= 32  : TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
+//   M >= 16  : TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
 //              tile of W (BN rows x 64 k) land in shared memory by cp.async.bulk.tensor with the 128-byte
 //              swizzle that tcgen05.mma reads; accumulators live in TMEM, double-buffered so that the
 //              epilogue of a tile overlaps the main loop of the next. The reference takes its matrix
 //              unit from 128 rows on (exec_matmul_f16_hmx, kernels/src/runtime/oplist_exec.c:1600-1706).
-//   M <  32  : streaming GEMV, one warp per output column, 16-byte loads along K, fp32 accumulation,
+//   M <  16  (and below 32 where the GEMM does not take N or K): streaming GEMV, one warp per output column, 16-byte loads along K, fp32 accumulation,
 //              shuffle reduction (exec_matmul_f16_gemv, :1483-1590).
 //
 // Sums are formed in another order than the reference's ascending-k scalar loop, so results agree with
@@ -36,7 +36,6 @@ using namespace sm100;
 
 namespace {
 
-constexpr uint32_t kF16GemmRows = 32;
 constexpr int BK = 64, HALF_A_BYTES = 128 * BK * 2, NTHREADS = 384, EPI_WARPS = 8, MAX_STAGES = 6;
 
 template <int MH, int BN>
@@ -571,10 +570,14 @@ bool launch_tiles(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16
 
 }  // namespace
 
+// From 16 rows on a round over the weights for every 8 rows costs more than the GEMM. Four layers of the 28-layer shape, four
+// steps, us, GEMV / GEMM: 9 rows 1242 / 1340, 12 rows 1288 / 1287, 16 rows 1369 / 1343, 17 rows 1690 / 1395, 31 rows 2272 / 1538.
+static bool gemm_takes(uint32_t M, uint32_t K, uint32_t N) { return M >= 16 && K % BK == 0 && N % 128 == 0; }
+
 // y = gated feed-forward of two matrices of one shape, M < 32; gate and up get the two products. false: not taken
 bool k_matmul_f16_swiglu(cudaStream_t st, const uint16_t* a, const uint16_t* wg, const uint16_t* wu, uint16_t* gate, uint16_t* up, uint16_t* y,
                          uint32_t M, uint32_t K, uint32_t N) {
-    if (!M || M >= kF16GemmRows || !K || !N || (K & 31u) || ((((uintptr_t)a) | ((uintptr_t)wg) | ((uintptr_t)wu)) & 15u)) return false;
+    if (!M || M >= 32 || gemm_takes(M, K, N) || !K || !N || (K & 31u) || ((((uintptr_t)a) | ((uintptr_t)wg) | ((uintptr_t)wu)) & 15u)) return false;
     const GemvDual du{wu, gate, up};
     // the shares of launch_gemv_mma_any, up to what a CTA of 8 warps has for two matrices: the same sums
     const uint32_t KC = K / 32, groups = (N + 7) / 8;
@@ -588,13 +591,11 @@ bool k_matmul_f16_swiglu(cudaStream_t st, const uint16_t* a, const uint16_t* wg,
 bool k_matmul_f16_nk(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N,
                      uint32_t ldy, unsigned int* status) {
     if (!M || !K || !N || (K & 7u) || ((((uintptr_t)a) | ((uintptr_t)w)) & 15u)) return false;
-    if (M < kF16GemmRows) {
-        static const int mma_on = [] { const char* e = std::getenv("GEHTP_CUDA_F16_GEMV_MMA"); return e ? std::atoi(e) : 1; }();
-        if (mma_on && launch_gemv_mma_any(st, a, w, y, M, K, N, ldy)) return true;
-        return M <= 4 ? launch_gemv<4>(st, a, w, y, M, K, N, ldy) : launch_gemv<8>(st, a, w, y, M, K, N, ldy);
-    }
-    if (K % BK || N % 128 || (ldy & 7u) || ((uintptr_t)y & 15u)) return false;
-    return launch_tiles(st, a, K, w, EpiF16{y, ldy}, M, K, N, status);
+    if (gemm_takes(M, K, N) && (ldy & 7u) == 0 && ((uintptr_t)y & 15u) == 0) return launch_tiles(st, a, K, w, EpiF16{y, ldy}, M, K, N, status);
+    if (M >= 32) return false;
+    static const int mma_on = [] { const char* e = std::getenv("GEHTP_CUDA_F16_GEMV_MMA"); return e ? std::atoi(e) : 1; }();
+    if (mma_on && launch_gemv_mma_any(st, a, w, y, M, K, N, ldy)) return true;
+    return M <= 4 ? launch_gemv<4>(st, a, w, y, M, K, N, ldy) : launch_gemv<8>(st, a, w, y, M, K, N, ldy);
 }
 
 // The same kernel on bf16 operands with the outputs of a row-count projection: any N, K a multiple of 8 (16-byte rows),
