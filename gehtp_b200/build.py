@@ -40,6 +40,7 @@ UNITS = {
     "linear_f32.cu": [],
     "latent_attn.cu": [],
     "latent_prefill.cu": [],
+    "latent_attn_sm100.cu": [],
     "window_attn.cu": [],
     "window_f32.cu": [],
     "window_prefill.cu": [],

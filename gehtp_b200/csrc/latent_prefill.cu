@@ -1,5 +1,6 @@
 // Latent attention over many rows (bf16): keys and values of every cached position are expanded by one projection of
-// the state rows (all heads' key and value up-projections side by side), then a flash kernel on mma.sync runs per head:
+// the state rows (all heads' key and value up-projections side by side), then attention per head: latent_attn_sm100.cu for heads
+// of 128 + 64 / 128, a flash kernel on mma.sync for the others:
 // 128 query rows, tiles of 64 positions by cp.async in two stages, the rotated key part read from the state row that
 // all heads share. Scores and weights are fp32; the weights enter the value product as hi + lo bf16 pairs.
 #include "launchers_rows.h"
@@ -202,6 +203,7 @@ bool k_latent_prefill(cudaStream_t st, const LatentArgs& a, uint32_t rows, uint3
     lin.x_bf16 = lin.y_bf16 = true;
     k_linear(st, lin, n_past + rows, false, a.status);
     const uint16_t* kv = (const uint16_t*)a.work;
+    if (k_latent_sm100(st, a, kv, rows, n_past)) return true;
     const bool vec = a.dim % 8 == 0 && a.rot % 8 == 0 && a.vdim % 8 == 0 && a.rank % 8 == 0;
     const uint32_t vt = (a.vdim + 15) / 16 * 2;
     if (vec) {

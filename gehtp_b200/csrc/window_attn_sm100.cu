@@ -22,7 +22,7 @@
 #include <cuda_runtime.h>
 #include "launchers_rows.h"
 #include "rows_common.cuh"
-#include "sm100_umma.cuh"
+#include "sm100_attn.cuh"
 
 namespace gehtp {
 
@@ -39,116 +39,6 @@ struct __align__(8) WBars {
     uint32_t tmem_base, abort_flag;
 };
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-// waits for the loads in flight; the registers of the last one pass through, so that nothing reads them ahead of it
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-          "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
-          "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
-          "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
-        :: "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};"
-        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// two fp32 operations in one instruction
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
-        " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 d, a, b;\n mov.b64 {%0, %1}, d;\n}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-
-// bit i: column c0 + i lies in [lo, hi]
-__device__ __forceinline__ uint32_t visible32(int c0, int lo, int hi) {
-    const int a = lo - c0, b = hi - c0;
-    const uint32_t from = a <= 0 ? 0xFFFFFFFFu : a > 31 ? 0u : 0xFFFFFFFFu << a, to = b < 0 ? 0u : b >= 31 ? 0xFFFFFFFFu : 0xFFFFFFFFu >> (31 - b);
-    return from & to;
-}
-
-// largest of 32 scores, EDGE: of those whose bit is set
-template <bool EDGE>
-__device__ __forceinline__ float max32(const uint32_t (&v)[32], uint32_t see) {
-    float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-    for (int i = 0; i < 32; i++) m[i & 3] = fmaxf(m[i & 3], !EDGE || ((see >> i) & 1u) ? __uint_as_float(v[i]) : -INFINITY);
-    return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
-}
-
-// 2^(s sc + off) of 32 scores (EDGE: 0 where the bit is not set), as 16 words of hi and 16 of lo bf16 pairs; adds the
-// values to l
-template <bool EDGE>
-__device__ __forceinline__ void probs32(const uint32_t (&v)[32], uint32_t (&w)[32], float sc, float off, uint32_t see, float2 (&l)[2]) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const float2 x = fma2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(sc, sc), make_float2(off, off));
-        float2 e = make_float2(ex2(x.x), ex2(x.y));
-        if (EDGE) {
-            e.x = (see >> (2 * i)) & 1u ? e.x : 0.0f;
-            e.y = (see >> (2 * i + 1)) & 1u ? e.y : 0.0f;
-        }
-        l[i & 1] = add2(l[i & 1], e);
-        const uint32_t p = pack_bf2(e.x, e.y);
-        w[i] = p;
-        const float2 r = fma2(make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)), make_float2(-1.0f, -1.0f), e);
-        w[16 + i] = pack_bf2(r.x, r.y);
-    }
-}
-
-// D[tmem] (+)= A[tmem] B[smem]
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// B operand of a value tile as it lies in memory ([position][value], value contiguous): boxes of 64 positions x 64 values
-// with the 128-byte swizzle, 8-position groups 1024 bytes apart, the second 64 values one box further
-__device__ __forceinline__ uint64_t umma_desc_v(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)(BOX >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-constexpr uint32_t IDESC_BF16 = (1u << 7) | (1u << 10);          // A and B are bf16
 
 // DB, VB: key and value size in units of 64
 template <int DB, int VB>
