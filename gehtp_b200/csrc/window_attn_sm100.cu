@@ -184,33 +184,43 @@ window_attn_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         const uint32_t pos = past + qrow, w_first = pos - lane, w_last = w_first + 31;
         const uint32_t ts = tmem + ((quarter * 32) << 16) + t * 128, to = ts + 256;
         const float sc = A.scale * 1.44269504088896340736f;      // scores in powers of two
+        const bool gate = A.gate_col != 0xFFFFFFFFu;
+        const uint32_t first_row = q0 + (by_head ? 0 : t * BQ) + quarter * 32;
+        constexpr bool GATES_AHEAD = DB >= VB;                   // a Q tile has room for the gates of its rows
+        uint4* gates = (uint4*)(sQ + t * Q_BYTES) + quarter * (32 * VB * 8);
         float m = -INFINITY;
         float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         bool ok = true;
         asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll 1
         for (uint32_t j = 0; j < n_kt; j++) {
             ok = !__any_sync(0xffffffffu, *abort_flag != 0) && __all_sync(0xffffffffu, mbar_wait_or_abort(&bars->s_full[t], j & 1, abort_flag));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (GATES_AHEAD && gate && j + 1 == n_kt) {          // every product of this Q tile is done: the gates come in over it
+#pragma unroll 1
+                for (uint32_t i = lane; i < 32 * VB * 8; i += 32) {
+                    const uint32_t r = i / (VB * 8), p = i % (VB * 8);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(gates + i)),
+                                 "l"((const uint4*)((const uint16_t*)A.y + (size_t)min(first_row + r, rows - 1) * A.y_cols + A.gate_col + h * (VB * 64)) + p) : "memory");
+                }
+            }
             const uint32_t j0 = (kt0 + j) * BKV;
             const bool edge = j0 + BKV - 1 > w_first || j0 + A.window <= w_last;      // some key of the tile is hidden from some row
             // columns [lo, hi] of the tile are visible to this row
             const int hi = (int)(pos - j0), lo = (int)(pos + 1 - A.window - j0);
-            // the next 32 columns are on their way while 32 are worked on
-            uint32_t va[32], vb[32];
-            auto largest = [&](const uint32_t (&v)[32], int c) { return edge ? max32<true>(v, visible32(c * 32, lo, hi)) : max32<false>(v, 0u); };
-            tmem_ld32(ts, va);
-            tmem_ld_wait(va);
-            tmem_ld32(ts + 32, vb);
-            float mt = largest(va, 0);
-            tmem_ld_wait(vb);
-            tmem_ld32(ts + 64, va);
-            mt = fmaxf(mt, largest(vb, 1));
-            tmem_ld_wait(va);
-            tmem_ld32(ts + 96, vb);
-            mt = fmaxf(mt, largest(va, 2));
-            tmem_ld_wait(vb);
-            mt = fmaxf(mt, largest(vb, 3)) * sc;
+            float mt = -INFINITY;
+#pragma unroll 1
+            for (int c = 0; c < 2; c++) {
+                uint32_t va[32], vb[32];
+                tmem_ld32(ts + c * 64, va);
+                tmem_ld32(ts + c * 64 + 32, vb);
+                tmem_ld_wait(va);
+                tmem_ld_wait(vb);
+                if (edge) mt = fmaxf(mt, fmaxf(max32<true>(va, visible32(c * 64, lo, hi)), max32<true>(vb, visible32(c * 64 + 32, lo, hi))));
+                else mt = fmaxf(mt, fmaxf(max32<false>(va, 0u), max32<false>(vb, 0u)));
+            }
+            mt *= sc;
             // s_full of this tile came after the products of the tile before: O is at rest
             const bool raise = mt > m + kRaise;
             if (__any_sync(0xffffffffu, raise)) {
@@ -232,59 +242,61 @@ window_attn_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 }
             }
             const float off = m == -INFINITY ? 0.0f : -m;        // a row that has seen no key yet: zeros
-            auto weigh = [&](const uint32_t (&v)[32], int c) {
-                uint32_t w[32];
-                if (edge) probs32<true>(v, w, sc, off, visible32(c * 32, lo, hi), l2);
-                else probs32<false>(v, w, sc, off, 0u, l2);
-                tmem_st32(ts + c * 32, w);
-            };
-            tmem_ld32(ts, va);
-            tmem_ld_wait(va);
-            tmem_ld32(ts + 32, vb);
-            weigh(va, 0);
-            tmem_ld_wait(vb);
-            tmem_ld32(ts + 64, va);
-            weigh(vb, 1);
-            tmem_ld_wait(va);
-            tmem_ld32(ts + 96, vb);
-            weigh(va, 2);
-            tmem_ld_wait(vb);
-            weigh(vb, 3);
+#pragma unroll 1
+            for (int c = 0; c < 2; c++) {
+                uint32_t va[32], vb[32], w[32];
+                tmem_ld32(ts + c * 64, va);
+                tmem_ld_wait(va);
+                tmem_ld32(ts + c * 64 + 32, vb);
+                if (edge) probs32<true>(va, w, sc, off, visible32(c * 64, lo, hi), l2);
+                else probs32<false>(va, w, sc, off, 0u, l2);
+                tmem_st32(ts + c * 64, w);
+                tmem_ld_wait(vb);
+                if (edge) probs32<true>(vb, w, sc, off, visible32(c * 64 + 32, lo, hi), l2);
+                else probs32<false>(vb, w, sc, off, 0u, l2);
+                tmem_st32(ts + c * 64 + 32, w);
+            }
             tmem_st_wait();
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->p_full[t]);
         }
-        // the gates come in while the last products run
-        const bool gate = A.gate_col != 0xFFFFFFFFu, live = qrow < rows;
-        const uint4* yg = (const uint4*)((const uint16_t*)A.y + (size_t)qrow * A.y_cols + A.gate_col + h * (VB * 64));
-        uint4 g[VB * 8];
-#pragma unroll
-        for (int q = 0; q < VB * 8; q++) g[q] = live && gate ? __ldcg(yg + q) : make_uint4(0, 0, 0, 0);
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait_or_abort(&bars->o_full, 0, abort_flag));
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float inv = 1.0f / ((l2[0].x + l2[0].y) + (l2[1].x + l2[1].y));
-            uint4* out = (uint4*)((uint16_t*)A.out + ((size_t)qrow * A.heads + h) * (VB * 64));
-#pragma unroll
-            for (int c = 0; c < VB * 2; c++) {
+            // The warp's 32 rows by way of shared memory (every operand has been read), so that requests for gates and results
+            // touch whole rows; loops stay rolled, since code that runs once a CTA costs its fetch.
+            constexpr uint32_t CH = VB * 16;                     // pieces of 4 values a row
+            float4* stage = (float4*)(GATES_AHEAD ? sK : sQ) + (warp - 4) * (32 * CH);
+#pragma unroll 1
+            for (uint32_t c = 0; c < VB * 2; c++) {
                 uint32_t v[32];
                 tmem_ld32(to + c * 32, v);
                 tmem_ld_wait(v);
-                if (!live) continue;
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const uint4 gq = g[c * 4 + q];
-                    const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
-                    uint32_t w[4];
+                for (uint32_t q = 0; q < 8; q++)
+                    stage[lane * CH + ((c * 8 + q) ^ (lane & 7))] = make_float4(__uint_as_float(v[4 * q]) * inv, __uint_as_float(v[4 * q + 1]) * inv,
+                                                                               __uint_as_float(v[4 * q + 2]) * inv, __uint_as_float(v[4 * q + 3]) * inv);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+#pragma unroll 2
+            for (uint32_t i = lane; i < 32 * CH / 2; i += 32) {
+                const uint32_t r = i / (CH / 2), p = i % (CH / 2), gr = first_row + r;
+                if (gr >= rows) continue;
+                const float4 a = stage[r * CH + ((2 * p) ^ (r & 7))], b = stage[r * CH + ((2 * p + 1) ^ (r & 7))];
+                float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                if (gate) {
+                    const uint4 g = GATES_AHEAD ? gates[i] : __ldcg((const uint4*)((const uint16_t*)A.y + (size_t)gr * A.y_cols + A.gate_col + h * (VB * 64)) + p);
+                    const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        float a = __uint_as_float(v[8 * q + 2 * i]) * inv, b = __uint_as_float(v[8 * q + 2 * i + 1]) * inv;
-                        if (gate) { a *= sigmoid_fast(__uint_as_float(gw[i] << 16)); b *= sigmoid_fast(__uint_as_float(gw[i] & 0xffff0000u)); }
-                        w[i] = pack_bf2(a, b);
+                    for (int e = 0; e < 4; e++) {
+                        x[2 * e] *= sigmoid_fast(__uint_as_float(gw[e] << 16));
+                        x[2 * e + 1] *= sigmoid_fast(__uint_as_float(gw[e] & 0xffff0000u));
                     }
-                    out[c * 4 + q] = make_uint4(w[0], w[1], w[2], w[3]);
                 }
+                ((uint4*)((uint16_t*)A.out + ((size_t)gr * A.heads + h) * (VB * 64)))[p] = make_uint4(pack_bf2(x[0], x[1]), pack_bf2(x[2], x[3]), pack_bf2(x[4], x[5]), pack_bf2(x[6], x[7]));
             }
         } else {
             *abort_flag = 1;
