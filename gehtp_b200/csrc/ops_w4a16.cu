@@ -421,6 +421,110 @@ bool k_w4a16_skinny_qkv_rope(cudaStream_t st, const uint16_t* a, const uint32_t*
     return true;
 }
 
+// Gate and up of up to 8 rows where there are more strips than CTAs fit the GPU: CTAs stay and walk the strips blockIdx.x,
+// + gridDim.x, ... Every register slot is refilled with the next strip's group as soon as its own has been used, so that
+// requests stay in flight across the reduction of a strip, and a warp's activations are staged once. Same sums as WALK_ONE:
+// the warp's GW groups of 64, then the warps in order. 8 rows, 2560 x 9728 (608 strips, two CTAs an SM: a third round of 16
+// CTAs before): 11.9 -> 8.4 us a launch. (The vocabulary projection the same way, 9496 strips of one matrix: 52 us for 51;
+// scales through shared memory instead of registers: 9.0 and 60.)
+template <int GW>
+__global__ void __launch_bounds__(640)
+w4a16_swiglu_strips_kernel(const uint16_t* __restrict__ a, const uint4* __restrict__ wg, const uint16_t* __restrict__ sg, const uint4* __restrict__ wu,
+                           const uint16_t* __restrict__ su, uint16_t* __restrict__ y, uint32_t M, uint32_t K, uint32_t N) {
+    extern __shared__ __align__(16) float red[];  // [2][nwarps][8][32], then the activations [nwarps][GW][rows][144 B]
+    constexpr uint32_t AROW = 144;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t NB = N / 16, kg0 = warp * GW, wstride = NB * 512u, sstride = N * 2u;      // bytes per k group
+    const char *wl = (const char*)(wg + (size_t)kg0 * NB * 32 + lane), *wl2 = (const char*)(wu + (size_t)kg0 * NB * 32 + lane);
+    const char *sl = (const char*)(sg + (size_t)kg0 * N + g), *sl2 = (const char*)(su + (size_t)kg0 * N + g);
+    uint4 wq[GW], wq2[GW];
+    uint16_t s0[GW], s1[GW], t0[GW], t1[GW];
+    auto fetch = [&](int u, uint32_t nb) {
+        const uint32_t wo = u * wstride + nb * 512u, so = u * sstride + nb * 32u;
+        wq[u] = __ldcs((const uint4*)(wl + wo));
+        s0[u] = __ldg((const uint16_t*)(sl + so));
+        s1[u] = __ldg((const uint16_t*)(sl + so) + 8);
+        wq2[u] = __ldcs((const uint4*)(wl2 + wo));
+        t0[u] = __ldg((const uint16_t*)(sl2 + so));
+        t1[u] = __ldg((const uint16_t*)(sl2 + so) + 8);
+    };
+#pragma unroll
+    for (int u = 0; u < GW; u++) fetch(u, blockIdx.x);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    unsigned char* stage = (unsigned char*)(red + 2 * nwarps * 8 * 32) + (size_t)warp * GW * M * AROW;
+    for (uint32_t c = lane; c < GW * M * 8; c += 32) {
+        const uint32_t col = c & 7, u = (c >> 3) / M, r = (c >> 3) % M;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + (c >> 3) * AROW + col * 16);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(a + (size_t)r * K + (size_t)(kg0 + u) * 64 + col * 8) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    const unsigned char* arow = stage + min(g, M - 1) * AROW + t * 32;        // rows past M read the last; never stored
+    uint32_t flip = 0;
+    for (uint32_t nb = blockIdx.x; nb < NB; nb += gridDim.x, flip ^= 1) {
+        const uint32_t next = nb + gridDim.x;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int u = 0; u < GW; u++) {
+            const uint4 b0 = *(const uint4*)(arow + u * M * AROW), b1 = *(const uint4*)(arow + u * M * AROW + 16);
+            uint32_t af[4][4];
+            dequant_word(wq[u].x, af[0]); dequant_word(wq[u].y, af[1]); dequant_word(wq[u].z, af[2]); dequant_word(wq[u].w, af[3]);
+            mma_group(acc, af, b0, b1, h2f(s0[u]), h2f(s1[u]));
+            dequant_word(wq2[u].x, af[0]); dequant_word(wq2[u].y, af[1]); dequant_word(wq2[u].z, af[2]); dequant_word(wq2[u].w, af[3]);
+            mma_group(acc2, af, b0, b1, h2f(t0[u]), h2f(t1[u]));
+            if (next < NB) fetch(u, next);
+        }
+        float* rd = red + flip * nwarps * 8 * 32;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            rd[(warp * 8 + c) * 32 + lane] = acc[c];
+            rd[(warp * 8 + 4 + c) * 32 + lane] = acc2[c];
+        }
+        __syncthreads();                                // this half is read until the barrier after next
+        for (uint32_t idx = threadIdx.x; idx < 4 * 32; idx += blockDim.x) {
+            float s = 0.0f, s2 = 0.0f;
+            for (uint32_t w = 0; w < nwarps; w++) {
+                s += rd[w * 8 * 32 + idx];
+                s2 += rd[w * 8 * 32 + 4 * 32 + idx];
+            }
+            const uint32_t ln = idx & 31, c = idx >> 5, n = nb * 16 + (ln >> 2) + ((c & 2) ? 8 : 0), m = (ln & 3) * 2 + (c & 1);
+            if (m < M) y[(size_t)m * N + n] = swiglu_chain(s, s2);
+        }
+    }
+}
+
+// false: the strips fit beside one another, or a size the kernel does not take; nothing launched
+template <int GW>
+static bool launch_swiglu_strips(cudaStream_t st, const uint16_t* a, const uint32_t* pg, const uint16_t* sg, const uint32_t* pu, const uint16_t* su,
+                                 uint16_t* y, uint32_t M, uint32_t K, uint32_t N) {
+    const uint32_t nwarps = K / 64 / GW, threads = nwarps * 32;
+    if (M > 8 || K % (64 * GW) || nwarps > 20 || (uint64_t)K * N / 2 > 0xFFFFFFFFull || ((uintptr_t)a & 15u)) return false;
+    const size_t smem = (size_t)nwarps * (2 * 8 * 32 * sizeof(float) + GW * M * 144);
+    static int have[64], sms[64], per_sm[64][21][9];
+    int dev = 0;
+    if (smem > 200 * 1024 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    if (!ensure_dyn_smem(w4a16_swiglu_strips_kernel<GW>, 200 * 1024, have)) return false;
+    int fit = per_sm[dev][nwarps][M];
+    if (!fit) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, w4a16_swiglu_strips_kernel<GW>, (int)threads, smem) != cudaSuccess || fit < 1) {
+            cudaGetLastError();
+            return false;
+        }
+        sms[dev] = n;
+        per_sm[dev][nwarps][M] = fit;
+    }
+    const uint32_t grid = (uint32_t)(fit * sms[dev]);
+    if (N / 16 <= grid) return false;
+    if (launch_pdl(w4a16_swiglu_strips_kernel<GW>, dim3(grid), dim3(threads), smem, st, a, (const uint4*)pg, sg, (const uint4*)pu, su, y, M, K, N) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 // y = swiglu(a.Wg, a.Wu): two weight matrices of the same shape in one pass.
 void k_w4a16_skinny_swiglu(cudaStream_t st, const uint16_t* a, const uint32_t* pg, const uint16_t* sg,
                            const uint32_t* pu, const uint16_t* su, uint16_t* y, uint32_t M, uint32_t K,
@@ -434,7 +538,8 @@ void k_w4a16_skinny_swiglu(cudaStream_t st, const uint16_t* a, const uint32_t* p
         if (KG % 4 == 0 && KG / 4 <= 20) {   // whole 4-group warps: the branch-free variant
             kgw = 4;
             nwarps = KG / 4;
-            launch_skinny1<4, true, WALK_ONE, false>(grid, dim3(nwarps * 32), M, st, SKINNY_ARGS(pg, sg, pu, su));
+            if (!launch_swiglu_strips<4>(st, a, pg, sg, pu, su, y, M, K, N))
+                launch_skinny1<4, true, WALK_ONE, false>(grid, dim3(nwarps * 32), M, st, SKINNY_ARGS(pg, sg, pu, su));
         } else {
             launch_skinny1<4, true, WALK_ANY, false>(grid, dim3(nwarps * 32), M, st, SKINNY_ARGS(pg, sg, pu, su));
         }
