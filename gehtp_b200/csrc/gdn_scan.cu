@@ -67,14 +67,10 @@ delta_chunks_kernel(const DeltaChunk* __restrict__ chunks, unsigned char* scratc
     if (tid < 3 * C) ((float*)(item + 3 * MAT * 2))[tid] = vec[tid];
 }
 
-// A fragment (16 rows x 16 k) and B fragment (8 rows x 16 k) of row-major shared-memory operands
-__device__ __forceinline__ void frag_a(uint32_t (&a)[4], const uint16_t* A, int ld, int k0, int g, int t) {
-    const uint16_t *lo = A + g * ld + k0 + 2 * t, *hi = lo + 8 * ld;
-    a[0] = *(const uint32_t*)lo; a[1] = *(const uint32_t*)hi; a[2] = *(const uint32_t*)(lo + 8); a[3] = *(const uint32_t*)(hi + 8);
-}
-__device__ __forceinline__ void frag_b(uint32_t (&b)[2], const uint16_t* B, int ld, int k0, int g, int t) {
-    const uint16_t* p = B + g * ld + k0 + 2 * t;
-    b[0] = *(const uint32_t*)p; b[1] = *(const uint32_t*)(p + 8);
+__device__ __forceinline__ uint32_t smem_of(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// four 8 x 8 tiles of a row-major operand, one row address per lane
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
 template <int D>
@@ -102,9 +98,12 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
     const float scale = q_raw ? 1.0f : 1.0f / sqrtf((float)D);
     float* Sglob = Sg + ((size_t)h * D + m0) * D;
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The operands' addresses are read a chunk before they are used: read where they are needed, each chunk waited for them once
+    // for its copies and once for its result.
+    DeltaChunk ck = chunks[0];
+    uint16_t* y_next = ck.y;
     auto fetch = [&](int ch) {
         ScanBuf<D>& b = sm.buf[ch & 1];
-        const DeltaChunk ck = chunks[ch];
         const size_t off = (size_t)h * ntok * D;
 #pragma unroll
         for (int u = 0; u < C * (D / 8) / 256; u++) {
@@ -123,6 +122,7 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
         if (tid < 128) cp_async16(b.V + (tid >> 1) * VP + (tid & 1) * 8, ck.v + off + (size_t)(tid >> 1) * D + m0 + (tid & 1) * 8);
         else if (tid < 128 + 3 * C / 4) cp_async16(b.vec + (tid - 128) * 4, item + 3 * MAT * 2 + (size_t)(tid - 128) * 16);
         asm volatile("cp.async.commit_group;" ::: "memory");
+        ck = chunks[min(ch + 1, n - 1)];
     };
     fetch(0);
     // this warp's tiles of S: columns (warp + 8 j) * 8 + 2 t, + 1 of rows g and g + 8
@@ -138,22 +138,33 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
     for (int ch = 0; ch < n; ch++) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                            // chunk ch and S are in shared memory, the other buffer has been read
+        uint16_t* yh = y_next + (size_t)h * ntok * D + m0;
+        y_next = ck.y;
         if (ch + 1 < n) fetch(ch + 1);
         const ScanBuf<D>& b = sm.buf[ch & 1];
         const float *bj = b.vec, *eG = b.vec + C, *wd = b.vec + 2 * C;
         // ---- b and the state's part of y: S k and S q, hi and lo apart
         float kh[4] = {}, kl[4] = {}, qh[4] = {}, ql[4] = {};
-#pragma unroll 4
-        for (int k0 = 0; k0 < D; k0 += 16) {
-            uint32_t ak[4], aq[4], bh[2], bl[2];
-            frag_a(ak, b.K + mi * 16 * DP, DP, k0, g, t);
-            frag_a(aq, b.Q + mi * 16 * DP, DP, k0, g, t);
-            frag_b(bh, sm.Shi + ni * 8 * DP, DP, k0, g, t);
-            frag_b(bl, sm.Slo + ni * 8 * DP, DP, k0, g, t);
-            mma16816(kh, ak, bh[0], bh[1]);
-            mma16816(kl, ak, bl[0], bl[1]);
-            mma16816(qh, aq, bh[0], bh[1]);
-            mma16816(ql, aq, bl[0], bl[1]);
+        {
+            // rows of an operand by ldmatrix: 16 rows x 16 columns of k and q, 8 rows x 32 columns of S
+            const uint32_t arow = (mi * 16 + (lane & 15)) * DP + (lane >> 4) * 8, brow = (ni * 8 + (lane & 7)) * DP + (lane >> 3) * 8;
+            const uint32_t pk = smem_of(b.K + arow), pq = smem_of(b.Q + arow), ph = smem_of(sm.Shi + brow), pl = smem_of(sm.Slo + brow);
+#pragma unroll
+            for (int k0 = 0; k0 < D; k0 += 32) {
+                uint32_t bh[4], bl[4];
+                ldsm(bh, ph + k0 * 2);
+                ldsm(bl, pl + k0 * 2);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    uint32_t ak[4], aq[4];
+                    ldsm(ak, pk + (k0 + 16 * i) * 2);
+                    ldsm(aq, pq + (k0 + 16 * i) * 2);
+                    mma16816(kh, ak, bh[2 * i], bh[2 * i + 1]);
+                    mma16816(kl, ak, bl[2 * i], bl[2 * i + 1]);
+                    mma16816(qh, aq, bh[2 * i], bh[2 * i + 1]);
+                    mma16816(ql, aq, bl[2 * i], bl[2 * i + 1]);
+                }
+            }
         }
 #pragma unroll
         for (int e = 0; e < 4; e++) {
@@ -163,14 +174,21 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
         __syncthreads();
         // ---- u = T b, also weighted with the decay to the end of the chunk
         float uh[4] = {}, ul[4] = {};
+        const uint32_t crow = (mi * 16 + (lane & 15)) * CP + (lane >> 4) * 8, drow = (ni * 8 + (lane & 7)) * CP + (lane >> 3) * 8;
+        {
+            const uint32_t pt = smem_of(b.T + crow), ph = smem_of(sm.bThi + drow), pl = smem_of(sm.bTlo + drow);
 #pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16) {
-            uint32_t a[4], bh[2], bl[2];
-            frag_a(a, b.T + mi * 16 * CP, CP, k0, g, t);
-            frag_b(bh, sm.bThi + ni * 8 * CP, CP, k0, g, t);
-            frag_b(bl, sm.bTlo + ni * 8 * CP, CP, k0, g, t);
-            mma16816(uh, a, bh[0], bh[1]);
-            mma16816(ul, a, bl[0], bl[1]);
+            for (int k0 = 0; k0 < C; k0 += 32) {
+                uint32_t bh[4], bl[4], a0[4], a1[4];
+                ldsm(bh, ph + k0 * 2);
+                ldsm(bl, pl + k0 * 2);
+                ldsm(a0, pt + k0 * 2);
+                ldsm(a1, pt + k0 * 2 + 32);
+                mma16816(uh, a0, bh[0], bh[1]);
+                mma16816(ul, a0, bl[0], bl[1]);
+                mma16816(uh, a1, bh[2], bh[3]);
+                mma16816(ul, a1, bl[2], bl[3]);
+            }
         }
 #pragma unroll
         for (int e = 0; e < 4; e++) {
@@ -182,18 +200,24 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
         __syncthreads();
         // ---- y = e^G S q + QK u
         float y0[4] = {}, y1[4] = {}, y2[4] = {};
+        {
+            const uint32_t pa = smem_of(b.QKhi + crow), pb = smem_of(b.QKlo + crow), ph = smem_of(sm.uThi + drow), pl = smem_of(sm.uTlo + drow);
 #pragma unroll
-        for (int k0 = 0; k0 < C; k0 += 16) {
-            uint32_t ah[4], al[4], bh[2], bl[2];
-            frag_a(ah, b.QKhi + mi * 16 * CP, CP, k0, g, t);
-            frag_a(al, b.QKlo + mi * 16 * CP, CP, k0, g, t);
-            frag_b(bh, sm.uThi + ni * 8 * CP, CP, k0, g, t);
-            frag_b(bl, sm.uTlo + ni * 8 * CP, CP, k0, g, t);
-            mma16816(y0, ah, bh[0], bh[1]);
-            mma16816(y1, ah, bl[0], bl[1]);
-            mma16816(y2, al, bh[0], bh[1]);
+            for (int k0 = 0; k0 < C; k0 += 32) {
+                uint32_t bh[4], bl[4];
+                ldsm(bh, ph + k0 * 2);
+                ldsm(bl, pl + k0 * 2);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    uint32_t ah[4], al[4];
+                    ldsm(ah, pa + (k0 + 16 * i) * 2);
+                    ldsm(al, pb + (k0 + 16 * i) * 2);
+                    mma16816(y0, ah, bh[2 * i], bh[2 * i + 1]);
+                    mma16816(y1, ah, bl[2 * i], bl[2 * i + 1]);
+                    mma16816(y2, al, bh[2 * i], bh[2 * i + 1]);
+                }
+            }
         }
-        uint16_t* yh = chunks[ch].y + (size_t)h * ntok * D + m0;
 #pragma unroll
         for (int e = 0; e < 4; e += 2) {
             const int j = mi * 16 + g + (e >> 1) * 8, m = ni * 8 + 2 * t;
@@ -211,10 +235,11 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
 #pragma unroll
         for (int k0 = 0; k0 < C; k0 += 32) {
             uint32_t a0[4], a1[4], l0[4], l1[4];
-            frag_a(a0, sm.wuhi, CP, k0, g, t);
-            frag_a(a1, sm.wuhi, CP, k0 + 16, g, t);
-            frag_a(l0, sm.wulo, CP, k0, g, t);
-            frag_a(l1, sm.wulo, CP, k0 + 16, g, t);
+            const uint32_t wrow = ((lane & 15) * CP + (lane >> 4) * 8 + k0) * 2;
+            ldsm(a0, smem_of(sm.wuhi) + wrow);
+            ldsm(a1, smem_of(sm.wuhi) + wrow + 32);
+            ldsm(l0, smem_of(sm.wulo) + wrow);
+            ldsm(l1, smem_of(sm.wulo) + wrow + 32);
 #pragma unroll
             for (int j = 0; j < TPW; j++) {
                 uint32_t r[4];
