@@ -106,8 +106,8 @@ struct Engine {
     uint32_t* d_st_count = nullptr;     // device: WT_MAX_STATES counters, then WT_MAX_STATES arrival counts of the merge kernel
     KvGeom kv[WT_MAX_STATES];
 
-    unsigned int* d_status = nullptr;   // first failing op (1-based) raised by a kernel
-    unsigned int* h_status = nullptr;   // pinned
+    unsigned int* h_status = nullptr;   // pinned and mapped: first failing op (1-based) or a code raised by a kernel
+    unsigned int* d_status = nullptr;   // the same word as the device sees it
 
     std::vector<PlanOp> plan;
     uint32_t fused_ops = 0;
