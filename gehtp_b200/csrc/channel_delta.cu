@@ -352,7 +352,11 @@ gated_norm_kernel(const float* o, const float* __restrict__ w, const float* gate
 constexpr uint32_t STEP_ROWS = 4, STEP_COLS = 32;
 inline uint32_t step_floats(const DeltaArgs& a, uint32_t dp, uint32_t r) { return r * (3 * dp + ((a.rank_a + 3) & ~3u) + ((a.rank_g + 3) & ~3u)) + 8 * STEP_COLS * 2; }
 
-// elements k .. k + 3 of row `row` of w [.., n], zeros past n
+// elements k .. k + 3 of row `row` of w [.., n], zeros past n; rows that are no multiple of 8 bytes go through a call: their code
+// stays out of the kernel's straight line, whose fetch costs as much as its work
+__device__ __noinline__ float4 low_rank_edge(const uint16_t* __restrict__ p, uint32_t k, uint32_t n) {
+    return make_float4(k < n ? bf2f(__ldg(p)) : 0.f, k + 1 < n ? bf2f(__ldg(p + 1)) : 0.f, k + 2 < n ? bf2f(__ldg(p + 2)) : 0.f, k + 3 < n ? bf2f(__ldg(p + 3)) : 0.f);
+}
 __device__ __forceinline__ float4 low_rank4(const uint16_t* __restrict__ w, size_t row, uint32_t k, uint32_t n) {
     const uint16_t* p = w + row * n + k;
     if ((n & 3u) == 0) {
@@ -360,7 +364,7 @@ __device__ __forceinline__ float4 low_rank4(const uint16_t* __restrict__ w, size
         const uint2 q = __ldg((const uint2*)p);
         return make_float4(bf2f((uint16_t)(q.x & 0xffffu)), bf2f((uint16_t)(q.x >> 16)), bf2f((uint16_t)(q.y & 0xffffu)), bf2f((uint16_t)(q.y >> 16)));
     }
-    return make_float4(k < n ? bf2f(__ldg(p)) : 0.f, k + 1 < n ? bf2f(__ldg(p + 1)) : 0.f, k + 2 < n ? bf2f(__ldg(p + 2)) : 0.f, k + 3 < n ? bf2f(__ldg(p + 3)) : 0.f);
+    return low_rank_edge(p, k, n);
 }
 
 template <class A, int RPL, int R>
@@ -497,17 +501,10 @@ delta_step_kernel(const DeltaArgs a, uint32_t rows_arg) {
             dg[j] = dot4(wg[j], s_g1 + r * rg4, c * 4, rg4);
             for (uint32_t k = 128 + c * 4; k < rg4; k += 128) dg[j] += dot4(low_rank4(a.g2, h * V + v, k, a.rank_g), s_g1 + r * rg4, k, rg4);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int i = 0; i < RPL; i++) da[i] += __shfl_xor_sync(0xffffffffu, da[i], o);
-#pragma unroll
-            for (int j = 0; j < (int)STEP_COLS / 8; j++) dg[j] += __shfl_xor_sync(0xffffffffu, dg[j], o);
-        }
-#pragma unroll
-        for (int i = 0; i < RPL; i++) if (c == (i & 31)) s_g[r * DP + l + 8 * i] = da[i];
-#pragma unroll
-        for (int j = 0; j < (int)STEP_COLS / 8; j++) if (c == j) s_gate[r][l + 8 * j] = dg[j];
+        // lane v * 32 / N ends up with sum v of N
+        const float va = fold_sum(da), vg = fold_sum(dg);
+        if (c % (32 / RPL) == 0) s_g[r * DP + l + 8 * (c / (32 / RPL))] = va;
+        if (c % (32 / (STEP_COLS / 8)) == 0) s_gate[r][l + 8 * (c / (32 / (STEP_COLS / 8)))] = vg;
     }
     __syncthreads();
     for (uint32_t r = 0; r < rows; r++)

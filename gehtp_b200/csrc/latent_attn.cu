@@ -405,6 +405,7 @@ latent_split_kernel(const LatentArgs a, const uint16_t* qh, const uint16_t* ql, 
     const uint32_t past = *(volatile const uint32_t*)a.counter, n = min(past + rows, a.nslots);
     const uint32_t tiles = (n + TP - 1) / TP, per = (tiles + nsplit - 1) / nsplit;
     const uint32_t t0 = min(blockIdx.x * per, tiles), t1 = min(t0 + per, tiles);
+    if (t0 >= t1) return;                                             // the merge knows how many slices there are
     const uint16_t* st = (const uint16_t*)a.state;
     const uint32_t ch = ls / 8;
     auto fetch = [&](uint32_t t) {
@@ -576,30 +577,37 @@ latent_merge_kernel(const LatentArgs a, const float* part_o, const float* part_m
     }
     pdl_wait();
     pdl_release();          // after the wait, like the merge of the KV-ring attention
-    // nsplit <= kMaxSplit: one slice per thread here, at most kMaxSplit / 4 slices of a column per thread below; the
-    // partial latents are requested before the weights are known
-    const float2 ml = tid < nsplit ? __ldcg((const float2*)part_ml + (size_t)pr * nsplit + tid) : make_float2(-INFINITY, 0.0f);
+    // One slice per thread here (nsplit <= kMaxSplit), every fourth slice of a column below; the first of the partial latents are
+    // requested before the weights are known. Slices past the last one with a position have not been written.
+    const uint32_t n = min(*(volatile const uint32_t*)a.counter + gridDim.x / a.heads, a.nslots), tiles = (n + TP - 1) / TP, per = (tiles + nsplit - 1) / nsplit;
+    const uint32_t slices = (tiles + per - 1) / per;
+    const float2 ml = tid < slices ? __ldcg((const float2*)part_ml + (size_t)pr * nsplit + tid) : make_float2(-INFINITY, 0.0f);
     const uint32_t cper = (a.rank + MC - 1) / MC, c = part * cper + tid % MCOLS, q = tid / MCOLS;     // cper <= MCOLS
     const bool live = tid % MCOLS < cper && c < a.rank;
     const float* po = part_o + (size_t)pr * nsplit * a.rank + c;
-    float v[kMaxSplit / 4];
+    constexpr int AHEAD = 8;
+    float v[AHEAD];
+    auto request = [&](uint32_t s0) {
 #pragma unroll
-    for (int i = 0; i < (int)kMaxSplit / 4; i++) {
-        const uint32_t s = q + 4 * i;
-        v[i] = live && s < nsplit ? __ldcg(po + (size_t)s * a.rank) : 0.0f;
-    }
+        for (int i = 0; i < AHEAD; i++) v[i] = live && s0 + 4 * i < slices ? __ldcg(po + (size_t)(s0 + 4 * i) * a.rank) : 0.0f;
+    };
+    request(q);
     float m = warp_max(ml.x);
     if (lane == 0) red[warp] = m;
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < 8; w++) m = fmaxf(m, red[w]);
-    const float wt = ml.y > 0.0f ? expf(ml.x - m) : 0.0f;          // an empty slice has sum 0 (and a zero latent)
+    const float wt = ml.y > 0.0f ? expf(ml.x - m) : 0.0f;          // a slice without a visible position has sum 0
     if (tid < kMaxSplit) sw[tid] = wt;
     const float l = block_sum(wt * ml.y, red);
     {
         float o = 0.0f;
+#pragma unroll 1
+        for (uint32_t s0 = q; s0 < slices; s0 += 4 * AHEAD) {
+            if (s0 > q) request(s0);
 #pragma unroll
-        for (int i = 0; i < (int)kMaxSplit / 4; i++) o = fmaf(sw[q + 4 * i], v[i], o);
+            for (int i = 0; i < AHEAD; i++) o = s0 + 4 * i < slices ? fmaf(sw[s0 + 4 * i], v[i], o) : o;
+        }
         quarter[q][tid % MCOLS] = o;
         __syncthreads();
         cluster_wait();                                // every CTA of the cluster has started

@@ -16,7 +16,8 @@ constexpr int PB = 4;                         // positions a warp takes at a tim
 // once for all pairs in rows of 512 bytes; the P * PB dot products are folded over the warp until each lane has one score,
 // one exponential and its part of the softmax. Warps meet in shared memory, CTAs of a cluster in distributed shared memory.
 // Bound by the latency of one row's loads (one row), by its shuffles (many). 16 heads of 128 over
-// 8 key heads: 6.5 us for one row behind 150 positions, 30 us for 150 rows (a thread per position walking its key alone, one CTA
+// 8 key heads: 4.8 us for one row behind 150 positions (8.4 with positions of earlier runs requested behind the wait and one trip
+// to each CTA of the cluster after the other), 30 us for 150 rows (a thread per position walking its key alone, one CTA
 // per head and row, in its place before: 89 us for both).
 template <int P, int DI>
 __global__ void __launch_bounds__(256)
@@ -31,25 +32,13 @@ window_f32_kernel(const WindowArgs a, uint32_t rows, uint32_t hg) {
     const uint32_t R = P / hg, r0 = blockIdx.z * R, row = a.row();
     auto pair_row = [&](uint32_t p) { return min(r0 + p / hg, rows - 1); };        // pairs past the last repeat it; never stored
     auto pair_head = [&](uint32_t p) { return g * rep + min(hp + p % hg, rep - 1); };
-    pdl_wait();
+    // the counter moves at the end of a run only: it is read, and what earlier runs have left is requested, before the wait
     const uint32_t past = *(volatile const uint32_t*)a.counter;
     auto first_of = [&](uint32_t pos) { return pos + 1 > a.window ? pos + 1 - a.window : 0; };
     const uint32_t first = first_of(past + r0), last = past + pair_row(P - 1);
-    float4 q[P][DI], o[P][DI];
-#pragma unroll
-    for (int p = 0; p < P; p++)
-#pragma unroll
-        for (int i = 0; i < DI; i++) {
-            const uint32_t d = lane * 4 + 128 * i;
-            o[p][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            q[p][i] = d < a.dim ? __ldcg((const float4*)((const float*)a.q + ((size_t)pair_row(p) * a.heads + pair_head(p)) * a.dim + d)) : o[p][i];
-        }
     const float *keys = (const float*)a.state + g * a.dim, *vals = (const float*)a.state + a.kv_heads * a.dim + g * a.vdim;
-    // this lane's pair and place among the PB positions
-    const uint32_t mp = lane / LPV / PB, mb = lane / LPV % PB, mpos = past + pair_row(mp), mfirst = first_of(mpos);
-    float m = -INFINITY, l = 0.0f;
-    for (uint32_t j0 = first + PB * (blockIdx.x * FW + warp); j0 <= last; j0 += PB * FW * C) {
-        float4 k[PB][DI], v[PB][DI];
+    float4 k[PB][DI], v[PB][DI];
+    auto load = [&](uint32_t j0) {
 #pragma unroll
         for (int b = 0; b < PB; b++) {
             const size_t at = (size_t)((j0 + b) % a.ring) * row;
@@ -61,6 +50,27 @@ window_f32_kernel(const WindowArgs a, uint32_t rows, uint32_t hg) {
                 v[b][i] = j0 + b <= last && d < a.vdim ? __ldcg((const float4*)(vals + at + d)) : z;
             }
         }
+    };
+    const uint32_t step = PB * FW * C;
+    uint32_t j0 = first + PB * (blockIdx.x * FW + warp);
+    bool early = j0 + PB <= past;
+    if (early) load(j0);
+    pdl_wait();
+    float4 q[P][DI], o[P][DI];
+#pragma unroll
+    for (int p = 0; p < P; p++)
+#pragma unroll
+        for (int i = 0; i < DI; i++) {
+            const uint32_t d = lane * 4 + 128 * i;
+            o[p][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            q[p][i] = d < a.dim ? __ldcg((const float4*)((const float*)a.q + ((size_t)pair_row(p) * a.heads + pair_head(p)) * a.dim + d)) : o[p][i];
+        }
+    // this lane's pair and place among the PB positions
+    const uint32_t mp = lane / LPV / PB, mb = lane / LPV % PB, mpos = past + pair_row(mp), mfirst = first_of(mpos);
+    float m = -INFINITY, l = 0.0f;
+    for (; j0 <= last; j0 += step) {
+        if (!early) load(j0);                                     // past the last: zeros
+        early = false;
         float s[NV];
 #pragma unroll
         for (int p = 0; p < P; p++)
@@ -126,20 +136,42 @@ window_f32_kernel(const WindowArgs a, uint32_t rows, uint32_t hg) {
         sm[i] = num;                                              // only this thread reads element i of any warp
         if (i % a.vdim == 0) { cm[p] = mx; cl[p] = sum; }
     }
-    if (C > 1) cluster.sync(); else __syncthreads();
     const uint32_t per = (P * a.vdim + C - 1) / C, e0 = blockIdx.x * per, e1 = min(e0 + per, P * a.vdim);
+    auto gate_of = [&](uint32_t i) {
+        const uint32_t p = i / a.vdim;
+        return a.gate_col == 0xFFFFFFFFu || i >= e1 ? 0.0f : __ldcg((const float*)a.y + (size_t)pair_row(p) * a.y_cols + a.gate_col + pair_head(p) * a.vdim + i % a.vdim);
+    };
+    const float gate0 = gate_of(e0 + tid);
+    if (C > 1) cluster.sync(); else __syncthreads();
     for (uint32_t i = e0 + tid; i < e1; i += 256) {
         const uint32_t p = i / a.vdim, c = i % a.vdim;
         if (r0 + p / hg >= rows || hp + p % hg >= rep) continue;
-        float mx = -INFINITY, num = 0.0f, den = 0.0f, pm[FC];
-        for (uint32_t k = 0; k < C; k++) { pm[k] = C > 1 ? *cluster.map_shared_rank(cm + p, k) : cm[p]; mx = fmaxf(mx, pm[k]); }
-        for (uint32_t k = 0; k < C; k++) {
-            const float f = pm[k] > -INFINITY ? expf(pm[k] - mx) : 0.0f;
-            num = fmaf(f, C > 1 ? *cluster.map_shared_rank(sm + i, k) : sm[i], num);
-            den = fmaf(f, C > 1 ? *cluster.map_shared_rank(cl + p, k) : cl[p], den);
+        float num = 0.0f, den = 0.0f;
+        if (C == 1) {
+            num = sm[i]; den = cl[p];
+        } else {
+            // what the CTAs of the cluster have, requested together: one trip after the other cost 0.1 us each
+            float mx = -INFINITY, pm[FC], pn[FC], pl[FC];
+#pragma unroll
+            for (uint32_t k = 0; k < FC; k++) {
+                pm[k] = -INFINITY; pn[k] = pl[k] = 0.0f;
+                if (k >= C) continue;
+                pm[k] = *cluster.map_shared_rank(cm + p, k);
+                pn[k] = *cluster.map_shared_rank(sm + i, k);
+                pl[k] = *cluster.map_shared_rank(cl + p, k);
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < FC; k++) mx = fmaxf(mx, pm[k]);
+#pragma unroll
+            for (uint32_t k = 0; k < FC; k++) {
+                const float f = pm[k] > -INFINITY ? expf(pm[k] - mx) : 0.0f;
+                if (k >= C) continue;
+                num = fmaf(f, pn[k], num);
+                den = fmaf(f, pl[k], den);
+            }
         }
         const uint32_t r = pair_row(p), h = pair_head(p);
-        const float gate = a.gate_col == 0xFFFFFFFFu ? 1.0f : sigmoid_f(__ldcg((const float*)a.y + (size_t)r * a.y_cols + a.gate_col + h * a.vdim + c));
+        const float gate = a.gate_col == 0xFFFFFFFFu ? 1.0f : sigmoid_f(i == e0 + tid ? gate0 : gate_of(i));
         ((float*)a.out)[((size_t)r * a.heads + h) * a.vdim + c] = num / den * gate;
     }
     if (C > 1) cluster.sync();                                    // nobody leaves while its results are being read
