@@ -30,8 +30,11 @@ void k_add_rmsnorm(cudaStream_t st, const uint16_t* a, const uint16_t* r, const 
     const uintptr_t ptrs = (uintptr_t)a | (uintptr_t)r | (uintptr_t)g | (uintptr_t)b | (uintptr_t)sum_out | (uintptr_t)y;
     if (width > 512 && norm_in_registers<256, 1>(width, ptrs))
         launch_pdl(rmsnorm_kernel<256, 1, true>, dim3(rows), dim3(256), 0, st, a, r, g, b, sum_out, y, width);
-    else if (width > 512 && norm_in_registers<256, 2>(width, ptrs))
-        launch_pdl(rmsnorm_kernel<256, 2, true>, dim3(rows), dim3(256), 0, st, a, r, g, b, sum_out, y, width);
+    // eight values a thread: with 16 the code, which runs once, is twice as long to fetch
+    else if (width > 512 && norm_in_registers<320, 1>(width, ptrs))
+        launch_pdl(rmsnorm_kernel<320, 1, true>, dim3(rows), dim3(320), 0, st, a, r, g, b, sum_out, y, width);
+    else if (width > 512 && norm_in_registers<512, 1>(width, ptrs))
+        launch_pdl(rmsnorm_kernel<512, 1, true>, dim3(rows), dim3(512), 0, st, a, r, g, b, sum_out, y, width);
     else if (width <= 512)
         launch_pdl(rmsnorm_kernel<64>, dim3(rows), dim3(64), width * sizeof(float), st, a, r, g, b, sum_out, y, width);
     else

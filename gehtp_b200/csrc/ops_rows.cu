@@ -25,16 +25,17 @@ embed_rows_kernel(const uint16_t* __restrict__ table, const int32_t* ids, float*
 }
 
 // One CTA per row: x_out = x + y / sqrt(mean(y^2) + eps) * (base + w), act = x_out in the activation type. A thread
-// keeps up to KEEP values of the row in registers between the two passes; longer rows are read twice.
-template <class Y, class A, int VEC>
-__global__ void __launch_bounds__(256)
+// keeps up to KEEP values of the row in registers between the two passes; longer rows are read twice. Four values a thread and
+// as many threads as that takes, up to 4096 columns: with 256 threads of up to 16 the fetch of code that runs once, or not at
+// all, was a third of a launch.
+template <class Y, class A, int VEC, int KEEP>
+__global__ void __launch_bounds__(VEC == 4 ? 1024 : 256)
 norm_resid_kernel(const typename Y::T* y, const float* __restrict__ w, const float* x, float* x_out, typename A::T* act,
                   uint32_t width, float eps, float base) {
-    __shared__ float part[8];
-    constexpr int KEEP = 16;
+    __shared__ float part[32];
     pdl_release();
     const size_t off = (size_t)blockIdx.x * width;
-    const uint32_t tid = threadIdx.x, step = 256 * VEC;
+    const uint32_t tid = threadIdx.x, step = blockDim.x * VEC;
     pdl_wait();
     float keep[KEEP], res[KEEP];
     float ss = 0.0f;
@@ -59,7 +60,7 @@ norm_resid_kernel(const typename Y::T* y, const float* __restrict__ w, const flo
 #pragma unroll
         for (int k = 0; k < VEC; k++) ss = fmaf(keep[u * VEC + k], keep[u * VEC + k], ss);
     }
-    for (uint32_t i = tid + 256 * KEEP; i < width; i += 256) { const float v = Y::ld(y + off + i); ss = fmaf(v, v, ss); }
+    for (uint32_t i = tid + blockDim.x * KEEP; i < width; i += blockDim.x) { const float v = Y::ld(y + off + i); ss = fmaf(v, v, ss); }
     ss = block_sum(ss, part);
     const float inv = 1.0f / sqrtf(ss / (float)width + eps);
 #pragma unroll
@@ -84,7 +85,7 @@ norm_resid_kernel(const typename Y::T* y, const float* __restrict__ w, const flo
             }
         }
     }
-    for (uint32_t i = tid + 256 * KEEP; i < width; i += 256) {
+    for (uint32_t i = tid + blockDim.x * KEEP; i < width; i += blockDim.x) {
         const float o = (x ? __ldcg(x + off + i) : 0.0f) + Y::ld(y + off + i) * inv * (base + __ldg(w + i));
         if (x_out) x_out[off + i] = o;
         if (act) A::st(act + off + i, o);
@@ -191,9 +192,9 @@ void launch_norm(cudaStream_t st, const NormResidArgs& a, uint32_t rows) {
     const typename Y::T* y = (const typename Y::T*)a.y;
     typename A::T* act = (typename A::T*)a.act;
     if (a.width % 4 == 0 && a.width <= 4096 && (al & 15u) == 0)
-        launch_pdl(norm_resid_kernel<Y, A, 4>, dim3(rows), dim3(256), 0, st, y, a.w, a.x, a.x_out, act, a.width, a.eps, a.base);
+        launch_pdl(norm_resid_kernel<Y, A, 4, 4>, dim3(rows), dim3((a.width / 4 + 31) / 32 * 32), 0, st, y, a.w, a.x, a.x_out, act, a.width, a.eps, a.base);
     else
-        launch_pdl(norm_resid_kernel<Y, A, 1>, dim3(rows), dim3(256), 0, st, y, a.w, a.x, a.x_out, act, a.width, a.eps, a.base);
+        launch_pdl(norm_resid_kernel<Y, A, 1, 16>, dim3(rows), dim3(256), 0, st, y, a.w, a.x, a.x_out, act, a.width, a.eps, a.base);
 }
 
 }  // namespace
