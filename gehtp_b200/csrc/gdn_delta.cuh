@@ -55,11 +55,12 @@ __device__ __forceinline__ void chunk_decays(const uint16_t* gh, const uint16_t*
 }
 
 // T = (I + L)^-1 (Th, and transposed Tt) and the decayed q.k matrix (hi, lo) of one chunk, by 256 threads. Shared memory:
-// Kh, Qh [C][D + 8], Lh, Th, Tt, QKhi, QKlo [C][CP], xs [3][768]. `stage3` is run beside the first products, before the
-// first barrier; the matrices are complete when the function returns (the last barrier is behind them).
-template <int D, class Stage3>
-__device__ __forceinline__ void chunk_matrices(const uint16_t* Kh, const uint16_t* Qh, uint16_t* Lh, uint16_t* Th, uint16_t* Tt, uint16_t* QKhi,
-                                               uint16_t* QKlo, uint16_t* xs, const float* G, const float* bj, float scale, Stage3 stage3) {
+// Kh, Qh [C][D + 8], Lh, Th, Tt [C][CP], xs [3][768]; Th, Tt and xs may lie on Kh and Qh, which are read up to the first
+// barrier. Two neighbouring values of the q.k matrix, packed, go to put_qk(row, column, hi, lo). `stage3` is run beside the
+// first products, before the first barrier; the matrices are complete when the function returns (the last barrier is behind them).
+template <int D, class Stage3, class PutQK>
+__device__ __forceinline__ void chunk_matrices(const uint16_t* Kh, const uint16_t* Qh, uint16_t* Lh, uint16_t* Th, uint16_t* Tt, uint16_t* xs,
+                                               const float* G, const float* bj, float scale, Stage3 stage3, PutQK put_qk) {
     constexpr int DP = D + 8;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     // ---- stage 1 (with 3 and 5 below): L[j][i] = f16(exp(G_j - G_i) (k_j . k_i) beta_j) for i < j, else 0
@@ -79,9 +80,9 @@ __device__ __forceinline__ void chunk_matrices(const uint16_t* Kh, const uint16_
             Lh[j * CP + i] = i < j ? f2h(expf(G[j] - G[i]) * acc[e] * bj[j]) : (uint16_t)0;
         }
     }
-    for (int e = tid; e < C * C; e += 256) {          // the tiles above: L = 0, QK = 0
-        const int r = e / C, i = e % C;
-        if (i >= ((r >> 4) + 1) * 16) { Lh[r * CP + i] = 0; QKhi[r * CP + i] = 0; QKlo[r * CP + i] = 0; }
+    for (int e = tid; e < C * C / 2; e += 256) {      // the tiles above: L = 0, QK = 0
+        const int r = e / (C / 2), i = e % (C / 2) * 2;
+        if (i >= ((r >> 4) + 1) * 16) { *(uint32_t*)(Lh + r * CP + i) = 0; put_qk(r, i, 0u, 0u); }
     }
     // stages 3 and 5 need the operands only, not L or T: same phase, one barrier for the three
     stage3();
@@ -92,9 +93,17 @@ __device__ __forceinline__ void chunk_matrices(const uint16_t* Kh, const uint16_
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         mma_rows(acc, Qh + mi * 16 * DP, DP, Kh + ni * 8 * DP, DP, D, g, t);
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int tt = mi * 16 + g + (e >> 1) * 8, i = ni * 8 + 2 * t + (e & 1);
-            split_store(QKhi + tt * CP + i, QKlo + tt * CP + i, i <= tt ? acc[e] * scale * expf(G[tt] - G[i]) : 0.0f);
+        for (int e = 0; e < 4; e += 2) {
+            const int tt = mi * 16 + g + (e >> 1) * 8, i = ni * 8 + 2 * t;
+            uint32_t hi = 0, lo = 0;
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                const float x = i + b <= tt ? acc[e + b] * scale * expf(G[tt] - G[i + b]) : 0.0f;
+                const uint16_t h = f2h(x);
+                hi |= (uint32_t)h << (16 * b);
+                lo |= (uint32_t)f2h(x - h2f(h)) << (16 * b);
+            }
+            put_qk(tt, i, hi, lo);
         }
     }
     __syncthreads();

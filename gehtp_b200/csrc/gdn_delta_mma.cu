@@ -116,7 +116,7 @@ delta_chunk_mma_kernel(const uint16_t* __restrict__ k, const uint16_t* __restric
     }
     __syncthreads();
 
-    chunk_matrices<D>(Kh, Qh, Lh, Th, Tt, QKhi, QKlo, xs, G, bj, scale, [&] {
+    chunk_matrices<D>(Kh, Qh, Lh, Th, Tt, xs, G, bj, scale, [&] {
         // ---- stage 3: b[j][m] = beta_j (v[j][m] - e^{G_j} (S0 k_j)[m]), stored transposed as hi + lo
         for (int tile = warp; tile < (C / 16) * (DM / 8); tile += 8) {
             const int mi = tile / (DM / 8), ni = tile % (DM / 8);
@@ -130,6 +130,9 @@ delta_chunk_mma_kernel(const uint16_t* __restrict__ k, const uint16_t* __restric
                 split_store(bThi + m * CP + j, bTlo + m * CP + j, bj[j] * (vv - eG[j] * acc[e]));
             }
         }
+    }, [&](int r, int i, uint32_t hi, uint32_t lo) {
+        *(uint32_t*)(QKhi + r * CP + i) = hi;
+        *(uint32_t*)(QKlo + r * CP + i) = lo;
     });
 
     // ---- stage 4: u = T b ; also u_i weighted with the decay to the end of the chunk (for the state update)

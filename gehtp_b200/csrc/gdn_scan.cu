@@ -9,6 +9,7 @@
 // One launch per chunk is bound by the chain of all seven stages (15 us, 32 times in 2048 tokens); the walk's own chain is
 // three barriers a chunk. Its products are read from shared memory: k, q and S fragments are taken once for the two
 // products and the hi and lo halves that use them.
+#include <algorithm>
 #include "gdn_delta.cuh"
 #include "launchers.h"
 
@@ -36,12 +37,11 @@ delta_chunks_kernel(const DeltaChunk* __restrict__ chunks, unsigned char* scratc
     extern __shared__ __align__(16) unsigned char smem[];
     uint16_t* Kh = (uint16_t*)smem;                 // [C][DP]
     uint16_t* Qh = Kh + C * DP;
-    uint16_t* Lh = Qh + C * DP;                     // [C][CP] each
-    uint16_t* Th = Lh + C * CP;
-    uint16_t* Tt = Th + C * CP;
-    uint16_t* QKhi = Tt + C * CP;
-    uint16_t* QKlo = QKhi + C * CP;
-    uint16_t* xs = QKlo + C * CP;                   // [3][768]
+    uint16_t* Lh = Qh + C * DP;                     // [C][CP]
+    uint16_t* xs = Lh + C * CP;                     // [3][768]
+    // T over k and q, which have been read by then; q.k goes straight to scratch. Four CTAs fit an SM, and the 512 of 2048 tokens
+    // and 16 heads are one round; with every matrix in a place of its own they were two.
+    uint16_t *Th = Kh, *Tt = Th + C * CP;           // [C][CP] each
     float* G = (float*)(xs + 3 * 768);
     float* vec = G + C;                             // bj, eG, wd
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -57,13 +57,13 @@ delta_chunks_kernel(const DeltaChunk* __restrict__ chunks, unsigned char* scratc
     if (warp == 0) chunk_decays(ck.g + (size_t)h * ntok, ck.beta + (size_t)h * ntok, C, lane, G, vec, vec + C, vec + 2 * C);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    chunk_matrices<D>(Kh, Qh, Lh, Th, Tt, QKhi, QKlo, xs, G, vec, q_raw ? 1.0f : 1.0f / sqrtf((float)D), [] {});
     unsigned char* item = scratch + ((size_t)h * gridDim.y + blockIdx.y) * ITEM_BYTES;
-    const uint16_t* mats[3] = {Th, QKhi, QKlo};
-#pragma unroll
-    for (int m = 0; m < 3; m++)
-        for (int e = tid; e < C * C / 8; e += 256)
-            *(uint4*)(item + m * MAT * 2 + (size_t)e * 16) = *(const uint4*)(mats[m] + (e >> 3) * CP + (e & 7) * 8);
+    chunk_matrices<D>(Kh, Qh, Lh, Th, Tt, xs, G, vec, q_raw ? 1.0f : 1.0f / sqrtf((float)D), [] {}, [&](int r, int i, uint32_t hi, uint32_t lo) {
+        uint32_t* at = (uint32_t*)(item + MAT * 2 + (r * C + i) * 2);
+        at[0] = hi;
+        at[MAT / 2] = lo;
+    });
+    for (int e = tid; e < C * C / 8; e += 256) *(uint4*)(item + (size_t)e * 16) = *(const uint4*)(Th + (e >> 3) * CP + (e & 7) * 8);
     if (tid < 3 * C) ((float*)(item + 3 * MAT * 2))[tid] = vec[tid];
 }
 
@@ -270,7 +270,11 @@ delta_scan_mma_kernel(const DeltaChunk* __restrict__ chunks, const unsigned char
 template <int D>
 bool launch(cudaStream_t st, const DeltaChunk* chunks, unsigned char* scratch, float* S, uint32_t n, uint32_t ntok, uint32_t H, uint32_t q_raw) {
     static int have_a[64], have_b[64];
-    const size_t sa = (size_t)(2 * C * (D + 8) + 5 * C * CP + 3 * 768) * 2 + 4 * C * sizeof(float);
+    // No more CTAs to an SM than an even spread needs: those that come up while the kernel before still holds SMs would pile up on
+    // the ones it has left (256 tokens: 76 us a layer for 70). An SM has 228 KB.
+    const uint32_t per_sm = (H * n + 147) / 148;
+    const size_t need = (size_t)(2 * C * (D + 8) + C * CP + 3 * 768) * 2 + 4 * C * sizeof(float);
+    const size_t sa = std::max(need, per_sm < 4 ? (size_t)228 * 1024 / (per_sm + 1) + 1024 : 0);
     if (!ensure_dyn_smem(delta_chunks_kernel<D>, sa, have_a) || !ensure_dyn_smem(delta_scan_mma_kernel<D>, sizeof(ScanSmem<D>), have_b)) return false;
     if (launch_pdl(delta_chunks_kernel<D>, dim3(H, n), dim3(256), sa, st, chunks, scratch, (int)ntok, (int)q_raw) != cudaSuccess ||
         launch_pdl(delta_scan_mma_kernel<D>, dim3(H, D / DM), dim3(256), sizeof(ScanSmem<D>), st, chunks, (const unsigned char*)scratch, S, (int)n, (int)ntok, (int)q_raw) != cudaSuccess) {
