@@ -27,35 +27,50 @@ __device__ __forceinline__ float conv_in(const typename A::T* y, const float* ba
     return r >= 0 ? A::ld(y + (size_t)r * ys + c) : bank[(size_t)(keep + r) * C + c];
 }
 
-template <class A>
+template <class A, bool PAIRS>
 __global__ void __launch_bounds__(256)
 short_conv_kernel(const typename A::T* y, const float* __restrict__ w, float* state, const uint32_t* count, float* out,
                   uint32_t rows, uint32_t C, uint32_t taps, uint32_t ys) {
     pdl_release();
     pdl_wait();
-    const uint32_t c = blockIdx.x * 256 + threadIdx.x;
-    if (c >= C) return;
     const int keep = (int)taps - 1;
     const uint32_t par = *count & 1u;
     const float* bank = state + (size_t)par * keep * C;
-    const float* wc = w + (size_t)c * taps;
     const uint32_t r0 = blockIdx.y * CONV_ROWS, r1 = min(r0 + CONV_ROWS, rows);
-    if (taps == 4) {
-        const float w0 = __ldg(wc), w1 = __ldg(wc + 1), w2 = __ldg(wc + 2), w3 = __ldg(wc + 3);
-        float x0 = conv_in<A>(y, bank, (int)r0 - 3, c, ys, C, 3), x1 = conv_in<A>(y, bank, (int)r0 - 2, c, ys, C, 3),
-              x2 = conv_in<A>(y, bank, (int)r0 - 1, c, ys, C, 3);
+    if (PAIRS) {                                    // four taps, two neighbouring channels a thread
+        const uint32_t c = (blockIdx.x * 256 + threadIdx.x) * 2;
+        if (c >= C) return;
+        const float4 w0 = __ldg((const float4*)w + c), w1 = __ldg((const float4*)w + c + 1);
+        auto in = [&](int r) -> float2 {
+            if (r < 0) return __ldcg((const float2*)(bank + (size_t)(3 + r) * C + c));
+            if constexpr (sizeof(typename A::T) == 2) {
+                const uint32_t p = __ldcg((const uint32_t*)(y + (size_t)r * ys + c));
+                return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+            } else {
+                return __ldcg((const float2*)(y + (size_t)r * ys + c));
+            }
+        };
+        float2 x0 = in((int)r0 - 3), x1 = in((int)r0 - 2), x2 = in((int)r0 - 1);
 #pragma unroll 4
         for (uint32_t r = r0; r < r1; r++) {
-            const float x3 = A::ld(y + (size_t)r * ys + c);
-            out[(size_t)r * C + c] = silu_f(fmaf(w3, x3, fmaf(w2, x2, fmaf(w1, x1, w0 * x0))));
+            const float2 x3 = in((int)r);
+            *(float2*)(out + (size_t)r * C + c) = make_float2(silu_f(fmaf(w0.w, x3.x, fmaf(w0.z, x2.x, fmaf(w0.y, x1.x, w0.x * x0.x)))),
+                                                             silu_f(fmaf(w1.w, x3.y, fmaf(w1.z, x2.y, fmaf(w1.y, x1.y, w1.x * x0.y)))));
             x0 = x1; x1 = x2; x2 = x3;
         }
-    } else {
-        for (uint32_t r = r0; r < r1; r++) {
-            float s = 0.0f;
-            for (int j = 0; j < (int)taps; j++) s = fmaf(__ldg(wc + j), conv_in<A>(y, bank, (int)r - keep + j, c, ys, C, keep), s);
-            out[(size_t)r * C + c] = silu_f(s);
+        if (r1 == rows) {
+            float* next = state + (size_t)(par ^ 1u) * 3 * C + c;
+            *(float2*)next = in((int)rows - 3); *(float2*)(next + C) = in((int)rows - 2); *(float2*)(next + 2 * (size_t)C) = in((int)rows - 1);
         }
+        return;
+    }
+    const uint32_t c = blockIdx.x * 256 + threadIdx.x;
+    if (c >= C) return;
+    const float* wc = w + (size_t)c * taps;
+    for (uint32_t r = r0; r < r1; r++) {
+        float s = 0.0f;
+        for (int j = 0; j < (int)taps; j++) s = fmaf(__ldg(wc + j), conv_in<A>(y, bank, (int)r - keep + j, c, ys, C, keep), s);
+        out[(size_t)r * C + c] = silu_f(s);
     }
     if (r1 == rows) {
         float* next = state + (size_t)(par ^ 1u) * keep * C;
@@ -339,6 +354,16 @@ gated_norm_kernel(const float* o, const float* __restrict__ w, const float* gate
     if (i >= n) return;
     const size_t off = (size_t)i * V;
     float ss = 0.0f;
+    // 16 bytes a lane: 15.6 -> 9.3 us at 2048 rows of 16 heads
+    if (V == 128 && (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15u) == 0) {
+        const float4 v = __ldcg((const float4*)(o + off) + lane), g = __ldcg((const float4*)(gate + off) + lane), x = __ldg((const float4*)w + lane);
+        ss = warp_sum(fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))));
+        const float inv = 1.0f / sqrtf(ss / 128.0f + eps);
+        const float r[4] = {v.x * inv * x.x * sigmoid_f(g.x), v.y * inv * x.y * sigmoid_f(g.y), v.z * inv * x.z * sigmoid_f(g.z), v.w * inv * x.w * sigmoid_f(g.w)};
+        if constexpr (sizeof(typename A::T) == 2) *((uint2*)(out + off) + lane) = make_uint2(pack_bf2(r[0], r[1]), pack_bf2(r[2], r[3]));
+        else *((float4*)(out + off) + lane) = make_float4(r[0], r[1], r[2], r[3]);
+        return;
+    }
     for (uint32_t c = lane; c < V; c += 32) { const float v = __ldcg(o + off + c); ss = fmaf(v, v, ss); }
     ss = warp_sum(ss);
     const float inv = 1.0f / sqrtf(ss / (float)V + eps);
@@ -621,9 +646,14 @@ void launch_scan_128(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, ui
 void k_short_conv(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
     if (!rows) return;
     const uint32_t C = a.channels();
-    const dim3 grid((C + 255) / 256, (rows + CONV_ROWS - 1) / CONV_ROWS);
-    if (a.bf16) launch_pdl(short_conv_kernel<ActBf16>, grid, dim3(256), 0, st, (const uint16_t*)a.y, a.conv_w, a.conv_state, a.conv_count, a.qkv, rows, C, a.taps, a.ys);
-    else launch_pdl(short_conv_kernel<ActF32>, grid, dim3(256), 0, st, (const float*)a.y, a.conv_w, a.conv_state, a.conv_count, a.qkv, rows, C, a.taps, a.ys);
+    // two channels a thread where they lie aligned, with the last rows in registers; 30 us one at a time, 24.6 so,
+    // at 6144 channels, 2048 rows
+    const bool pairs = a.taps == 4 && C % 2 == 0 && a.ys % 2 == 0 &&
+                       (((uintptr_t)a.conv_w & 15u) | (((uintptr_t)a.y | (uintptr_t)a.conv_state | (uintptr_t)a.qkv) & 7u)) == 0;
+    const dim3 grid((C / (pairs ? 2 : 1) + 255) / 256, (rows + CONV_ROWS - 1) / CONV_ROWS);
+    auto go = [&](auto kernel, auto y) { launch_pdl(kernel, grid, dim3(256), 0, st, y, a.conv_w, a.conv_state, a.conv_count, a.qkv, rows, C, a.taps, a.ys); };
+    if (a.bf16) pairs ? go(short_conv_kernel<ActBf16, true>, (const uint16_t*)a.y) : go(short_conv_kernel<ActBf16, false>, (const uint16_t*)a.y);
+    else pairs ? go(short_conv_kernel<ActF32, true>, (const float*)a.y) : go(short_conv_kernel<ActF32, false>, (const float*)a.y);
     g_launches++;
 }
 
