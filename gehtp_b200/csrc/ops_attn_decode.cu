@@ -695,11 +695,13 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap, AttnDecodeArgs 
 }
 
 // out[h][d] = sum_s O_s[d] e^{m_s - m} / sum_s l_s e^{m_s - m}.
-// One CTA per query head, or one warp (MERGE_WARPS = 1, eight to a CTA) while there are no more than eight slices. A warp takes eight neighbouring slices at a time, their vectors requested before anything else;
+// One CTA per query head, or one warp (MERGE_WARPS = 1, eight to a CTA) while there are no more than eight slices. A warp takes
+// eight neighbouring slices at a time, their vectors requested before anything else;
 // beside them every warp reads the maxima and sums of all slices, lanes along the slices, and has the common maximum and the
 // denominator to itself: warps meet once, to add their vectors. Every slice of the scratch buffers is written by the split-KV
 // kernel (an empty one as max = -inf, sum = 0), so nothing here depends on the position counter.
-// Bound by two trips to L2, the launch and the fetch of its code.
+// Bound by two trips to L2, the launch and the fetch of its code. Against maxima folded slice by slice, a launch behind the other:
+// 4.0 -> 3.2 us (one sequence at context 4096), 7.2 -> 5.3 (eight at 8192).
 template <int MERGE_WARPS>
 __global__ void __launch_bounds__(MERGE_WARPS == 1 ? 256 : MERGE_WARPS * 32)
 attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* out, uint32_t heads, uint32_t rep, uint32_t hd,
