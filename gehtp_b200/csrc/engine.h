@@ -191,7 +191,9 @@ constexpr uint32_t kGraphRows = 8;
 // the value of a row argument in the coming run
 inline uint32_t rows_of(uint32_t arg) { return arg == WT_ROWS_AUTO ? g.run_rows : arg == WT_SEL_AUTO ? g.run_sel : arg; }
 // fuse.cu
-void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector<uint8_t>& internal, std::vector<uint8_t>& dead);
+// `holds`: temps that a chain reads until its last op, whatever its ops by themselves do (temp, from op, to op)
+struct LiveHold { uint32_t temp, from, to; };
+void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector<uint8_t>& internal, std::vector<uint8_t>& dead, std::vector<LiveHold>& holds);
 void fuse_materialize(const wt_blob* b);
 // Marks the ops whose result is a constant of the blob (PlanOp::const_fold). addr / maxb: device address and capacity
 // of every temp id of the plan.

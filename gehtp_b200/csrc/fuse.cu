@@ -35,6 +35,7 @@
 #include <functional>
 #include <map>
 #include <utility>
+#include "common.cuh"
 #include "engine.h"
 #include "launchers.h"
 #include "launchers_attn.h"
@@ -457,6 +458,9 @@ bool match_qkv_split_rope(const Graph& G, const std::vector<PlanOp>& meas, uint3
     return true;
 }
 
+// kind 6: both W4A16 projections and the tail run as one GEMM that stores neither product
+bool one_launch(const Span& sp) { return !sp.f16 && sp.K && !g.exact_ops && w4a16_gemm_sm100_swiglu_takes(sp.M, sp.K, sp.N); }
+
 // The SwiGLU chain of match_swiglu with more rows than the fused GEMV form takes, or with fp16 weights: the two
 // projections keep their own launches (GEMMs) and the three elementwise ops become one kernel.
 bool match_swiglu_tail(const Graph& G, uint32_t ip, Span& sp) {
@@ -487,7 +491,8 @@ bool match_swiglu_tail(const Graph& G, uint32_t ip, Span& sp) {
     // one input and one K: the pair can also run as the gate | up GEMM
     sp.M = gt.args[3]; sp.N = gt.args[5]; sp.K = (gt.args[0] == u.args[0] && gt.args[4] == u.args[4]) ? gt.args[4] : 0;
     sp.wg = gt.args[1]; sp.wu = u.args[1]; sp.f16 = proj == OP_MATMUL_F16;
-    return true;
+    // one temp for the gate, the up projection and the result: the tail has no place to keep the gate's part
+    return one_launch(sp) || sp.gate_t != sp.up_t || sp.y != sp.up_t;
 }
 
 // TRANSPOSE_GEN of a [heads][rows][d] tensor to [rows][heads * d] whose only reader is the W4A16 GEMM right behind it
@@ -679,8 +684,9 @@ bool touch(const uint16_t* a, size_t n, const uint16_t* b, size_t m) { return a 
 
 // Finds the chains. `internal[t]` is set for temp ids written only inside
 // fused chains (and not among a chain's outputs): they need no memory.
-void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector<uint8_t>& internal, std::vector<uint8_t>& dead) {
+void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector<uint8_t>& internal, std::vector<uint8_t>& dead, std::vector<LiveHold>& holds) {
     g_spans.clear();
+    holds.clear();
     internal.assign(kMaxTemps, 0);
     dead.assign(b->n_ops, 0);
     Graph G;
@@ -738,6 +744,12 @@ void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector
     for (uint32_t i = 0; i + 1 < b->n_ops; i++) {
         Span sp{};
         if (!taken[i] && !taken[i + 1] && (match_tanh_resid(G, i, sp) || match_window_step(G, i, sp) || match_picked_norm(G, i, sp))) claim(sp);
+    }
+    // A chain reads some inputs later than its ops do: their bytes are not another's before the chain is done. SwiGLU behind two
+    // launches reads the gate once the up projection is there; its result may still take the gate's place, whole.
+    for (const Span& sp : g_spans) {
+        const uint32_t first = sp.ops.front(), last = sp.ops.back();
+        if (sp.kind == 6 && !one_launch(sp) && g.static_off[sp.gate_t] != g.static_off[sp.y]) holds.push_back({sp.gate_t, first, last});
     }
     // temps written only by interior ops of chains
     std::vector<int> writes_in(kMaxTemps, 0), writes_out(kMaxTemps, 0);
@@ -989,10 +1001,25 @@ void fuse_materialize(const wt_blob* b) {
             if ((((uintptr_t)gt) | ((uintptr_t)up) | ((uintptr_t)y)) & 15u) continue;
             auto lg = pg.launch, lu = pu.launch;
             size_t n = sp.n;
-            // the result may lie where the gate lay, whole; where it covers the gate in part, the ops stay apart
-            if (y != gt && touch(y, n, gt, n)) continue;
-            // both projections and the elementwise tail in one launch when they share input and shape, and the result does not lie
-            // on the input, which other CTAs still read
+            // Two projections and the elementwise tail, as far as the places allow: the result may lie where the gate lay, whole. The gate
+            // is dead once it has met its sigmoid, so a sound table may lay the up projection on it; then the three elementwise
+            // ops run where they stand, by way of the result's place.
+            const uint32_t K_up = b->ops[sp.up_op].args[4];
+            const uint16_t* in = (const uint16_t*)resolve(b, b->ops[sp.up_op].args[0]);
+            const bool over = touch(gt, n, up, n), at_gate = touch(y, n, gt, n), at_up = touch(y, n, up, n);
+            std::function<void(cudaStream_t)> apart;
+            if (!over && (y == gt || !at_gate) && (y == up || !at_up))
+                apart = [=](cudaStream_t st) { lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n); };
+            else if (over && !at_gate && !at_up && in && !touch(y, n, in, (size_t)sp.M * K_up))
+                apart = [=](cudaStream_t st) {
+                    lg(st);
+                    k_unary(st, gt, y, (uint32_t)n, 8);
+                    k_binary(st, gt, y, y, (uint32_t)n, 2, false);
+                    lu(st);
+                    k_binary(st, y, up, y, (uint32_t)n, 2, false);
+                };
+            // both projections and the tail in one launch when they share input and shape, and the result does not lie on the input, which
+            // other CTAs still read
             const uint16_t* act = sp.K ? (const uint16_t*)resolve(b, sp.a_ref) : nullptr;
             if (act && touch(y, n, act, (size_t)sp.M * sp.K)) act = nullptr;
             auto find = [&](uint32_t wref) -> const W4Packed* {
@@ -1000,27 +1027,30 @@ void fuse_materialize(const wt_blob* b) {
                 auto it = g.w4.find(key);
                 return it == g.w4.end() ? nullptr : &it->second;
             };
+            const uint32_t M = sp.M, K = sp.K, N = sp.N;
+            if (apart) head.fused = apart;
             if (sp.f16) {
-                const uint16_t *wg = act ? (const uint16_t*)resolve(b, sp.wg) : nullptr, *wu = act ? (const uint16_t*)resolve(b, sp.wu) : nullptr;
+                // this form stores both products
+                const bool clear = act && !over && !touch(gt, n, act, (size_t)M * K) && !touch(up, n, act, (size_t)M * K);
+                const uint16_t *wg = (const uint16_t*)resolve(b, sp.wg), *wu = (const uint16_t*)resolve(b, sp.wu);
                 uint16_t *gw = (uint16_t*)gt, *uw = (uint16_t*)up;
-                const uint32_t M = sp.M, K = sp.K, N = sp.N;
-                head.fused = [=](cudaStream_t st) {
-                    if (wg && wu && !g.exact_ops && k_matmul_f16_swiglu(st, act, wg, wu, gw, uw, y, M, K, N)) return;
-                    lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n);
-                };
-            }
-            const W4Packed *wg = act && !sp.f16 ? find(sp.wg) : nullptr, *wu = act && !sp.f16 ? find(sp.wu) : nullptr;
-            if (!sp.f16 && wg && wu && !g.exact_ops && w4a16_gemm_sm100_swiglu_takes(sp.M, sp.K, sp.N) && !(((uintptr_t)act) & 15u)) {
-                const uint32_t *qg = wg->packed, *qu = wu->packed;
-                const uint16_t *sg = wg->scales, *su = wu->scales;
-                const uint32_t M = sp.M, K = sp.K, N = sp.N;
-                unsigned int* status = g.d_status;
-                head.fused = [=](cudaStream_t st) {
-                    if (k_w4a16_gemm_sm100_swiglu(st, act, qg, sg, qu, su, y, M, K, N, status)) return;
-                    lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n);
-                };
-            } else if (!sp.f16) {
-                head.fused = [=](cudaStream_t st) { lg(st); lu(st); k_swiglu_tail(st, gt, up, y, n); };
+                if (apart && clear && wg && wu)
+                    head.fused = [=](cudaStream_t st) {
+                        if (g.exact_ops || !k_matmul_f16_swiglu(st, act, wg, wu, gw, uw, y, M, K, N)) apart(st);
+                    };
+            } else if (act && !g.exact_ops && w4a16_gemm_sm100_swiglu_takes(M, K, N) && !(((uintptr_t)act) & 15u)) {
+                const W4Packed *wg = find(sp.wg), *wu = find(sp.wu);
+                if (wg && wu) {
+                    const uint32_t *qg = wg->packed, *qu = wu->packed;
+                    const uint16_t *sg = wg->scales, *su = wu->scales;
+                    unsigned int* status = g.d_status;
+                    unsigned int* failed = g.h_status;
+                    head.fused = [=](cudaStream_t st) {
+                        if (k_w4a16_gemm_sm100_swiglu(st, act, qg, sg, qu, su, y, M, K, N, status)) return;
+                        if (apart) apart(st);
+                        else *(volatile unsigned int*)failed = kStatusGemmTimeout;      // places that no other form takes: the run fails
+                    };
+                }
             }
         } else if (sp.kind == 4) {
             const uint16_t *q = (const uint16_t*)resolve(b, sp.pq), *k = (const uint16_t*)resolve(b, sp.pk),

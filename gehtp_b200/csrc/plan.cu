@@ -754,7 +754,9 @@ int build_plan(const wt_blob* b, char* err, size_t errn) {
     std::vector<uint8_t> dead_ops;
     if (fusing) {
         std::vector<uint8_t> internal;
-        fuse_analyze(b, meas, internal, dead_ops);
+        std::vector<LiveHold> holds;
+        fuse_analyze(b, meas, internal, dead_ops, holds);
+        for (const LiveHold& h : holds) P.live[h.temp].push_back({h.from, h.to});
         for (uint32_t i = 0; i < kMaxTemps; i++) P.internal[i] = internal[i] != 0;
     }
 
