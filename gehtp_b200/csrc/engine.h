@@ -190,6 +190,8 @@ bool tp_p2p_add_rmsnorm(cudaStream_t st, const uint16_t* a, uint16_t* r, const u
 constexpr uint32_t kGraphRows = 8;
 // the value of a row argument in the coming run
 inline uint32_t rows_of(uint32_t arg) { return arg == WT_ROWS_AUTO ? g.run_rows : arg == WT_SEL_AUTO ? g.run_sel : arg; }
+// `arg` names a slot that keeps its bytes for a whole run: only memory-planner ops write slots
+bool const_slot(const wt_blob* b, uint32_t arg);
 // fuse.cu
 // `holds`: temps that a chain reads until its last op, whatever its ops by themselves do (temp, from op, to op)
 struct LiveHold { uint32_t temp, from, to; };

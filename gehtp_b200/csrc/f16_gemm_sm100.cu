@@ -406,7 +406,8 @@ f16_gemv_nk_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* 
 // 8 values feed two MMAs. Which of the 16 k slots of an MMA a value takes does not matter as long as A and B
 // agree, so no shuffling into the fragment order is needed: one 16-byte load per operand and chunk, 2 MMAs,
 // where the scalar form above spends some 140 instructions on the same 8 weights at 8 rows.
-// The first batch of weights (constants) is requested before the dependency wait.
+// The first batch of weights is requested before the dependency wait where they are constants of the run; a second operand that the
+// launch in front may have written is read behind it.
 // Bound by DRAM where the matrix is large (vocabulary) and by the latency of one warp's share of K where it is small:
 // one warp per 8 columns left a projection to 1024 columns on 16 SMs.
 // DUAL: the gate and the up matrix of a gated feed-forward in one launch, as many warps again behind each group for the
@@ -414,7 +415,7 @@ f16_gemv_nk_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* 
 struct GemvDual { const uint16_t* w; uint16_t *gate, *up; };
 template <int KS, int UNR, bool DUAL>
 __global__ void __launch_bounds__(256)
-f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, const GemvDual du) {
+f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, bool w_const, const GemvDual du) {
     extern __shared__ __align__(16) unsigned char smem_a[];      // [rows][K * 2 + 64] bytes: rows 64 bytes apart in the banks
     __shared__ float part[KS > 1 || DUAL ? 8 : 1][64];
     constexpr int WG = DUAL ? 2 * KS : KS;                       // warps of a group of 8 columns
@@ -425,6 +426,7 @@ f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t*
     const uint16_t* wm = DUAL && warp % WG >= KS ? du.w : w;
     const uint4* wr = (const uint4*)(wm + (size_t)min(n0 + g, N - 1) * K) + t;     // chunk kc lies 4 * kc further
     uint4 wq[UNR];
+    if (!w_const) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
     for (int u = 0; u < UNR; u++) wq[u] = (active && ks + u * KS < KC) ? __ldcs(wr + 4 * (ks + u * KS)) : make_uint4(0, 0, 0, 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -483,12 +485,12 @@ f16_gemv_mma_kernel(const uint16_t* a, const uint16_t* __restrict__ w, uint16_t*
 }
 
 template <int KS, bool DUAL = false>
-bool launch_gemv_mma(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, const GemvDual& du = {}) {
+bool launch_gemv_mma(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, bool w_const, const GemvDual& du = {}) {
     const size_t smem = (size_t)(M < 8 ? M : 8) * (K * 2 + 64);
     static int have[64] = {};
     if (K % 32 || smem > 200 * 1024 || (smem > 40 * 1024 && !ensure_dyn_smem(f16_gemv_mma_kernel<KS, 8, DUAL>, smem, have))) return false;
     const uint32_t cols = 8 * (8 / KS) / (DUAL ? 2 : 1);
-    if (launch_pdl(f16_gemv_mma_kernel<KS, 8, DUAL>, dim3((N + cols - 1) / cols, (M + 7) / 8), dim3(256), smem, st, a, w, y, M, K, N, ldy, du) != cudaSuccess) {
+    if (launch_pdl(f16_gemv_mma_kernel<KS, 8, DUAL>, dim3((N + cols - 1) / cols, (M + 7) / 8), dim3(256), smem, st, a, w, y, M, K, N, ldy, w_const, du) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -497,12 +499,12 @@ bool launch_gemv_mma(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint
 }
 
 // K shares per column group: enough CTAs for two per SM, a share of at least one batch of chunks
-bool launch_gemv_mma_any(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy) {
+bool launch_gemv_mma_any(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N, uint32_t ldy, bool w_const) {
     const uint32_t KC = K / 32, groups = (N + 7) / 8;
-    if (groups >= 8 * 296 || KC < 16) return launch_gemv_mma<1>(st, a, w, y, M, K, N, ldy);
-    if (groups >= 4 * 296 || KC < 32) return launch_gemv_mma<2>(st, a, w, y, M, K, N, ldy);
-    if (groups >= 2 * 296 || KC < 64) return launch_gemv_mma<4>(st, a, w, y, M, K, N, ldy);
-    return launch_gemv_mma<8>(st, a, w, y, M, K, N, ldy);
+    if (groups >= 8 * 296 || KC < 16) return launch_gemv_mma<1>(st, a, w, y, M, K, N, ldy, w_const);
+    if (groups >= 4 * 296 || KC < 32) return launch_gemv_mma<2>(st, a, w, y, M, K, N, ldy, w_const);
+    if (groups >= 2 * 296 || KC < 64) return launch_gemv_mma<4>(st, a, w, y, M, K, N, ldy, w_const);
+    return launch_gemv_mma<8>(st, a, w, y, M, K, N, ldy, w_const);
 }
 
 template <int MR>
@@ -574,27 +576,27 @@ bool launch_tiles(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16
 // steps, us, GEMV / GEMM: 9 rows 1242 / 1340, 12 rows 1288 / 1287, 16 rows 1369 / 1343, 17 rows 1690 / 1395, 31 rows 2272 / 1538.
 static bool gemm_takes(uint32_t M, uint32_t K, uint32_t N) { return M >= 16 && K % BK == 0 && N % 128 == 0; }
 
-// y = gated feed-forward of two matrices of one shape, M < 32; gate and up get the two products. false: not taken
+// y = gated feed-forward of two matrices of one shape, constants of the run, M < 32; gate and up get the two products. false: not taken
 bool k_matmul_f16_swiglu(cudaStream_t st, const uint16_t* a, const uint16_t* wg, const uint16_t* wu, uint16_t* gate, uint16_t* up, uint16_t* y,
                          uint32_t M, uint32_t K, uint32_t N) {
     if (!M || M >= 32 || gemm_takes(M, K, N) || !K || !N || (K & 31u) || ((((uintptr_t)a) | ((uintptr_t)wg) | ((uintptr_t)wu)) & 15u)) return false;
     const GemvDual du{wu, gate, up};
     // the shares of launch_gemv_mma_any, up to what a CTA of 8 warps has for two matrices: the same sums
     const uint32_t KC = K / 32, groups = (N + 7) / 8;
-    if (groups >= 8 * 296 || KC < 16) return launch_gemv_mma<1, true>(st, a, wg, y, M, K, N, N, du);
-    if (groups >= 4 * 296 || KC < 32) return launch_gemv_mma<2, true>(st, a, wg, y, M, K, N, N, du);
-    return launch_gemv_mma<4, true>(st, a, wg, y, M, K, N, N, du);
+    if (groups >= 8 * 296 || KC < 16) return launch_gemv_mma<1, true>(st, a, wg, y, M, K, N, N, true, du);
+    if (groups >= 4 * 296 || KC < 32) return launch_gemv_mma<2, true>(st, a, wg, y, M, K, N, N, true, du);
+    return launch_gemv_mma<4, true>(st, a, wg, y, M, K, N, N, true, du);
 }
 
 // Y[M, N] (rows ldy apart) = A[M, K] . W^T, W stored [N, K]. false: shape or alignment outside what the
-// tensor-core forms take (the caller then runs the exact kernel); nothing launched.
+// tensor-core forms take (the caller then runs the exact kernel); nothing launched. w_const: W is a constant of the run.
 bool k_matmul_f16_nk(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M, uint32_t K, uint32_t N,
-                     uint32_t ldy, unsigned int* status) {
+                     uint32_t ldy, bool w_const, unsigned int* status) {
     if (!M || !K || !N || (K & 7u) || ((((uintptr_t)a) | ((uintptr_t)w)) & 15u)) return false;
     if (gemm_takes(M, K, N) && (ldy & 7u) == 0 && ((uintptr_t)y & 15u) == 0) return launch_tiles(st, a, K, w, EpiF16{y, ldy}, M, K, N, status);
     if (M >= 32) return false;
     static const int mma_on = [] { const char* e = std::getenv("GEHTP_CUDA_F16_GEMV_MMA"); return e ? std::atoi(e) : 1; }();
-    if (mma_on && launch_gemv_mma_any(st, a, w, y, M, K, N, ldy)) return true;
+    if (mma_on && launch_gemv_mma_any(st, a, w, y, M, K, N, ldy, w_const)) return true;
     return M <= 4 ? launch_gemv<4>(st, a, w, y, M, K, N, ldy) : launch_gemv<8>(st, a, w, y, M, K, N, ldy);
 }
 

@@ -236,13 +236,10 @@ bool slot_row(const Graph& G, int bc, uint32_t n, uint32_t rows, uint32_t& slot_
         src = q.args[0];
         first = q.args[4];
     }
-    if (!(src & 0x8000u) || (src & 0x4000u)) return false;
+    if (!(src & 0x8000u)) return false;
     const uint32_t s = src & 0x7FFFu;
     if (s >= b->n_slots || (b->slots[s].addr != 0 && b->slots[s].addr != WT_SLOT_EXT_IN) || ((uint64_t)first + n) * 2 > b->slots[s].len) return false;
-    for (uint32_t i = 0; i < b->n_ops; i++) {
-        const uint32_t oc = b->ops[i].opcode;
-        if (oc == OP_SPILL || oc == OP_FILL || oc == OP_DMA) return false;
-    }
+    if (!const_slot(b, src)) return false;
     slot_ref = src;
     return true;
 }
@@ -1030,8 +1027,8 @@ void fuse_materialize(const wt_blob* b) {
             const uint32_t M = sp.M, K = sp.K, N = sp.N;
             if (apart) head.fused = apart;
             if (sp.f16) {
-                // this form stores both products
-                const bool clear = act && !over && !touch(gt, n, act, (size_t)M * K) && !touch(up, n, act, (size_t)M * K);
+                // this form stores both products, and reads the weights ahead of the launch in front
+                const bool clear = act && const_slot(b, sp.wg) && const_slot(b, sp.wu) && !over && !touch(gt, n, act, (size_t)M * K) && !touch(up, n, act, (size_t)M * K);
                 const uint16_t *wg = (const uint16_t*)resolve(b, sp.wg), *wu = (const uint16_t*)resolve(b, sp.wu);
                 uint16_t *gw = (uint16_t*)gt, *uw = (uint16_t*)up;
                 if (apart && clear && wg && wu)

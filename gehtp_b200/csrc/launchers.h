@@ -72,10 +72,11 @@ void k_matmul_f16(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_
                   uint32_t Bn);
 
 // W stored [N, K] on the tensor cores (M >= 16: TMA-fed tcgen05 GEMM) or as a streaming GEMV,
-// f16_gemm_sm100.cu; y rows are ldy elements apart. false: shape not taken, nothing launched.
+// f16_gemm_sm100.cu; y rows are ldy elements apart. w_const: no op of the run writes W, which is then read ahead of the launch
+// in front. false: shape not taken, nothing launched.
 bool k_matmul_f16_nk(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M,
-                     uint32_t K, uint32_t N, uint32_t ldy, unsigned int* status);
-// two such products and their SwiGLU chain in one launch (M < 32); the products go to gate and up. false: not taken
+                     uint32_t K, uint32_t N, uint32_t ldy, bool w_const, unsigned int* status);
+// two such products with constant W and their SwiGLU chain in one launch (M < 32); the products go to gate and up. false: not taken
 bool k_matmul_f16_swiglu(cudaStream_t st, const uint16_t* a, const uint16_t* wg, const uint16_t* wu, uint16_t* gate, uint16_t* up, uint16_t* y,
                          uint32_t M, uint32_t K, uint32_t N);
 

@@ -461,11 +461,11 @@ void plan_op(Planner& P, const wt_op& op, PlanOp& p) {
         p.engine = WT_ENG_HVX;
         // Weights stored [N, K], one matrix: tensor cores (M >= 16) or the streaming GEMV, unless
         // the one-kernel-per-op plan or a dump hook asks for the reference's summation order bit for bit.
-        const bool nk = t1 && !t0 && !(flags & 4u);
+        const bool nk = t1 && !t0 && !(flags & 4u), w_const = const_slot(b, a[1]);
         if (nk) p.engine = M >= 128 ? WT_ENG_HMX : WT_ENG_HVX;
         if (P.build) p.launch = [=](cudaStream_t st) {
             if (nk && g.opt_fuse && !g.exact_ops &&
-                k_matmul_f16_nk(st, x, w + (size_t)n0 * K, y + n0, M, K, N, N_full, g.d_status)) return;
+                k_matmul_f16_nk(st, x, w + (size_t)n0 * K, y + n0, M, K, N, N_full, w_const, g.d_status)) return;
             k_matmul_f16(st, x, w, y, M, K, N, n0, N_full, t0, t1, Bn);
         };
         return;
@@ -706,6 +706,15 @@ bool ranges_clash(const std::vector<LiveRange>& x, const std::vector<LiveRange>&
 }
 
 }  // namespace
+
+bool const_slot(const wt_blob* b, uint32_t arg) {
+    if (!(arg & 0x8000u) || (arg & 0x4000u)) return false;
+    for (uint32_t i = 0; i < b->n_ops; i++) {
+        const uint32_t oc = b->ops[i].opcode;
+        if (oc == OP_SPILL || oc == OP_FILL || oc == OP_DMA) return false;
+    }
+    return true;
+}
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
