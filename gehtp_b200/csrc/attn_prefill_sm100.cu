@@ -416,7 +416,7 @@ attn_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
             const float M = fmaxf(ml0.x, ml1.x);
             float f0 = ml0.x == -INFINITY ? 0.0f : ex2(ml0.x - M), f1 = ml1.x == -INFINITY ? 0.0f : ex2(ml1.x - M);
             const float l = ml0.y * f0 + ml1.y * f1;
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+            const float inv = l == 0.0f ? 0.0f : 1.0f / l;       // a sum that is no number makes no number of the row
             f0 *= inv; f1 *= inv;
             const uint32_t ta = tmem + ((quarter * 32) << 16) + 256 + t * 64;
             // the warp's 32 rows of 128 bytes by way of shared memory: 8 lanes to a row, a request touches four (a row to a lane touched

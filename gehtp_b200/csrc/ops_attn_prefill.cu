@@ -192,7 +192,7 @@ attn_prefill_kernel(PrefillArgs A) {
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 const float mr = m_run[c >> 1];
-                const float e = (mr == -INFINITY) ? 0.0f : __expf(s[nb][c] - mr);
+                const float e = __expf(s[nb][c] - (mr == -INFINITY ? 0.0f : mr));      // 0 for -inf; a score that is no number stays one
                 s[nb][c] = e;
                 l_run[c >> 1] += e;
             }
@@ -231,7 +231,7 @@ attn_prefill_kernel(PrefillArgs A) {
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
     }
-    const float inv0 = l_run[0] > 0.0f ? 1.0f / l_run[0] : 0.0f, inv1 = l_run[1] > 0.0f ? 1.0f / l_run[1] : 0.0f;
+    const float inv0 = l_run[0] == 0.0f ? 0.0f : 1.0f / l_run[0], inv1 = l_run[1] == 0.0f ? 0.0f : 1.0f / l_run[1];
 #pragma unroll
     for (int i = 0; i < DBLK; i++) {
         const int d = i * 8 + 2 * t;
