@@ -230,7 +230,7 @@ attn_decode_split_kernel(AttnDecodeArgs A, uint32_t kv_heads_total) {
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         float mr = m_run[c >> 1];
-                        float e = (mr == -INFINITY) ? 0.0f : __expf(x[nb][c] - mr);
+                        float e = __expf(x[nb][c] - (mr == -INFINITY ? 0.0f : mr));
                         pv[nb][c] = e;
                         l_run[c >> 1] += e;
                     }
@@ -424,7 +424,7 @@ attn_decode_group_kernel(AttnDecodeArgs A, uint32_t kv_heads_total) {
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         float mr = m_run[c >> 1];
-                        float e = (mr == -INFINITY) ? 0.0f : __expf(x[nb][c] - mr);
+                        float e = __expf(x[nb][c] - (mr == -INFINITY ? 0.0f : mr));
                         pv[nb][c] = e;
                         l_run[c >> 1] += e;
                     }
@@ -647,7 +647,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap, AttnDecodeArgs 
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     float mr = m_run[c >> 1];
-                    float e = (mr == -INFINITY) ? 0.0f : __expf(x[nb][c] - mr);
+                    float e = __expf(x[nb][c] - (mr == -INFINITY ? 0.0f : mr));
                     pv[nb][c] = e;
                     l_run[c >> 1] += e;
                 }
@@ -699,7 +699,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap, AttnDecodeArgs 
 // eight neighbouring slices at a time, their vectors requested before anything else;
 // beside them every warp reads the maxima and sums of all slices, lanes along the slices, and has the common maximum and the
 // denominator to itself: warps meet once, to add their vectors. Every slice of the scratch buffers is written by the split-KV
-// kernel (an empty one as max = -inf, sum = 0), so nothing here depends on the position counter.
+// kernel (an empty one as max = -inf, sum = 0), so nothing here depends on the position counter. Scores that are no numbers leave
+// the maximum as it is and make the sum one: a sum behind a maximum of -inf counts as it stands.
 // Bound by two trips to L2, the launch and the fetch of its code. Against maxima folded slice by slice, a launch behind the other:
 // 4.0 -> 3.2 us (one sequence at context 4096), 7.2 -> 5.3 (eight at 8192).
 template <int MERGE_WARPS>
@@ -748,7 +749,7 @@ attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* ou
                 den *= m == -INFINITY ? 0.0f : __expf(m - m_new);
                 m = m_new;
 #pragma unroll
-                for (uint32_t u = 0; u < 4; u++) den += v[u].x == -INFINITY ? 0.0f : v[u].y * __expf(v[u].x - m);
+                for (uint32_t u = 0; u < 4; u++) den += v[u].x == -INFINITY ? v[u].y : v[u].y * __expf(v[u].x - m);
             }
             den = warp_sum(den);
         }
@@ -764,7 +765,7 @@ attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* ou
     if (MERGE_WARPS == 1) {                                   // heads past the last: the last one again, the same values
         uint16_t o[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) o[e] = f2h(den > 0.0f ? acc[e] / den : 0.0f);
+        for (int e = 0; e < 4; e++) o[e] = f2h(den == 0.0f ? 0.0f : acc[e] / den);
         uint32_t* dst = (uint32_t*)(out + (size_t)h * hd + at);
         dst[0] = o[0] | ((uint32_t)o[1] << 16);
         if (hd == 128) dst[1] = o[2] | ((uint32_t)o[3] << 16);
@@ -778,7 +779,7 @@ attn_decode_merge_kernel(const float* part_o, const float* part_ml, uint16_t* ou
         float num = 0.0f;
 #pragma unroll
         for (int w = 0; w < MERGE_WARPS; w++) num += s_acc[w][d];
-        out[(size_t)h * hd + d] = f2h(den > 0.0f ? num / den : 0.0f);
+        out[(size_t)h * hd + d] = f2h(den == 0.0f ? 0.0f : num / den);
     }
     // all readers of the counter in this launch must be done before it moves: the
     // last block to finish advances it
