@@ -283,14 +283,17 @@ chunk_walk_kernel(const ChunkArgs c) {
     auto x_of = [&](uint32_t ch) { return sm + ch % NB * O_K; };
     auto rest_of = [&](uint32_t ch) { return sm + NB * O_K + ch % NB * (STAGE - O_K) - O_K; };     // indexed like an item
     bool lost = false;
+    uint32_t asked[2] = {0, 0};                               // chunks whose copies thread 0 has requested
     auto fetch_x = [&](uint32_t ch) {                         // one thread
         if (ch >= n || lost) return;
+        asked[0] = ch + 1;
         uint64_t* bar = &full[0][ch % NB];
         sm100::mbar_expect_tx(bar, O_K * 4);
         sm100::bulk_load(x_of(ch), items + ch * item_floats(V), O_K * 4, bar);
     };
     auto fetch_rest = [&](uint32_t ch) {
         if (ch >= n || lost) return;
+        asked[1] = ch + 1;
         const float* src = items + ch * item_floats(V);
         uint64_t* bar = &full[1][ch % NB];
         sm100::mbar_expect_tx(bar, (STAGE - O_K) * 4);
@@ -406,7 +409,13 @@ chunk_walk_kernel(const ChunkArgs c) {
     for (int m = 0; m < 2; m++)
 #pragma unroll
         for (int e = 0; e < 4; e++) bad |= !finite(S[m][e]);
-    if (__syncthreads_or(lost)) return;
+    if (__syncthreads_or(lost)) {                             // copies on their way land before the CTA's shared memory is another's
+        if (tid == 0)
+            for (int part = 0; part < 2; part++)
+                for (uint32_t ch = asked[part] > NB ? asked[part] - NB : 0; ch < asked[part]; ch++) sm100::mbar_wait(&full[part][ch % NB], ch / NB & 1);
+        __syncthreads();
+        return;
+    }
     if (__syncthreads_or(bad)) { walk_tokens<A>(c, sm, h, c0); return; }
 #pragma unroll
     for (int m = 0; m < 2; m++)
