@@ -39,7 +39,7 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 constexpr unsigned int kStatusAllReduceTimeout = 0x80000001u;   // peer-memory all-reduce: a rank never wrote
 constexpr unsigned int kStatusAttnTimeout = 0x80000002u;        // decode attention: a K/V tile copy never arrived
 constexpr unsigned int kStatusGemmTimeout = 0x80000003u;        // tcgen05 GEMM: a pipeline barrier never completed
-constexpr unsigned int kStatusDeltaTimeout = 0x80000004u;       // channel-decay recurrence: a chunk's copy never arrived
+constexpr unsigned int kStatusDeltaTimeout = 0x80000004u;       // channel-decay recurrence: a chunk's copy never arrived; the state is a mix of old and new
 
 // Device status word: first failing op (1-based) wins.
 __device__ __forceinline__ void raise_status(unsigned int* status, unsigned int code) {

@@ -349,7 +349,7 @@ int status_message(unsigned int code, char* m, size_t mn) {
         std::snprintf(m, mn, "tcgen05 GEMM timed out on a pipeline barrier (output incomplete)");
         return -1;
     case kStatusDeltaTimeout:
-        std::snprintf(m, mn, "channel-decay recurrence timed out waiting for a chunk's copy (state unchanged)");
+        std::snprintf(m, mn, "channel-decay recurrence timed out waiting for a chunk's copy (output and state incomplete: reset the state)");
         return -1;
     default:
         if (code & 0x80000000u) { std::snprintf(m, mn, "device status 0x%08x", code); return -1; }

@@ -5,7 +5,7 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
-from .wtop import Engine
+from .wtop import Engine, EngineError
 
 
 class Session:
@@ -32,7 +32,12 @@ class Session:
         self._face[:n] = tokens
         self._face[self.man["max_rows"]:self.man["max_rows"] + len(sel)] = sel
         self.engine.set_rows(n, len(sel))
-        self.engine.run_io(self._face, out_temp, out)
+        try:
+            self.engine.run_io(self._face, out_temp, out)
+        except EngineError as e:
+            if e.rc < 0:          # failed on the device: states between two runs, of which no sequence can go on
+                self.reset()
+            raise
         self.position += n
 
     def _check(self, tokens):

@@ -150,6 +150,8 @@ def test_status_word_messages(cuda):
         assert frag in msg.value, msg.value
         seen.add(msg.value)
     assert len(seen) == 3
+    # the recurrence's CTAs store their columns by themselves: nothing vouches for the state
+    assert cuda.gehtp_cuda_status_message(0x80000004, msg, 160) == -1 and b"recurrence timed out" in msg.value and b"reset the state" in msg.value
     assert cuda.gehtp_cuda_status_message(7, msg, 160) == 7 and b"kv gather miss" in msg.value and b"op 6" in msg.value
     assert cuda.gehtp_cuda_status_message(0x80000077, msg, 160) == -1 and b"0x80000077" in msg.value
 
