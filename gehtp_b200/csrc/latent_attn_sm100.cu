@@ -7,6 +7,8 @@
 //   S = Q K^T   three boxes of 64 values, into TMEM
 //   P           fp32 scores, one thread per row; 2^(s - m) as hi + lo bf16 over S (as window_attn_sm100.cu)
 //   O += P V    P as the A operand from TMEM, V as it lies in memory
+// Hidden keys have weight 0, which a value that is no number turns into one. A row whose result is no number although the tiles held
+// keys it does not see is worked out once more over its own keys alone.
 // 2048 tokens of 16 heads: 36 us a layer, 146 with mma.sync products; 1500 tokens of 32 heads 46, 140; 64 tokens 7.9, 10.9.
 // Every mbarrier wait is bounded; on a timeout the CTA raises the engine's status word and winds down.
 #include <cuda.h>
@@ -31,9 +33,54 @@ struct __align__(8) LBars {
     float2 ml[2][BQ];                                           // row maximum and sum of the two groups
 };
 
+// Values 64 t .. + 63 of a row's result, two a lane, over the keys up to its position alone: a key per lane for the scores, a warp per
+// key for the values. Rows beside a value that is no number come here, no others.
+__device__ __noinline__ float2 row_alone(const LatentArgs& A, const uint16_t* kv, uint32_t h, uint32_t row, uint32_t pos, uint32_t t, float sc) {
+    const uint32_t lane = threadIdx.x & 31;
+    const size_t kw = (size_t)A.heads * (DIM + VD), ls = A.ls();
+    const uint4* q = (const uint4*)((const uint16_t*)A.q + ((size_t)row * A.heads + h) * (DIM + ROT));
+    const uint16_t* rot = (const uint16_t*)A.state + A.rank;
+    const uint16_t* val = kv + (size_t)A.heads * DIM + h * VD + t * 64 + 2 * lane;
+    auto dot = [](float s, uint4 x, uint4 y) {
+        const uint32_t a[4] = {x.x, x.y, x.z, x.w}, b[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            s = fmaf(__uint_as_float(a[i] & 0xffff0000u), __uint_as_float(b[i] & 0xffff0000u), fmaf(__uint_as_float(a[i] << 16), __uint_as_float(b[i] << 16), s));
+        return s;
+    };
+    float m = -INFINITY, l = 0.0f;
+    float2 o = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (uint32_t j0 = 0; j0 <= pos; j0 += 32) {
+        const uint32_t j = j0 + lane, n = min(32u, pos - j0 + 1);
+        float s = 0.0f;
+        if (lane < n) {
+            const uint4 *k = (const uint4*)(kv + j * kw + h * DIM), *r = (const uint4*)(rot + j * ls);
+#pragma unroll 4
+            for (uint32_t i = 0; i < DIM / 8; i++) s = dot(s, __ldcg(q + i), __ldcg(k + i));
+#pragma unroll 4
+            for (uint32_t i = 0; i < ROT / 8; i++) s = dot(s, __ldcg(q + DIM / 8 + i), __ldcg(r + i));
+        }
+        s = lane < n ? s * sc : -INFINITY;
+        const float mx = fmaxf(m, warp_max(s)), off = mx == -INFINITY ? 0.0f : mx, f = ex2(m - off), p = ex2(s - off);
+        m = mx;
+        l = l * f + p;
+        o.x *= f; o.y *= f;
+#pragma unroll 1
+        for (uint32_t i = 0; i < n; i++) {
+            const float w = __shfl_sync(0xffffffffu, p, i);
+            const uint32_t v = __ldcg((const uint32_t*)(val + (j0 + i) * kw));
+            o.x = fmaf(w, __uint_as_float(v << 16), o.x);
+            o.y = fmaf(w, __uint_as_float(v & 0xffff0000u), o.y);
+        }
+    }
+    const float f = A.gate[(size_t)row * A.heads + h] / warp_sum(l);
+    return make_float2(o.x * f, o.y * f);
+}
+
 __global__ void __launch_bounds__(NTHREADS, 1)
 latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_rot,
-                         const LatentArgs A, uint32_t rows, uint32_t past) {
+                         const LatentArgs A, const uint16_t* kv, uint32_t rows, uint32_t past) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sQ = smem;                                    // at the end the rows on their way out
@@ -233,6 +280,7 @@ latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             f0 *= f; f1 *= f;
             const uint32_t ta = tmem + ((quarter * 32) << 16) + 256 + t * 64;
             uint4* stage = (uint4*)sQ + (t * 4 + quarter) * 256;     // Q has been read by all products
+            float sum = 0.0f;                                        // no number if one of the row's values is none
 #pragma unroll 1
             for (int c = 0; c < 4; c++) {
                 uint32_t v[16], u[16], w[8];
@@ -245,12 +293,19 @@ latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 for (int e = 0; e < 8; e++) {
                     float x = __uint_as_float(v[2 * e]) * f0, y = __uint_as_float(v[2 * e + 1]) * f0;
                     if (two) { x = fmaf(__uint_as_float(u[2 * e]), f1, x); y = fmaf(__uint_as_float(u[2 * e + 1]), f1, y); }
+                    sum += (x - x) + (y - y);
                     w[e] = pack_bf2(x, y);
                 }
 #pragma unroll
                 for (int q = 0; q < 2; q++) stage[lane * 8 + ((c * 2 + q) ^ (lane & 7))] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
             }
             __syncwarp();
+            for (uint32_t bad = __ballot_sync(0xffffffffu, sum != 0.0f && row < rows && pos + 1 < min(n_kt * BKV, past + rows)); bad; bad &= bad - 1) {
+                const uint32_t r = __ffs(bad) - 1;
+                const float2 x = row_alone(A, kv, h, row - lane + r, pos - lane + r, t, sc);
+                ((uint32_t*)(stage + r * 8 + ((lane >> 2) ^ (r & 7))))[lane & 3] = pack_bf2(x.x, x.y);
+                __syncwarp();
+            }
             const uint32_t p = lane & 7;
 #pragma unroll 2
             for (uint32_t r = lane >> 3; r < 32; r += 4)
@@ -290,7 +345,7 @@ bool k_latent_sm100(cudaStream_t st, const LatentArgs& a, const uint16_t* kv, ui
     const size_t smem = 1024 + 3 * (size_t)K_BYTES + 2 * (size_t)V_BYTES + sizeof(LBars) + 16;
     static int have[64] = {};
     if (!ensure_dyn_smem(latent_attn_sm100_kernel, smem, have)) return false;
-    if (launch_pdl(latent_attn_sm100_kernel, dim3(a.heads, (rows + BQ - 1) / BQ), dim3(NTHREADS), smem, st, tq, tkv, trot, a, rows, past) != cudaSuccess) {
+    if (launch_pdl(latent_attn_sm100_kernel, dim3(a.heads, (rows + BQ - 1) / BQ), dim3(NTHREADS), smem, st, tq, tkv, trot, a, kv, rows, past) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -5,6 +5,7 @@ import pytest
 
 import ripidra_oracle
 import test_ripidra as rip
+from test_nonfinite_rows import _with_bad_token
 
 
 @pytest.mark.gpu
@@ -21,3 +22,21 @@ def test_rows(cuda, heads, kv_rank, sharp, cut):
         at += n
     s.close()
     assert rip.close(np.concatenate(got), want, "bfloat16")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("past,rows,bad", [(0, 96, 1), (0, 96, 95), (0, 200, 127), (0, 200, 128), (150, 200, 120), (1, 40, 17)])
+def test_rows_before_a_bad_token(cuda, value, past, rows, bad):
+    """Rows of a run in front of a token whose latent is no number, in its tile and in others."""
+    mt = _with_bad_token(rip.make([rip.latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=72, ff=None)], seed=bad, sharp=2.0), value)
+    tok = rip.ids(past + rows, seed=bad)
+    tok[past + bad] = mt[0]["vocab"] - 1
+    want = ripidra_oracle.run(*mt, tok[:past + bad])[0][past:, :-1]
+    s = rip.session(cuda, mt, "bfloat16", max_tokens=640)
+    if past:
+        s.feed(tok[:past], [0])
+    got = s.feed(tok[past:], range(rows))
+    s.close()
+    assert rip.close(got[:bad, :-1], want, "bfloat16")
+    assert not np.isfinite(got[bad:, :-1]).any()
