@@ -134,7 +134,7 @@ int gehtp_dev_w4a16_matmul(const uint16_t* a_dev, const uint32_t* packed_dev, co
     return 0;
 }
 
-// y[M, N] = a[M, K] . w^T with w stored [N, K] (fp16): tcgen05 GEMM for M >= 16, streaming GEMV for fewer
+// y[M, N] = a[M, K] . w^T with w stored [N, K] (fp16): tcgen05 GEMM from 32 rows, from 16 for large matrices, streaming GEMV for fewer
 int gehtp_dev_matmul_f16_nk(const uint16_t* a_dev, const uint16_t* w_dev, uint16_t* y_dev, uint32_t M, uint32_t K, uint32_t N) {
     if (!ensure_device(nullptr, 0)) return -1;
     if (!k_matmul_f16_nk(g.stream, a_dev, w_dev, y_dev, M, K, N, N, false, g.d_status)) return fail("matmul_f16 [N,K]: shape not taken by the tensor-core forms");

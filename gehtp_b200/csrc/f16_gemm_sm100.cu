@@ -2,12 +2,12 @@
 // (flags bit 1, the layout the reference's emitter gives every FullyConnected weight,
 // compiler/tools/wtop_ops/op_matmul.cpp:50):
 //
-//   M >= 16  : TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
+//   M >= 16  (below 32 by the size of the matrix, see gemm_takes): TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
 //              tile of W (BN rows x 64 k) land in shared memory by cp.async.bulk.tensor with the 128-byte
 //              swizzle that tcgen05.mma reads; accumulators live in TMEM, double-buffered so that the
 //              epilogue of a tile overlaps the main loop of the next. The reference takes its matrix
 //              unit from 128 rows on (exec_matmul_f16_hmx, kernels/src/runtime/oplist_exec.c:1600-1706).
-//   M <  16  (and below 32 where the GEMM does not take N or K): streaming GEMV, one warp per output column, 16-byte loads along K, fp32 accumulation,
+//   M <  32  otherwise: streaming GEMV, one warp per output column, 16-byte loads along K, fp32 accumulation,
 //              shuffle reduction (exec_matmul_f16_gemv, :1483-1590).
 //
 // Sums are formed in another order than the reference's ascending-k scalar loop, so results agree with
@@ -572,9 +572,19 @@ bool launch_tiles(cudaStream_t st, const uint16_t* a, uint32_t lda, const uint16
 
 }  // namespace
 
-// From 16 rows on a round over the weights for every 8 rows costs more than the GEMM. Four layers of the 28-layer shape, four
-// steps, us, GEMV / GEMM: 9 rows 1242 / 1340, 12 rows 1288 / 1287, 16 rows 1369 / 1343, 17 rows 1690 / 1395, 31 rows 2272 / 1538.
-static bool gemm_takes(uint32_t M, uint32_t K, uint32_t N) { return M >= 16 && K % BK == 0 && N % 128 == 0; }
+// The GEMV goes over the weights once for every 8 rows, the GEMM of one row tile takes 5 to 8 us whatever the matrix (runs of K, a
+// second launch for their sums). One product of a captured run, weights from HBM, us, GEMV / GEMM (K x N, rows):
+//     1024 x 1024  16: 2.6 / 6.5   31: 2.6 / 6.7       2048 x 1024  16: 4.1 / 6.9   20: 6.2 / 7.1   24: 7.7 / 7.2   31: 7.4 / 7.0
+//     1024 x 3072  16: 5.7 / 7.3   24: 6.2 / 7.6   25: 7.2 / 7.7   31: 8.3 / 8.2
+//     3072 x 1024  16: 5.6 / 6.9   17: 8.0 / 7.0   31: 10.6 / 7.0       1024 x 4096  16: 6.1 / 7.6   20: 7.7 / 7.6   31: 11.3 / 8.6
+//     4096 x 1024  16: 6.9 / 7.5   17: 9.6 / 7.5       1024 x 6144  16: 8.7 / 8.1       6144 x 1024  16: 11.6 / 8.2
+//     2560 x 2560  16: 13.8 / 8.6       9728 x 2560  16: 63.6 / 14.2   31: 110 / 15.2       1024 x 16384  16: 16.6 / 12.2   31: 27.7 / 11.6
+// The line below follows the rows and the matrix, N with what a warp pays whatever its columns; two rounds (16 rows) pay off later
+// than it says. From 32 rows on there is no GEMV.
+static bool gemm_takes(uint32_t M, uint32_t K, uint32_t N) {
+    if (M < 16 || K % BK || N % 128) return false;
+    return M >= 32 || ((uint64_t)M * K * (N + 1024) >= 105000000ull && (M > 16 || (uint64_t)K * N >= 5000000ull));
+}
 
 // y = gated feed-forward of two matrices of one shape, constants of the run, M < 32; gate and up get the two products. false: not taken
 bool k_matmul_f16_swiglu(cudaStream_t st, const uint16_t* a, const uint16_t* wg, const uint16_t* wu, uint16_t* gate, uint16_t* up, uint16_t* y,

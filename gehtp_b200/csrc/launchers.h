@@ -71,7 +71,7 @@ void k_matmul_f16(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_
                   uint32_t K, uint32_t N, uint32_t n0, uint32_t N_full, int t0, int t1,
                   uint32_t Bn);
 
-// W stored [N, K] on the tensor cores (M >= 16: TMA-fed tcgen05 GEMM) or as a streaming GEMV,
+// W stored [N, K] on the tensor cores (TMA-fed tcgen05 GEMM: from 32 rows, from 16 for large matrices) or as a streaming GEMV,
 // f16_gemm_sm100.cu; y rows are ldy elements apart. w_const: no op of the run writes W, which is then read ahead of the launch
 // in front. false: shape not taken, nothing launched.
 bool k_matmul_f16_nk(cudaStream_t st, const uint16_t* a, const uint16_t* w, uint16_t* y, uint32_t M,

@@ -459,7 +459,7 @@ void plan_op(Planner& P, const wt_op& op, PlanOp& p) {
         uint16_t* y = (uint16_t*)P.temp_get(a[2], (uint64_t)M * N_full * Balloc * 2u, p);
         if (!x || !w || !y) FAIL("matmul_f16 ref fail");
         p.engine = WT_ENG_HVX;
-        // Weights stored [N, K], one matrix: tensor cores (M >= 16) or the streaming GEMV, unless
+        // Weights stored [N, K], one matrix: tcgen05 GEMM or streaming GEMV by its size, unless
         // the one-kernel-per-op plan or a dump hook asks for the reference's summation order bit for bit.
         const bool nk = t1 && !t0 && !(flags & 4u), w_const = const_slot(b, a[1]);
         if (nk) p.engine = M >= 128 ? WT_ENG_HMX : WT_ENG_HVX;

@@ -42,6 +42,28 @@ def test_decode(cuda, hidden, ffn):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("hidden,ffn", [(256, 512), (1024, 3072), (2048, 2048)])
+@pytest.mark.parametrize("batch", [15, 16, 17, 25, 26, 31, 32])
+def test_decode_at_the_line_between_gemv_and_gemm(cuda, hidden, ffn, batch):
+    """Widths that both forms take; 1024 x 3072 changes between 25 and 26 rows, 2048 x 2048 between 16 and 17."""
+    cfg = _cfg(hidden, ffn)
+    blob, man = build_decode_runlist(cfg, batch, 64, quant="f16")
+    out = []
+    for fusion in (1, 0):
+        cuda.gehtp_cuda_set_fusion(fusion)
+        cuda.wt_exec_state_reset()
+        eng = Engine(cuda, blob)
+        for pos in range(2):
+            eng.run_io(decode_face(man, np.arange(batch) * 5 + pos, pos, cfg.head_dim, cfg.rope_theta), man["token_temp"])
+        out.append([eng.temp(man["logits_temp"])] + [eng.temp(t) for t in _products(eng)])
+        eng.shutdown()
+        cuda.wt_exec_state_reset()
+    cuda.gehtp_cuda_set_fusion(1)
+    for k, (a, b) in enumerate(zip(*out)):
+        assert_fp16_close(a, b, "batch %d, %s" % (batch, ("logits", "gate", "up")[k]))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tokens", [16, 33, 64, 100, 127, 128])
 def test_prefill(cuda, tokens):
     cfg = _cfg(256, 512)
