@@ -444,10 +444,12 @@ void launch(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
 
 }  // namespace
 
-// From two chunks on: 64 tokens of 16 heads, two layers, 430 -> 420 us a prompt; 40 tokens in fp32 636 -> 624. Below, what a chunk
-// costs in the two launches is not made up for.
+// From two chunks on while a CTA has an SM to itself, from four where two share one and a chunk takes longer; below, what a chunk costs
+// in the two launches is not made up for. A prompt of two such layers, token by token / in chunks, us: 16 heads, 32 tokens 427 / 417,
+// 64 tokens 432 / 414, fp32 40 tokens 628 / 619; 32 heads, 33 tokens 588 / 600, 47 tokens 597 / 606, 56 tokens 611 / 619, 64 tokens
+// 626 / 628, 80 tokens 638 / 632, 112 tokens 674 / 656.
 bool delta_chunks_take(const DeltaArgs& a, uint32_t rows) {
-    return a.dim == D && a.vdim % VC == 0 && rows >= 2 * T && (((uintptr_t)a.qkv | (uintptr_t)a.a | (uintptr_t)a.dt_bias | (uintptr_t)a.work) & 15) == 0;
+    return a.dim == D && a.vdim % VC == 0 && rows >= (a.vdim / VC * a.heads <= 148 ? 2 : 4) * T && (((uintptr_t)a.qkv | (uintptr_t)a.a | (uintptr_t)a.dt_bias | (uintptr_t)a.work) & 15) == 0;
 }
 
 size_t delta_chunks_floats(const DeltaArgs& a, uint32_t max_rows) {

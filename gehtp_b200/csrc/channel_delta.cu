@@ -3,14 +3,15 @@
 //   short_conv_kernel    causal depthwise convolution + silu; the last taps - 1 inputs are kept in the state, two banks:
 //                        a run reads the bank of its parity and writes the other, so that no CTA overwrites what
 //                        another still reads
-//   (heads of 128 key channels, runs of 32 rows and more: channel_chunks.cu)
+//   (heads of 128 key channels, runs of 32 or 64 rows and more: chunks of 16 tokens, channel_chunks.cu)
 //   delta_prep_kernel    unit vectors, decays, step sizes and the products of the vectors of four tokens, fp32
 //   delta_scan_kernel    the recurrence, four tokens at a time: S lives in registers, all reductions of the four run side
 //                        by side
 //   gated_norm_kernel    RMS norm of a head's read-out, weight, sigmoid gate
 //   delta_step_kernel    all of it for up to 4 rows, with the second halves of the low-rank decay and gate projections
 //
-// All of it is fp32, token after token: a cut of the prompt changes nothing but roundings.
+// All of it is fp32 here, token after token; the chunks work on three bf16 terms of fp32 values, sixteen tokens at a time. A cut of
+// the prompt changes nothing but roundings.
 #include <algorithm>
 #include <cooperative_groups.h>
 #include "launchers_rows.h"
@@ -630,7 +631,7 @@ void launch_scan(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, uint32
     else launch_scan_t<L, RPL, WIDE, true>(st, a, w, rows);
 }
 
-// 65 to 128 channels (128 of them only below 32 rows, see delta_chunks_take): 32 lanes of 4 rows while CTAs of 16 columns fit one to an SM. Beyond that the SM's issue slots count, and
+// 65 to 128 channels (128 of them only where delta_chunks_take refuses the rows): 32 lanes of 4 rows while CTAs of 16 columns fit one to an SM. Beyond that the SM's issue slots count, and
 // 16 lanes of 8 rows spend fewer exchanges on a token; of their two widths the one with less of a last round. 1024 tokens,
 // heads of 128 x 128, us: 16 heads 217 (16 lanes, 32 columns: 252; 16 lanes, 16 columns: 218), 32 heads 296 (253; 272),
 // 64 heads 591 (403; 441); two tokens at a time, before: 249, 263, 410.

@@ -27,6 +27,22 @@ def test_chunked_recurrence(cuda, heads, kv_heads, vdim, slow, cut):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("cut", [[31, 32, 33], [63, 64], [65, 16]])
+def test_lines_between_the_forms(cuda, cut):
+    """9 heads (72 CTAs) change to chunks at 32 rows, 19 heads (152 CTAs) at 64."""
+    for heads in (9, 19):
+        mt = rip.make([rip.delta(heads=heads, kv_heads=heads, dim=128, vdim=128, ff=None)], seed=heads, slow=1.0)
+        tok = rip.ids(sum(cut), seed=cut[0])
+        want = ripidra_oracle.run(*mt, tok)[0]
+        s, got, at = rip.session(cuda, mt, "bfloat16", max_tokens=256), [], 0
+        for n in cut:
+            got.append(s.feed(tok[at:at + n], range(n)))
+            at += n
+        s.close()
+        assert rip.close(np.concatenate(got), want, "bfloat16"), heads
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("value", [np.inf, np.nan])
 @pytest.mark.parametrize("rows,bad", [(32, 1), (40, 39), (60, 23), (50, 16)])
 def test_rows_in_front_of_a_bad_token(cuda, value, rows, bad):
