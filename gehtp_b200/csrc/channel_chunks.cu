@@ -445,9 +445,9 @@ void launch(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
 }  // namespace
 
 // From two chunks on while a CTA has an SM to itself, from four where two share one and a chunk takes longer; below, what a chunk costs
-// in the two launches is not made up for. A prompt of two such layers, token by token / in chunks, us: 16 heads, 32 tokens 427 / 417,
-// 64 tokens 432 / 414, fp32 40 tokens 628 / 619; 32 heads, 33 tokens 588 / 600, 47 tokens 597 / 606, 56 tokens 611 / 619, 64 tokens
-// 626 / 628, 80 tokens 638 / 632, 112 tokens 674 / 656.
+// in the two launches is not made up for. A run of two such layers and two of latent attention without the head, token by token /
+// in chunks, us: 16 heads, 32 tokens 314 / 308, 64 tokens 338 / 322, fp32 40 tokens 540 / 533; 32 heads, 33 tokens 438 / 450,
+// 40 tokens 442 / 447, 56 tokens 466 / 471, 64 tokens 478 / 477, 80 tokens 500 / 494, 128 tokens 559 / 534.
 bool delta_chunks_take(const DeltaArgs& a, uint32_t rows) {
     return a.dim == D && a.vdim % VC == 0 && rows >= (a.vdim / VC * a.heads <= 148 ? 2 : 4) * T && (((uintptr_t)a.qkv | (uintptr_t)a.a | (uintptr_t)a.dt_bias | (uintptr_t)a.work) & 15) == 0;
 }
