@@ -69,10 +69,21 @@ short_conv_kernel(const typename A::T* y, const float* __restrict__ w, float* st
     const uint32_t c = blockIdx.x * 256 + threadIdx.x;
     if (c >= C) return;
     const float* wc = w + (size_t)c * taps;
-    for (uint32_t r = r0; r < r1; r++) {
-        float s = 0.0f;
-        for (int j = 0; j < (int)taps; j++) s = fmaf(__ldg(wc + j), conv_in<A>(y, bank, (int)r - keep + j, c, ys, C, keep), s);
-        out[(size_t)r * C + c] = silu_f(s);
+    if (taps == 4) {
+        const float w0 = __ldg(wc), w1 = __ldg(wc + 1), w2 = __ldg(wc + 2), w3 = __ldg(wc + 3);
+        float x0 = conv_in<A>(y, bank, (int)r0 - 3, c, ys, C, 3), x1 = conv_in<A>(y, bank, (int)r0 - 2, c, ys, C, 3), x2 = conv_in<A>(y, bank, (int)r0 - 1, c, ys, C, 3);
+#pragma unroll 4
+        for (uint32_t r = r0; r < r1; r++) {
+            const float x3 = A::ld(y + (size_t)r * ys + c);
+            out[(size_t)r * C + c] = silu_f(fmaf(w3, x3, fmaf(w2, x2, fmaf(w1, x1, w0 * x0))));
+            x0 = x1; x1 = x2; x2 = x3;
+        }
+    } else {
+        for (uint32_t r = r0; r < r1; r++) {
+            float s = 0.0f;
+            for (int j = 0; j < (int)taps; j++) s = fmaf(__ldg(wc + j), conv_in<A>(y, bank, (int)r - keep + j, c, ys, C, keep), s);
+            out[(size_t)r * C + c] = silu_f(s);
+        }
     }
     if (r1 == rows) {
         float* next = state + (size_t)(par ^ 1u) * keep * C;
