@@ -659,9 +659,11 @@ void launch_scan_128(cudaStream_t st, const DeltaArgs& a, const DeltaWork& w, ui
 void k_short_conv(cudaStream_t st, const DeltaArgs& a, uint32_t rows) {
     if (!rows) return;
     const uint32_t C = a.channels();
-    // two channels a thread where they lie aligned, with the last rows in registers; 30 us one at a time, 24.6 so,
-    // at 6144 channels, 2048 rows
-    const bool pairs = a.taps == 4 && C % 2 == 0 && a.ys % 2 == 0 &&
+    // Two channels a thread where they lie aligned and one a thread would be more than six CTAs an SM; fewer are bound by their own chain,
+    // and half as many of them is no help. A run of two layers and two of latent attention, one / two channels, us: 6144 channels,
+    // 128 rows 357 / 359, 500 rows 458 / 464, 700 rows 559 / 556, 1200 rows 783 / 774, 2048 rows 1080 / 1063; 12288 channels, 200 rows
+    // 618 / 625, 300 rows 726 / 725, 350 rows 749 / 744, 1000 rows 1407 / 1389.
+    const bool pairs = (uint64_t)((C + 255) / 256) * ((rows + CONV_ROWS - 1) / CONV_ROWS) > 6 * 148 && a.taps == 4 && C % 2 == 0 && a.ys % 2 == 0 &&
                        (((uintptr_t)a.conv_w & 15u) | (((uintptr_t)a.y | (uintptr_t)a.conv_state | (uintptr_t)a.qkv) & 7u)) == 0;
     const dim3 grid((C / (pairs ? 2 : 1) + 255) / 256, (rows + CONV_ROWS - 1) / CONV_ROWS);
     auto go = [&](auto kernel, auto y) { launch_pdl(kernel, grid, dim3(256), 0, st, y, a.conv_w, a.conv_state, a.conv_count, a.qkv, rows, C, a.taps, a.ys); };

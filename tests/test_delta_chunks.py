@@ -43,6 +43,23 @@ def test_lines_between_the_forms(cuda, cut):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("cut", [[490, 3], [497, 2, 500]])
+def test_convolution_at_the_line_between_one_and_two_channels_a_thread(cuda, cut):
+    """7296 channels: 899 CTAs of one channel a thread at 496 rows and more."""
+    mt = rip.make([rip.delta(heads=19, kv_heads=19, dim=128, vdim=128, ff=None)], seed=4, slow=1.0)
+    tok = rip.ids(sum(cut), seed=cut[0])
+    want = ripidra_oracle.run(*mt, tok)[0]
+    for dtype in rip.DTYPES:
+        s, got, at = rip.session(cuda, mt, dtype, max_tokens=1024), [], 0
+        for n in cut:
+            got.append(s.feed(tok[at:at + n], [0, 1, n - 1]))
+            at += n
+        s.close()
+        at = np.cumsum([0] + cut[:-1])
+        assert rip.close(np.concatenate(got), np.concatenate([want[[a, a + 1, a + n - 1]] for a, n in zip(at, cut)]), dtype), dtype
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("value", [np.inf, np.nan])
 @pytest.mark.parametrize("rows,bad", [(32, 1), (40, 39), (60, 23), (50, 16)])
 def test_rows_in_front_of_a_bad_token(cuda, value, rows, bad):
