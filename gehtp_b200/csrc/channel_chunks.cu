@@ -282,18 +282,16 @@ chunk_walk_kernel(const ChunkArgs c) {
     const float* items = a.work + (size_t)h * n * item_floats(V);
     auto x_of = [&](uint32_t ch) { return sm + ch % NB * O_K; };
     auto rest_of = [&](uint32_t ch) { return sm + NB * O_K + ch % NB * (STAGE - O_K) - O_K; };     // indexed like an item
-    bool lost = false;
-    uint32_t asked[2] = {0, 0};                               // chunks whose copies thread 0 has requested
+    constexpr int NEVER = 0x7FFFFFFF;
+    int lost = NEVER;                                         // the chunk of the walk at which a wait ran out
     auto fetch_x = [&](uint32_t ch) {                         // one thread
-        if (ch >= n || lost) return;
-        asked[0] = ch + 1;
+        if (ch >= n || lost != NEVER) return;
         uint64_t* bar = &full[0][ch % NB];
         sm100::mbar_expect_tx(bar, O_K * 4);
         sm100::bulk_load(x_of(ch), items + ch * item_floats(V), O_K * 4, bar);
     };
     auto fetch_rest = [&](uint32_t ch) {
-        if (ch >= n || lost) return;
-        asked[1] = ch + 1;
+        if (ch >= n || lost != NEVER) return;
         const float* src = items + ch * item_floats(V);
         uint64_t* bar = &full[1][ch % NB];
         sm100::mbar_expect_tx(bar, (STAGE - O_K) * 4);
@@ -301,7 +299,7 @@ chunk_walk_kernel(const ChunkArgs c) {
         sm100::bulk_load(rest_of(ch) + SHARED, src + SHARED + blockIdx.x * UV, UV * 4, bar);
     };
     auto arrived = [&](int part, uint32_t ch) {
-        if (!lost && !sm100::mbar_wait(&full[part][ch % NB], ch / NB & 1)) { lost = true; raise_status(a.status, kStatusDeltaTimeout); }
+        if (lost == NEVER && !sm100::mbar_wait(&full[part][ch % NB], ch / NB & 1)) { lost = (int)ch - (part == 0); raise_status(a.status, kStatusDeltaTimeout); }
     };
     if (tid == 0) {
         for (int i = 0; i < 2 * NB; i++) sm100::mbar_init(&full[i / NB][i % NB], 1);
@@ -409,10 +407,14 @@ chunk_walk_kernel(const ChunkArgs c) {
     for (int m = 0; m < 2; m++)
 #pragma unroll
         for (int e = 0; e < 4; e++) bad |= !finite(S[m][e]);
-    if (__syncthreads_or(lost)) {                             // copies on their way land before the CTA's shared memory is another's
+    if (__syncthreads_or(lost != NEVER)) {
+        // Copies on their way land before the CTA's shared memory is another's. Thread 0 has requested what the walk asks for up to the
+        // chunk at which it gave up (-1: the first), or all of it; the last copy of each buffer is behind all earlier ones.
         if (tid == 0)
-            for (int part = 0; part < 2; part++)
-                for (uint32_t ch = asked[part] > NB ? asked[part] - NB : 0; ch < asked[part]; ch++) sm100::mbar_wait(&full[part][ch % NB], ch / NB & 1);
+            for (int part = 0; part < 2; part++) {
+                const uint32_t asked = lost == NEVER ? n : min(n, (uint32_t)(lost + NB + 1 - part));
+                for (uint32_t ch = asked > NB ? asked - NB : 0; ch < asked; ch++) sm100::mbar_wait(&full[part][ch % NB], ch / NB & 1);
+            }
         __syncthreads();
         return;
     }
