@@ -80,7 +80,7 @@ __device__ __noinline__ float2 row_alone(const LatentArgs& A, const uint16_t* kv
 
 __global__ void __launch_bounds__(NTHREADS, 1)
 latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_rot,
-                         const LatentArgs A, const uint16_t* kv, uint32_t rows, uint32_t past) {
+                         const __grid_constant__ LatentArgs A, const uint16_t* kv, uint32_t rows, uint32_t past) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sQ = smem;                                    // at the end the rows on their way out
