@@ -401,6 +401,14 @@ bool match_prefill_attention(const Graph& G, uint32_t ism, Span& sp) {
     return true;
 }
 
+// Operands that share bytes wherever the plan lays its temps: one temp, or places in the on-chip region.
+bool share_bytes(uint32_t t, uint64_t nt, uint32_t u, uint64_t nu) {
+    if (!is_temp_ref(t) || !is_temp_ref(u)) return false;
+    if (t == u) return true;
+    const uint64_t a = g.vtcm_off[t], b = g.vtcm_off[u];
+    return a != kNoOff && b != kNoOff && a < b + nu && b < a + nt;
+}
+
 bool match_swiglu(const Graph& G, uint32_t ip, Span& sp) {
     const wt_blob* b = G.b;
     const wt_op& pr = b->ops[ip];
@@ -414,6 +422,7 @@ bool match_swiglu(const Graph& G, uint32_t ip, Span& sp) {
     if (gt.args[0] != u.args[0] || gt.args[3] != u.args[3] || gt.args[4] != u.args[4] || gt.args[5] != u.args[5]) return false;
     uint32_t M = gt.args[3], n = M * gt.args[5];
     if (M > 64 || M >= w4_gemm_min_rows() || pr.args[3] != n || b->ops[act].args[3] != n || b->ops[sig].args[2] != n) return false;
+    if (share_bytes(pr.args[2], 2ull * n, gt.args[0], 2ull * M * gt.args[4])) return false;      // other CTAs still read the input
     std::vector<uint32_t> ops = {(uint32_t)gate, (uint32_t)sig, (uint32_t)act, (uint32_t)up, ip};
     uint32_t first;
     if (!contiguous(ops, first) || !closed(G, ops, {ip})) return false;
@@ -746,6 +755,8 @@ void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector
     // launches reads the gate once the up projection is there; its result may still take the gate's place, whole.
     for (const Span& sp : g_spans) {
         const uint32_t first = sp.ops.front(), last = sp.ops.back();
+        // both projections read the input in the launch that writes the result
+        if ((sp.kind == 1 || (sp.kind == 6 && sp.K)) && is_temp_ref(sp.a_ref)) holds.push_back({sp.a_ref, first, last});
         if (sp.kind == 6 && !one_launch(sp) && g.static_off[sp.gate_t] != g.static_off[sp.y]) holds.push_back({sp.gate_t, first, last});
     }
     // temps written only by interior ops of chains

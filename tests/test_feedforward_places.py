@@ -24,7 +24,7 @@ def _blob(quant, rows, N, ids, offsets):
         else:
             w.append(b.add_slot(np.ascontiguousarray(dequant_f16(nib, sc).T)))
     n = rows * N
-    if offsets:
+    if offsets:                                                   # entries for temps apart from one another keep their places
         size = {t: 2 * rows * K if t == X else 2 * n for t in offsets}
         b.add_tempoff(max(o + size[t] for t, o in offsets.items()), [(t, o, size[t]) for t, o in offsets.items()], bump_kb=64)
     op, flags = (OP.MATMUL_W4A16, []) if quant == "w4" else (OP.MATMUL_F16, [2])
@@ -86,3 +86,18 @@ def test_result_over_the_gate(cuda, quant, rows, N):
 @pytest.mark.parametrize("quant,rows,N", FORMS)
 def test_one_temp_for_gate_up_and_result(cuda, quant, rows, N):
     _check(cuda, quant, rows, N, ids={UP: GATE, Y: GATE}, fused=5 if (quant, N) == ("w4", 256) else 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("quant,rows,N", FORMS + [("w4", 3, 256)])
+def test_result_over_the_input(cuda, quant, rows, N):
+    """The input is dead behind the up projection; the forms of one launch read it until they are done."""
+    at = _far(rows, N)
+    _check(cuda, quant, rows, N, offsets={X: 0, GATE: at(0), UP: at(1), Y: 0})
+    _check(cuda, quant, rows, N, offsets={X: 512, GATE: at(0), UP: at(1), Y: 0})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("quant,rows,N", FORMS + [("w4", 3, 256)])
+def test_one_temp_for_input_and_result(cuda, quant, rows, N):
+    _check(cuda, quant, rows, N, ids={Y: X}, fused=0 if (quant, rows) == ("w4", 3) else 5)
