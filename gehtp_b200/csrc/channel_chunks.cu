@@ -39,7 +39,7 @@ constexpr int O_XL = 2 * T * XS, O_K = O_XL + 2 * T * XL, O_KL = O_K + D * T, O_
 constexpr int UV = 2 * T * VC, STAGE = SHARED + UV;                         // of which O_K words are W | qF
 constexpr int RS = 36, US = 20;
 constexpr int walk_words(int nb) { return nb * STAGE + 8 * VC * RS + VC * US; }
-constexpr uint32_t WINDOW = 1024;                             // rows a pair of launches takes: the scratch of 16 heads (51 MB) stays in L2
+constexpr uint32_t WINDOW = 1024;                             // rows a pair of launches takes: the scratch of 16 heads (59 MB) stays in L2, that of 32 (118 MB) nearly fills it
 
 __host__ __device__ inline size_t item_floats(uint32_t V) { return SHARED + (size_t)2 * T * V; }
 

@@ -2,9 +2,9 @@
 // (flags bit 1, the layout the reference's emitter gives every FullyConnected weight,
 // compiler/tools/wtop_ops/op_matmul.cpp:50):
 //
-//   M >= 16  (below 32 by the size of the matrix, see gemm_takes): TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A (128 rows x 64 k) and a
-//              tile of W (BN rows x 64 k) land in shared memory by cp.async.bulk.tensor with the 128-byte
-//              swizzle that tcgen05.mma reads; accumulators live in TMEM, double-buffered so that the
+//   M >= 32, from 16 for large matrices (gemm_takes): TMA-fed tcgen05 GEMM. Both operands are K-major, so a tile of A
+//              (128 rows x 64 k) and a tile of W (BN rows x 64 k) land in shared memory by cp.async.bulk.tensor with the
+//              128-byte swizzle that tcgen05.mma reads; accumulators live in TMEM, double-buffered so that the
 //              epilogue of a tile overlaps the main loop of the next. The reference takes its matrix
 //              unit from 128 rows on (exec_matmul_f16_hmx, kernels/src/runtime/oplist_exec.c:1600-1706).
 //   M <  32  otherwise: streaming GEMV, one warp per output column, 16-byte loads along K, fp32 accumulation,
