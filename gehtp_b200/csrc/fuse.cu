@@ -751,12 +751,24 @@ void fuse_analyze(const wt_blob* b, const std::vector<PlanOp>& meas, std::vector
         Span sp{};
         if (!taken[i] && !taken[i + 1] && (match_tanh_resid(G, i, sp) || match_window_step(G, i, sp) || match_picked_norm(G, i, sp))) claim(sp);
     }
-    // A chain reads some inputs later than its ops do: their bytes are not another's before the chain is done. SwiGLU behind two
-    // launches reads the gate once the up projection is there; its result may still take the gate's place, whole.
+    // A chain reads some temps later than its ops do: their bytes are not another's before the chain is done. Its launches read what
+    // comes in from outside while they write what goes out. SwiGLU behind two launches reads the gate once the up
+    // projection is there; its result may still take the gate's place, whole.
     for (const Span& sp : g_spans) {
         const uint32_t first = sp.ops.front(), last = sp.ops.back();
-        // both projections read the input in the launch that writes the result
-        if ((sp.kind == 1 || (sp.kind == 6 && sp.K)) && is_temp_ref(sp.a_ref)) holds.push_back({sp.a_ref, first, last});
+        auto hold_inputs = [&](uint32_t op) {
+            int ia[8];
+            const int n = input_args(b->ops[op], ia);
+            for (int k = 0; k < n; k++) {
+                const uint32_t t = b->ops[op].args[ia[k]];
+                const int from = G.producer_of_arg[ia[k]][op];
+                if (is_temp_ref(t) && !(from >= 0 && std::find(sp.ops.begin(), sp.ops.end(), (uint32_t)from) != sp.ops.end())) holds.push_back({t, std::min(op, first), last});
+            }
+        };
+        for (uint32_t o : sp.ops) hold_inputs(o);
+        // the projection in front may take the chain into its own launch
+        if (sp.kind == 0 && sp.qkv_lin >= 0) hold_inputs((uint32_t)sp.qkv_lin);
+        if (sp.kind == 2 && first > 0 && b->ops[first - 1].opcode == OP_MATMUL_W4A16) hold_inputs(first - 1);
         if (sp.kind == 6 && !one_launch(sp) && g.static_off[sp.gate_t] != g.static_off[sp.y]) holds.push_back({sp.gate_t, first, last});
     }
     // temps written only by interior ops of chains
